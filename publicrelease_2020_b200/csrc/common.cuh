@@ -16,6 +16,7 @@ constexpr int NMOM = 49;          // (LM+1)^2
 constexpr int NANG = 146;         // Lebedev degree-19 mesh used by ANGMSH(LMAX=18)
 constexpr int NCOEF = 46;         // potential polynomial coefficients per pair
 constexpr int COEF_LD = 52;       // coefficient row stride (zero padded; 52 = 4 mod 16 doubles)
+constexpr int NEAR_K = 48;        // rows of a pair in the per-FO kernel's MMA order
 constexpr int MOM_LD = 52;        // normalised-moment row stride (zero padded)
 constexpr int TILE = 128;         // mesh points per spatial tile
 constexpr int BOYS_NT = 1601;     // Boys table rows (T = 0..16 step 0.01)
@@ -64,6 +65,21 @@ struct CallShare {
   int32_t kf;         // moment columns of the far segment: (lmax over FOs + 1)^2 rounded up to 4; 0 = none
   int32_t shared;     // 1 when the geometry is FO independent
   int32_t ksum;       // multipole terms kept by the skip rule, summed over the FOs
+};
+
+// One pair of the per-FO calls, in call order.
+struct __align__(16) PerfoPair {
+  int32_t pair, call;
+  int32_t fmt;            // largest Boys variant over the FOs (3, 4 or 5)
+  int16_t first, last;    // of its call
+};
+
+// Spheres around one call's mean pair centre: within rin every FO is near,
+// beyond rout none is (squared radii; DBL_MAX where a call has no far points).
+struct CallBound {
+  double c[3];
+  double rin2, rout2;
+  int32_t p0, np;     // the call's pairs
 };
 
 #define FLOSIC_HD __host__ __device__ __forceinline__

@@ -19,19 +19,17 @@
 //                     over all such calls, on the FP64 tensor cores
 //                     (mma.sync m8n8k4 .f64).  A CTA owns 128 points and up to
 //                     128 FOs.
-//   k_coulomb_perfo   the remaining calls, whose CG (charge weighted,
-//                     poisson1.f:503-520) differs per FO: the near field of the
-//                     FOs with near points in the tile as a GEMM over compacted
-//                     FO slots, added per (FO, point); the far field per
-//                     (FO, point).
+//   k_perfo_near, k_perfo_far (csrc/coulomb_perfo.cu)  the remaining calls,
+//                     whose CG (charge weighted, poisson1.f:503-520) differs
+//                     per FO.
 //
-// Both near-field GEMMs run warp specialised: producer warps build the G / H
+// The shared-geometry GEMM runs warp specialised: producer warps build the G / H
 // columns and copy the A rows (cp.async) into double-buffered shared memory,
 // packing consecutive segments into stages of up to 52 rows, while consumer
 // warps keep the accumulators and issue only the tensor-core MMAs.
 //
-// Both walk their calls in order, so every per-point sum is deterministic.
-// Both count the evaluations they perform: near (pair, point, FO), far
+// All walk their calls in order, so every per-point sum is deterministic.
+// All count the evaluations they perform: near (pair, point, FO), far
 // (call, point, FO) and the multipole terms the far evaluations keep, the
 // units of the reference's POISSON1 work.
 #include "coulomb_common.cuh"
@@ -387,293 +385,6 @@ __device__ __forceinline__ void shared_tile(int tile, int fob, int ncalls, const
   count_add(cnt, my_near * (unsigned long long)nk, my_far * (unsigned long long)nk, my_terms);
 }
 
-// ---------------------------------------------------------------------------
-// Per-FO-geometry calls
-// ---------------------------------------------------------------------------
-// A CTA owns 128 points and up to 32*WM FOs and walks the per-FO calls in
-// order.  For each call it classifies the tile against every FO's sphere and
-// compacts the FOs with near points into slots; the producers stream the G
-// columns of the call's pairs and the slots' coefficient rows, the consumers
-// contract them on the active slot m-tiles only (up to 32*WC slots per pass),
-// so the tensor work follows the FOs that are near rather than the whole FO
-// block.  The call's near field is added, masked per (FO, point), to the CTA's
-// own slice of vh (L2 resident); its far field follows, one FO per warp with
-// lanes over points.
-template <int WM>
-struct PerFOSmem {
-  static constexpr int WC = WM < 2 ? WM : 2;  // consumer warp rows: slot capacity 32*WC per pass
-  double A[2][32 * WC * KSEG];  // slot rows of the stage's coefficients
-  double B[2][KSEG * G_LD];     // G columns
-  double MV[32 * WM * MOM_LD];  // far phase: the FOs' moments
-  double px[TILE], py[TILE], pz[TILE];
-  double cg[32 * WM][3];
-  double rc2[32 * WM];
-  int stat[32 * WM];
-  int npot[32 * WM];
-  int lmax[32 * WM];
-  int nkeep[32 * WM];
-  int fo_of[32 * WM];           // slot -> FO (block-local)
-  double lo[3], hi[3];          // tile bounding box
-  unsigned bal[WM];             // per warp of the status phase: FOs with near points
-  unsigned balf[WM];            // per warp of the status phase: FOs with far points
-  int na;
-  int rows[2];
-};
-
-// Physical A row of pass-local slot s: slots fill m-tiles round robin over the
-// WC warp rows, so that a few active FOs keep several warps busy.
-template <int WC>
-__device__ __forceinline__ int slot_row(int s) {
-  const int g = s >> 3;
-  return (g % WC) * 32 + (g / WC) * 8 + (s & 7);
-}
-
-// Far-field potential of one FO at one point, sum_lm MV[lm] Y_lm(u) / r^(l+1),
-// summed per degree l and scaled once per degree; degree LMX at compile time.
-template <typename T, int LMX>
-__device__ __forceinline__ T multipole(const T* __restrict__ mv, T ux, T uy, T uz, T hn) {
-  T acc[LMX + 1];
-#pragma unroll
-  for (int l = 0; l <= LMX; ++l) acc[l] = T(0);
-  harmonics_mmajor(ux, uy, uz, LMX, [&](int row, int l, T v) { acc[l] += mv[row] * v; });
-  T pot = T(0), rec = hn;
-#pragma unroll
-  for (int l = 0; l <= LMX; ++l) {
-    pot += acc[l] * rec;
-    rec *= hn;
-  }
-  return pot;
-}
-
-// Far field of one FO over the tile's points, lanes over points with the
-// TILE/32 points of a lane evaluated together (independent chains; points
-// that are near or past np are evaluated on a dummy radius and not added).
-// The near/far decision is the FP64 distance test of poisson1.f; T is the
-// arithmetic of the expansion.
-template <typename T, int LMX>
-__device__ __forceinline__ void far_points(const T* __restrict__ mv, const double* __restrict__ px,
-                                           const double* __restrict__ py, const double* __restrict__ pz, int np,
-                                           double cx, double cy, double cz, double rc2, double* __restrict__ vk,
-                                           int lane, unsigned long long& nfar) {
-#pragma unroll
-  for (int j = 0; j < TILE / 32; ++j) {
-    const int p = lane + 32 * j;
-    const double x = px[p], y = py[p], z = pz[p];
-    const double r2 = sqdist_rn2(x, y, z, cx, cy, cz);
-    const bool f = p < np && r2 > rc2;
-    T pot;
-    if constexpr (sizeof(T) == 4) {
-      const float hn = rsqrtf(f ? (float)r2 : 1.f);
-      pot = multipole<float, LMX>(mv, hn * (float)(x - cx), hn * (float)(y - cy), hn * (float)(z - cz), hn);
-    } else {
-      const double hn = 1.0 / sqrt(f ? r2 : 1.0);
-      pot = multipole<double, LMX>(mv, hn * (x - cx), hn * (y - cy), hn * (z - cz), hn);
-    }
-    if (f) {
-      vk[p] += (double)pot;
-      ++nfar;
-    }
-  }
-}
-
-// One (tile, FO block) of the per-FO-geometry calls; the body of
-// k_coulomb_perfo and of k_coulomb_perfo_batch.
-template <int WM, bool MIXED>
-__device__ __forceinline__ void perfo_tile(int tile, int fob, int ncalls, const int* __restrict__ lists,
-                                           int accumulate, const CallInfo* __restrict__ calls,
-                                           const PairGeo* __restrict__ pairs, int nfo,
-                                           const double* __restrict__ coef, const int8_t* __restrict__ pair_fmt,
-                                           const CallFO* __restrict__ cfo, const double* __restrict__ momv,
-                                           const MeshDev& M, const double* __restrict__ boys_tab,
-                                           double* __restrict__ vh, int ldv, unsigned long long* __restrict__ cnt) {
-  constexpr int FOB = 32 * WM, WC = PerFOSmem<WM>::WC, SC = 32 * WC;
-  using PT = typename std::conditional<MIXED, float, double>::type;  // producer and far-field arithmetic
-  constexpr int WN = CONS_WARPS / WC, WPTS = TILE / WN, NT = WPTS / 8;
-  const int* list = lists + ncalls;
-  const int nl = lists[2 * ncalls + 1];
-  if (accumulate && nl == 0) return;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  PerFOSmem<WM>& S = *reinterpret_cast<PerFOSmem<WM>*>(smraw);
-  const int k0 = fob * FOB;
-  const int nk = min(FOB, nfo - k0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int p0 = tile * TILE;
-  const int np = min(TILE, M.n - p0);
-  for (int i = tid; i < TILE; i += WS_THREADS) {
-    const bool a = i < np;
-    S.px[i] = a ? M.x[p0 + i] : 0.0;
-    S.py[i] = a ? M.y[p0 + i] : 0.0;
-    S.pz[i] = a ? M.z[p0 + i] : 0.0;
-  }
-  if (!accumulate)
-    for (int e = tid; e < nk * TILE; e += WS_THREADS) {
-      const int k = e / TILE, p = e - k * TILE;
-      if (p < np) vh[(size_t)(k0 + k) * ldv + p0 + p] = 0.0;
-    }
-  if (tid < 3) {
-    S.lo[tid] = M.tile_lo[3 * tile + tid];
-    S.hi[tid] = M.tile_hi[3 * tile + tid];
-  }
-  unsigned long long my_near = 0, my_far = 0, my_terms = 0;
-
-  for (int li = 0; li < nl; ++li) {
-    const int c = list[li];
-    const CallInfo ci = calls[c];
-    __syncthreads();  // the previous call is done with every shared buffer and with vh
-    // status of every FO of the block for this tile, and the active slots
-    if (tid < FOB) {
-      int st = 1, npot = 2, lmx = 0, nkeep = 0;
-      double cgx = 0, cgy = 0, cgz = 0, rc2 = 0;
-      if (tid < nk) {
-        const CallFO f = cfo[(size_t)c * nfo + k0 + tid];
-        cgx = f.cg[0];
-        cgy = f.cg[1];
-        cgz = f.cg[2];
-        rc2 = f.rcut2;
-        npot = f.npot;
-        st = (npot == 1) ? 0 : tile_class(S.lo, S.hi, cgx, cgy, cgz, rc2);
-        if (st != 0 && npot == 2) {
-          lmx = f.lmax;
-          nkeep = __popcll(f.keep);
-        }
-      }
-      S.stat[tid] = st;
-      S.npot[tid] = npot;
-      S.cg[tid][0] = cgx;
-      S.cg[tid][1] = cgy;
-      S.cg[tid][2] = cgz;
-      S.rc2[tid] = rc2;
-      S.lmax[tid] = lmx;
-      S.nkeep[tid] = nkeep;
-      const unsigned b = __ballot_sync(0xffffffffu, tid < nk && st != 1);
-      const unsigned bf = __ballot_sync(0xffffffffu, tid < nk && st != 0 && npot == 2);
-      if (lane == 0) {
-        S.bal[warp] = b;
-        S.balf[warp] = bf;
-      }
-    }
-    __syncthreads();
-    if (tid < FOB) {
-      int before = 0;
-      for (int w = 0; w < warp; ++w) before += __popc(S.bal[w]);
-      const unsigned b = S.bal[warp];
-      if ((b >> lane) & 1u) S.fo_of[before + __popc(b & ((1u << lane) - 1u))] = tid;
-      if (tid == FOB - 1) S.na = before + __popc(b);
-    }
-    __syncthreads();
-    const int na = S.na;
-    bool anyfar = false;
-#pragma unroll
-    for (int w = 0; w < WM; ++w) anyfar = anyfar || S.balf[w] != 0u;
-
-    for (int c0 = 0; c0 < na; c0 += SC) {
-      const int nac = min(SC, na - c0);
-      const int* fo = S.fo_of + c0;
-      if (warp >= CONS_WARPS) {
-        // ---- producers: the call's pairs, packed into stages
-        const int pt = tid - NCONS;
-        const bool leader = pt == 0;
-        StagePacker P;
-        for (int qi = 0; qi < ci.np; ++qi) {
-          const int q = ci.p0 + qi;
-          const int kq = near_rows(pair_fmt[q]);
-          const int off = P.place(S.rows, kq, leader);
-          const int b = P.b;
-          const double* src = coef + ((size_t)q * nfo + k0) * COEF_LD;
-          copy_rows(S.A[b], off, nac, kq, pt, [&](int s) { return src + (size_t)fo[s] * COEF_LD; },
-                    [](int s) { return slot_row<WC>(s); });
-          cp_async_commit();
-          const PairGeo& pg = pairs[q];
-          for (int j = 0; j < PTS_PER_PROD; ++j) {
-            const int p = pt + j * NPROD;
-            double* g = &S.B[b][(size_t)off * G_LD + p];
-            if (p < np) write_g_point<PT>(g, kq, pg, S.px[p], S.py[p], S.pz[p], boys_tab);
-            else zero_rows(g, kq);
-          }
-        }
-        P.end(S.rows, leader);
-      } else {
-        // ---- consumers
-        const int wn = warp % WN, wm = warp / WN;
-        double T[4][NT][2];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < NT; ++b) T[a][b][0] = T[a][b][1] = 0.0;
-        bool mt_active[4];
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt) mt_active[mt] = (mt * WC + wm) * 8 < nac;
-        for (int qi = 0;; ++qi) {
-          const int b = qi & 1;
-          named_sync(BAR_FULL + b);
-          const int r = S.rows[b];
-          if (r > 0)
-            stage_mma(T, &S.A[b][(wm * 32 + (lane >> 2)) * KSEG + (lane & 3)],
-                      &S.B[b][(lane & 3) * G_LD + wn * WPTS + (lane >> 2)], r, mt_active);
-          named_arrive(BAR_EMPTY + b);
-          if (r < 0) break;
-        }
-        // masked add of the call's near field to vh
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
-          const int s = (mt * WC + wm) * 8 + (lane >> 2);
-          if (s >= nac) continue;
-          const int k = fo[s];
-          const int st = S.stat[k];
-          const double cx = S.cg[k][0], cy = S.cg[k][1], cz = S.cg[k][2], rc2 = S.rc2[k];
-          double* vk = vh + (size_t)(k0 + k) * ldv + p0;
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int p = wn * WPTS + nt * 8 + 2 * (lane & 3) + i;
-              if (p >= np) continue;
-              bool nr = (st == 0);
-              if (st == 2) nr = !(sqdist_rn2(S.px[p], S.py[p], S.pz[p], cx, cy, cz) > rc2);
-              if (nr) {
-                vk[p] += T[mt][nt][i];
-                my_near += (unsigned long long)ci.np;
-              }
-            }
-        }
-      }
-    }
-
-    if (anyfar) {
-      __syncthreads();  // the near phase is done with vh
-      // the FOs' moments in the arithmetic of the expansion (FP32 in the mixed path)
-      PT* MVp = reinterpret_cast<PT*>(S.MV);
-      const double* mg = momv + ((size_t)c * nfo + k0) * MOM_LD;
-      for (int e = tid; e < nk * MOM_LD; e += WS_THREADS) MVp[e] = (PT)mg[e];
-      __syncthreads();
-      for (int k = warp; k < nk; k += WS_THREADS / 32) {
-        if (S.stat[k] == 0 || S.npot[k] == 1) continue;
-        const double cx = S.cg[k][0], cy = S.cg[k][1], cz = S.cg[k][2], rc2 = S.rc2[k];
-        const PT* mv = MVp + k * MOM_LD;
-        double* vk = vh + (size_t)(k0 + k) * ldv + p0;
-        unsigned long long nf = 0;
-        switch (S.lmax[k]) {
-#define FAR_CASE(L)                                                                          \
-  case L:                                                                                    \
-    far_points<PT, L>(mv, S.px, S.py, S.pz, np, cx, cy, cz, rc2, vk, lane, nf); \
-    break;
-          FAR_CASE(0)
-          FAR_CASE(1)
-          FAR_CASE(2)
-          FAR_CASE(3)
-          FAR_CASE(4)
-          FAR_CASE(5)
-          default: FAR_CASE(6)
-#undef FAR_CASE
-        }
-        my_far += nf;
-        my_terms += nf * (unsigned long long)S.nkeep[k];
-      }
-    }
-  }
-  count_add(cnt, my_near, my_far, my_terms);
-}
-
 template <int WM, bool MIXED>
 __global__ void __launch_bounds__(WS_THREADS, 1)
 k_coulomb_shared(int ncalls, const int* __restrict__ lists, const CallShare* __restrict__ share,
@@ -683,17 +394,6 @@ k_coulomb_shared(int ncalls, const int* __restrict__ lists, const CallShare* __r
                  double* __restrict__ vh, int ldv, unsigned long long* __restrict__ cnt) {
   shared_tile<WM, MIXED>(blockIdx.x, blockIdx.y, ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M,
                          boys_tab, vh, ldv, cnt);
-}
-
-template <int WM, bool MIXED>
-__global__ void __launch_bounds__(WS_THREADS, 1)
-k_coulomb_perfo(int ncalls, const int* __restrict__ lists, int accumulate, const CallInfo* __restrict__ calls,
-                const PairGeo* __restrict__ pairs, int nfo, const double* __restrict__ coef,
-                const int8_t* __restrict__ pair_fmt, const CallFO* __restrict__ cfo,
-                const double* __restrict__ momv, MeshDev M, const double* __restrict__ boys_tab,
-                double* __restrict__ vh, int ldv, unsigned long long* __restrict__ cnt) {
-  perfo_tile<WM, MIXED>(blockIdx.x, blockIdx.y, ncalls, lists, accumulate, calls, pairs, nfo, coef, pair_fmt, cfo,
-                        momv, M, boys_tab, vh, ldv, cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -722,19 +422,6 @@ k_coulomb_shared_batch(const CoulombJob* __restrict__ jobs, const int4* __restri
     const CoulombJob J = jobs[w.x];
     shared_tile<WM, MIXED>(w.y, w.z, J.ncalls, J.lists, J.share, J.calls, J.nfo, J.coef, J.pair_fmt, J.pairs,
                            J.momv, J.M, boys_tab, J.vh, J.ldv, J.cnt);
-  }
-}
-
-template <int WM, bool MIXED>
-__global__ void __launch_bounds__(WS_THREADS, 1)
-k_coulomb_perfo_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__ items, int nitems,
-                      int* __restrict__ counter, const double* __restrict__ boys_tab) {
-  __shared__ int slot;
-  for (int it = next_item(counter, &slot); it < nitems; it = next_item(counter, &slot)) {
-    const int4 w = items[it];
-    const CoulombJob J = jobs[w.x];
-    perfo_tile<WM, MIXED>(w.y, w.z, J.ncalls, J.lists, 1, J.calls, J.pairs, J.nfo, J.coef, J.pair_fmt, J.cfo,
-                          J.momv, J.M, boys_tab, J.vh, J.ldv, J.cnt);
   }
 }
 
@@ -790,41 +477,62 @@ __global__ void k_call_share(int ncalls, int nfo, const CallFO* __restrict__ cfo
 
 // Stable partition of the calls into lists[0..ns) (shared geometry) and
 // lists[ncalls..ncalls+nf) (per-FO geometry); lists[2 ncalls] = ns,
-// lists[2 ncalls + 1] = nf.  One block.
+// lists[2 ncalls + 1] = nf, lists[2 ncalls + 2] = the pairs of the per-FO calls,
+// listed in plist in call order.  One block.
 constexpr int LIST_THREADS = 1024;
 __global__ void __launch_bounds__(LIST_THREADS) k_call_lists(int ncalls, int per_fo_only,
                                                              const CallShare* __restrict__ share,
-                                                             int* __restrict__ lists) {
-  __shared__ int wsum[LIST_THREADS / 32];
-  __shared__ int base;
+                                                             const CallInfo* __restrict__ calls,
+                                                             const int8_t* __restrict__ pair_fmt,
+                                                             int* __restrict__ lists, PerfoPair* __restrict__ plist) {
+  __shared__ int wsum[LIST_THREADS / 32], wpair[LIST_THREADS / 32];
+  __shared__ int base, pbase;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid == 0) base = 0;
+  if (tid == 0) base = pbase = 0;
   __syncthreads();
   for (int c0 = 0; c0 < ncalls; c0 += LIST_THREADS) {
     const int c = c0 + tid;
     const bool valid = c < ncalls;
     const bool sh = valid && !per_fo_only && share[c].shared;
+    const CallInfo ci = valid ? calls[c] : CallInfo{};
+    const int np = valid && !sh ? ci.np : 0;
+    int scan = np;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, scan, o);
+      if (lane >= o) scan += v;
+    }
     const unsigned bal = __ballot_sync(0xffffffffu, sh);
-    if (lane == 0) wsum[wid] = __popc(bal);
+    if (lane == 31) {
+      wsum[wid] = __popc(bal);
+      wpair[wid] = scan;
+    }
     __syncthreads();
-    int before = base;
-    for (int w = 0; w < wid; ++w) before += wsum[w];
+    int before = base, pb = pbase + scan - np;
+    for (int w = 0; w < wid; ++w) {
+      before += wsum[w];
+      pb += wpair[w];
+    }
     const int rank_s = before + __popc(bal & ((1u << lane) - 1u));
     if (valid) {
       if (sh) lists[rank_s] = c;
       else lists[ncalls + (c - rank_s)] = c;  // c minus the shared calls before it
     }
+    for (int i = 0; i < np; ++i)
+      plist[pb + i] = PerfoPair{ci.p0 + i, c, max((int)pair_fmt[ci.p0 + i], 3), (int16_t)(i == 0), (int16_t)(i == np - 1)};
     __syncthreads();
     if (tid == 0) {
-      int t = 0;
-      for (int w = 0; w < LIST_THREADS / 32; ++w) t += wsum[w];
-      base += t;
+      for (int w = 0; w < LIST_THREADS / 32; ++w) {
+        base += wsum[w];
+        pbase += wpair[w];
+      }
     }
     __syncthreads();
   }
   if (tid == 0) {
     lists[2 * ncalls] = base;
     lists[2 * ncalls + 1] = ncalls - base;
+    lists[2 * ncalls + 2] = pbase;
   }
 }
 
@@ -842,18 +550,6 @@ static void set_batch_attr() {
                        (int)sizeof(SharedSmem<WM>));
   cudaFuncSetAttribute(k_coulomb_shared_batch<WM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(SharedSmem<WM>));
-  cudaFuncSetAttribute(k_coulomb_perfo_batch<WM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(PerFOSmem<WM>));
-  cudaFuncSetAttribute(k_coulomb_perfo_batch<WM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(PerFOSmem<WM>));
-}
-
-template <int WM>
-static void set_perfo_attr() {
-  cudaFuncSetAttribute(k_coulomb_perfo<WM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(PerFOSmem<WM>));
-  cudaFuncSetAttribute(k_coulomb_perfo<WM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(PerFOSmem<WM>));
 }
 
 // Per-device set-up: the dynamic shared-memory opt-ins.
@@ -861,9 +557,6 @@ void init_coulomb_mma() {
   set_shared_attr<1>();
   set_shared_attr<2>();
   set_shared_attr<4>();
-  set_perfo_attr<1>();
-  set_perfo_attr<2>();
-  set_perfo_attr<4>();
   set_batch_attr<1>();
   set_batch_attr<2>();
   set_batch_attr<4>();
@@ -883,51 +576,33 @@ static void launch_shared(int ncalls, const int* lists, const CallShare* share, 
         ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh, ldv, cnt);
 }
 
-template <int WM>
-static void launch_perfo(int ncalls, const int* lists, int acc, const CallInfo* calls, const PairGeo* pairs, int nfo,
-                         const double* coef, const int8_t* pair_fmt, const CallFO* cfo, const double* momv,
-                         const MeshDev& M, const double* boys_tab, double* vh, int ldv, unsigned long long* cnt,
-                         bool mixed, cudaStream_t st) {
-  dim3 grid(M.ntiles, (nfo + 32 * WM - 1) / (32 * WM));
-  if (mixed)
-    k_coulomb_perfo<WM, true><<<grid, WS_THREADS, sizeof(PerFOSmem<WM>), st>>>(
-        ncalls, lists, acc, calls, pairs, nfo, coef, pair_fmt, cfo, momv, M, boys_tab, vh, ldv, cnt);
-  else
-    k_coulomb_perfo<WM, false><<<grid, WS_THREADS, sizeof(PerFOSmem<WM>), st>>>(
-        ncalls, lists, acc, calls, pairs, nfo, coef, pair_fmt, cfo, momv, M, boys_tab, vh, ldv, cnt);
-}
-
-void launch_coulomb_classify(int ncalls, int npairs, int nfo, const int8_t* maxfmt, const CallFO* cfo,
-                             const CoulombScratch& scr, bool per_fo_only, cudaStream_t st) {
+void launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
+                             const CallFO* cfo, const CoulombScratch& scr, bool per_fo_only, cudaStream_t st) {
   if (npairs > 0) k_pair_fmt<<<(npairs + 127) / 128, 128, 0, st>>>(npairs, nfo, maxfmt, scr.pair_fmt);
   if (ncalls > 0) k_call_share<<<(ncalls + 7) / 8, 256, 0, st>>>(ncalls, nfo, cfo, scr.share);
-  k_call_lists<<<1, LIST_THREADS, 0, st>>>(ncalls, per_fo_only ? 1 : 0, scr.share, scr.lists);
+  k_call_lists<<<1, LIST_THREADS, 0, st>>>(ncalls, per_fo_only ? 1 : 0, scr.share, calls, scr.pair_fmt, scr.lists,
+                                           scr.plist);
 }
 
 template <int WM>
-static void launch_batch_wm(const CoulombJob* jobs, const int4* items, int nitems, int* counters, bool mixed,
+static void launch_batch_wm(const CoulombJob* jobs, const int4* items, int nitems, int* counter, bool mixed,
                             const double* boys_tab, int nctas, cudaStream_t st) {
-  if (mixed) {
-    k_coulomb_shared_batch<WM, true><<<nctas, WS_THREADS, sizeof(SharedSmem<WM>), st>>>(jobs, items, nitems,
-                                                                                          counters, boys_tab);
-    k_coulomb_perfo_batch<WM, true><<<nctas, WS_THREADS, sizeof(PerFOSmem<WM>), st>>>(jobs, items, nitems,
-                                                                                        counters + 1, boys_tab);
-  } else {
-    k_coulomb_shared_batch<WM, false><<<nctas, WS_THREADS, sizeof(SharedSmem<WM>), st>>>(jobs, items, nitems,
-                                                                                           counters, boys_tab);
-    k_coulomb_perfo_batch<WM, false><<<nctas, WS_THREADS, sizeof(PerFOSmem<WM>), st>>>(jobs, items, nitems,
-                                                                                         counters + 1, boys_tab);
-  }
+  if (mixed)
+    k_coulomb_shared_batch<WM, true><<<nctas, WS_THREADS, sizeof(SharedSmem<WM>), st>>>(jobs, items, nitems, counter,
+                                                                                          boys_tab);
+  else
+    k_coulomb_shared_batch<WM, false><<<nctas, WS_THREADS, sizeof(SharedSmem<WM>), st>>>(jobs, items, nitems, counter,
+                                                                                           boys_tab);
 }
 
-void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counters, int wm, bool mixed,
+void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
                           const double* boys_tab, int nctas, cudaStream_t st) {
   if (nitems <= 0) return;
   nctas = std::max(1, std::min(nctas, nitems));
-  cudaMemsetAsync(counters, 0, 2 * sizeof(int), st);
-  if (wm == 4) launch_batch_wm<4>(jobs, items, nitems, counters, mixed, boys_tab, nctas, st);
-  else if (wm == 2) launch_batch_wm<2>(jobs, items, nitems, counters, mixed, boys_tab, nctas, st);
-  else launch_batch_wm<1>(jobs, items, nitems, counters, mixed, boys_tab, nctas, st);
+  cudaMemsetAsync(counter, 0, sizeof(int), st);
+  if (wm == 4) launch_batch_wm<4>(jobs, items, nitems, counter, mixed, boys_tab, nctas, st);
+  else if (wm == 2) launch_batch_wm<2>(jobs, items, nitems, counter, mixed, boys_tab, nctas, st);
+  else launch_batch_wm<1>(jobs, items, nitems, counter, mixed, boys_tab, nctas, st);
 }
 
 cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo* pairs, int npairs, int nfo,
@@ -936,8 +611,7 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
                                unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st) {
   const bool per_fo_only = cfg.per_fo_only;
-  unsigned long long* cnt_perfo = cnt + 3;  // the per-FO kernel counts apart from the shared-geometry one
-  launch_coulomb_classify(ncalls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
+  launch_coulomb_classify(ncalls, calls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
   if (!per_fo_only && mixed && cfg.shared_tc) {
     const size_t nc = (size_t)npairs * nfo * COEF_LD, nm = (size_t)ncalls * nfo * MOM_LD;
     launch_split_tf32((size_t)npairs, nfo, coef, scr.coef_hl, st);
@@ -958,17 +632,28 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                        ldv, cnt, mixed, st);
   }
   if (mid) cudaEventRecord(mid, st);
-  const int acc = per_fo_only ? 0 : 1;
-  const int wm = cfg.perfo_wm > 0 ? cfg.perfo_wm : (nfo > 64 ? 4 : (nfo > 32 ? 2 : 1));
-  if (wm == 4)
-    launch_perfo<4>(ncalls, scr.lists, acc, calls, pairs, nfo, coef, scr.pair_fmt, cfo, momv, M, boys_tab, vh, ldv,
-                    cnt_perfo, mixed, st);
-  else if (wm == 2)
-    launch_perfo<2>(ncalls, scr.lists, acc, calls, pairs, nfo, coef, scr.pair_fmt, cfo, momv, M, boys_tab, vh, ldv,
-                    cnt_perfo, mixed, st);
-  else
-    launch_perfo<1>(ncalls, scr.lists, acc, calls, pairs, nfo, coef, scr.pair_fmt, cfo, momv, M, boys_tab, vh, ldv,
-                    cnt_perfo, mixed, st);
+  if (per_fo_only) cudaMemset2DAsync(vh, sizeof(double) * ldv, 0, sizeof(double) * M.n, nfo, st);
+  launch_perfo_setup(ncalls, npairs, nfo, calls, pairs, cfo, scr.share, per_fo_only, mixed, coef, momv, scr.coefp,
+                     scr.momp, scr.bound, st);
+  CoulombJob J{};
+  J.ncalls = ncalls;
+  J.nfo = nfo;
+  J.ldv = ldv;
+  J.lists = scr.lists;
+  J.share = scr.share;
+  J.calls = calls;
+  J.pairs = pairs;
+  J.pair_fmt = scr.pair_fmt;
+  J.cfo = cfo;
+  J.momv = momv;
+  J.coefp = scr.coefp;
+  J.momp = scr.momp;
+  J.bound = scr.bound;
+  J.plist = scr.plist;
+  J.M = M;
+  J.vh = vh;
+  J.cnt_perfo = cnt + 3;  // counted apart from the shared-geometry kernel
+  launch_perfo(J, cfg.perfo_wm > 0 ? cfg.perfo_wm : perfo_default_wm(nfo), mixed, boys_tab, st);
   return cudaGetLastError();
 }
 

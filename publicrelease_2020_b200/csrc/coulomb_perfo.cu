@@ -1,0 +1,952 @@
+// Coulomb potential of the calls whose near/far geometry differs per FO
+// (every call with more than one POISSON1 slot: its CG is charge weighted,
+// poisson1.f:503-520).  Near field and far field are two kernels.
+//
+//   k_perfo_near  A CTA owns 64 mesh points (8 warps x 8) and up to 32, 64 or
+//                 128 FOs and walks the pairs of the calls in order, 128 at a
+//                 time: it drops the calls with no near point of any FO in its
+//                 box, lists the FOs that have some, and streams those FOs'
+//                 coefficient rows through two shared-memory buffers.  A warp
+//                 forms the G columns of its points in registers, directly as B
+//                 fragments of mma.sync m8n8k4 .f64 (lane 4 n + q holds row q of
+//                 each k-step at point n; one column per (pair, point), the Boys
+//                 values of four pairs at once over the four lanes of a point),
+//                 and multiplies the coefficient rows of its own near FOs into
+//                 FP64 accumulators.  Calls near for every FO accumulate on;
+//                 the others are added masked, point by point.
+//   k_perfo_far   One warp owns 64 points (two per lane) and one FO and adds
+//                 the L <= 6 multipole expansions of the far calls as Clenshaw
+//                 sums.
+//
+// What bounds it: the FP64 pipe (tensor and FMA path share ~37 TF/s), 92 flops
+// per near (pair, point, FO), ~100-260 per far (call, point, FO), and beside it
+// the instructions that form a column (~150 per warp and pair).  The form before,
+// one 384-thread CTA per 128 points with producer and consumer warps, spent 9-14
+// us per (call, tile) in CTA barriers, stage hand-overs and per-call FO status,
+// whatever the call's size; with NSPN=2 most calls are one 16-48-row pair.
+// Measured, FP64, both kernels: benzene (37,843 points, 21 + 21 FOs) 85.9 -> 35.2
+// ms, the 40-atom system (100,003 points, 128 FOs) 108 -> 66 ms (near 46, far
+// 20), water (3,942 points) 2.0 -> 0.8 ms.
+#include <algorithm>
+
+#include "coulomb_common.cuh"
+
+namespace flosic {
+
+// Columns of one pair in MMA order: k-step s (0..11), lane residue q.  Row of
+// COEFICIENT order at position 4 s + q (-1: zero).  Residues 1, 2, 3 hold the
+// monomials of one cyclic permutation (a,b,c) of (x,y,z) each, so their values
+// have one formula; residue 0, with (a,b,c) = (x,y,z), holds the rest:
+//   F_0..F_2 group   a F1 | a F2 | aa F2 | ab F2      (0: F0, F1, F2, none)
+//   F_3 group        aa | ab | aaa | aab              (0: xyz, xxz, xyy, yzz)
+//   F_4 group        aaaa | aaab | aaac | aabb        (0: xxyz, xyyz, xyzz, none)
+// The first 4, 8 and 12 k-steps are the pairs of Boys variant 3, 4 and 5.
+__constant__ int8_t c_mma_row[NEAR_K] = {0,  5,  4,  3,  1,  8,  7,  6,  2,  14, 11, 9,  -1, 13, 10, 12,
+                                         26, 20, 17, 15, 28, 19, 16, 18, 27, 30, 24, 21, 22, 29, 23, 25,
+                                         41, 45, 35, 31, 38, 44, 34, 36, 37, 43, 39, 32, -1, 42, 33, 40};
+
+// Coefficient rows of the per-FO calls' pairs in the order the lanes read them:
+// [pair][group g of four k-steps][FO][16].  The 16-byte piece of a row that
+// holds k-steps 4 g + 2 h and 4 g + 2 h + 1 of residue q is number 4 h + q.
+__global__ void __launch_bounds__(256) k_perfo_pack(int nfo, const PairGeo* __restrict__ pairs,
+                                                    const CallShare* __restrict__ share, int per_fo_only,
+                                                    const double* __restrict__ coef, double* __restrict__ out) {
+  const int pr = blockIdx.x;
+  if (!per_fo_only && share[pairs[pr].call].shared) return;
+  const double* src = coef + (size_t)pr * nfo * COEF_LD;
+  double* dst = out + (size_t)pr * nfo * NEAR_K;
+  for (int e = threadIdx.x; e < nfo * NEAR_K; e += blockDim.x) {
+    const int g = e / (nfo * 16), f = e - g * nfo * 16, k = f >> 4;
+    const int row = c_mma_row[4 * (4 * g + 2 * ((f >> 3) & 1) + (f & 1)) + ((f >> 1) & 3)];
+    dst[e] = row >= 0 ? src[(size_t)k * COEF_LD + row] : 0.0;
+  }
+}
+
+// Spheres around the mean pair centre c of each call: a point within rin is
+// near for every FO, a point beyond rout for none.  One warp per call.
+__global__ void __launch_bounds__(256) k_perfo_bounds(int ncalls, int nfo, const CallInfo* __restrict__ calls,
+                                                      const PairGeo* __restrict__ pairs,
+                                                      const CallFO* __restrict__ cfo, CallBound* __restrict__ out) {
+  const int c = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (c >= ncalls) return;
+  const CallInfo ci = calls[c];
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int q = lane; q < ci.np; q += 32)
+    for (int d = 0; d < 3; ++d) s[d] += pairs[ci.p0 + q].C[d];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    for (int o = 16; o > 0; o >>= 1) s[d] += __shfl_xor_sync(0xffffffffu, s[d], o);
+    s[d] /= ci.np;
+  }
+  double rin = DBL_MAX, rout = 0.0;
+  for (int k = lane; k < nfo; k += 32) {
+    const CallFO& f = cfo[(size_t)c * nfo + k];
+    if (f.npot == 1) {
+      rout = DBL_MAX;
+      continue;
+    }
+    const double dx = f.cg[0] - s[0], dy = f.cg[1] - s[1], dz = f.cg[2] - s[2];
+    const double d = sqrt(dx * dx + dy * dy + dz * dz);
+    rin = fmin(rin, f.rcut * (1.0 - 1e-12) - d * (1.0 + 1e-12));
+    rout = fmax(rout, (f.rcut + d) * (1.0 + 1e-12));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    rin = fmin(rin, __shfl_xor_sync(0xffffffffu, rin, o));
+    rout = fmax(rout, __shfl_xor_sync(0xffffffffu, rout, o));
+  }
+  if (lane == 0) {
+    CallBound b;
+    for (int d = 0; d < 3; ++d) b.c[d] = s[d];
+    rin = fmax(rin, 0.0);
+    b.rin2 = rin < 1e150 ? rin * rin : DBL_MAX;
+    b.rout2 = rout < 1e150 ? rout * rout : DBL_MAX;
+    b.p0 = ci.p0;
+    b.np = ci.np;
+    out[c] = b;
+  }
+}
+
+// Box of a warp's points (each lane gives one point that exists).
+__device__ __forceinline__ void warp_box(double x, double y, double z, double lo[3], double hi[3]) {
+  lo[0] = hi[0] = x;
+  lo[1] = hi[1] = y;
+  lo[2] = hi[2] = z;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+}
+
+// 0: every point near for every FO; 1: no point near for any FO; 2: neither.
+__device__ __forceinline__ int bound_class(const double lo[3], const double hi[3], const CallBound& b) {
+  const int in = tile_class(lo, hi, b.c[0], b.c[1], b.c[2], b.rin2);
+  if (in == 0) return 0;
+  return tile_class(lo, hi, b.c[0], b.c[1], b.c[2], b.rout2) == 1 ? 1 : 2;
+}
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// ---------------------------------------------------------------------------
+// Near field
+// ---------------------------------------------------------------------------
+constexpr int NEAR_WARPS = 8;                  // warps per CTA
+constexpr int NEAR_PTS = 8;                    // points per warp
+constexpr int NEAR_THREADS = 32 * NEAR_WARPS;
+constexpr int NEAR_CTA_PTS = NEAR_WARPS * NEAR_PTS;
+constexpr int NEAR_PER_TILE = TILE / NEAR_CTA_PTS;
+constexpr int NEAR_WIN = 128;                  // pairs classified at once
+constexpr int near_rows_cap(int mt) { return mt <= 4 ? 192 : (mt <= 8 ? 224 : 384); }
+
+struct __align__(16) NearEntry {
+  int pre;                                     // coefficient rows of the entries before it
+  int call, pair;
+  uint8_t lead, nl, fmt, flags;                // index into lead, listed FOs, Boys variant, 1 first + 2 last of its call
+};
+
+template <int MT>
+struct NearSmem {
+  static constexpr int ROWS = near_rows_cap(MT);  // coefficient rows (16 doubles) per buffer
+  static_assert(ROWS >= 3 * 8 * MT, "a pair's rows of all FOs fit");
+  double A[2][ROWS * 16];
+  double V[NEAR_WARPS][8 * MT * NEAR_PTS];     // the warps' potentials, [FO][point]
+  double p[NEAR_CTA_PTS][3];
+  double box[NEAR_WARPS + 1][6];               // of each warp's points, and of all
+  double geo[NEAR_WIN][6];                     // queue: pair centre x y z x y, exponent sum
+  NearEntry queue[NEAR_WIN + 1];               // the window's pairs with near points in this CTA
+  int lead[NEAR_WIN];                          // the window's calls; + (1 << 30) when all FOs are near
+  int cnt[NEAR_WIN];                           // FOs of the block with near points in the CTA's box
+  int wcount[NEAR_WIN / 32][2];
+  uint8_t list[NEAR_WIN][8 * MT];              // those FOs, ascending
+  uint8_t slot[NEAR_WARPS][8 * MT];            // a warp's slots: position in list, + 128 when all points are near
+};
+
+// The column values of one (pair, point) for lane residue q: four k-steps of
+// group g, products in the association of poisson1.f:925-959.  Positions whose
+// coefficient row is padding hold any finite value.
+template <typename T>
+struct NearLane {
+  T a, b, c, aa, ab, bb;
+  __device__ __forceinline__ NearLane(T a_, T b_, T c_) : a(a_), b(b_), c(c_), aa(a_ * a_), ab(a_ * b_), bb(b_ * b_) {}
+};
+template <typename T, int g>
+__device__ __forceinline__ void near_group(const NearLane<T>& L, const T (&F)[5], bool q0, double (&o)[4]) {
+  if constexpr (g == 0) {
+    o[0] = (double)(q0 ? F[0] : F[1] * L.a);
+    o[1] = (double)(q0 ? F[1] : F[2] * L.a);
+    o[2] = (double)(q0 ? F[2] : F[2] * L.aa);
+    o[3] = (double)(F[2] * L.ab);
+  } else if constexpr (g == 1) {
+    o[0] = (double)(F[3] * (q0 ? L.a * (L.b * L.c) : L.aa));
+    o[1] = (double)(F[3] * (q0 ? L.c * L.aa : L.ab));
+    o[2] = (double)(F[3] * (L.a * (q0 ? L.bb : L.aa)));
+    o[3] = (double)(F[3] * (L.b * (q0 ? L.c * L.c : L.aa)));
+  } else {
+    const T t = q0 ? L.b * L.c : L.aa;
+    o[0] = (double)(F[4] * (L.aa * t));
+    o[1] = (double)(F[4] * (L.ab * t));
+    o[2] = (double)(F[4] * (q0 ? L.ab * (L.c * L.c) : (L.a * L.c) * L.aa));
+    o[3] = (double)(F[4] * (L.aa * L.bb));
+  }
+}
+
+// Boys values F_0..F_{fmt-1} (absent orders zero) by the steps of boys_fmt, with
+// the variant chosen by selection: the lanes of a warp hold different pairs.
+template <typename T>
+__device__ __forceinline__ void near_boys(const double* __restrict__ tab, T x, T ex, int fmt, T (&F)[5]) {
+  if (x > T(16)) {
+    if constexpr (sizeof(T) == 8) {  // as boys_fmt, from one reciprocal square root
+      const double h = rsqrt(x), r = 0.5 * h * h;
+      F[0] = r * (x * h * 1.77245385090551602728 - ex);
+      F[1] = r * (F[0] - ex);
+      F[2] = r * (3.0 * F[1] - ex);
+      F[3] = r * (5.0 * F[2] - ex);
+      F[4] = r * (7.0 * F[3] - ex);
+    } else {
+      boys_fmt<T>(tab, x, ex, fmt, F);
+    }
+    return;
+  }
+  const int it = (int)(T(100) * x + T(1.5));
+  const T rect1 = T(2) * x, dt = T(1.0e-2) * T(it - 1) - x;
+  const double* f = tab + (size_t)(it - 1) * BOYS_NC + (fmt - 3);
+  const T o7 = T(1) / T(7), o5 = T(1) / T(5), o3 = T(1) / T(3);
+  const T top = T(f[0]) + dt * (T(f[1]) + dt * (T(f[4]) + dt * T(f[7])));
+  F[4] = fmt == 5 ? top : T(0);
+  F[3] = fmt == 5 ? (top * rect1 + ex) * o7 : (fmt == 4 ? top : T(0));
+  F[2] = fmt == 3 ? top : (F[3] * rect1 + ex) * o5;
+  F[1] = (F[2] * rect1 + ex) * o3;
+  F[0] = F[1] * rect1 + ex;
+}
+
+// Four k-steps of one group: two 16-byte fragment loads and four MMAs per eight
+// FO slots.  row[mt]: double offset of the
+// slot's coefficient row, with the lane's piece.
+template <int MT, typename T, int g>
+__device__ __forceinline__ void near_mma(double (&acc)[MT][2], const double* __restrict__ A, const int (&row)[MT],
+                                         int nmt, const NearLane<T>& L, const T (&F)[5], bool q0) {
+  double b[4];
+  near_group<T, g>(L, F, q0, b);
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+    if (mt >= nmt) break;
+    const double2 a0 = *reinterpret_cast<const double2*>(A + row[mt]);
+    const double2 a1 = *reinterpret_cast<const double2*>(A + (row[mt] ^ 8));
+    dmma(acc[mt], a0.x, b[0]);
+    dmma(acc[mt], a0.y, b[1]);
+    dmma(acc[mt], a1.x, b[2]);
+    dmma(acc[mt], a1.y, b[3]);
+  }
+}
+
+// delta |r|^2 (poisson1.f:640-650); the single-precision form fixes its roundings
+template <typename T>
+__device__ __forceinline__ T near_arg(T delta, T x, T y, T z) {
+  if constexpr (sizeof(T) == 4) return delta * __fadd_rn(__fadd_rn(__fmul_rn(z, z), __fmul_rn(y, y)), __fmul_rn(x, x));
+  else return delta * (z * z + y * y + x * x);
+}
+
+template <int MT, bool MIXED>
+__device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob,
+                                           const double* __restrict__ tab) {
+  using PT = typename std::conditional<MIXED, float, double>::type;
+  constexpr int FOB = 8 * MT;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  NearSmem<MT>& S = *reinterpret_cast<NearSmem<MT>*>(smraw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = lane >> 2, q = lane & 3;
+  const int k0 = fob * FOB, nk = min(FOB, J.nfo - k0);
+  const int cta0 = blk * NEAR_CTA_PTS;
+  if (cta0 >= J.M.n) return;  // whole CTA
+  const int npl = J.lists[2 * J.ncalls + 2];
+  if (npl == 0) return;
+  const int pb = cta0 + warp * NEAR_PTS;
+  const int npt = min(NEAR_PTS, J.M.n - pb);  // <= 0: this warp only helps with the copies
+  double* V = S.V[warp];
+  for (int e = lane; e < nk * NEAR_PTS; e += 32) V[e] = 0.0;
+  {
+    // points past the end repeat the last one and are not stored
+    const int p = min(pb + (lane & 7), J.M.n - 1);
+    const double x = J.M.x[p], y = J.M.y[p], z = J.M.z[p];
+    double lo[3], hi[3];
+    warp_box(x, y, z, lo, hi);
+    if (lane < NEAR_PTS) {
+      S.p[warp * NEAR_PTS + lane][0] = x;
+      S.p[warp * NEAR_PTS + lane][1] = y;
+      S.p[warp * NEAR_PTS + lane][2] = z;
+    }
+    if (lane == 0)
+      for (int d = 0; d < 3; ++d) {
+        S.box[warp][d] = lo[d];
+        S.box[warp][3 + d] = hi[d];
+      }
+  }
+  __syncthreads();
+  if (tid < 6) {
+    double v = S.box[0][tid];
+    for (int w = 1; w < NEAR_WARPS; ++w) v = tid < 3 ? fmin(v, S.box[w][tid]) : fmax(v, S.box[w][tid]);
+    S.box[NEAR_WARPS][tid] = v;
+  }
+  __syncthreads();
+  const double(*pts)[3] = &S.p[warp * NEAR_PTS];
+  const double* box = S.box[warp];
+  double T[MT][2];
+  int row[MT];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) T[mt][0] = T[mt][1] = 0.0, row[mt] = 0;
+  bool dirty = false;
+  int na = 0;
+  PT Fq[5] = {};  // Boys values of one pair of the current four
+  const int cyc = max(q - 1, 0);  // the lane's coordinates: (x,y,z), (x,y,z), (y,z,x), (z,x,y)
+  const double pa = pts[n][cyc], pb_ = pts[n][cyc == 2 ? 0 : cyc + 1], pc = pts[n][cyc == 0 ? 2 : cyc - 1];
+  unsigned long long near = 0;
+  // V += T for slots that are the block's FOs in order
+  auto flush = [&] {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const int k = mt * 8 + n;
+      if (k < nk) {
+        double2* ch = reinterpret_cast<double2*>(V + k * NEAR_PTS + 2 * q);
+        double2 v = *ch;
+        v.x += T[mt][0];
+        v.y += T[mt][1];
+        *ch = v;
+      }
+      T[mt][0] = T[mt][1] = 0.0;
+    }
+    dirty = false;
+  };
+  // asynchronous copy of the coefficient rows of queue entries [e0, e1) into
+  // buffer b, one warp per entry: [group][listed FO][16], the halves of odd rows
+  // exchanged so that the eight lanes of two rows read all 32 banks
+  auto copy = [&](int e0, int e1, int b) {
+    for (int e = e0 + warp; e < e1; e += NEAR_WARPS) {
+      const NearEntry w = S.queue[e];
+      const int nl = w.nl;
+      const uint8_t* list = S.list[w.lead];
+      double* dst = S.A[b] + (w.pre - S.queue[e0].pre) * 16;
+      for (int g = 0; g < w.fmt - 2; ++g, dst += nl * 16) {
+        const double* src = J.coefp + (((size_t)w.pair * 3 + g) * J.nfo + k0) * 16;
+        for (int i = lane; i < nl * 8; i += 32) {
+          const int r = i >> 3, pc = i & 7;
+          cp_async16(dst + r * 16 + 2 * (pc ^ ((r & 1) << 2)), src + (int)list[r] * 16 + 2 * pc);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+
+  for (int w0 = 0; w0 < npl; w0 += NEAR_WIN) {
+    // 1. the window's calls with near points of some FO in the CTA's box
+    bool act = false, leads = false;
+    int cls = 1;
+    PerfoPair my{};
+    const double* bx = S.box[NEAR_WARPS];
+    const double clo[3] = {bx[0], bx[1], bx[2]}, chi[3] = {bx[3], bx[4], bx[5]};
+    if (tid < NEAR_WIN && w0 + tid < npl) {
+      my = J.plist[w0 + tid];
+      cls = bound_class(clo, chi, J.bound[my.call]);
+      act = cls != 1;
+      leads = act && (tid == 0 || my.first);
+    }
+    unsigned bal = __ballot_sync(0xffffffffu, leads);
+    if (lane == 0 && warp < NEAR_WIN / 32) S.wcount[warp][0] = __popc(bal);
+    __syncthreads();  // and every warp is done with the previous window
+    int before = 0, nlead = 0;
+#pragma unroll
+    for (int w = 0; w < NEAR_WIN / 32; ++w) {
+      const int cw = S.wcount[w][0];
+      before += w < warp ? cw : 0;
+      nlead += cw;
+    }
+    const int mycall = before + __popc(bal & (lane == 31 ? 0xffffffffu : (2u << lane) - 1u)) - 1;
+    if (leads) S.lead[mycall] = my.call | (cls == 0 ? 1 << 30 : 0);
+    __syncthreads();
+    // 2. per call, the block's FOs with near points in the CTA's box
+    for (int u = warp; u < nlead; u += NEAR_WARPS) {
+      const int cc = S.lead[u];
+      const bool allnear = cc >> 30;
+      const CallFO* cf = J.cfo + (size_t)(cc & ((1 << 30) - 1)) * J.nfo + k0;
+      int n1 = 0;
+#pragma unroll
+      for (int kb = 0; kb < FOB; kb += 32) {
+        const int k = kb + lane;
+        bool on = k < nk;
+        if (on && !allnear) {
+          const CallFO& f = cf[k];
+          on = f.npot == 1 || tile_class(clo, chi, f.cg[0], f.cg[1], f.cg[2], f.rcut2) != 1;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) S.list[u][n1 + __popc(m & ((1u << lane) - 1u))] = (uint8_t)k;
+        n1 += __popc(m);
+      }
+      if (lane == 0) S.cnt[u] = n1;
+    }
+    __syncthreads();
+    // 3. the queue: the pairs of the calls that keep an FO
+    act = act && S.cnt[mycall] > 0;
+    bal = __ballot_sync(0xffffffffu, act);
+    int rows = act ? S.cnt[mycall] * (my.fmt - 2) : 0;
+    const int mine = rows;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, rows, o);
+      if (lane >= o) rows += v;
+    }
+    if (lane == 31 && warp < NEAR_WIN / 32) {
+      S.wcount[warp][0] = __popc(bal);
+      S.wcount[warp][1] = rows;
+    }
+    __syncthreads();
+    before = 0;
+    int qn = 0, rbefore = 0, rtotal = 0;
+#pragma unroll
+    for (int w = 0; w < NEAR_WIN / 32; ++w) {
+      const int cw = S.wcount[w][0], rw = S.wcount[w][1];
+      before += w < warp ? cw : 0;
+      rbefore += w < warp ? rw : 0;
+      qn += cw;
+      rtotal += rw;
+    }
+    if (act) {
+      const int e = before + __popc(bal & ((1u << lane) - 1u));
+      S.queue[e] = NearEntry{rbefore + rows - mine, my.call, my.pair, (uint8_t)mycall, (uint8_t)S.cnt[mycall],
+                             (uint8_t)my.fmt, (uint8_t)(my.first + 2 * my.last)};
+      const PairGeo& g = J.pairs[my.pair];
+      S.geo[e][0] = S.geo[e][3] = g.C[0];
+      S.geo[e][1] = S.geo[e][4] = g.C[1];
+      S.geo[e][2] = g.C[2];
+      S.geo[e][5] = g.delta;
+    }
+    if (tid == 0) S.queue[qn].pre = rtotal;
+    __syncthreads();
+    // 4. chunks of at most 32 entries whose rows fill a buffer
+    auto chunk_end = [&](int e0) {
+      int e = e0;
+      while (e < qn && e - e0 < 32 && S.queue[e + 1].pre - S.queue[e0].pre <= NearSmem<MT>::ROWS) ++e;
+      return e;
+    };
+    int e0 = 0, e1 = chunk_end(0), b = 0, fquad = -1;
+    if (e1 > 0) copy(0, e1, 0);
+    while (e0 < qn) {
+      const int e2 = chunk_end(e1);
+      cp_async_wait_all();
+      __syncthreads();  // this chunk has arrived and the other buffer is free
+      if (e1 < qn) copy(e1, e2, b ^ 1);
+      if (npt > 0) {
+        int wc = 1;
+        if (lane < e1 - e0) {
+          const double lo[3] = {box[0], box[1], box[2]}, hi[3] = {box[3], box[4], box[5]};
+          wc = bound_class(lo, hi, J.bound[S.queue[e0 + lane].call]);
+        }
+        const double* A = S.A[b] - S.queue[e0].pre * 16;
+        unsigned todo = __ballot_sync(0xffffffffu, wc != 1);
+        const unsigned full = __ballot_sync(0xffffffffu, wc == 0);
+        while (todo) {
+          const int i = __ffs(todo) - 1, e = e0 + i;
+          todo &= todo - 1;
+          const NearEntry w = S.queue[e];
+          const int nl = w.nl;
+          const uint8_t* list = S.list[w.lead];
+          const double* Ae = A + w.pre * 16;
+          const bool isfull = (full >> i) & 1u;
+          if (w.flags & 1) {
+            na = nk;  // a call that is near for every FO lists them all
+            if (!isfull) {  // the FOs with near points of this warp, compacted into slots
+              if (dirty) flush();
+              const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
+              const double lo[3] = {box[0], box[1], box[2]}, hi[3] = {box[3], box[4], box[5]};
+              na = 0;
+              for (int sb = 0; sb < nl; sb += 32) {
+                const int s = sb + lane;
+                int st = 1;
+                if (s < nl) {
+                  const CallFO& f = cf[list[s]];
+                  st = (f.npot == 1) ? 0 : tile_class(lo, hi, f.cg[0], f.cg[1], f.cg[2], f.rcut2);
+                }
+                const unsigned on = __ballot_sync(0xffffffffu, st != 1);
+                if (st != 1) S.slot[warp][na + __popc(on & ((1u << lane) - 1u))] = (uint8_t)(s | (st == 0 ? 128 : 0));
+                na += __popc(on);
+              }
+              __syncwarp();
+            }
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+              const int s = max(min(mt * 8 + n, na - 1), 0);
+              const int r = isfull ? s : (int)(S.slot[warp][s] & 127);
+              row[mt] = r * 16 + 2 * (q ^ ((r & 1) << 2));
+            }
+          }
+          if (na == 0) continue;
+          const int nmt = (na + 7) >> 3;
+          if ((e >> 2) != fquad) {
+            // Boys values of four pairs at once: lane residue q takes pair 4 fquad + q
+            fquad = e >> 2;
+            const int eq = min(4 * fquad + q, qn - 1);
+            const double* gq = S.geo[eq];
+            const double* pp = pts[n];
+            const PT arg = near_arg<PT>(PT(gq[5]), PT(pp[0] - gq[0]), PT(pp[1] - gq[1]), PT(pp[2] - gq[2]));
+            PT ex;
+            if constexpr (MIXED) ex = expf(-arg);
+            else ex = exp(-arg);
+            near_boys<PT>(tab, arg, ex, S.queue[eq].fmt, Fq);
+          }
+          const double* gq = S.geo[e] + cyc;
+          const NearLane<PT> L(PT(pa - gq[0]), PT(pb_ - gq[1]), PT(pc - gq[2]));
+          const int src = (lane & 28) | (e & 3);
+          PT F[5];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) F[j] = __shfl_sync(0xffffffffu, Fq[j], src);
+          near_mma<MT, PT, 0>(T, Ae, row, nmt, L, F, q == 0);
+          if (w.fmt >= 4) {
+            F[3] = __shfl_sync(0xffffffffu, Fq[3], src);
+            near_mma<MT, PT, 1>(T, Ae + nl * 16, row, nmt, L, F, q == 0);
+          }
+          if (w.fmt >= 5) {
+            F[4] = __shfl_sync(0xffffffffu, Fq[4], src);
+            near_mma<MT, PT, 2>(T, Ae + 2 * nl * 16, row, nmt, L, F, q == 0);
+          }
+          if (isfull) {
+            dirty = true;
+            if (lane == 0) near += (unsigned)(nk * npt);
+          } else if (w.flags & 2) {
+            // masked add: a point counts for an FO when it is inside the FO's sphere
+            const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
+            const int np = J.bound[w.call].np;
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+              const int s = mt * 8 + n;
+              if (s < na) {
+                const int sl = S.slot[warp][s], k = list[sl & 127];
+                const bool all = sl >= 128;
+                const CallFO& f = cf[k];
+                const double cx = f.cg[0], cy = f.cg[1], cz = f.cg[2], rc2 = f.rcut2;
+                const double *p0 = pts[2 * q], *p1 = pts[2 * q + 1];
+                const bool n0 = 2 * q < npt && (all || !(sqdist_rn2(p0[0], p0[1], p0[2], cx, cy, cz) > rc2));
+                const bool n1 = 2 * q + 1 < npt && (all || !(sqdist_rn2(p1[0], p1[1], p1[2], cx, cy, cz) > rc2));
+                double2* ch = reinterpret_cast<double2*>(V + k * NEAR_PTS + 2 * q);
+                double2 v = *ch;
+                if (n0) v.x += T[mt][0];
+                if (n1) v.y += T[mt][1];
+                *ch = v;
+                near += (unsigned long long)(((int)n0 + (int)n1) * np);
+              }
+              T[mt][0] = T[mt][1] = 0.0;
+            }
+            __syncwarp();
+          }
+        }
+      }
+      e0 = e1;
+      e1 = e2;
+      b ^= 1;
+    }
+  }
+  if (npt > 0) {
+    if (dirty) flush();
+    __syncwarp();
+    for (int e = lane; e < nk * NEAR_PTS; e += 32) {
+      const int k = e / NEAR_PTS, p = e - k * NEAR_PTS;
+      if (p < npt) J.vh[(size_t)(k0 + k) * J.ldv + pb + p] += V[e];
+    }
+    count_add(J.cnt_perfo, near, 0, 0);
+  }
+}
+
+// resident CTAs per SM the registers are limited for
+template <int MT>
+constexpr int near_ctas() { return MT <= 8 ? 2 : 1; }
+
+template <int MT, bool MIXED>
+__global__ void __launch_bounds__(NEAR_THREADS, near_ctas<MT>())
+k_perfo_near(const __grid_constant__ CoulombJob J, const double* __restrict__ tab) {
+  near_block<MT, MIXED>(J, blockIdx.x, blockIdx.y, tab);
+}
+
+// Many (molecule, spin) jobs: items[i] = {job, 128-point tile, FO block, 0}.
+template <int MT, bool MIXED>
+__global__ void __launch_bounds__(NEAR_THREADS, near_ctas<MT>())
+k_perfo_near_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__ items,
+                   const double* __restrict__ tab) {
+  __shared__ CoulombJob J;
+  const int4 w = items[blockIdx.x / NEAR_PER_TILE];
+  if (threadIdx.x == 0) J = jobs[w.x];
+  __syncthreads();
+  near_block<MT, MIXED>(J, w.y * NEAR_PER_TILE + blockIdx.x % NEAR_PER_TILE, w.z, tab);
+}
+
+// ---------------------------------------------------------------------------
+// Far field
+// ---------------------------------------------------------------------------
+// Potential of one FO at one point, sum_lm MV[lm] Y_lm(u) / r^(l+1), degree LMX
+// at compile time.
+//
+// FP64: Clenshaw sums.  With w = d / r^2 and s = 1/r^2 the terms are solid
+// harmonics of w over r; per order m, Q_l = z Q_{l-1} - c_lm s Q_{l-2} once the
+// moments carry the recursion's leading factors (k_perfo_pack_mom), so a term
+// costs two fused multiply-adds instead of the four operations of forming the
+// harmonic and adding it (131 against ~250 FP64 operations at LMX = 6).
+// Moments: mv[l] for m = 0, then per m the (cos, sin) pairs of l = m..6.
+__host__ __device__ constexpr int far_pos(int l, int m) { return m == 0 ? l : 8 + 2 * ((m - 1) * 6 - (m - 1) * (m - 2) / 2 + l - m); }
+// c_lm = B_lm / (A_lm A_{l-1,m}), A = (2l-1)/(l-m), B = (l+m-1)/(l-m)
+__host__ __device__ constexpr double far_c(int l, int m) {
+  return (double)((l + m - 1) * (l - 1 - m)) / (double)((2 * l - 1) * (2 * l - 3));
+}
+
+template <int LMX>
+__device__ __forceinline__ double far_sum(const double* __restrict__ mv, double wx, double wy, double wz, double s) {
+  double pot;
+  {
+    double b1 = mv[LMX], b2 = 0.0;
+#pragma unroll
+    for (int l = LMX - 1; l >= 0; --l) {
+      double b = fma(wz, b1, mv[l]);
+      if (l + 2 <= LMX) b = fma(-far_c(l + 2, 0) * s, b2, b);
+      b2 = b1;
+      b1 = b;
+    }
+    pot = b1;
+  }
+  double c = wx, t = wy;
+#pragma unroll
+  for (int m = 1; m <= LMX; ++m) {
+    const double2 top = *reinterpret_cast<const double2*>(mv + far_pos(LMX, m));
+    double b1 = top.x, b2 = 0.0, d1 = top.y, d2 = 0.0;
+#pragma unroll
+    for (int l = LMX - 1; l >= m; --l) {
+      const double2 a = *reinterpret_cast<const double2*>(mv + far_pos(l, m));
+      double b = fma(wz, b1, a.x), d = fma(wz, d1, a.y);
+      if (l + 2 <= LMX) {
+        const double cs = -far_c(l + 2, m) * s;
+        b = fma(cs, b2, b);
+        d = fma(cs, d2, d);
+      }
+      b2 = b1;
+      b1 = b;
+      d2 = d1;
+      d1 = d;
+    }
+    pot = fma(c, b1, pot);
+    pot = fma(t, d1, pot);
+    const double nc = c * wx - t * wy;
+    t = c * wy + t * wx;
+    c = nc;
+  }
+  return pot;
+}
+
+// FP32: the harmonics of harmonics.f, summed per degree and scaled once per degree.
+template <int LMX>
+__device__ __forceinline__ float far_sum(const float* __restrict__ mv, float ux, float uy, float uz, float hn) {
+  float acc[LMX + 1];
+#pragma unroll
+  for (int l = 0; l <= LMX; ++l) acc[l] = 0.f;
+  harmonics_mmajor(ux, uy, uz, LMX, [&](int row, int l, float v) { acc[l] += mv[row] * v; });
+  float pot = 0.f, rec = hn;
+#pragma unroll
+  for (int l = 0; l <= LMX; ++l) {
+    pot += acc[l] * rec;
+    rec *= hn;
+  }
+  return pot;
+}
+
+// Moments of the per-FO calls for k_perfo_far, rows of MOM_LD doubles: in FP64
+// times the leading factors of far_sum's recursion, prod_{i=m+1..l} (2i-1)/(i-m)
+// and prod_{i=2..m} (2i-1), in its order; in the mixed path rounded to FP32 in
+// the order of the moments (MOM_LD floats, then unused space).
+__global__ void __launch_bounds__(64) k_perfo_pack_mom(int nfo, int mixed, int per_fo_only,
+                                                       const CallShare* __restrict__ share,
+                                                       const double* __restrict__ momv, double* __restrict__ out) {
+  const int c = blockIdx.x, j = threadIdx.x;
+  if ((!per_fo_only && share[c].shared) || j >= MOM_LD) return;
+  int pos = j;
+  double f = j < NMOM ? 1.0 : 0.0;
+  if (!mixed && j < NMOM) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= j) ++l;
+    const int m = (j - l * l + 1) / 2;
+    pos = far_pos(l, m) + (m > 0 && j == l * l + 2 * m);
+    for (int i = m + 1; i <= l; ++i) f *= (double)(2 * i - 1) / (double)(i - m);
+    for (int i = 2; i <= m; ++i) f *= (double)(2 * i - 1);
+  } else if (!mixed) {
+    pos = j == NMOM ? 7 : j;  // the positions far_pos leaves out
+  }
+  for (int k = blockIdx.y; k < nfo; k += gridDim.y) {
+    const size_t r = ((size_t)c * nfo + k) * MOM_LD;
+    const double v = j < NMOM ? momv[r + j] * f : 0.0;
+    if (mixed) reinterpret_cast<float*>(out + r)[j] = (float)v;
+    else out[r + pos] = v;
+  }
+}
+
+constexpr int FAR_FOS = 4;             // FOs per CTA: a warp has one FO and 64 points, two per lane
+constexpr int FAR_THREADS = 2 * 32 * FAR_FOS;
+constexpr int FAR_CALLS = 8;           // calls per buffer
+static_assert(sizeof(CallFO) == 64 && MOM_LD % 4 == 0, "copied in 16-byte pieces");
+static_assert(far_pos(6, 6) + 1 < MOM_LD, "moment positions");
+
+template <bool MIXED>
+struct FarSmem {
+  using PT = typename std::conditional<MIXED, float, double>::type;
+  CallFO f[2][FAR_CALLS][FAR_FOS];
+  PT mv[2][FAR_CALLS][FAR_FOS][MOM_LD];
+  double box[FAR_THREADS / 32 + 1][6];
+  int queue[FAR_THREADS];
+  int wcount[FAR_THREADS / 32];
+};
+
+template <bool MIXED>
+__device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp) {
+  using PT = typename std::conditional<MIXED, float, double>::type;
+  __shared__ __align__(16) FarSmem<MIXED> S;
+  constexpr int NW = FAR_THREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int k0 = grp * FAR_FOS, nk = min(FAR_FOS, J.nfo - k0);
+  const int p0 = tile * TILE, npt = min(TILE, J.M.n - p0);
+  const int* list = J.lists + J.ncalls;
+  const int nl = J.lists[2 * J.ncalls + 1];
+  if (nl == 0) return;
+  const int k = warp >> 1;                       // this warp's FO
+  const int pl = (warp & 1) * 64 + lane;         // and points pl, pl + 32
+  double x[2], y[2], z[2], V[2] = {0.0, 0.0};
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int p = p0 + min(pl + 32 * j, npt - 1);
+    x[j] = J.M.x[p];
+    y[j] = J.M.y[p];
+    z[j] = J.M.z[p];
+  }
+  {
+    double lo[3], hi[3], lo1[3], hi1[3];
+    warp_box(x[0], y[0], z[0], lo, hi);
+    warp_box(x[1], y[1], z[1], lo1, hi1);
+    if (lane == 0)
+      for (int d = 0; d < 3; ++d) {
+        S.box[warp][d] = fmin(lo[d], lo1[d]);
+        S.box[warp][3 + d] = fmax(hi[d], hi1[d]);
+      }
+  }
+  __syncthreads();
+  if (tid < 6) {
+    double v = S.box[0][tid];
+    for (int w = 1; w < NW; ++w) v = tid < 3 ? fmin(v, S.box[w][tid]) : fmax(v, S.box[w][tid]);
+    S.box[NW][tid] = v;
+  }
+  __syncthreads();
+  unsigned long long far = 0, terms = 0;
+  auto copy = [&](int e0, int e1, int b) {
+    constexpr int MP = MOM_LD * sizeof(PT) / 16;  // 16-byte pieces of one FO's moments
+    const int per = nk * (MP + 4);
+    for (int e = tid; e < (e1 - e0) * per; e += FAR_THREADS) {
+      const int i = e / per, r = e - i * per;
+      const size_t ck = (size_t)S.queue[e0 + i] * J.nfo + k0;
+      if (r < nk * MP) {
+        const int kk = r / MP, o = r - kk * MP;
+        cp_async16(reinterpret_cast<char*>(S.mv[b][i][kk]) + 16 * o,
+                   reinterpret_cast<const char*>(J.momp + (ck + kk) * MOM_LD) + 16 * o);
+      } else {
+        cp_async16(reinterpret_cast<char*>(S.f[b][i]) + 16 * (r - nk * MP),
+                   reinterpret_cast<const char*>(J.cfo + ck) + 16 * (r - nk * MP));
+      }
+    }
+    cp_async_commit();
+  };
+  for (int l0 = 0; l0 < nl; l0 += FAR_THREADS) {
+    // the window's calls with far points in the tile, in order
+    bool act = false;
+    int c = 0;
+    if (l0 + tid < nl) {
+      c = list[l0 + tid];
+      const double* bx = S.box[NW];
+      const double lo[3] = {bx[0], bx[1], bx[2]}, hi[3] = {bx[3], bx[4], bx[5]};
+      const CallBound& b = J.bound[c];
+      act = tile_class(lo, hi, b.c[0], b.c[1], b.c[2], b.rin2) != 0;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, act);
+    if (lane == 0) S.wcount[warp] = __popc(bal);
+    __syncthreads();  // and every warp is done with the previous window
+    int before = 0, qn = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const int cw = S.wcount[w];
+      before += w < warp ? cw : 0;
+      qn += cw;
+    }
+    if (act) S.queue[before + __popc(bal & ((1u << lane) - 1u))] = c;
+    __syncthreads();
+    if (qn > 0) copy(0, min(FAR_CALLS, qn), 0);
+    for (int e0 = 0, b = 0; e0 < qn; e0 += FAR_CALLS, b ^= 1) {
+      const int ne = min(FAR_CALLS, qn - e0);
+      cp_async_wait_all();
+      __syncthreads();  // this chunk has arrived and the other buffer is free
+      if (e0 + FAR_CALLS < qn) copy(e0 + FAR_CALLS, min(e0 + 2 * FAR_CALLS, qn), b ^ 1);
+      if (k >= nk) continue;
+#pragma unroll 1
+      for (int i = 0; i < ne; ++i) {
+        const CallFO& f = S.f[b][i][k];
+        if (f.npot == 1) continue;
+        const double cx = f.cg[0], cy = f.cg[1], cz = f.cg[2], rc2 = f.rcut2;
+        double r2[2];
+        bool isfar[2];
+        int nf = 0;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          r2[j] = sqdist_rn2(x[j], y[j], z[j], cx, cy, cz);
+          isfar[j] = pl + 32 * j < npt && r2[j] > rc2;
+          nf += __popc(__ballot_sync(0xffffffffu, isfar[j]));
+        }
+        if (nf == 0) continue;
+        const PT* mv = S.mv[b][i][k];
+        PT a[2][4], pot[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const PT dx = PT(x[j] - cx), dy = PT(y[j] - cy), dz = PT(z[j] - cz);
+          if constexpr (MIXED) {
+            const float hn = rsqrtf(isfar[j] ? (float)r2[j] : 1.f);
+            a[j][0] = hn * dx;
+            a[j][1] = hn * dy;
+            a[j][2] = hn * dz;
+            a[j][3] = hn;
+          } else {
+            const double hn = rsqrt(isfar[j] ? r2[j] : 1.0), s = hn * hn;
+            a[j][0] = s * dx;
+            a[j][1] = s * dy;
+            a[j][2] = s * dz;
+            a[j][3] = s;
+            r2[j] = hn;
+          }
+        }
+        switch (f.lmax) {
+#define FAR_CASE(L)                                                              \
+  {                                                                              \
+    pot[0] = far_sum<L>(mv, a[0][0], a[0][1], a[0][2], a[0][3]);                 \
+    pot[1] = far_sum<L>(mv, a[1][0], a[1][1], a[1][2], a[1][3]);                 \
+    break;                                                                       \
+  }
+          case 0: FAR_CASE(0)
+          case 1: FAR_CASE(1)
+          case 2: FAR_CASE(2)
+          case 3: FAR_CASE(3)
+          case 4: FAR_CASE(4)
+          case 5: FAR_CASE(5)
+          default: FAR_CASE(6)
+#undef FAR_CASE
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          double v;
+          if constexpr (MIXED) v = (double)pot[j];
+          else v = r2[j] * pot[j];
+          if (isfar[j]) V[j] += v;
+        }
+        if (lane == 0) {
+          far += (unsigned long long)nf;
+          terms += (unsigned long long)nf * (unsigned long long)__popcll(f.keep);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (k < nk && pl + 32 * j < npt) J.vh[(size_t)(k0 + k) * J.ldv + p0 + pl + 32 * j] += V[j];
+  count_add(J.cnt_perfo, 0, far, terms);
+}
+
+template <bool MIXED>
+__global__ void __launch_bounds__(FAR_THREADS) k_perfo_far(const __grid_constant__ CoulombJob J) {
+  far_block<MIXED>(J, blockIdx.x, blockIdx.y);
+}
+
+// items[i] = {job, tile, FO block of fob FOs, 0}; blockIdx.y: group of FAR_FOS FOs of the block.
+template <bool MIXED>
+__global__ void __launch_bounds__(FAR_THREADS)
+k_perfo_far_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__ items, int fob) {
+  __shared__ CoulombJob J;
+  const int4 w = items[blockIdx.x];
+  if (threadIdx.x == 0) J = jobs[w.x];
+  __syncthreads();
+  const int grp = w.z * (fob / FAR_FOS) + blockIdx.y;
+  if (grp * FAR_FOS >= J.nfo) return;
+  far_block<MIXED>(J, w.y, grp);
+}
+
+// ---------------------------------------------------------------------------
+// Launches
+// ---------------------------------------------------------------------------
+template <int MT>
+static cudaError_t near_attr() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto* f) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NearSmem<MT>));
+  };
+  set(k_perfo_near<MT, false>);
+  set(k_perfo_near<MT, true>);
+  set(k_perfo_near_batch<MT, false>);
+  set(k_perfo_near_batch<MT, true>);
+  return e;
+}
+
+cudaError_t init_coulomb_perfo() {
+  cudaError_t e = near_attr<4>();
+  if (e == cudaSuccess) e = near_attr<8>();
+  if (e == cudaSuccess) e = near_attr<16>();
+  return e;
+}
+
+void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
+                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed,
+                        const double* coef, const double* momv, double* coefp, double* momp, CallBound* bound,
+                        cudaStream_t st) {
+  if (ncalls <= 0 || npairs <= 0) return;
+  k_perfo_bounds<<<(ncalls + 7) / 8, 256, 0, st>>>(ncalls, nfo, calls, pairs, cfo, bound);
+  k_perfo_pack<<<npairs, 256, 0, st>>>(nfo, pairs, share, per_fo_only ? 1 : 0, coef, coefp);
+  k_perfo_pack_mom<<<dim3(ncalls, std::min(nfo, 32)), 64, 0, st>>>(nfo, mixed ? 1 : 0, per_fo_only ? 1 : 0, share, momv,
+                                                                  momp);
+}
+
+template <int MT>
+static void launch_near(const CoulombJob& J, bool mixed, const double* tab, cudaStream_t st) {
+  const dim3 grid(J.M.ntiles * NEAR_PER_TILE, (J.nfo + 8 * MT - 1) / (8 * MT));
+  if (mixed) k_perfo_near<MT, true><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(J, tab);
+  else k_perfo_near<MT, false><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(J, tab);
+}
+
+void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* tab, cudaStream_t st) {
+  if (J.M.ntiles <= 0 || J.nfo <= 0) return;
+  const dim3 grid(J.M.ntiles, (J.nfo + FAR_FOS - 1) / FAR_FOS);
+  if (mixed) k_perfo_far<true><<<grid, FAR_THREADS, 0, st>>>(J);
+  else k_perfo_far<false><<<grid, FAR_THREADS, 0, st>>>(J);
+  if (wm == 4) launch_near<16>(J, mixed, tab, st);
+  else if (wm == 2) launch_near<8>(J, mixed, tab, st);
+  else launch_near<4>(J, mixed, tab, st);
+}
+
+template <int MT>
+static void launch_near_batch(const CoulombJob* jobs, const int4* items, int nitems, bool mixed, const double* tab,
+                              cudaStream_t st) {
+  const int grid = nitems * NEAR_PER_TILE;
+  if (mixed) k_perfo_near_batch<MT, true><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(jobs, items, tab);
+  else k_perfo_near_batch<MT, false><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(jobs, items, tab);
+}
+
+void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int wm, bool mixed,
+                        const double* tab, cudaStream_t st) {
+  if (nitems <= 0) return;
+  const dim3 grid(nitems, 32 * wm / FAR_FOS);
+  if (mixed) k_perfo_far_batch<true><<<grid, FAR_THREADS, 0, st>>>(jobs, items, 32 * wm);
+  else k_perfo_far_batch<false><<<grid, FAR_THREADS, 0, st>>>(jobs, items, 32 * wm);
+  if (wm == 4) launch_near_batch<16>(jobs, items, nitems, mixed, tab, st);
+  else if (wm == 2) launch_near_batch<8>(jobs, items, nitems, mixed, tab, st);
+  else launch_near_batch<4>(jobs, items, nitems, mixed, tab, st);
+}
+
+}  // namespace flosic

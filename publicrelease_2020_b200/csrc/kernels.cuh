@@ -77,10 +77,14 @@ void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo*
 struct CoulombScratch {
   int8_t* pair_fmt;    // npairs
   CallShare* share;    // ncalls
-  int* lists;          // 2*ncalls + 2: shared calls, per-FO calls, the two counts
+  int* lists;          // 2*ncalls + 3: shared calls, per-FO calls, the two counts, pairs of the per-FO calls
+  PerfoPair* plist;    // npairs: the pairs of the per-FO calls
   float* coef_hl;      // mixed path: TF32 hi/lo split of the coefficients (2 x npairs*nfo*COEF_LD)
   float* momv_hl;      // mixed path: TF32 hi/lo split of the moments (2 x ncalls*nfo*MOM_LD)
   int* err;            // mixed path: set when a tensor-core pipeline wait reached its limit
+  double* coefp;       // npairs*nfo*NEAR_K: the per-FO calls' coefficients in MMA order
+  double* momp;        // ncalls*nfo*MOM_LD: their moments as the far kernel reads them
+  CallBound* bound;    // ncalls
 };
 // Kernel choices (all evaluate the same sums; the results differ only by the
 // rounding of the chosen arithmetic).  per_fo_only: every call through the
@@ -107,21 +111,36 @@ struct CoulombJob {
   const int8_t* pair_fmt;
   const CallFO* cfo;
   const double* momv;
+  const double* coefp;
+  const double* momp;
+  const CallBound* bound;
+  const PerfoPair* plist;
   MeshDev M;
   double* vh;
-  unsigned long long* cnt;
+  unsigned long long* cnt;        // work counts of the shared-geometry calls
+  unsigned long long* cnt_perfo;  // and of the per-FO calls
 };
 void init_coulomb_mma();
 // Pair Boys variants, shared-geometry flags and the two call lists (the set-up
 // of launch_coulomb_mma before its kernels).
-void launch_coulomb_classify(int ncalls, int npairs, int nfo, const int8_t* maxfmt, const CallFO* cfo,
-                             const CoulombScratch& scr, bool per_fo_only, cudaStream_t st);
-// Every (job, tile, FO block) item of a batch in two persistent launches
-// (shared-geometry calls, then per-FO calls added): items[i] = {job, tile,
-// FO block of 32*wm FOs, 0}, taken in list order from two device counters
-// (counters[0..1], zeroed here); nctas persistent CTAs.
-void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counters, int wm, bool mixed,
+void launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
+                             const CallFO* cfo, const CoulombScratch& scr, bool per_fo_only, cudaStream_t st);
+// The shared-geometry calls of every (job, tile, FO block) item of a batch in
+// one persistent launch: items[i] = {job, tile, FO block of 32*wm FOs, 0}, taken
+// in list order from a device counter (zeroed here) by nctas CTAs.
+void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
                           const double* boys_tab, int nctas, cudaStream_t st);
+// Per-FO calls (csrc/coulomb_perfo.cu): spheres of the calls and coefficients
+// in MMA order, then the far and the near field added to vh.
+cudaError_t init_coulomb_perfo();
+void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
+                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed,
+                        const double* coef, const double* momv, double* coefp, double* momp, CallBound* bound,
+                        cudaStream_t st);
+inline int perfo_default_wm(int nfo) { return nfo > 32 ? 2 : 1; }
+void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* boys_tab, cudaStream_t st);
+void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int wm, bool mixed,
+                        const double* boys_tab, cudaStream_t st);
 void init_coulomb_tc();
 // TF32 hi/lo split of nrow x nfo rows of KSEG doubles into the chunk-major
 // [nrow][KSEG/4][nfo][4] layout (hi, then lo at + nrow*nfo*KSEG floats).

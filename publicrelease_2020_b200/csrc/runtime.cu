@@ -249,7 +249,9 @@ struct TypeInfo {
 // Coulomb inputs of one spin for a batched launch over many molecules (the
 // per-molecule path keeps them in the context and reuses them per spin).
 struct CoulBufs {
-  DevBuf<double> coef, cgp, mom;
+  DevBuf<double> coef, cgp, mom, coefp, momp;
+  DevBuf<CallBound> bound;
+  DevBuf<PerfoPair> plist;
   DevBuf<int8_t> maxfmt, pairfmt;
   DevBuf<CallFO> callfo;
   DevBuf<CallShare> share;
@@ -259,6 +261,10 @@ struct CoulBufs {
     coef.release();
     cgp.release();
     mom.release();
+    coefp.release();
+    momp.release();
+    bound.release();
+    plist.release();
     maxfmt.release();
     pairfmt.release();
     callfo.release();
@@ -351,6 +357,9 @@ struct flosic_ctx {
   DevBuf<double> d_basis, d_fodpts, d_psig, d_tmat, d_u, d_coef, d_cgp, d_mom, d_part, d_sums, d_sic, d_tmp;
   DevBuf<int8_t> d_maxfmt, d_pairfmt;
   DevBuf<CallShare> d_share;
+  DevBuf<double> d_coefp, d_momp;
+  DevBuf<CallBound> d_bound;
+  DevBuf<PerfoPair> d_plist;
   DevBuf<int> d_lists, d_tc_err;
   DevBuf<int> d_setup_list;  // one-slot calls first (nsingle), then the others
   int nsingle = 0;
@@ -776,7 +785,8 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
   CUDA_CHECK(cudaEventRecord(c->ev[3], st));
   c->d_pairfmt.ensure((size_t)std::max(npairs, 1));
   c->d_share.ensure((size_t)std::max(ncalls, 1));
-  c->d_lists.ensure((size_t)2 * ncalls + 2);
+  c->d_lists.ensure((size_t)2 * ncalls + 3);
+  c->d_plist.ensure((size_t)std::max(npairs, 1));
   c->d_cnt.ensure(6);
   CUDA_CHECK(cudaMemsetAsync(c->d_cnt.p, 0, 6 * sizeof(unsigned long long), st));
   const bool mixed = c->precision == FLOSIC_PRECISION_MIXED;
@@ -786,12 +796,17 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
     c->d_tc_err.ensure(1);
     CUDA_CHECK(cudaMemsetAsync(c->d_tc_err.p, 0, sizeof(int), st));
   }
-  CoulombScratch scr{c->d_pairfmt.p, c->d_share.p, c->d_lists.p, c->d_coef_hl.p, c->d_momv_hl.p, c->d_tc_err.p};
+  c->d_coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
+  c->d_momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
+  c->d_bound.ensure((size_t)std::max(ncalls, 1));
+  CoulombScratch scr{c->d_pairfmt.p, c->d_share.p,  c->d_lists.p, c->d_plist.p, c->d_coef_hl.p,
+                     c->d_momv_hl.p, c->d_tc_err.p, c->d_coefp.p, c->d_momp.p,
+                     c->d_bound.p};
   CUDA_CHECK(launch_coulomb_mma(ncalls, c->d_calls.p, c->d_pairs.p, npairs, nf, c->d_coef.p, c->d_maxfmt.p,
                                 c->d_callfo.p, c->d_mom.p, c->eval_mesh(), c->d_boys.p, vh, P, c->coulomb_cfg, mixed,
                                 scr, c->d_cnt.p, c->ev[8], st));
   CUDA_CHECK(cudaEventRecord(c->ev[9], st));
-  c->launches += c->coulomb_cfg.per_fo_only ? 4 : 5;
+  c->launches += c->coulomb_cfg.per_fo_only ? 8 : 9;
   unsigned long long cnt[6];
   int tc_err = 0;
   CUDA_CHECK(cudaMemcpyAsync(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost, st));
@@ -1152,16 +1167,23 @@ CoulombJob batch_prepare(flosic_ctx* c, int s) {
   B.mom.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
   B.pairfmt.ensure((size_t)std::max(npairs, 1));
   B.share.ensure((size_t)std::max(ncalls, 1));
-  B.lists.ensure((size_t)2 * ncalls + 2);
+  B.lists.ensure((size_t)2 * ncalls + 3);
+  B.plist.ensure((size_t)std::max(npairs, 1));
   B.cnt.ensure(3);
   launch_pair_coef(npairs, c->d_pairs.p, c->d_calls.p, nf, c->nprim, c->d_u.p, nullptr, c->nspn, B.coef.p,
                    B.maxfmt.p, B.cgp.p, st);
   launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn, B.coef.p,
                     B.maxfmt.p, B.cgp.p, c->mesh_dev(), c->d_boys.p, B.callfo.p, B.mom.p, st);
   CUDA_CHECK(cudaMemsetAsync(B.cnt.p, 0, 3 * sizeof(unsigned long long), st));
-  CoulombScratch scr{B.pairfmt.p, B.share.p, B.lists.p, nullptr, nullptr, nullptr};
-  launch_coulomb_classify(ncalls, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
-  c->launches += 6;
+  B.coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
+  B.momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
+  B.bound.ensure((size_t)std::max(ncalls, 1));
+  CoulombScratch scr{B.pairfmt.p, B.share.p, B.lists.p, B.plist.p, nullptr, nullptr, nullptr, B.coefp.p, B.momp.p,
+                     B.bound.p};
+  launch_coulomb_classify(ncalls, c->d_calls.p, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
+  launch_perfo_setup(ncalls, npairs, nf, c->d_calls.p, c->d_pairs.p, B.callfo.p, B.share.p, false,
+                     c->precision == FLOSIC_PRECISION_MIXED, B.coef.p, B.mom.p, B.coefp.p, B.momp.p, B.bound.p, st);
+  c->launches += 9;
   pair_density(c, s, B.callfo.p);
   S.vh.ensure((size_t)nf * P);
   CoulombJob J{};
@@ -1176,9 +1198,14 @@ CoulombJob batch_prepare(flosic_ctx* c, int s) {
   J.pair_fmt = B.pairfmt.p;
   J.cfo = B.callfo.p;
   J.momv = B.mom.p;
+  J.coefp = B.coefp.p;
+  J.momp = B.momp.p;
+  J.bound = B.bound.p;
+  J.plist = B.plist.p;
   J.M = c->eval_mesh();
   J.vh = S.vh.p;
   J.cnt = B.cnt.p;
+  J.cnt_perfo = B.cnt.p;
   return J;
 }
 
@@ -1259,6 +1286,7 @@ int flosic_sic_create(int device, flosic_ctx** out) {
     upload_constants(ang.data(), w.data());
     init_call_setup();
     init_coulomb_mma();
+    CUDA_CHECK(init_coulomb_perfo());
     init_coulomb_tc();
     CUDA_CHECK(init_sym_eigen());
     CUDA_CHECK(init_contract());
@@ -1286,6 +1314,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_basis.release(); c->d_fodpts.release(); c->d_psig.release(); c->d_tmat.release(); c->d_u.release();
   c->d_coef.release(); c->d_cgp.release(); c->d_mom.release(); c->d_part.release(); c->d_sums.release();
   c->d_sic.release(); c->d_tmp.release(); c->d_maxfmt.release(); c->d_callfo.release(); c->d_cnt.release(); c->d_pairfmt.release();
+  c->d_coefp.release(); c->d_momp.release(); c->d_bound.release(); c->d_plist.release();
   c->d_share.release(); c->d_lists.release(); c->d_setup_list.release();
   c->d_eig_a.release(); c->d_eig_w.release(); c->d_eig_v.release(); c->d_eig_work.release(); c->d_eig_info.release();
   c->d_coef_hl.release(); c->d_momv_hl.release(); c->d_tc_err.release(); c->d_dens_coef.release();
@@ -1957,7 +1986,7 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       for (int t = 0; t < J.M.ntiles; ++t)
         for (int b = 0; b < nfb; ++b) items.push_back(make_int4(job, t, b, 0));
     }
-    // 2. all potentials of all molecules: two persistent launches on the first context's stream
+    // 2. all potentials of all molecules in three launches on the first context's stream
     int nsm = 148;
     CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c0->device));
     c0->d_jobs.ensure(std::max<size_t>(jobs.size(), 1));
@@ -1967,11 +1996,13 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
                                  c0->st));
       CUDA_CHECK(cudaMemcpyAsync(c0->d_items.p, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice,
                                  c0->st));
-      c0->d_batch_counters.ensure(2);
+      c0->d_batch_counters.ensure(1);
       launch_coulomb_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), c0->d_batch_counters.p, wm,
                            c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, nsm, c0->st);
+      launch_perfo_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), wm,
+                         c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, c0->st);
       CUDA_CHECK(cudaGetLastError());
-      c0->launches += 2;
+      c0->launches += 3;
     }
     CUDA_CHECK(cudaEventRecord(c0->ev[4], c0->st));
     for (int m = 1; m < n; ++m) CUDA_CHECK(cudaStreamWaitEvent(ctxs[m]->st, c0->ev[4], 0));
