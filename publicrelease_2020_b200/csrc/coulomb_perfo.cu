@@ -12,8 +12,8 @@
 //                 each k-step at point n; one column per (pair, point), the Boys
 //                 values of four pairs at once over the four lanes of a point),
 //                 and multiplies the coefficient rows of its own near FOs into
-//                 FP64 accumulators.  Calls near for every FO accumulate on;
-//                 the others are added masked, point by point.
+//                 FP64 accumulators, added call by call, masked point by
+//                 point where a sphere cuts the warp's box.
 //   k_perfo_far   One warp owns 64 points (two per lane) and one FO and adds
 //                 the L <= 6 multipole expansions of the far calls as Clenshaw
 //                 sums.
@@ -301,28 +301,11 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
   int row[MT];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) T[mt][0] = T[mt][1] = 0.0, row[mt] = 0;
-  bool dirty = false;
   int na = 0;
   PT Fq[5] = {};  // Boys values of one pair of the current four
   const int cyc = max(q - 1, 0);  // the lane's coordinates: (x,y,z), (x,y,z), (y,z,x), (z,x,y)
   const double pa = pts[n][cyc], pb_ = pts[n][cyc == 2 ? 0 : cyc + 1], pc = pts[n][cyc == 0 ? 2 : cyc - 1];
   unsigned long long near = 0;
-  // V += T for slots that are the block's FOs in order
-  auto flush = [&] {
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      const int k = mt * 8 + n;
-      if (k < nk) {
-        double2* ch = reinterpret_cast<double2*>(V + k * NEAR_PTS + 2 * q);
-        double2 v = *ch;
-        v.x += T[mt][0];
-        v.y += T[mt][1];
-        *ch = v;
-      }
-      T[mt][0] = T[mt][1] = 0.0;
-    }
-    dirty = false;
-  };
   // asynchronous copy of the coefficient rows of queue entries [e0, e1) into
   // buffer b, one warp per entry: [group][listed FO][16], the halves of odd rows
   // exchanged so that the eight lanes of two rows read all 32 banks
@@ -460,7 +443,6 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
           if (w.flags & 1) {
             na = nk;  // a call that is near for every FO lists them all
             if (!isfull) {  // the FOs with near points of this warp, compacted into slots
-              if (dirty) flush();
               const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
               const double lo[3] = {box[0], box[1], box[2]}, hi[3] = {box[3], box[4], box[5]};
               na = 0;
@@ -513,35 +495,42 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
             F[4] = __shfl_sync(0xffffffffu, Fq[4], src);
             near_mma<MT, PT, 2>(T, Ae + 2 * nl * 16, row, nmt, L, F, q == 0);
           }
-          if (isfull) {
-            dirty = true;
-            if (lane == 0) near += (unsigned)(nk * npt);
-          } else if (w.flags & 2) {
-            // masked add: a point counts for an FO when it is inside the FO's sphere
-            const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
-            const int np = J.bound[w.call].np;
+          if (!(w.flags & 2)) continue;
+          // the call's sum goes to V (call by call, so that no sum depends on how
+          // FOs are blocked); a point counts for an FO when it is inside the FO's sphere
+          const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
+          const int np = J.bound[w.call].np;
+          if (isfull && lane == 0) near += (unsigned long long)(nk * npt) * np;
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-              const int s = mt * 8 + n;
-              if (s < na) {
-                const int sl = S.slot[warp][s], k = list[sl & 127];
-                const bool all = sl >= 128;
-                const CallFO& f = cf[k];
-                const double cx = f.cg[0], cy = f.cg[1], cz = f.cg[2], rc2 = f.rcut2;
-                const double *p0 = pts[2 * q], *p1 = pts[2 * q + 1];
-                const bool n0 = 2 * q < npt && (all || !(sqdist_rn2(p0[0], p0[1], p0[2], cx, cy, cz) > rc2));
-                const bool n1 = 2 * q + 1 < npt && (all || !(sqdist_rn2(p1[0], p1[1], p1[2], cx, cy, cz) > rc2));
-                double2* ch = reinterpret_cast<double2*>(V + k * NEAR_PTS + 2 * q);
-                double2 v = *ch;
-                if (n0) v.x += T[mt][0];
-                if (n1) v.y += T[mt][1];
-                *ch = v;
-                near += (unsigned long long)(((int)n0 + (int)n1) * np);
+          for (int mt = 0; mt < MT; ++mt) {
+            if (mt >= nmt) break;
+            const int s = mt * 8 + n;
+            if (s < na) {
+              int k = s;
+              bool n0 = true, n1 = true;  // points past the end: never stored
+              if (!isfull) {
+                const int sl = S.slot[warp][s];
+                k = list[sl & 127];
+                n0 = 2 * q < npt;
+                n1 = 2 * q + 1 < npt;
+                if (sl < 128) {
+                  const CallFO& f = cf[k];
+                  const double cx = f.cg[0], cy = f.cg[1], cz = f.cg[2], rc2 = f.rcut2;
+                  const double *p0 = pts[2 * q], *p1 = pts[2 * q + 1];
+                  n0 = n0 && !(sqdist_rn2(p0[0], p0[1], p0[2], cx, cy, cz) > rc2);
+                  n1 = n1 && !(sqdist_rn2(p1[0], p1[1], p1[2], cx, cy, cz) > rc2);
+                }
+                near += (unsigned)(((int)n0 + (int)n1) * np);
               }
-              T[mt][0] = T[mt][1] = 0.0;
+              double2* ch = reinterpret_cast<double2*>(V + k * NEAR_PTS + 2 * q);
+              double2 v = *ch;
+              if (n0) v.x += T[mt][0];
+              if (n1) v.y += T[mt][1];
+              *ch = v;
             }
-            __syncwarp();
+            T[mt][0] = T[mt][1] = 0.0;
           }
+          if (!isfull) __syncwarp();
         }
       }
       e0 = e1;
@@ -550,7 +539,6 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
     }
   }
   if (npt > 0) {
-    if (dirty) flush();
     __syncwarp();
     for (int e = lane; e < nk * NEAR_PTS; e += 32) {
       const int k = e / NEAR_PTS, p = e - k * NEAR_PTS;

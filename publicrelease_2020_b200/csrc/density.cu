@@ -232,7 +232,7 @@ constexpr int DENS_NBUF = 4;
 template <int NCH, int LDC>
 __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int ncalls, const CallInfo* __restrict__ calls,
                                                                const PairGeo* __restrict__ pairs,
-                                                               const CallFO* __restrict__ cfo, int nfo,
+                                                               const CallFO* __restrict__ cfo, int cfo_ld, int nfo,
                                                                const double* __restrict__ dc,
                                                                double* __restrict__ rhog, size_t ldr) {
   static_assert(LDC % 2 == 0 && LDC / 2 <= DENS_THREADS, "one 16-byte chunk of a row per thread");
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int nc
     bool hit = false;
     CallFO cf;
     if (c < ncalls) {
-      cf = cfo[(size_t)c * nfo + k];
+      cf = cfo[(size_t)c * cfo_ld + k];
       hit = cf.npot == 1 || tile_class(lo, hi, cf.cg[0], cf.cg[1], cf.cg[2], cf.rcut2) != 1;
     }
     const unsigned b = __ballot_sync(0xffffffffu, hit);
@@ -349,18 +349,18 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int nc
 int pair_density_ld(int nch) { return nch == 1 ? 36 : (nch == 4 ? 96 : 156); }
 
 void launch_pair_density(int npairs, const PairGeo* pairs, int ncalls, const CallInfo* calls, const CallFO* cfo,
-                         int nfo, int nprim, const double* u, int nch, const MeshDev& M, double* dc, double* rhog,
+                         int cfo_ld, int nfo, int nprim, const double* u, int nch, const MeshDev& M, double* dc, double* rhog,
                          size_t ldr, cudaStream_t st) {
   if (nfo <= 0 || M.ntiles <= 0) return;
   const int ldc = pair_density_ld(nch);
   if (npairs > 0) k_pair_dens_coef<<<npairs, 128, 0, st>>>(pairs, nfo, nprim, u, nch, dc, ldc);
   dim3 grid(M.ntiles, nfo);
   if (nch == 1)
-    k_pair_density<1, 36><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, nfo, dc, rhog, ldr);
+    k_pair_density<1, 36><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
   else if (nch == 4)
-    k_pair_density<4, 96><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, nfo, dc, rhog, ldr);
+    k_pair_density<4, 96><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
   else
-    k_pair_density<10, 156><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, nfo, dc, rhog, ldr);
+    k_pair_density<10, 156><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
 }
 
 }  // namespace flosic

@@ -276,6 +276,7 @@ struct CoulBufs {
 
 struct SpinCache {
   bool fo_valid = false;       // FMAT/TMAT/CFO
+  bool vh_valid = false;       // raw Coulomb potentials at vhp
   bool pot_valid = false;      // potentials, RESULTS
   int nf = 0, nw = 0;
   std::vector<double> fmat;    // [(K*nf + jfm)*nw + jwf]
@@ -290,7 +291,9 @@ struct SpinCache {
   bool sic_valid = false;
   DevBuf<double> cfo;          // nb x nf
   DevBuf<double> phi;          // [ch][k][P]
-  DevBuf<double> vh;           // raw Coulomb [k][P]
+  DevBuf<double> vh;           // raw Coulomb [k][P]; of both spins when evaluated together (spin 0's buffer)
+  double* vhp = nullptr;       // this spin's part
+  int kofs = 0, kld = 0;       // this spin's first FO and the FO count of the Coulomb evaluation that made it
   DevBuf<double> vpot;         // SIC potential [k][P]
   DevBuf<double> y;            // w V phi [k][P]
   DevBuf<double> rhog;         // pair-route density channels [ch][k][P] (FLOSIC_DENSITY_PAIRS)
@@ -625,7 +628,7 @@ void sort_mesh(flosic_ctx* c, const double* rmsh, const double* wmsh) {
 
 void invalidate(flosic_ctx* c) {
   for (auto& s : c->spin) {
-    s.fo_valid = s.pot_valid = s.sic_valid = false;
+    s.fo_valid = s.vh_valid = s.pot_valid = s.sic_valid = false;
   }
 }
 
@@ -833,21 +836,48 @@ void pair_density(flosic_ctx* c, int s, const CallFO* cfo) {
   const int npairs = (int)c->pairs.size(), ncalls = (int)c->calls.size();
   c->d_dens_coef.ensure((size_t)std::max(npairs, 1) * nf * pair_density_ld(nch));
   S.rhog.ensure((size_t)nch * nf * P);
-  launch_pair_density(npairs, c->d_pairs.p, ncalls, c->d_calls.p, cfo, nf, c->nprim, c->d_u.p, nch, c->eval_mesh(),
-                      c->d_dens_coef.p, S.rhog.p, (size_t)P, c->st);
+  launch_pair_density(npairs, c->d_pairs.p, ncalls, c->d_calls.p, cfo + S.kofs, S.kld, nf, c->nprim,
+                      c->d_u.p + (size_t)S.kofs * c->nprim * 10, nch, c->eval_mesh(), c->d_dens_coef.p, S.rhog.p,
+                      (size_t)P, c->st);
   CUDA_CHECK(cudaGetLastError());
   c->launches += 2;
 }
 
-// COUPOT_SIC's Coulomb part for the FOs of spin s.
-void coulomb(flosic_ctx* c, int s) {
-  SpinCache& S = c->spin[s];
-  const int nf = S.nf;
+// The spins [s0, s0 + ns) as one set of FOs for a Coulomb evaluation: their
+// primitive projections one after another in d_u, their potentials in the
+// first spin's buffer.  Returns the FO count.
+int coulomb_set(flosic_ctx* c, int s0, int ns) {
+  int nf = 0;
+  for (int s = s0; s < s0 + ns; ++s) nf += c->spin[s].nf;
   c->d_u.ensure((size_t)nf * c->nprim * 10);
-  launch_prim_u(c->basis_dev(), nf, S.cfo.p, c->nbasis, c->d_u.p, c->st);
-  c->launches++;
-  S.vh.ensure((size_t)nf * c->eval_n);
-  coulomb_eval(c, nf, nullptr, S.vh.p);
+  c->spin[s0].vh.ensure((size_t)nf * c->eval_n);
+  int k = 0;
+  for (int s = s0; s < s0 + ns; ++s) {
+    SpinCache& S = c->spin[s];
+    launch_prim_u(c->basis_dev(), S.nf, S.cfo.p, c->nbasis, c->d_u.p + (size_t)k * c->nprim * 10, c->st);
+    c->launches++;
+    S.vhp = c->spin[s0].vh.p + (size_t)k * c->eval_n;
+    S.kofs = k;
+    S.kld = nf;
+    k += S.nf;
+  }
+  return nf;
+}
+
+// COUPOT_SIC's Coulomb part for the FOs of spins [s0, s0 + ns).
+void coulomb(flosic_ctx* c, int s0, int ns = 1) {
+  const int nf = coulomb_set(c, s0, ns);
+  coulomb_eval(c, nf, nullptr, c->spin[s0].vh.p);
+  for (int s = s0; s < s0 + ns; ++s) c->spin[s].vh_valid = true;
+}
+
+// Whether a cycle evaluates the Coulomb potentials of both spins together: the
+// columns of a (pair, point) do not depend on the FO, so when the FOs of both
+// spins fit one FO block of the per-FO kernel (64) they are formed once instead
+// of twice (benzene, 21 + 21 FOs: 35.2 -> 30.8 ms; with 37 + 37 there are two
+// blocks either way).
+bool spins_together(const flosic_ctx* c) {
+  return c->nspn == 2 && c->nfrm[0] > 0 && c->nfrm[1] > 0 && c->nfrm[0] + c->nfrm[1] <= 64;
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
@@ -871,32 +901,48 @@ void spin_potentials(flosic_ctx* c, int s) {
   CUDA_CHECK(cudaEventRecord(c->ev[1], st));
   fo_values(c, s);
   CUDA_CHECK(cudaEventRecord(c->ev[7], st));
-  coulomb(c, s);
+  const bool eval = !S.vh_valid;
+  if (eval) coulomb(c, s);
   CUDA_CHECK(cudaEventRecord(c->ev[4], st));
   pair_density(c, s, c->d_callfo.p);  // FLOSIC_DENSITY_PAIRS only; timed with XC
   spin_xc(c, s);
   c->stage_ms[0] += elapsed(c->ev[0], c->ev[1]);
   c->stage_ms[1] += elapsed(c->ev[1], c->ev[7]);
-  c->stage_ms[2] += elapsed(c->ev[7], c->ev[3]);
-  c->stage_ms[3] += elapsed(c->ev[3], c->ev[4]);
+  if (eval) {
+    c->stage_ms[2] += elapsed(c->ev[7], c->ev[3]);
+    c->stage_ms[3] += elapsed(c->ev[3], c->ev[4]);
+  }
   c->stage_ms[4] += elapsed(c->ev[4], c->ev[5]);
 }
 
+// FO construction and Coulomb potentials of both spins in one evaluation.
+void cycle_coulomb(flosic_ctx* c) {
+  cudaStream_t st = c->st;
+  CUDA_CHECK(cudaEventRecord(c->ev[0], st));
+  for (int s = 0; s < 2; ++s) fo_setup(c, s);
+  CUDA_CHECK(cudaEventRecord(c->ev[7], st));
+  coulomb(c, 0, 2);
+  CUDA_CHECK(cudaEventRecord(c->ev[4], st));
+  CUDA_CHECK(cudaEventSynchronize(c->ev[4]));
+  c->stage_ms[0] += elapsed(c->ev[0], c->ev[7]);
+  c->stage_ms[2] += elapsed(c->ev[7], c->ev[3]);
+  c->stage_ms[3] += elapsed(c->ev[3], c->ev[4]);
+}
+
 // XC and the APOTNL_SIC mesh sums of spin s from its FO values and raw
-// Coulomb potentials (S.phi, S.vh), then RESULTS; marks the potentials valid.
+// Coulomb potentials (S.phi, S.vhp), then RESULTS; marks the potentials valid.
 void spin_xc(flosic_ctx* c, int s) {
   SpinCache& S = c->spin[s];
   cudaStream_t st = c->st;
   const int nf = S.nf, P = c->eval_n;
   S.vpot.ensure((size_t)nf * P);
   S.y.ensure((size_t)(c->mgga ? 4 : 1) * nf * P);
-  S.vh.ensure((size_t)nf * P);
   const int nblk = std::min(1024, (P + 255) / 256);
   c->d_part.ensure((size_t)nf * nblk * NPART);
   c->d_sums.ensure((size_t)nf * NPART);
   // XC reads the raw Coulomb potential; keep a scaled copy out of place
   c->d_tmp.ensure((size_t)nf * P);
-  CUDA_CHECK(cudaMemcpyAsync(c->d_tmp.p, S.vh.p, sizeof(double) * nf * P, cudaMemcpyDeviceToDevice, st));
+  CUDA_CHECK(cudaMemcpyAsync(c->d_tmp.p, S.vhp, sizeof(double) * nf * P, cudaMemcpyDeviceToDevice, st));
   const double* rhog = c->density == FLOSIC_DENSITY_PAIRS ? S.rhog.p : nullptr;
   launch_xc(c->eval_mesh(), nf, c->gga, c->mgga, c->nspn, c->xc, S.phi.p, P, rhog, c->d_tmp.p, S.vpot.p, S.y.p,
             c->d_part.p, nblk, st);
@@ -1146,20 +1192,20 @@ void adjoint_device(flosic_ctx* c, int s, DevBuf<double>& dg) {
 //   dE/dT = (W + W^T) T + (M S^-1/2)^T,  dE/da_m = sum_j (dE/dT)_mj dT_mj/da_m.
 // This is the reference's FOD force (frmorb2.F:586-717, times 2/NSPN) reached
 // through the basis-space adjoint instead of the SIC matrix.
-// Batch of molecules: everything of spin s before its Coulomb evaluation --
-// FO construction, FO values, pair coefficients, POISSON1 call set-up and
-// call classification -- into the spin's own buffers, on the context's stream.
-// Returns the spin's job for the batched Coulomb launch.
-CoulombJob batch_prepare(flosic_ctx* c, int s) {
-  SpinCache& S = c->spin[s];
-  fo_setup(c, s);
-  fo_values(c, s);
-  const int nf = S.nf, P = c->eval_n;
+// Batch of molecules: everything of spins [s0, s0 + ns) before their Coulomb
+// evaluation -- FO construction, FO values, pair coefficients, POISSON1 call
+// set-up and call classification -- into the first spin's own buffers, on the
+// context's stream.  Returns their job for the batched Coulomb launch.
+CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
+  for (int s = s0; s < s0 + ns; ++s) {
+    fo_setup(c, s);
+    fo_values(c, s);
+  }
+  const int P = c->eval_n;
   const int npairs = (int)c->pairs.size(), ncalls = (int)c->calls.size();
   cudaStream_t st = c->st;
-  c->d_u.ensure((size_t)nf * c->nprim * 10);
-  launch_prim_u(c->basis_dev(), nf, S.cfo.p, c->nbasis, c->d_u.p, st);
-  CoulBufs& B = S.bc;
+  const int nf = coulomb_set(c, s0, ns);
+  CoulBufs& B = c->spin[s0].bc;
   B.coef.ensure((size_t)std::max(npairs, 1) * nf * COEF_LD);
   B.maxfmt.ensure((size_t)std::max(npairs, 1) * nf);
   B.cgp.ensure((size_t)std::max(npairs, 1) * nf * 4);
@@ -1183,9 +1229,8 @@ CoulombJob batch_prepare(flosic_ctx* c, int s) {
   launch_coulomb_classify(ncalls, c->d_calls.p, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
   launch_perfo_setup(ncalls, npairs, nf, c->d_calls.p, c->d_pairs.p, B.callfo.p, B.share.p, false,
                      c->precision == FLOSIC_PRECISION_MIXED, B.coef.p, B.mom.p, B.coefp.p, B.momp.p, B.bound.p, st);
-  c->launches += 9;
-  pair_density(c, s, B.callfo.p);
-  S.vh.ensure((size_t)nf * P);
+  c->launches += 8;
+  for (int s = s0; s < s0 + ns; ++s) pair_density(c, s, B.callfo.p);
   CoulombJob J{};
   J.ncalls = ncalls;
   J.nfo = nf;
@@ -1203,7 +1248,7 @@ CoulombJob batch_prepare(flosic_ctx* c, int s) {
   J.bound = B.bound.p;
   J.plist = B.plist.p;
   J.M = c->eval_mesh();
-  J.vh = S.vh.p;
+  J.vh = c->spin[s0].vh.p;
   J.cnt = B.cnt.p;
   J.cnt_perfo = B.cnt.p;
   return J;
@@ -1614,7 +1659,7 @@ int flosic_sic_coupot_sic(flosic_ctx* c, int kxxs, int kxxo, double* coulomb, do
     SpinCache& S = c->spin[s];
     const int P = c->nmsh, k = kxxo - 1;
     std::vector<double> v(P), r((size_t)10 * P, 0.0);
-    CUDA_CHECK(cudaMemcpyAsync(v.data(), S.vh.p + (size_t)k * P, sizeof(double) * P, cudaMemcpyDeviceToHost, c->st));
+    CUDA_CHECK(cudaMemcpyAsync(v.data(), S.vhp + (size_t)k * P, sizeof(double) * P, cudaMemcpyDeviceToHost, c->st));
     if (c->density == FLOSIC_DENSITY_PAIRS) {
       // the channels POISSON1 accumulated (meta-GGA: 4, the rest of the 10-channel layout zero)
       CUDA_CHECK(cudaMemcpy2DAsync(r.data(), sizeof(double) * P, S.rhog.p + (size_t)k * P,
@@ -1725,7 +1770,7 @@ int flosic_sic_set_density_mode(flosic_ctx* c, int mode) {
     if (mode != c->density) {
       c->density = mode;
       for (auto& s : c->spin) {
-        s.pot_valid = false;
+        s.vh_valid = s.pot_valid = false;
         s.sic_valid = false;
         if (mode == FLOSIC_DENSITY_PHI2) s.rhog.release();
       }
@@ -1741,7 +1786,7 @@ int flosic_sic_set_precision(flosic_ctx* c, int mode) {
     if (mode != c->precision) {
       c->precision = mode;
       for (auto& s : c->spin) {
-        s.pot_valid = false;
+        s.vh_valid = s.pot_valid = false;
         s.sic_valid = false;
       }
     }
@@ -1761,12 +1806,20 @@ int flosic_sic_autotune(flosic_ctx* c, int reps, int* perfo_fos, float* ms) {
     require(c, true);
     if (reps < 1 || reps > 100) fail(FLOSIC_ERR_ARG, "REPS must be in 1..100");
     if (!perfo_fos) fail(FLOSIC_ERR_ARG, "null output pointer");
-    const int s = (c->nspn == 2 && c->nfrm[1] > c->nfrm[0]) ? 1 : 0;
+    // the evaluation a cycle makes: of both spins together, or of the spin with the most FOs
+    bool both = spins_together(c);
+    if (both) {
+      try {
+        for (int t = 0; t < 2; ++t) fo_setup(c, t);
+      } catch (const Fail&) {
+        both = false;  // one spin's FODs cannot be used: tune on the other
+      }
+    }
+    const int s = !both && c->nspn == 2 && c->nfrm[1] > c->nfrm[0] ? 1 : 0, ns = both ? 2 : 1;
     if (c->nfrm[s] < 1) fail(FLOSIC_ERR_STATE, "no FOs to tune on");
-    // The timing runs overwrite this spin's potentials: drop the cached ones
-    // first, and put the width and counters back on every way out.
-    c->spin[s].pot_valid = false;
-    c->spin[s].sic_valid = false;
+    // The timing runs overwrite these potentials: drop the cached ones first,
+    // and put the width and counters back on every way out.
+    for (int t = s; t < s + ns; ++t) c->spin[t].vh_valid = c->spin[t].pot_valid = c->spin[t].sic_valid = false;
     struct Restore {
       flosic_ctx* c;
       int wm;
@@ -1781,7 +1834,7 @@ int flosic_sic_autotune(flosic_ctx* c, int reps, int* perfo_fos, float* ms) {
       }
     } restore{c, c->coulomb_cfg.perfo_wm, c->work_near, c->work_far, c->work_terms, c->launches};
     fo_setup(c, s);
-    const int nf = c->spin[s].nf;
+    const int nf = c->spin[s].nf + (both ? c->spin[1].nf : 0);
     cudaStream_t st = c->st;
     float best = std::numeric_limits<float>::infinity();
     int best_wm = 0;
@@ -1790,11 +1843,11 @@ int flosic_sic_autotune(flosic_ctx* c, int reps, int* perfo_fos, float* ms) {
       if (ms) ms[i] = -1.f;
       if (wm > 1 && 16 * wm >= nf) continue;  // half the block or more would stay empty
       c->coulomb_cfg.perfo_wm = wm;
-      coulomb(c, s);
+      coulomb(c, s, ns);
       float t = std::numeric_limits<float>::infinity();
       for (int r = 0; r < reps; ++r) {
         CUDA_CHECK(cudaEventRecord(c->ev[5], st));
-        coulomb(c, s);
+        coulomb(c, s, ns);
         CUDA_CHECK(cudaEventRecord(c->ev[6], st));
         CUDA_CHECK(cudaEventSynchronize(c->ev[6]));
         t = std::min(t, elapsed(c->ev[5], c->ev[6]));
@@ -1908,6 +1961,7 @@ int flosic_sic_cycle(flosic_ctx* c, int ld, double* results, double* sic, double
     c->kernel_ms[0] = c->kernel_ms[1] = 0.0;
     for (auto& w : c->kernel_work) w = 0;
     invalidate(c);
+    if (spins_together(c)) cycle_coulomb(c);
     double zsic = 0.0;
     for (int s = 0; s < c->nspn; ++s) {
       const int nf = c->nfrm[s];
@@ -1949,13 +2003,16 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
     CUDA_CHECK(cudaSetDevice(c0->device));
     if (wm == 0) {  // widest block that the largest FO count fills at least half
       int nfmax = 1;
-      for (int m = 0; m < n; ++m)
-        for (int s = 0; s < ctxs[m]->nspn; ++s) nfmax = std::max(nfmax, ctxs[m]->nfrm[s]);
+      for (int m = 0; m < n; ++m) {
+        const flosic_ctx* c = ctxs[m];
+        for (int s = 0; s < c->nspn; ++s) nfmax = std::max(nfmax, c->nfrm[s]);
+        if (spins_together(c)) nfmax = std::max(nfmax, c->nfrm[0] + c->nfrm[1]);
+      }
       wm = nfmax > 64 ? 4 : (nfmax > 32 ? 2 : 1);
     }
     // 1. every (molecule, spin) up to its Coulomb evaluation, on its own stream
     std::vector<CoulombJob> jobs;
-    std::vector<std::pair<int, int>> owner;  // (molecule, spin) of each job
+    std::vector<std::pair<int, int>> owner;  // (molecule, first spin) of each job
     std::vector<int4> items;
     for (int m = 0; m < n; ++m) {
       flosic_ctx* c = ctxs[m];
@@ -1968,8 +2025,10 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       CUDA_CHECK(cudaEventRecord(c->ev[0], c->st));
       for (int s = 0; s < c->nspn; ++s) {
         if (c->nfrm[s] == 0) continue;
-        jobs.push_back(batch_prepare(c, s));
+        const int ns = spins_together(c) ? 2 : 1;
+        jobs.push_back(batch_prepare(c, s, ns));
         owner.push_back({m, s});
+        s += ns - 1;
       }
       CUDA_CHECK(cudaEventRecord(c->ev[3], c->st));
       if (m > 0) CUDA_CHECK(cudaStreamWaitEvent(c0->st, c->ev[3], 0));
@@ -2016,7 +2075,11 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       c->work_near += cnt[0];
       c->work_far += cnt[1];
       c->work_terms += cnt[2];
-      spin_xc(c, owner[j].second);
+      const int s0 = owner[j].second;
+      for (int s = s0; s < s0 + (spins_together(c) ? 2 : 1); ++s) {
+        c->spin[s].vh_valid = true;
+        spin_xc(c, s);
+      }
     }
     for (int m = 0; m < n; ++m) {
       flosic_ctx* c = ctxs[m];
@@ -2347,6 +2410,7 @@ int flosic_sic_cycle_partial(flosic_ctx* c, double* d_partial) {
     c->kernel_ms[0] = c->kernel_ms[1] = 0.0;
     for (auto& w : c->kernel_work) w = 0;
     invalidate(c);
+    if (spins_together(c)) cycle_coulomb(c);
     std::vector<double> h(partial_doubles(c), 0.0);
     size_t o = 0;
     for (int s = 0; s < c->nspn; ++s) {
