@@ -131,7 +131,7 @@ __device__ __forceinline__ void monomials(double x, double y, double z, double p
 // Real spherical harmonics of harmonics.f for a unit vector, degrees 0..lm
 // (lm <= 6), storage order of the reference (l^2 .. (l+1)^2-1 per degree),
 // including the normalisation prefactors.
-__device__ __forceinline__ void harmonics6(int lm, double x, double y, double z, double Y[NMOM]) {
+__host__ __device__ inline void harmonics6(int lm, double x, double y, double z, double Y[NMOM]) {
   Y[0] = 1.0;
   if (lm >= 1) {
     Y[1] = z;

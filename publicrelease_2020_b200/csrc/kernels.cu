@@ -5,23 +5,50 @@
 //                    factor of the pair density matrix of coupot_sic.F:366-482)
 //   k_pair_coef      Gaussian-pair Coulomb polynomial coefficients (polyx.F,
 //                    poisson1.f:259-501) and centre-of-gravity moments (ginted.F)
-//   k_call_setup     per POISSON1 call and FO: CG, RCUT, NPOT, sphere potential
-//                    and L<=6 multipole moments (poisson1.f:503-1230)
+//   k_call_geom, k_call_moments, k_call_setup_single  per POISSON1 call and FO:
+//                    CG, RCUT, NPOT, sphere potential and L<=6 multipole
+//                    moments (poisson1.f:503-1230)
 //   k_xc             XC potential of the FO density, SIC potential, energy
 //                    partial sums (getvlxc.F, subvlxc_libxc.F90, apotnl_sic.F)
 #include <cfloat>
+#include <cmath>
 #include <cstdio>
+#include <vector>
 
-#include "device_math.cuh"
+#include "coulomb_common.cuh"
 #include "kernels.cuh"
 #include "xc_functionals.cuh"
 #include "xc_scan.cuh"
 
 namespace flosic {
 
+// Per Lebedev point the harmonics times the weight, rows and columns padded with
+// zeros to the call set-up's k-steps and n-tiles, and the moments' normalisation
+// sqrt(NRUN (2l+1)/4pi (l-m)!/(l+m)!).
+constexpr int WY_K = 148, WY_N = 56;
+__device__ double g_leb_wy[WY_K * WY_N];
+__constant__ double c_mom_vf[NMOM];
+
 void upload_constants(const double* leb_ang, const double* leb_w) {
   cudaMemcpyToSymbol(c_leb_ang, leb_ang, sizeof(double) * NANG * 3);
   cudaMemcpyToSymbol(c_leb_w, leb_w, sizeof(double) * NANG);
+  std::vector<double> wy((size_t)WY_K * WY_N, 0.0);
+  double vf[NMOM];
+  for (int i = 0; i < NANG; ++i) {
+    double Y[NMOM];
+    harmonics6(LM, leb_ang[3 * i], leb_ang[3 * i + 1], leb_ang[3 * i + 2], Y);
+    for (int m = 0; m < NMOM; ++m) wy[(size_t)i * WY_N + m] = leb_w[i] * Y[m];
+  }
+  for (int j = 0; j < NMOM; ++j) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= j) ++l;
+    const int m = (j - l * l + 1) / 2;
+    double facfc = (2 * l + 1) * (1.0 / (16 * std::atan(1.0)));
+    for (int mm = 0; mm < m; ++mm) facfc = facfc / ((l - mm > 1 ? l - mm : 1) * (l + mm + 1));
+    vf[j] = std::sqrt((m == 0 ? 1 : 2) * facfc);
+  }
+  cudaMemcpyToSymbol(g_leb_wy, wy.data(), sizeof(double) * wy.size());
+  cudaMemcpyToSymbol(c_mom_vf, vf, sizeof(vf));
 }
 
 __constant__ int c_pow[10][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0},
@@ -434,11 +461,18 @@ __device__ __forceinline__ void box_dist2(const double lo[3], const double hi[3]
   }
 }
 
-constexpr int SETUP_THREADS = 160;
 constexpr int SETUP1_THREADS = 128;
 constexpr int GEO_LD = 48;  // per sphere point: 35 monomials, F_0..2 (s3), F_0..3 (s4), F_0..4 (s5)
 
-// RCUT of a call around its centre of gravity (poisson1.f:522-538).
+// RCUT of a call whose pair centres lie within dmax of its centre of gravity
+// (poisson1.f:522-538).
+__device__ double call_rcut(double delta_min, double dmax) {
+  double rcut = sqrt(30.0 / delta_min) + dmax;
+  const double pirc = 1.0 / (4 * atan(1.0));
+  const double fact = sqrt(pirc / (pirc + LM + 1));
+  const double dist = 2 * dmax / pow(1.0e-6 / fact, 1.0 / (LM + 1));
+  return fmax(rcut, dist);
+}
 __device__ double call_rcut(const CallInfo& ci, const PairGeo* __restrict__ pairs, const double cgr[3]) {
   double dmax = 0.0;
   for (int q = 0; q < ci.np; ++q) {
@@ -446,11 +480,7 @@ __device__ double call_rcut(const CallInfo& ci, const PairGeo* __restrict__ pair
     const double dist = sqrt(sqdist_rn(C[0], C[1], C[2], cgr));
     if (dist > dmax) dmax = dist;
   }
-  double rcut = sqrt(30.0 / ci.delta_min) + dmax;
-  const double pirc = 1.0 / (4 * atan(1.0));
-  const double fact = sqrt(pirc / (pirc + LM + 1));
-  const double dist = 2 * dmax / pow(1.0e-6 / fact, 1.0 / (LM + 1));
-  return fmax(rcut, dist);
+  return call_rcut(ci.delta_min, dmax);
 }
 
 // Far-point count of a call (all threads of the block), with early exit once
@@ -501,139 +531,208 @@ __device__ int call_far_count(const CallInfo& ci, const MeshDev& M, const double
   return npot;
 }
 
-__global__ void __launch_bounds__(SETUP_THREADS) k_call_setup(const int* __restrict__ list,
+// CG, RCUT and NPOT of every call of more than one slot and FO (poisson1.f:503-583),
+// one warp each.  The far count first adds the tiles that lie wholly outside the
+// sphere and stops once NPOT=2 is certain; only a call with few of them looks at
+// the points of the tiles its sphere cuts.
+__global__ void __launch_bounds__(256) k_call_geom(int nmulti, const int* __restrict__ list,
+                                                   const CallInfo* __restrict__ calls,
+                                                   const PairGeo* __restrict__ pairs, int nfo, int nspn,
+                                                   const double* __restrict__ cgp, MeshDev M,
+                                                   CallFO* __restrict__ out, double* __restrict__ momv) {
+  const size_t wi = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (wi >= (size_t)nmulti * nfo) return;
+  const int c = list[wi / nfo], k = (int)(wi % nfo);
+  const CallInfo ci = calls[c];
+  // lanes 0-3: the charge-weighted sums in pair order; lanes 4-6: the plain centre sums
+  double s = 0.0;
+  if (lane < 4) {
+    const double* p = cgp + ((size_t)ci.p0 * nfo + k) * 4 + lane;
+#pragma unroll 8
+    for (int q = 0; q < ci.np; ++q) s += p[(size_t)q * nfo * 4];
+  } else if (lane < 7) {
+#pragma unroll 8
+    for (int q = 0; q < ci.np; ++q) s = s - (-pairs[ci.p0 + q].C[lane - 4]);
+  }
+  const double chg = __shfl_sync(0xffffffffu, s, 3);
+  double cg[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double w = __shfl_sync(0xffffffffu, s, d), plain = __shfl_sync(0xffffffffu, s, 4 + d);
+    cg[d] = chg != 0.0 && ci.slots > 1 ? w / chg : (nspn * plain) / ci.slots;
+  }
+  double dmax = 0.0;
+  for (int q = lane; q < ci.np; q += 32) {
+    const double* C = pairs[ci.p0 + q].C;
+    dmax = fmax(dmax, sqrt(sqdist_rn(C[0], C[1], C[2], cg)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  const double rcut = call_rcut(ci.delta_min, dmax);
+  const double rcut2 = __dmul_rn(rcut, rcut);
+  const double slots = (double)ci.slots;
+  const double thr = 1.36 * slots * NANG / (1.36 * slots - 0.99) + 2.0;
+  int nfar = 0;
+  bool sure = false;
+  for (int pass = 0; pass < 2 && !sure; ++pass) {
+    for (int t0 = 0; t0 < M.ntiles && !sure; t0 += 32) {
+      const int t = t0 + lane;
+      int cls = 0, n = 0;
+      if (t < M.ntiles) {
+        const double lo[3] = {M.tile_lo[3 * t], M.tile_lo[3 * t + 1], M.tile_lo[3 * t + 2]};
+        const double hi[3] = {M.tile_hi[3 * t], M.tile_hi[3 * t + 1], M.tile_hi[3 * t + 2]};
+        cls = tile_class(lo, hi, cg[0], cg[1], cg[2], rcut2);
+        n = min(M.n - t * TILE, TILE);
+      }
+      if (pass == 0) {
+        nfar += __reduce_add_sync(0xffffffffu, cls == 1 ? n : 0);
+      } else {
+        for (unsigned cut = __ballot_sync(0xffffffffu, cls == 2); cut; cut &= cut - 1) {
+          const int tt = t0 + __ffs(cut) - 1, p1 = min(M.n, (tt + 1) * TILE);
+          for (int p = tt * TILE + lane; p < tt * TILE + TILE; p += 32)
+            nfar += __popc(__ballot_sync(0xffffffffu, p < p1 && sqdist_rn(M.x[min(p, p1 - 1)], M.y[min(p, p1 - 1)],
+                                                                          M.z[min(p, p1 - 1)], cg) > rcut2));
+        }
+      }
+      sure = (double)nfar > thr;
+    }
+  }
+  int npot = 2;
+  if (!sure) {
+    const double cls = (double)(M.n - nfar);
+    const double cost1 = 1.36 * (cls + NANG) * slots + 0.99 * (double)nfar;
+    const double cost2 = 1.36 * ((double)nfar + cls) * slots;
+    if (cost2 < cost1) npot = 1;
+  }
+  const size_t ck = (size_t)c * nfo + k;
+  if (lane == 0) {
+    CallFO f;
+    for (int d = 0; d < 3; ++d) f.cg[d] = cg[d];
+    f.rcut = rcut;
+    f.rcut2 = (npot == 1) ? DBL_MAX : rcut2;
+    f.npot = npot;
+    f.nfar = (npot == 1) ? 0 : nfar;
+    f.keep = 0ull;
+    f.lmax = 0;
+    f.pad = 0;
+    out[ck] = f;
+  }
+  if (npot == 1 || nfar == 0)
+    for (int m = lane; m < MOM_LD; m += 32) momv[ck * MOM_LD + m] = 0.0;
+}
+
+// Moments of eight FOs of one call: the exact potential on the Lebedev sphere of
+// radius RCUT around each FO's CG (poisson1.f:1100-1230), one (FO, point) per
+// thread, then projected on the weighted harmonics as an 8 x 49 x 146 product on
+// the FP64 tensor cores, scaled, and the skip rule applied.  Bounded by the FP64
+// pipe (~200 operations per (pair, FO, point)); the block-per-FO form before it
+// rebuilt the harmonics and their normalisation in every thread and summed the
+// moments serially: benzene (68,670 call-FO pairs) 5.7 -> 0.9 ms, the 40-atom
+// system 5.7 -> 2.8 ms, both kernels.
+constexpr int MOM_FOS = 8;
+constexpr int MOM_THREADS = 256;
+constexpr int MOM_VLD = WY_K;  // 148 = 4 mod 16 doubles: conflict-free A fragments
+
+__global__ void __launch_bounds__(MOM_THREADS) k_call_moments(const int* __restrict__ list,
                                                               const CallInfo* __restrict__ calls,
                                                               const PairGeo* __restrict__ pairs, int nfo,
-                                                              int nspn, const double* __restrict__ coef,
+                                                              const double* __restrict__ coef,
                                                               const int8_t* __restrict__ maxfmt,
-                                                              const double* __restrict__ cgp, MeshDev M,
                                                               const double* __restrict__ boys_tab,
-                                                              CallFO* __restrict__ out,
-                                                              double* __restrict__ momv) {
-  extern __shared__ double sm[];  // [NANG][NMOM] products, then NANG potentials
-  double* prod = sm;
-  double* vang = sm + NANG * NMOM;
-  __shared__ double s_cg[3], s_rcut;
-  __shared__ int s_far, s_stop;
-  const int c = list[blockIdx.x], k = blockIdx.y, tid = threadIdx.x;
+                                                              CallFO* __restrict__ out, double* __restrict__ momv) {
+  __shared__ double v[MOM_FOS * MOM_VLD];
+  __shared__ double mom[MOM_FOS][WY_N];
+  __shared__ double s_cg[MOM_FOS][3], s_rcut[MOM_FOS];
+  __shared__ int s_on[MOM_FOS];
+  const int c = list[blockIdx.x], k0 = blockIdx.y * MOM_FOS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nk = min(MOM_FOS, nfo - k0);
   const CallInfo ci = calls[c];
-  if (tid == 0) {
-    double cg[4] = {0, 0, 0, 0};
-    for (int q = 0; q < ci.np; ++q) {
-      const double* p = cgp + ((size_t)(ci.p0 + q) * nfo + k) * 4;
-      for (int i = 0; i < 4; ++i) cg[i] += p[i];
+  bool on = false;
+  if (tid < MOM_FOS) {
+    if (tid < nk) {
+      const CallFO& f = out[(size_t)c * nfo + k0 + tid];
+      on = f.npot == 2 && f.nfar > 0;
+      for (int d = 0; d < 3; ++d) s_cg[tid][d] = f.cg[d];
+      s_rcut[tid] = f.rcut;
     }
-    double cgr[3];
-    if (cg[3] != 0.0 && ci.slots > 1) {
-      for (int d = 0; d < 3; ++d) cgr[d] = cg[d] / cg[3];
-    } else {
-      for (int d = 0; d < 3; ++d) {
-        double s = 0.0;
-        for (int q = 0; q < ci.np; ++q) s = s - (-pairs[ci.p0 + q].C[d]);
-        cgr[d] = (nspn * s) / ci.slots;
+    s_on[tid] = on;
+  }
+  if (!__syncthreads_or(on)) return;
+  for (int e = tid; e < MOM_FOS * MOM_VLD; e += MOM_THREADS) {
+    const int f = e / MOM_VLD, i = e - f * MOM_VLD;
+    double pot = 0.0;
+    if (i < NANG && s_on[f]) {
+      const double rcut = s_rcut[f];
+      const double qx = s_cg[f][0] + c_leb_ang[3 * i] * rcut, qy = s_cg[f][1] + c_leb_ang[3 * i + 1] * rcut,
+                   qz = s_cg[f][2] + c_leb_ang[3 * i + 2] * rcut;
+      for (int qq = 0; qq < ci.np; ++qq) {
+        const PairGeo& g = pairs[ci.p0 + qq];
+        const double rx = qx - g.C[0], ry = qy - g.C[1], rz = qz - g.C[2];
+        const double xx = g.delta * (rz * rz + ry * ry + rx * rx);
+        const size_t pk = (size_t)(ci.p0 + qq) * nfo + k0 + f;
+        const int fmt = maxfmt[pk];
+        double F[5], mono[35];
+        boys_fmt<double>(boys_tab, xx, exp(-xx), fmt, F);
+        monomials(rx, ry, rz, mono);
+        pot += pair_potential(coef + pk * COEF_LD, mono, fmt, F, F, F);
       }
     }
-    const double rcut = call_rcut(ci, pairs, cgr);
-    for (int d = 0; d < 3; ++d) s_cg[d] = cgr[d];
-    s_rcut = rcut;
+    v[e] = pot;
   }
   __syncthreads();
-  const double cg[3] = {s_cg[0], s_cg[1], s_cg[2]};
-  const double rcut = s_rcut;
-  const double rcut2 = __dmul_rn(rcut, rcut);
-  int nfar = 0;
-  const int npot = call_far_count(ci, M, cg, rcut2, &s_far, &s_stop, nfar);
-  CallFO* o = out + (size_t)c * nfo + k;
-  if (tid == 0) {
-    o->cg[0] = cg[0];
-    o->cg[1] = cg[1];
-    o->cg[2] = cg[2];
-    o->rcut = rcut;
-    o->rcut2 = (npot == 1) ? DBL_MAX : rcut2;
-    o->npot = npot;
-    o->nfar = (npot == 1) ? 0 : nfar;
+  if (warp < WY_N / 8) {
+    double d0 = 0.0, d1 = 0.0;
+    const double* a = v + (lane >> 2) * MOM_VLD + (lane & 3);
+    const double* b = g_leb_wy + (lane & 3) * WY_N + warp * 8 + (lane >> 2);
+#pragma unroll 4
+    for (int kk = 0; kk < WY_K; kk += 4)
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                   : "+d"(d0), "+d"(d1)
+                   : "d"(a[kk]), "d"(__ldg(b + kk * WY_N)));
+    mom[lane >> 2][warp * 8 + 2 * (lane & 3)] = d0;
+    mom[lane >> 2][warp * 8 + 2 * (lane & 3) + 1] = d1;
   }
-  double* mv = momv + ((size_t)c * nfo + k) * MOM_LD;
-  if (npot == 1 || nfar == 0) {
-    if (tid < MOM_LD) mv[tid] = 0.0;
-    if (tid == 0) {
-      o->keep = 0ull;
-      o->lmax = 0;
+  __syncthreads();
+  // one warp per FO: radial factors, skip rule of poisson1.f:1252-1270 with
+  // RI1 = 1/RCUT, an upper bound of 1/r over every far point (keeps every term
+  // the reference keeps), normalisation with the skipped terms zeroed
+  const int f = warp;
+  if (f >= nk || !s_on[f]) return;
+  const double rcut = s_rcut[f], h = sqrt(rcut * rcut), ri1 = 1.0 / rcut;
+  double val[2];
+  unsigned long long keep = 0ull;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int m = lane + 32 * j;
+    bool kept = false;
+    val[j] = 0.0;
+    if (m < NMOM) {
+      int l = 0;
+      while ((l + 1) * (l + 1) <= m) ++l;
+      double rl = h, rt = ri1;
+      for (int i = 1; i <= l; ++i) {
+        rl = h * rl;
+        rt *= ri1;
+      }
+      const double x = mom[f][m] * rl;
+      kept = !(fabs((2 * l + 1) * x * rt) < 1.0e-12);
+      val[j] = kept ? x * c_mom_vf[m] : 0.0;
     }
-    return;
+    keep |= (unsigned long long)__ballot_sync(0xffffffffu, kept) << (32 * j);
   }
-  // exact potential on the Lebedev sphere of radius RCUT around CG
-  if (tid < NANG) {
-    const double q[3] = {cg[0] + c_leb_ang[3 * tid] * rcut, cg[1] + c_leb_ang[3 * tid + 1] * rcut,
-                         cg[2] + c_leb_ang[3 * tid + 2] * rcut};
-    double v = 0.0;
-    for (int qq = 0; qq < ci.np; ++qq) {
-      const PairGeo& g = pairs[ci.p0 + qq];
-      const double rx = q[0] - g.C[0], ry = q[1] - g.C[1], rz = q[2] - g.C[2];
-      const double xx = g.delta * (rz * rz + ry * ry + rx * rx);
-      const double chgd = exp(-xx);
-      double s3[3], s4[4], s5[5], mono[35];
-      boys_all(boys_tab, xx, chgd, s3, s4, s5);
-      monomials(rx, ry, rz, mono);
-      const size_t pk = (size_t)(ci.p0 + qq) * nfo + k;
-      v += pair_potential(coef + pk * COEF_LD, mono, maxfmt[pk], s3, s4, s5);
+  const size_t ck = (size_t)c * nfo + k0 + f;
+  double* mv = momv + ck * MOM_LD;
+  mv[lane] = val[0];
+  if (lane + 32 < MOM_LD) mv[lane + 32] = val[1];
+  if (lane == 0) {
+    int lmx = 0;
+    if (keep) {
+      const int top = 63 - __clzll((long long)keep);
+      while ((lmx + 1) * (lmx + 1) <= top) ++lmx;
     }
-    vang[tid] = v;
-    // harmonics at the normalised sphere point
-    const double hn = 1.0 / sqrt(rcut * rcut);
-    double Y[NMOM];
-    harmonics6(LM, hn * (c_leb_ang[3 * tid] * rcut), hn * (c_leb_ang[3 * tid + 1] * rcut),
-               hn * (c_leb_ang[3 * tid + 2] * rcut), Y);
-    for (int m = 0; m < NMOM; ++m) prod[tid * NMOM + m] = c_leb_w[tid] * Y[m] * v;
-  }
-  __syncthreads();
-  __shared__ double s_mom[NMOM];
-  __shared__ unsigned long long s_keep_bits;
-  if (tid < NMOM) {
-    double s = 0.0;
-    for (int i = 0; i < NANG; ++i) s += prod[i * NMOM + tid];
-    int l = 0;
-    while ((l + 1) * (l + 1) <= tid) ++l;
-    const double h = sqrt(rcut * rcut);
-    double rl = h;
-    for (int j = 1; j <= l; ++j) rl = h * rl;
-    s_mom[tid] = s * rl;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    // skip rule of poisson1.f:1252-1270 with RI1 = 1/RCUT, an upper bound of
-    // 1/r over every far point: keeps every term the reference keeps
-    const double ri1 = 1.0 / rcut;
-    unsigned long long keep = 0ull;
-    int lmx = 0, m = 0;
-    double rt = ri1;
-    for (int l = 0; l <= LM; ++l) {
-      for (int j = -l; j <= l; ++j, ++m)
-        if (!(fabs((2 * l + 1) * s_mom[m] * rt) < 1.0e-12)) {
-          keep |= (1ull << m);
-          lmx = l;
-        }
-      rt *= ri1;
-    }
-    o->keep = keep;
-    o->lmax = lmx;
-    s_keep_bits = keep;
-  }
-  __syncthreads();
-  // normalised moments with the skipped terms zeroed: M_lm * sqrt(NRUN (2l+1)/4pi (l-m)!/(l+m)!)
-  if (tid < NMOM) {
-    int l = 0;
-    while ((l + 1) * (l + 1) <= tid) ++l;
-    const int j = tid - l * l;
-    const int m = (j + 1) / 2;
-    const int nrun = (m == 0) ? 1 : 2;
-    double facfc = (2 * l + 1) * (1.0 / (16 * atan(1.0)));
-    for (int mm = 0; mm < m; ++mm) facfc = facfc / ((l - mm > 1 ? l - mm : 1) * (l + mm + 1));
-    const double vf = sqrt(nrun * facfc);
-    const bool kept = (s_keep_bits >> tid) & 1ull;
-    mv[tid] = kept ? s_mom[tid] * vf : 0.0;
-  } else if (tid < MOM_LD) {
-    mv[tid] = 0.0;
+    out[ck].keep = keep;
+    out[ck].lmax = lmx;
   }
 }
 
@@ -641,8 +740,8 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_call_setup(const int* __restr
 // block: CG is the pair centre (poisson1.f:515-520), so CG, RCUT, the far
 // count and NPOT are the same for every FO and are formed once; the sphere
 // points' Boys values, monomials and weighted harmonics are formed once and
-// each thread (FO) contracts them with its coefficients.  Every FO's numbers
-// are bitwise those of k_call_setup: the same expressions, in the same order.
+// each thread (FO) contracts them with its coefficients.  The expressions
+// are those of the kernels above.
 __global__ void __launch_bounds__(SETUP1_THREADS) k_call_setup_single(
     const int* __restrict__ list, const CallInfo* __restrict__ calls, const PairGeo* __restrict__ pairs, int nfo,
     int nspn, const double* __restrict__ coef, const int8_t* __restrict__ maxfmt, MeshDev M,
@@ -655,7 +754,7 @@ __global__ void __launch_bounds__(SETUP1_THREADS) k_call_setup_single(
   const int c = list[blockIdx.x], tid = threadIdx.x;
   const CallInfo ci = calls[c];
   if (tid < NMOM) {
-    // normalisation sqrt(NRUN (2l+1)/4pi (l-m)!/(l+m)!) of moment tid, as k_call_setup
+    // normalisation sqrt(NRUN (2l+1)/4pi (l-m)!/(l+m)!) of moment tid
     int l = 0;
     while ((l + 1) * (l + 1) <= tid) ++l;
     const int j = tid - l * l;
@@ -739,7 +838,7 @@ __global__ void __launch_bounds__(SETUP1_THREADS) k_call_setup_single(
 #pragma unroll
       for (int m = 0; m < NMOM; ++m) acc[m] = __dadd_rn(acc[m], __dmul_rn(wyi[m], v));
     }
-    // moments, skip rule and normalisation as k_call_setup
+    // moments, skip rule and normalisation as k_call_moments
     unsigned long long keep = 0ull;
     int lmx = 0;
     double rt = ri1;
@@ -770,8 +869,6 @@ __global__ void __launch_bounds__(SETUP1_THREADS) k_call_setup_single(
 }
 
 void init_call_setup() {
-  cudaFuncSetAttribute(k_call_setup, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(sizeof(double) * (NANG * NMOM + NANG)));
   cudaFuncSetAttribute(k_call_setup_single, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)(sizeof(double) * NANG * (GEO_LD + NMOM)));
 }
@@ -783,11 +880,13 @@ void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo*
   if (nsingle > 0)
     k_call_setup_single<<<nsingle, SETUP1_THREADS, sizeof(double) * NANG * (GEO_LD + NMOM), st>>>(
         list, calls, pairs, nfo, nspn, coef, maxfmt, M, boys_tab, cfo, momv);
-  if (ncalls > nsingle) {
-    const size_t smem = sizeof(double) * (NANG * NMOM + NANG);
-    dim3 grid(ncalls - nsingle, nfo);
-    k_call_setup<<<grid, SETUP_THREADS, smem, st>>>(list + nsingle, calls, pairs, nfo, nspn, coef, maxfmt, cgp, M,
-                                                     boys_tab, cfo, momv);
+  const int nmulti = ncalls - nsingle;
+  if (nmulti > 0) {
+    const size_t warps = (size_t)nmulti * nfo;
+    k_call_geom<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(nmulti, list + nsingle, calls, pairs, nfo, nspn, cgp, M,
+                                                              cfo, momv);
+    k_call_moments<<<dim3(nmulti, (nfo + MOM_FOS - 1) / MOM_FOS), MOM_THREADS, 0, st>>>(
+        list + nsingle, calls, pairs, nfo, coef, maxfmt, boys_tab, cfo, momv);
   }
 }
 

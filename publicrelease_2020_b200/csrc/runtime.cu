@@ -877,7 +877,13 @@ void coulomb(flosic_ctx* c, int s0, int ns = 1) {
 // of twice (benzene, 21 + 21 FOs: 35.2 -> 30.8 ms; with 37 + 37 there are two
 // blocks either way).
 bool spins_together(const flosic_ctx* c) {
-  return c->nspn == 2 && c->nfrm[0] > 0 && c->nfrm[1] > 0 && c->nfrm[0] + c->nfrm[1] <= 64;
+  const int n0 = c->nfrm[0], n1 = c->nfrm[1];
+  if (c->nspn != 2 || n0 == 0 || n1 == 0 || n0 + n1 > 64) return false;
+  // In the mixed path the route of a call decides its arithmetic (TF32 products
+  // where CG is bitwise the same for every FO, FP32 columns otherwise).  A few FOs
+  // of one spin share a rounded CG by chance, both spins' FOs less often; with 16
+  // or more FOs per spin only calls that share it exactly remain, in either set.
+  return c->precision == FLOSIC_PRECISION_FP64 || std::min(n0, n1) >= 16;
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
