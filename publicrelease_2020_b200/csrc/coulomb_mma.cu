@@ -609,8 +609,9 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                                const double* coef, const int8_t* maxfmt, const CallFO* cfo, const double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
-                               unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st) {
-  const bool per_fo_only = cfg.per_fo_only;
+                               unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st, bool one_density) {
+  // one density in FP64: every call by k_one_near and k_perfo_far
+  const bool per_fo_only = cfg.per_fo_only || one_density;
   launch_coulomb_classify(ncalls, calls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
   if (!per_fo_only && mixed && cfg.shared_tc) {
     const size_t nc = (size_t)npairs * nfo * COEF_LD, nm = (size_t)ncalls * nfo * MOM_LD;
@@ -653,6 +654,14 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
   J.M = M;
   J.vh = vh;
   J.cnt_perfo = cnt + 3;  // counted apart from the shared-geometry kernel
+  J.seg = scr.seg;
+  J.coef = coef;
+  if (one_density) {
+    J.nseg = one_density_parts(M.ntiles);
+    launch_one_density(J, boys_tab, st);
+    return cudaGetLastError();
+  }
+  J.nseg = perfo_parts(M.ntiles);
   launch_perfo(J, cfg.perfo_wm > 0 ? cfg.perfo_wm : perfo_default_wm(nfo), mixed, boys_tab, st);
   return cudaGetLastError();
 }

@@ -255,7 +255,7 @@ __device__ __forceinline__ T near_arg(T delta, T x, T y, T z) {
 }
 
 template <int MT, bool MIXED>
-__device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob,
+__device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob, int part,
                                            const double* __restrict__ tab) {
   using PT = typename std::conditional<MIXED, float, double>::type;
   constexpr int FOB = 8 * MT;
@@ -265,8 +265,10 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
   const int k0 = fob * FOB, nk = min(FOB, J.nfo - k0);
   const int cta0 = blk * NEAR_CTA_PTS;
   if (cta0 >= J.M.n) return;  // whole CTA
-  const int npl = J.lists[2 * J.ncalls + 2];
-  if (npl == 0) return;
+  const int npairs = J.lists[2 * J.ncalls + 2];
+  if (npairs == 0) return;
+  // this part's pairs; a call cut by the part's ends begins and ends there
+  const int pl0 = (int)((long long)npairs * part / J.nseg), npl = (int)((long long)npairs * (part + 1) / J.nseg);
   const int pb = cta0 + warp * NEAR_PTS;
   const int npt = min(NEAR_PTS, J.M.n - pb);  // <= 0: this warp only helps with the copies
   double* V = S.V[warp];
@@ -301,7 +303,7 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
   int row[MT];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) T[mt][0] = T[mt][1] = 0.0, row[mt] = 0;
-  int na = 0;
+  int na = 0, np = 0;  // of the open call: FO slots, pairs
   PT Fq[5] = {};  // Boys values of one pair of the current four
   const int cyc = max(q - 1, 0);  // the lane's coordinates: (x,y,z), (x,y,z), (y,z,x), (z,x,y)
   const double pa = pts[n][cyc], pb_ = pts[n][cyc == 2 ? 0 : cyc + 1], pc = pts[n][cyc == 0 ? 2 : cyc - 1];
@@ -326,7 +328,7 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
     cp_async_commit();
   };
 
-  for (int w0 = 0; w0 < npl; w0 += NEAR_WIN) {
+  for (int w0 = pl0; w0 < npl; w0 += NEAR_WIN) {
     // 1. the window's calls with near points of some FO in the CTA's box
     bool act = false, leads = false;
     int cls = 1;
@@ -335,6 +337,8 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
     const double clo[3] = {bx[0], bx[1], bx[2]}, chi[3] = {bx[3], bx[4], bx[5]};
     if (tid < NEAR_WIN && w0 + tid < npl) {
       my = J.plist[w0 + tid];
+      if (w0 + tid == pl0) my.first = 1;
+      if (w0 + tid == npl - 1) my.last = 1;
       cls = bound_class(clo, chi, J.bound[my.call]);
       act = cls != 1;
       leads = act && (tid == 0 || my.first);
@@ -441,6 +445,7 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
           const double* Ae = A + w.pre * 16;
           const bool isfull = (full >> i) & 1u;
           if (w.flags & 1) {
+            np = 0;
             na = nk;  // a call that is near for every FO lists them all
             if (!isfull) {  // the FOs with near points of this warp, compacted into slots
               const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
@@ -466,6 +471,7 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
               row[mt] = r * 16 + 2 * (q ^ ((r & 1) << 2));
             }
           }
+          ++np;
           if (na == 0) continue;
           const int nmt = (na + 7) >> 3;
           if ((e >> 2) != fquad) {
@@ -499,7 +505,6 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
           // the call's sum goes to V (call by call, so that no sum depends on how
           // FOs are blocked); a point counts for an FO when it is inside the FO's sphere
           const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
-          const int np = J.bound[w.call].np;
           if (isfull && lane == 0) near += (unsigned long long)(nk * npt) * np;
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
@@ -542,7 +547,9 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
     __syncwarp();
     for (int e = lane; e < nk * NEAR_PTS; e += 32) {
       const int k = e / NEAR_PTS, p = e - k * NEAR_PTS;
-      if (p < npt) J.vh[(size_t)(k0 + k) * J.ldv + pb + p] += V[e];
+      if (p >= npt) continue;
+      if (J.nseg > 1) J.seg[((size_t)part * J.nfo + k0 + k) * J.ldv + pb + p] = V[e];
+      else J.vh[(size_t)(k0 + k) * J.ldv + pb + p] += V[e];
     }
     count_add(J.cnt_perfo, near, 0, 0);
   }
@@ -555,10 +562,10 @@ constexpr int near_ctas() { return MT <= 8 ? 2 : 1; }
 template <int MT, bool MIXED>
 __global__ void __launch_bounds__(NEAR_THREADS, near_ctas<MT>())
 k_perfo_near(const __grid_constant__ CoulombJob J, const double* __restrict__ tab) {
-  near_block<MT, MIXED>(J, blockIdx.x, blockIdx.y, tab);
+  near_block<MT, MIXED>(J, blockIdx.x, blockIdx.y, blockIdx.z, tab);
 }
 
-// Many (molecule, spin) jobs: items[i] = {job, 128-point tile, FO block, 0}.
+// Many (molecule, spin) jobs: items[i] = {job, 128-point tile, FO block, 0}; blockIdx.y: part.
 template <int MT, bool MIXED>
 __global__ void __launch_bounds__(NEAR_THREADS, near_ctas<MT>())
 k_perfo_near_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__ items,
@@ -567,7 +574,8 @@ k_perfo_near_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__
   const int4 w = items[blockIdx.x / NEAR_PER_TILE];
   if (threadIdx.x == 0) J = jobs[w.x];
   __syncthreads();
-  near_block<MT, MIXED>(J, w.y * NEAR_PER_TILE + blockIdx.x % NEAR_PER_TILE, w.z, tab);
+  if ((int)blockIdx.y >= J.nseg) return;
+  near_block<MT, MIXED>(J, w.y * NEAR_PER_TILE + blockIdx.x % NEAR_PER_TILE, w.z, blockIdx.y, tab);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,33 +683,34 @@ __global__ void __launch_bounds__(64) k_perfo_pack_mom(int nfo, int mixed, int p
   }
 }
 
-constexpr int FAR_FOS = 4;             // FOs per CTA: a warp has one FO and 64 points, two per lane
-constexpr int FAR_THREADS = 2 * 32 * FAR_FOS;
+constexpr int FAR_FOS = 4;             // FOs per CTA (1 for one density): a warp has one FO and 64 points, two per lane
+constexpr int far_threads(int fos) { return 2 * 32 * fos; }
 constexpr int FAR_CALLS = 8;           // calls per buffer
 static_assert(sizeof(CallFO) == 64 && MOM_LD % 4 == 0, "copied in 16-byte pieces");
 static_assert(far_pos(6, 6) + 1 < MOM_LD, "moment positions");
 
-template <bool MIXED>
+template <int FOS, bool MIXED>
 struct FarSmem {
   using PT = typename std::conditional<MIXED, float, double>::type;
-  CallFO f[2][FAR_CALLS][FAR_FOS];
-  PT mv[2][FAR_CALLS][FAR_FOS][MOM_LD];
-  double box[FAR_THREADS / 32 + 1][6];
-  int queue[FAR_THREADS];
-  int wcount[FAR_THREADS / 32];
+  CallFO f[2][FAR_CALLS][FOS];
+  PT mv[2][FAR_CALLS][FOS][MOM_LD];
+  double box[far_threads(FOS) / 32 + 1][6];
+  int queue[far_threads(FOS)];
+  int wcount[far_threads(FOS) / 32];
 };
 
-template <bool MIXED>
-__device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp) {
+template <int FOS, bool MIXED>
+__device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp, int part) {
   using PT = typename std::conditional<MIXED, float, double>::type;
-  __shared__ __align__(16) FarSmem<MIXED> S;
-  constexpr int NW = FAR_THREADS / 32;
+  __shared__ __align__(16) FarSmem<FOS, MIXED> S;
+  constexpr int NT = far_threads(FOS), NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int k0 = grp * FAR_FOS, nk = min(FAR_FOS, J.nfo - k0);
+  const int k0 = grp * FOS, nk = min(FOS, J.nfo - k0);
   const int p0 = tile * TILE, npt = min(TILE, J.M.n - p0);
   const int* list = J.lists + J.ncalls;
-  const int nl = J.lists[2 * J.ncalls + 1];
-  if (nl == 0) return;
+  const int ncall = J.lists[2 * J.ncalls + 1];
+  if (ncall == 0) return;
+  const int first = (int)((long long)ncall * part / J.nseg), nl = (int)((long long)ncall * (part + 1) / J.nseg);
   const int k = warp >> 1;                       // this warp's FO
   const int pl = (warp & 1) * 64 + lane;         // and points pl, pl + 32
   double x[2], y[2], z[2], V[2] = {0.0, 0.0};
@@ -733,7 +742,7 @@ __device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp
   auto copy = [&](int e0, int e1, int b) {
     constexpr int MP = MOM_LD * sizeof(PT) / 16;  // 16-byte pieces of one FO's moments
     const int per = nk * (MP + 4);
-    for (int e = tid; e < (e1 - e0) * per; e += FAR_THREADS) {
+    for (int e = tid; e < (e1 - e0) * per; e += NT) {
       const int i = e / per, r = e - i * per;
       const size_t ck = (size_t)S.queue[e0 + i] * J.nfo + k0;
       if (r < nk * MP) {
@@ -747,7 +756,7 @@ __device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp
     }
     cp_async_commit();
   };
-  for (int l0 = 0; l0 < nl; l0 += FAR_THREADS) {
+  for (int l0 = first; l0 < nl; l0 += NT) {
     // the window's calls with far points in the tile, in order
     bool act = false;
     int c = 0;
@@ -844,26 +853,169 @@ __device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp
   }
 #pragma unroll
   for (int j = 0; j < 2; ++j)
-    if (k < nk && pl + 32 * j < npt) J.vh[(size_t)(k0 + k) * J.ldv + p0 + pl + 32 * j] += V[j];
+    if (k < nk && pl + 32 * j < npt) {
+      const int p = p0 + pl + 32 * j;
+      if (J.nseg > 1) J.seg[((size_t)(J.nseg + part) * J.nfo + k0 + k) * J.ldv + p] = V[j];
+      else J.vh[(size_t)(k0 + k) * J.ldv + p] += V[j];
+    }
   count_add(J.cnt_perfo, 0, far, terms);
 }
 
-template <bool MIXED>
-__global__ void __launch_bounds__(FAR_THREADS) k_perfo_far(const __grid_constant__ CoulombJob J) {
-  far_block<MIXED>(J, blockIdx.x, blockIdx.y);
+template <int FOS, bool MIXED>
+__global__ void __launch_bounds__(far_threads(FOS)) k_perfo_far(const __grid_constant__ CoulombJob J) {
+  far_block<FOS, MIXED>(J, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// items[i] = {job, tile, FO block of fob FOs, 0}; blockIdx.y: group of FAR_FOS FOs of the block.
+// items[i] = {job, tile, FO block of fob FOs, 0}; blockIdx.y: group of FAR_FOS FOs of the block,
+// blockIdx.z: part.
 template <bool MIXED>
-__global__ void __launch_bounds__(FAR_THREADS)
+__global__ void __launch_bounds__(far_threads(FAR_FOS))
 k_perfo_far_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__ items, int fob) {
   __shared__ CoulombJob J;
   const int4 w = items[blockIdx.x];
   if (threadIdx.x == 0) J = jobs[w.x];
   __syncthreads();
   const int grp = w.z * (fob / FAR_FOS) + blockIdx.y;
-  if (grp * FAR_FOS >= J.nfo) return;
-  far_block<MIXED>(J, w.y, grp);
+  if (grp * FAR_FOS >= J.nfo || (int)blockIdx.z >= J.nseg) return;
+  far_block<FAR_FOS, MIXED>(J, w.y, grp, blockIdx.z);
+}
+
+// vh += the parts' sums in order: near parts, then far parts.  FOs [k0, k0 + nk) of one tile.
+__device__ __forceinline__ void add_parts(const CoulombJob& J, int tile, int k0, int nk) {
+  const bool any = J.lists[2 * J.ncalls + 1] > 0;
+  if (J.nseg <= 1 || !any) return;
+  const int p = tile * TILE + (int)threadIdx.x;
+  if (threadIdx.x >= TILE || p >= J.M.n) return;
+  for (int k = k0; k < k0 + nk; ++k) {
+    double v = 0.0;
+    for (int s = 0; s < 2 * J.nseg; ++s) v += J.seg[((size_t)s * J.nfo + k) * J.ldv + p];
+    J.vh[(size_t)k * J.ldv + p] += v;
+  }
+}
+__global__ void __launch_bounds__(TILE) k_perfo_add(const __grid_constant__ CoulombJob J) {
+  add_parts(J, blockIdx.x, blockIdx.y, 1);
+}
+__global__ void __launch_bounds__(TILE) k_perfo_add_batch(const CoulombJob* __restrict__ jobs,
+                                                          const int4* __restrict__ items, int fob) {
+  const int4 w = items[blockIdx.x];
+  __shared__ CoulombJob J;
+  if (threadIdx.x == 0) J = jobs[w.x];
+  __syncthreads();
+  add_parts(J, w.y, w.z * fob, min(fob, J.nfo - w.z * fob));
+}
+
+// ---------------------------------------------------------------------------
+// One density
+// ---------------------------------------------------------------------------
+// Near field of one density (COUPOT1): with a single row the tensor cores would
+// multiply seven rows of padding, so each thread evaluates the pairs at its own
+// point from coefficient rows staged in shared memory, and the pair list is cut
+// into parts until the chip is full.  ~200 FP64 operations per (pair, point).
+// C60 (17,520 points, 53,460 pairs, 19,020 calls), whole evaluation: 84 ms with
+// the shared-geometry kernel (137 CTAs, each walking every pair), now near 3.8 and far 2.1 ms.
+constexpr int ONE_CHUNK = 16;  // pairs per buffer
+
+__global__ void __launch_bounds__(TILE) k_one_near(const __grid_constant__ CoulombJob J,
+                                                   const double* __restrict__ tab) {
+  __shared__ __align__(16) double A[2][ONE_CHUNK][COEF_LD];
+  __shared__ double geo[TILE][4], sph[TILE][4];
+  __shared__ PerfoPair queue[TILE];
+  __shared__ double box[TILE / 32 + 1][6];
+  __shared__ int wcount[TILE / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = blockIdx.y;
+  const int p0 = blockIdx.x * TILE, npt = min(TILE, J.M.n - p0);
+  const int npairs = J.lists[2 * J.ncalls + 2];
+  const int pl0 = (int)((long long)npairs * part / J.nseg), npl = (int)((long long)npairs * (part + 1) / J.nseg);
+  const int p = p0 + min(tid, npt - 1);
+  const double x = J.M.x[p], y = J.M.y[p], z = J.M.z[p];
+  {
+    double lo[3], hi[3];
+    warp_box(x, y, z, lo, hi);
+    if (lane == 0)
+      for (int d = 0; d < 3; ++d) {
+        box[warp][d] = lo[d];
+        box[warp][3 + d] = hi[d];
+      }
+  }
+  __syncthreads();
+  double clo[3], chi[3];
+  for (int d = 0; d < 3; ++d) {
+    clo[d] = box[0][d];
+    chi[d] = box[0][3 + d];
+    for (int w = 1; w < TILE / 32; ++w) {
+      clo[d] = fmin(clo[d], box[w][d]);
+      chi[d] = fmax(chi[d], box[w][3 + d]);
+    }
+  }
+  double V = 0.0;
+  unsigned long long near = 0;
+  for (int w0 = pl0; w0 < npl; w0 += TILE) {
+    bool act = false;
+    PerfoPair my{};
+    if (w0 + tid < npl) {
+      my = J.plist[w0 + tid];
+      act = bound_class(clo, chi, J.bound[my.call]) != 1;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, act);
+    if (lane == 0) wcount[warp] = __popc(bal);
+    __syncthreads();  // and every thread is done with the previous window
+    int before = 0, qn = 0;
+#pragma unroll
+    for (int w = 0; w < TILE / 32; ++w) {
+      const int cw = wcount[w];
+      before += w < warp ? cw : 0;
+      qn += cw;
+    }
+    if (act) {
+      const int e = before + __popc(bal & ((1u << lane) - 1u));
+      queue[e] = my;
+      const PairGeo& g = J.pairs[my.pair];
+      geo[e][0] = g.C[0];
+      geo[e][1] = g.C[1];
+      geo[e][2] = g.C[2];
+      geo[e][3] = g.delta;
+      const CallFO& f = J.cfo[my.call];
+      sph[e][0] = f.cg[0];
+      sph[e][1] = f.cg[1];
+      sph[e][2] = f.cg[2];
+      sph[e][3] = f.rcut2;
+    }
+    __syncthreads();
+    auto copy = [&](int e0, int b) {
+      const int ne = min(ONE_CHUNK, qn - e0);
+      for (int i = tid; i < ne * (COEF_LD / 2); i += TILE) {
+        const int e = i / (COEF_LD / 2), o = i - e * (COEF_LD / 2);
+        cp_async16(&A[b][e][2 * o], J.coef + (size_t)queue[e0 + e].pair * COEF_LD + 2 * o);
+      }
+      cp_async_commit();
+    };
+    if (qn > 0) copy(0, 0);
+    for (int e0 = 0, b = 0; e0 < qn; e0 += ONE_CHUNK, b ^= 1) {
+      cp_async_wait_all();
+      __syncthreads();  // this chunk has arrived and the other buffer is free
+      if (e0 + ONE_CHUNK < qn) copy(e0 + ONE_CHUNK, b ^ 1);
+      const int ne = min(ONE_CHUNK, qn - e0);
+      for (int i = 0; i < ne; ++i) {
+        const double* s = sph[e0 + i];
+        const bool nr = tid < npt && !(sqdist_rn2(x, y, z, s[0], s[1], s[2]) > s[3]);
+        if (!__any_sync(0xffffffffu, nr)) continue;
+        const double* g = geo[e0 + i];
+        const int fmt = queue[e0 + i].fmt;
+        const double rx = x - g[0], ry = y - g[1], rz = z - g[2];
+        const double arg = near_arg<double>(g[3], rx, ry, rz);
+        double F[5], mono[35];
+        near_boys<double>(tab, arg, exp(-arg), fmt, F);
+        monomials(rx, ry, rz, mono);
+        const double v = pair_potential(A[b][i], mono, fmt, F, F, F);
+        if (nr) {
+          V += v;
+          ++near;
+        }
+      }
+    }
+  }
+  if (tid < npt) J.seg[(size_t)part * J.ldv + p0 + tid] = V;
+  count_add(J.cnt_perfo, near, 0, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -903,38 +1055,50 @@ void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, 
 
 template <int MT>
 static void launch_near(const CoulombJob& J, bool mixed, const double* tab, cudaStream_t st) {
-  const dim3 grid(J.M.ntiles * NEAR_PER_TILE, (J.nfo + 8 * MT - 1) / (8 * MT));
+  const dim3 grid(J.M.ntiles * NEAR_PER_TILE, (J.nfo + 8 * MT - 1) / (8 * MT), J.nseg);
   if (mixed) k_perfo_near<MT, true><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(J, tab);
   else k_perfo_near<MT, false><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(J, tab);
 }
 
 void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* tab, cudaStream_t st) {
   if (J.M.ntiles <= 0 || J.nfo <= 0) return;
-  const dim3 grid(J.M.ntiles, (J.nfo + FAR_FOS - 1) / FAR_FOS);
-  if (mixed) k_perfo_far<true><<<grid, FAR_THREADS, 0, st>>>(J);
-  else k_perfo_far<false><<<grid, FAR_THREADS, 0, st>>>(J);
+  const dim3 grid(J.M.ntiles, (J.nfo + FAR_FOS - 1) / FAR_FOS, J.nseg);
+  if (mixed) k_perfo_far<FAR_FOS, true><<<grid, far_threads(FAR_FOS), 0, st>>>(J);
+  else k_perfo_far<FAR_FOS, false><<<grid, far_threads(FAR_FOS), 0, st>>>(J);
   if (wm == 4) launch_near<16>(J, mixed, tab, st);
   else if (wm == 2) launch_near<8>(J, mixed, tab, st);
   else launch_near<4>(J, mixed, tab, st);
+  if (J.nseg > 1) k_perfo_add<<<dim3(J.M.ntiles, J.nfo), TILE, 0, st>>>(J);
+}
+
+// Enough CTAs for eight per SM, at least a window of pairs each.
+int one_density_parts(int ntiles) { return std::max(2, std::min(32, 8 * 148 / std::max(ntiles, 1))); }
+
+void launch_one_density(const CoulombJob& J, const double* tab, cudaStream_t st) {
+  if (J.M.ntiles <= 0) return;
+  k_perfo_far<1, false><<<dim3(J.M.ntiles, 1, J.nseg), far_threads(1), 0, st>>>(J);
+  k_one_near<<<dim3(J.M.ntiles, J.nseg), TILE, 0, st>>>(J, tab);
+  k_perfo_add<<<dim3(J.M.ntiles, 1), TILE, 0, st>>>(J);
 }
 
 template <int MT>
-static void launch_near_batch(const CoulombJob* jobs, const int4* items, int nitems, bool mixed, const double* tab,
-                              cudaStream_t st) {
-  const int grid = nitems * NEAR_PER_TILE;
+static void launch_near_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, bool mixed,
+                              const double* tab, cudaStream_t st) {
+  const dim3 grid(nitems * NEAR_PER_TILE, parts);
   if (mixed) k_perfo_near_batch<MT, true><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(jobs, items, tab);
   else k_perfo_near_batch<MT, false><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(jobs, items, tab);
 }
 
-void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int wm, bool mixed,
+void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, int wm, bool mixed,
                         const double* tab, cudaStream_t st) {
   if (nitems <= 0) return;
-  const dim3 grid(nitems, 32 * wm / FAR_FOS);
-  if (mixed) k_perfo_far_batch<true><<<grid, FAR_THREADS, 0, st>>>(jobs, items, 32 * wm);
-  else k_perfo_far_batch<false><<<grid, FAR_THREADS, 0, st>>>(jobs, items, 32 * wm);
-  if (wm == 4) launch_near_batch<16>(jobs, items, nitems, mixed, tab, st);
-  else if (wm == 2) launch_near_batch<8>(jobs, items, nitems, mixed, tab, st);
-  else launch_near_batch<4>(jobs, items, nitems, mixed, tab, st);
+  const dim3 grid(nitems, 32 * wm / FAR_FOS, parts);
+  if (mixed) k_perfo_far_batch<true><<<grid, far_threads(FAR_FOS), 0, st>>>(jobs, items, 32 * wm);
+  else k_perfo_far_batch<false><<<grid, far_threads(FAR_FOS), 0, st>>>(jobs, items, 32 * wm);
+  if (wm == 4) launch_near_batch<16>(jobs, items, nitems, parts, mixed, tab, st);
+  else if (wm == 2) launch_near_batch<8>(jobs, items, nitems, parts, mixed, tab, st);
+  else launch_near_batch<4>(jobs, items, nitems, parts, mixed, tab, st);
+  if (parts > 1) k_perfo_add_batch<<<nitems, TILE, 0, st>>>(jobs, items, 32 * wm);
 }
 
 }  // namespace flosic

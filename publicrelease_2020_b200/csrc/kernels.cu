@@ -630,26 +630,28 @@ __global__ void __launch_bounds__(256) k_call_geom(int nmulti, const int* __rest
 // rebuilt the harmonics and their normalisation in every thread and summed the
 // moments serially: benzene (68,670 call-FO pairs) 5.7 -> 0.9 ms, the 40-atom
 // system 5.7 -> 2.8 ms, both kernels.
-constexpr int MOM_FOS = 8;
-constexpr int MOM_THREADS = 256;
+// Few (call, FO) pairs: two FOs per block of 320 threads (one point each, the other
+// six rows of the product empty), since a thread then walks the call's pairs once
+// instead of five times (water, 112 calls x 10 FOs: 0.29 -> 0.09 ms).
 constexpr int MOM_VLD = WY_K;  // 148 = 4 mod 16 doubles: conflict-free A fragments
 
-__global__ void __launch_bounds__(MOM_THREADS) k_call_moments(const int* __restrict__ list,
+template <int FOS, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_call_moments(const int* __restrict__ list,
                                                               const CallInfo* __restrict__ calls,
                                                               const PairGeo* __restrict__ pairs, int nfo,
                                                               const double* __restrict__ coef,
                                                               const int8_t* __restrict__ maxfmt,
                                                               const double* __restrict__ boys_tab,
                                                               CallFO* __restrict__ out, double* __restrict__ momv) {
-  __shared__ double v[MOM_FOS * MOM_VLD];
-  __shared__ double mom[MOM_FOS][WY_N];
-  __shared__ double s_cg[MOM_FOS][3], s_rcut[MOM_FOS];
-  __shared__ int s_on[MOM_FOS];
-  const int c = list[blockIdx.x], k0 = blockIdx.y * MOM_FOS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nk = min(MOM_FOS, nfo - k0);
+  __shared__ double v[8 * MOM_VLD];
+  __shared__ double mom[8][WY_N];
+  __shared__ double s_cg[FOS][3], s_rcut[FOS];
+  __shared__ int s_on[FOS];
+  const int c = list[blockIdx.x], k0 = blockIdx.y * FOS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nk = min(FOS, nfo - k0);
   const CallInfo ci = calls[c];
   bool on = false;
-  if (tid < MOM_FOS) {
+  if (tid < FOS) {
     if (tid < nk) {
       const CallFO& f = out[(size_t)c * nfo + k0 + tid];
       on = f.npot == 2 && f.nfar > 0;
@@ -659,10 +661,10 @@ __global__ void __launch_bounds__(MOM_THREADS) k_call_moments(const int* __restr
     s_on[tid] = on;
   }
   if (!__syncthreads_or(on)) return;
-  for (int e = tid; e < MOM_FOS * MOM_VLD; e += MOM_THREADS) {
+  for (int e = tid; e < 8 * MOM_VLD; e += THREADS) {
     const int f = e / MOM_VLD, i = e - f * MOM_VLD;
     double pot = 0.0;
-    if (i < NANG && s_on[f]) {
+    if (f < FOS && i < NANG && s_on[f]) {
       const double rcut = s_rcut[f];
       const double qx = s_cg[f][0] + c_leb_ang[3 * i] * rcut, qy = s_cg[f][1] + c_leb_ang[3 * i + 1] * rcut,
                    qz = s_cg[f][2] + c_leb_ang[3 * i + 2] * rcut;
@@ -885,8 +887,12 @@ void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo*
     const size_t warps = (size_t)nmulti * nfo;
     k_call_geom<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(nmulti, list + nsingle, calls, pairs, nfo, nspn, cgp, M,
                                                               cfo, momv);
-    k_call_moments<<<dim3(nmulti, (nfo + MOM_FOS - 1) / MOM_FOS), MOM_THREADS, 0, st>>>(
-        list + nsingle, calls, pairs, nfo, coef, maxfmt, boys_tab, cfo, momv);
+    if ((size_t)nmulti * ((nfo + 7) / 8) < 4 * 148)  // less than two waves of the eight-FO blocks
+      k_call_moments<2, 320><<<dim3(nmulti, (nfo + 1) / 2), 320, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
+                                                                          maxfmt, boys_tab, cfo, momv);
+    else
+      k_call_moments<8, 256><<<dim3(nmulti, (nfo + 7) / 8), 256, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
+                                                                          maxfmt, boys_tab, cfo, momv);
   }
 }
 

@@ -1,6 +1,8 @@
 // Kernel declarations and device-side data descriptors.
 #pragma once
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace flosic {
@@ -85,6 +87,7 @@ struct CoulombScratch {
   double* coefp;       // npairs*nfo*NEAR_K: the per-FO calls' coefficients in MMA order
   double* momp;        // ncalls*nfo*MOM_LD: their moments as the far kernel reads them
   CallBound* bound;    // ncalls
+  double* seg;         // perfo_seg_size doubles
 };
 // Kernel choices (all evaluate the same sums; the results differ only by the
 // rounding of the chosen arithmetic).  per_fo_only: every call through the
@@ -117,6 +120,8 @@ struct CoulombJob {
   const PerfoPair* plist;
   MeshDev M;
   double* vh;
+  int nseg, spare;                // the per-FO calls in nseg parts, each a CTA of its own
+  double* seg;                    // nseg > 1: [part][FO][ldv], near parts then far parts
   unsigned long long* cnt;        // work counts of the shared-geometry calls
   unsigned long long* cnt_perfo;  // and of the per-FO calls
 };
@@ -138,8 +143,22 @@ void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, 
                         const double* coef, const double* momv, double* coefp, double* momp, CallBound* bound,
                         cudaStream_t st);
 inline int perfo_default_wm(int nfo) { return nfo > 32 ? 2 : 1; }
+// Parts of the call list: a small mesh does not fill the chip with one CTA per
+// 64 points, so its calls are walked in up to 8 parts whose sums are added in
+// order (from the mesh alone, so that every launch form makes the same sums).
+// Measured: water (31 tiles) near 0.34 -> 0.14 ms in 4 parts, far 0.10 -> 0.05.
+inline int perfo_parts(int ntiles) { return ntiles <= 0 ? 1 : std::max(1, std::min(8, 148 / ntiles)); }
+inline size_t perfo_seg_size(int ntiles, int nfo, int ldv) {
+  const int n = perfo_parts(ntiles);
+  return n > 1 ? (size_t)2 * n * nfo * ldv : 1;
+}
 void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* boys_tab, cudaStream_t st);
-void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int wm, bool mixed,
+// The potential of one density (nfo = 1, FP64) added to vh: near field by one
+// point per thread, far field as above; seg holds one_density_parts * 2 * ldv doubles.
+int one_density_parts(int ntiles);
+void launch_one_density(const CoulombJob& J, const double* boys_tab, cudaStream_t st);
+// parts: the largest nseg of the jobs
+void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, int wm, bool mixed,
                         const double* boys_tab, cudaStream_t st);
 void init_coulomb_tc();
 // TF32 hi/lo split of nrow x nfo rows of KSEG doubles into the chunk-major
@@ -158,7 +177,7 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                                const double* coef, const int8_t* maxfmt, const CallFO* cfo, const double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
-                               unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st);
+                               unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st, bool one_density = false);
 
 // Exchange-correlation of the FO densities (fully polarised, NSPN forced to 2 as
 // in apotnl_sic.F:419) from the FO values/derivatives phi[(ch*nfo+k)*ldp+p];

@@ -249,7 +249,7 @@ struct TypeInfo {
 // Coulomb inputs of one spin for a batched launch over many molecules (the
 // per-molecule path keeps them in the context and reuses them per spin).
 struct CoulBufs {
-  DevBuf<double> coef, cgp, mom, coefp, momp;
+  DevBuf<double> coef, cgp, mom, coefp, momp, seg;
   DevBuf<CallBound> bound;
   DevBuf<PerfoPair> plist;
   DevBuf<int8_t> maxfmt, pairfmt;
@@ -263,6 +263,7 @@ struct CoulBufs {
     mom.release();
     coefp.release();
     momp.release();
+    seg.release();
     bound.release();
     plist.release();
     maxfmt.release();
@@ -360,7 +361,7 @@ struct flosic_ctx {
   DevBuf<double> d_basis, d_fodpts, d_psig, d_tmat, d_u, d_coef, d_cgp, d_mom, d_part, d_sums, d_sic, d_tmp;
   DevBuf<int8_t> d_maxfmt, d_pairfmt;
   DevBuf<CallShare> d_share;
-  DevBuf<double> d_coefp, d_momp;
+  DevBuf<double> d_coefp, d_momp, d_seg;
   DevBuf<CallBound> d_bound;
   DevBuf<PerfoPair> d_plist;
   DevBuf<int> d_lists, d_tc_err;
@@ -802,12 +803,15 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
   c->d_coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
   c->d_momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
   c->d_bound.ensure((size_t)std::max(ncalls, 1));
+  // one density (COUPOT1) in FP64 has kernels of its own
+  const bool one = dm != nullptr && !mixed && !c->coulomb_cfg.per_fo_only;
+  c->d_seg.ensure(one ? (size_t)2 * one_density_parts(c->eval_nt) * P : perfo_seg_size(c->eval_nt, nf, P));
   CoulombScratch scr{c->d_pairfmt.p, c->d_share.p,  c->d_lists.p, c->d_plist.p, c->d_coef_hl.p,
                      c->d_momv_hl.p, c->d_tc_err.p, c->d_coefp.p, c->d_momp.p,
-                     c->d_bound.p};
+                     c->d_bound.p,   c->d_seg.p};
   CUDA_CHECK(launch_coulomb_mma(ncalls, c->d_calls.p, c->d_pairs.p, npairs, nf, c->d_coef.p, c->d_maxfmt.p,
                                 c->d_callfo.p, c->d_mom.p, c->eval_mesh(), c->d_boys.p, vh, P, c->coulomb_cfg, mixed,
-                                scr, c->d_cnt.p, c->ev[8], st));
+                                scr, c->d_cnt.p, c->ev[8], st, one));
   CUDA_CHECK(cudaEventRecord(c->ev[9], st));
   c->launches += c->coulomb_cfg.per_fo_only ? 8 : 9;
   unsigned long long cnt[6];
@@ -1230,8 +1234,9 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   B.coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
   B.momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
   B.bound.ensure((size_t)std::max(ncalls, 1));
+  B.seg.ensure(perfo_seg_size(c->eval_nt, nf, P));
   CoulombScratch scr{B.pairfmt.p, B.share.p, B.lists.p, B.plist.p, nullptr, nullptr, nullptr, B.coefp.p, B.momp.p,
-                     B.bound.p};
+                     B.bound.p, B.seg.p};
   launch_coulomb_classify(ncalls, c->d_calls.p, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
   launch_perfo_setup(ncalls, npairs, nf, c->d_calls.p, c->d_pairs.p, B.callfo.p, B.share.p, false,
                      c->precision == FLOSIC_PRECISION_MIXED, B.coef.p, B.mom.p, B.coefp.p, B.momp.p, B.bound.p, st);
@@ -1254,6 +1259,8 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   J.bound = B.bound.p;
   J.plist = B.plist.p;
   J.M = c->eval_mesh();
+  J.nseg = perfo_parts(c->eval_nt);
+  J.seg = B.seg.p;
   J.vh = c->spin[s0].vh.p;
   J.cnt = B.cnt.p;
   J.cnt_perfo = B.cnt.p;
@@ -1365,7 +1372,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_basis.release(); c->d_fodpts.release(); c->d_psig.release(); c->d_tmat.release(); c->d_u.release();
   c->d_coef.release(); c->d_cgp.release(); c->d_mom.release(); c->d_part.release(); c->d_sums.release();
   c->d_sic.release(); c->d_tmp.release(); c->d_maxfmt.release(); c->d_callfo.release(); c->d_cnt.release(); c->d_pairfmt.release();
-  c->d_coefp.release(); c->d_momp.release(); c->d_bound.release(); c->d_plist.release();
+  c->d_coefp.release(); c->d_momp.release(); c->d_seg.release(); c->d_bound.release(); c->d_plist.release();
   c->d_share.release(); c->d_lists.release(); c->d_setup_list.release();
   c->d_eig_a.release(); c->d_eig_w.release(); c->d_eig_v.release(); c->d_eig_work.release(); c->d_eig_info.release();
   c->d_coef_hl.release(); c->d_momv_hl.release(); c->d_tc_err.release(); c->d_dens_coef.release();
@@ -2064,7 +2071,9 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       c0->d_batch_counters.ensure(1);
       launch_coulomb_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), c0->d_batch_counters.p, wm,
                            c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, nsm, c0->st);
-      launch_perfo_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), wm,
+      int parts = 1;
+      for (const CoulombJob& J : jobs) parts = std::max(parts, J.nseg);
+      launch_perfo_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), parts, wm,
                          c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, c0->st);
       CUDA_CHECK(cudaGetLastError());
       c0->launches += 3;
