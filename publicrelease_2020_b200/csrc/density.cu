@@ -10,10 +10,15 @@
 // the points outside RCUT receive nothing from the call's pairs, so this
 // density is the reference's truncated one rather than phi^2.
 //
-//   k_pair_dens_coef   RHOC (35) and the RHOD entries the channels use, per
-//                      (pair, FO), thresholded as the reference skips them
-//   k_pair_density     all calls of one FO over one mesh tile: near test per
-//                      point, pair polynomials, channel sums in call order
+//   k_pair_dens_coef   RHOC (35) per (pair, FO), thresholded as the reference
+//                      skips its entries.  Every RHOD entry is a power times one
+//                      RHOC entry (gtdncf.F), so the derivative channels are the
+//                      derivatives of the one polynomial.  (The reference drops
+//                      an RHOD entry by its own magnitude: it keeps f RHOC with
+//                      f = 2..12 where RHOC is between 1e-14 / f and 1e-14.)
+//   k_pair_density     all pairs of one FO over one mesh tile: near test per
+//                      point, the polynomial with its derivatives, channel sums
+//                      in call order
 #include <cstddef>
 
 #include "coulomb_common.cuh"
@@ -29,6 +34,14 @@ __constant__ int c_dens_pow[10][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}
 
 constexpr double DENS_EPS = 1.0e-14;  // poisson1.f:860,870,880
 constexpr int DENS_THREADS = TILE;    // one mesh point per thread
+
+// A coefficient row: 35 entries in the order pair_channels reads them (x power
+// descending, then y, then z), one of padding.
+constexpr int DENS_LD = 36;
+__device__ __forceinline__ int dens_pos(int px, int py, int pz) {
+  const int n = 4 - px, u = n - py, s = u - pz;
+  return n * (n + 1) * (n + 2) / 6 + u * (u + 1) / 2 + s;
+}
 
 __device__ __forceinline__ double dens_keep(double v) { return fabs(v) > DENS_EPS ? v : 0.0; }
 
@@ -48,8 +61,7 @@ __device__ __forceinline__ void mono_powers(int m, int& px, int& py, int& pz) {
 }
 
 __global__ void __launch_bounds__(128) k_pair_dens_coef(const PairGeo* __restrict__ pairs, int nfo, int nprim,
-                                                        const double* __restrict__ u, int nch,
-                                                        double* __restrict__ dc, int ldc) {
+                                                        const double* __restrict__ u, double* __restrict__ dc) {
   __shared__ double P1[10][10][3][5];
   const int ip = blockIdx.x, tid = threadIdx.x;
   const PairGeo g = pairs[ip];
@@ -101,147 +113,107 @@ __global__ void __launch_bounds__(128) k_pair_dens_coef(const PairGeo* __restric
       }
     }
     const double rc = s * ex;
-    double* row = dc + ((size_t)ip * nfo + k) * ldc;
-    row[m] = dens_keep(rc);
+    double* row = dc + ((size_t)ip * nfo + k) * DENS_LD;
+    row[dens_pos(px, py, pz)] = dens_keep(rc);
     if (m == 0) row[35] = 0.0;
-    if (nch == 1) continue;
-    // RHOD: every entry is one power times one RHOC entry (gtdncf.F), so the
-    // thread of monomial m writes the entries that m feeds
-    const int p[3] = {px, py, pz};
-    for (int d = 0; d < 3; ++d)
-      if (p[d] > 0) {
-        int r[3] = {px, py, pz};
-        r[d] -= 1;
-        row[36 + mono_index(r[0], r[1], r[2]) * 3 + d] = dens_keep((double)p[d] * rc);
-      }
-    if (nch < 10) continue;
-    const int dd[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
-    for (int kk = 0; kk < 6; ++kk) {
-      int r[3] = {px, py, pz};
-      double f = r[dd[kk][0]];
-      r[dd[kk][0]] -= 1;
-      if (f <= 0) continue;
-      f *= r[dd[kk][1]];
-      r[dd[kk][1]] -= 1;
-      if (f <= 0) continue;
-      row[96 + mono_index(r[0], r[1], r[2]) * 6 + kk] = dens_keep(f * rc);
-    }
   }
 }
 
-// Monomials POLY(r - C) of poisson1.f:820-847 (formed by the same products)
-// and the pair Gaussian exp(-delta |r - C|^2) at one point.
-__device__ __forceinline__ double pair_poly(double x, double y, double z, const PairGeo& g, double (&p)[35]) {
-  p[0] = 1.0;
-  p[3] = x - g.C[0];
-  p[2] = y - g.C[1];
-  p[1] = z - g.C[2];
-  p[4] = p[1] * p[1];
-  p[6] = p[2] * p[2];
-  p[9] = p[3] * p[3];
-  p[5] = p[2] * p[1];
-  p[7] = p[3] * p[1];
-  p[8] = p[3] * p[2];
-  p[10] = p[1] * p[4];
-  p[11] = p[2] * p[4];
-  p[12] = p[1] * p[6];
-  p[13] = p[2] * p[6];
-  p[14] = p[3] * p[4];
-  p[15] = p[3] * p[5];
-  p[16] = p[3] * p[6];
-  p[17] = p[1] * p[9];
-  p[18] = p[2] * p[9];
-  p[19] = p[3] * p[9];
-  p[20] = p[4] * p[4];
-  p[21] = p[4] * p[5];
-  p[22] = p[6] * p[4];
-  p[23] = p[6] * p[5];
-  p[24] = p[6] * p[6];
-  p[25] = p[4] * p[7];
-  p[26] = p[8] * p[4];
-  p[27] = p[8] * p[5];
-  p[28] = p[6] * p[8];
-  p[29] = p[9] * p[4];
-  p[30] = p[9] * p[5];
-  p[31] = p[9] * p[6];
-  p[32] = p[7] * p[9];
-  p[33] = p[8] * p[9];
-  p[34] = p[9] * p[9];
-  return exp(-(g.delta * (p[4] + p[6] + p[9])));
-}
+// Value, first derivative and half the second derivative of a polynomial by
+// Horner's scheme, coefficients highest first; t counts them from 0 (a compile-
+// time constant after unrolling), ND the derivatives kept.
+template <int ND>
+struct Horner {
+  double v, d1, d2;
+  __device__ __forceinline__ void add(int t, double x, double c) {
+    if (ND >= 2 && t >= 2) d2 = t == 2 ? d1 : fma(d2, x, d1);
+    if (ND >= 1 && t >= 1) d1 = t == 1 ? v : fma(d1, x, v);
+    v = t == 0 ? c : fma(v, x, c);
+  }
+};
 
-// Channel values of one pair and one FO at one point before the Gaussian
-// factor (poisson1.f:849-940): the RHOC and RHOD sums in the reference's
-// order, then the product-rule terms of the Gaussian's derivatives.  row: the
-// pair's coefficient row, staged in shared memory.
+// Channels of one pair and one FO at offset (x, y, z) before the Gaussian
+// factor: the polynomial RHOC and its derivatives by nested Horner schemes (z
+// inside y inside x, 90 multiply-adds for all ten channels against 155 with the
+// monomials and RHOD tables), then the product-rule terms of the Gaussian's
+// derivatives (poisson1.f:849-940).  row: 36 coefficients in shared memory, read
+// in order.
 template <int NCH>
-__device__ __forceinline__ void pair_channels(const double (&p)[35], double delta, const double* row,
-                                              double (&a)[NCH]) {
+__device__ __forceinline__ void pair_channels(double x, double y, double z, double delta,
+                                              const double* __restrict__ row, double (&a)[NCH]) {
+  constexpr int ND = NCH == 1 ? 0 : (NCH == 4 ? 1 : 2);
   const double2* r2 = reinterpret_cast<const double2*>(row);
+  Horner<ND> X;                                  // the polynomial in x
+  Horner<(ND > 1 ? 1 : 0)> XY, XZ;               // its y and z derivatives
+  Horner<0> XYY, XZZ, XYZ;
+  double2 two = r2[0];
+  int at = 0;
 #pragma unroll
-  for (int c = 0; c < NCH; ++c) a[c] = 0.0;
+  for (int n = 0; n <= 4; ++n) {                 // x power 4 - n
+    Horner<ND> Y;
+    Horner<(ND > 1 ? 1 : 0)> YZ;
+    Horner<0> YZZ;
 #pragma unroll
-  for (int j = 0; j < 18; ++j) {
-    const double2 v = r2[j];
-    a[0] = fma(p[2 * j], v.x, a[0]);
-    if (2 * j + 1 < 35) a[0] = fma(p[2 * j + 1], v.y, a[0]);
-  }
-  if constexpr (NCH > 1) {
-    // gradient channels: 20 monomials x 3, row[36 + q*3 + d]
+    for (int u = 0; u <= n; ++u) {               // y power n - u
+      Horner<ND> Z;
 #pragma unroll
-    for (int j = 0; j < 30; ++j) {
-      const double2 v = r2[18 + j];
-      const int e0 = 2 * j, e1 = 2 * j + 1;
-      a[1 + e0 % 3] = fma(p[e0 / 3], v.x, a[1 + e0 % 3]);
-      a[1 + e1 % 3] = fma(p[e1 / 3], v.y, a[1 + e1 % 3]);
+      for (int s = 0; s <= u; ++s, ++at) {       // z power u - s
+        if (at > 0 && (at & 1) == 0) two = r2[at >> 1];
+        Z.add(s, z, (at & 1) ? two.y : two.x);
+      }
+      Y.add(u, y, Z.v);
+      if (ND >= 1 && u >= 1) YZ.add(u - 1, y, Z.d1);
+      if (ND >= 2 && u >= 2) YZZ.add(u - 2, y, Z.d2);
+    }
+    X.add(n, x, Y.v);
+    if (ND >= 1 && n >= 1) {
+      XY.add(n - 1, x, Y.d1);
+      XZ.add(n - 1, x, YZ.v);
+    }
+    if (ND >= 2 && n >= 2) {
+      XYY.add(n - 2, x, Y.d2);
+      XYZ.add(n - 2, x, YZ.d1);
+      XZZ.add(n - 2, x, YZZ.v);
     }
   }
-  if constexpr (NCH == 10) {
-    // second-derivative channels: 10 monomials x 6, row[96 + q*6 + kk]
-#pragma unroll
-    for (int j = 0; j < 30; ++j) {
-      const double2 v = r2[48 + j];
-      const int e0 = 2 * j, e1 = 2 * j + 1;
-      a[4 + e0 % 6] = fma(p[e0 / 6], v.x, a[4 + e0 % 6]);
-      a[4 + e1 % 6] = fma(p[e1 / 6], v.y, a[4 + e1 % 6]);
-    }
-    const double d1x4 = delta * 4.0, d2x4 = delta * delta * 4.0, d1x2 = delta * 2.0;
-    a[4] = a[4] - d1x4 * p[3] * a[1] + (d2x4 * p[9] - d1x2) * a[0];
-    a[5] = a[5] - d1x4 * p[2] * a[2] + (d2x4 * p[6] - d1x2) * a[0];
-    a[6] = a[6] - d1x4 * p[1] * a[3] + (d2x4 * p[4] - d1x2) * a[0];
-    a[7] = a[7] - d1x2 * p[2] * a[1] - d1x2 * p[3] * a[2] + d2x4 * p[8] * a[0];
-    a[8] = a[8] - d1x2 * p[1] * a[1] - d1x2 * p[3] * a[3] + d2x4 * p[7] * a[0];
-    a[9] = a[9] - d1x2 * p[2] * a[3] - d1x2 * p[1] * a[2] + d2x4 * p[5] * a[0];
-  }
+  a[0] = X.v;
   if constexpr (NCH > 1) {
-    const double d1x2 = delta * 2.0;
-    a[1] = a[1] - d1x2 * p[3] * a[0];
-    a[2] = a[2] - d1x2 * p[2] * a[0];
-    a[3] = a[3] - d1x2 * p[1] * a[0];
+    const double d1x2 = delta * 2.0, px = X.d1, py = XY.v, pz = XZ.v;
+    if constexpr (NCH == 10) {
+      const double d1x4 = delta * 4.0, d2x4 = delta * delta * 4.0;
+      a[4] = 2.0 * X.d2 - d1x4 * x * px + (d2x4 * (x * x) - d1x2) * a[0];
+      a[5] = 2.0 * XYY.v - d1x4 * y * py + (d2x4 * (y * y) - d1x2) * a[0];
+      a[6] = 2.0 * XZZ.v - d1x4 * z * pz + (d2x4 * (z * z) - d1x2) * a[0];
+      a[7] = XY.d1 - d1x2 * y * px - d1x2 * x * py + d2x4 * (x * y) * a[0];
+      a[8] = XZ.d1 - d1x2 * z * px - d1x2 * x * pz + d2x4 * (x * z) * a[0];
+      a[9] = XYZ.v - d1x2 * y * pz - d1x2 * z * py + d2x4 * (y * z) * a[0];
+    }
+    a[1] = px - d1x2 * x * a[0];
+    a[2] = py - d1x2 * y * a[0];
+    a[3] = pz - d1x2 * z * a[0];
   }
 }
 
-// Block = (mesh tile, FO k).  The calls whose sphere reaches the tile are
-// gathered in call order, 128 at a time, with their sphere and pair range in
-// shared memory; their pairs then stream through a DENS_NBUF-deep ring of
-// shared-memory stages (coefficient row and pair centre/exponent, copied with
-// cp.async DENS_NBUF-1 pairs ahead), and each is added at the tile's points
-// inside the call's sphere, in pair order, so each point sums its
-// contributions in the reference's order.
-constexpr int DENS_NBUF = 4;
-template <int NCH, int LDC>
-__global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int ncalls, const CallInfo* __restrict__ calls,
+// Block = (mesh tile, FO k), one point per thread.  The pairs are taken 128 at a
+// time: those whose call's sphere reaches the tile are queued in order with
+// their sphere and centre, their coefficient rows stream through two shared
+// buffers of DENS_CHUNK rows (cp.async one chunk ahead, one barrier per chunk),
+// and each is added at the points inside its sphere, so every point sums its
+// contributions in the reference's order.  Bounded by the FP64 pipe (~180
+// operations per (pair, point, FO) with ten channels).  Measured, 20 atoms, 64
+// FOs, 50,021 points, PBE: 90 -> 51 ms (before: one barrier per pair and rows of
+// 156 entries, 78 16-byte shared-memory loads each).
+constexpr int DENS_CHUNK = 16;
+template <int NCH>
+__global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int npairs,
                                                                const PairGeo* __restrict__ pairs,
                                                                const CallFO* __restrict__ cfo, int cfo_ld, int nfo,
                                                                const double* __restrict__ dc,
                                                                double* __restrict__ rhog, size_t ldr) {
-  static_assert(LDC % 2 == 0 && LDC / 2 <= DENS_THREADS, "one 16-byte chunk of a row per thread");
-  static_assert(sizeof(PairGeo) % 16 == 0 && offsetof(PairGeo, C) == 64 && offsetof(PairGeo, delta) == 88,
-                "pair centre and exponent are the 32 bytes at offset 64");
-  __shared__ __align__(16) double s_row[DENS_NBUF][LDC];
-  __shared__ __align__(16) double s_geo[DENS_NBUF][4];  // C[3], delta
-  __shared__ double s_cg[DENS_THREADS][4];              // CG, RCUT^2 of the listed calls
-  __shared__ int s_p0[DENS_THREADS], s_np[DENS_THREADS];
+  __shared__ __align__(16) double s_row[2][DENS_CHUNK][DENS_LD];
+  __shared__ double s_geo[DENS_THREADS][4];  // queue: C[3], delta
+  __shared__ double s_cg[DENS_THREADS][4];   // queue: CG, RCUT^2
+  __shared__ int s_pair[DENS_THREADS];
   __shared__ int s_cnt[DENS_THREADS / 32];
   const int tile = blockIdx.x, k = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double lo[3], hi[3];
@@ -256,87 +228,64 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int nc
   double acc[NCH];
 #pragma unroll
   for (int c = 0; c < NCH; ++c) acc[c] = 0.0;
-  for (int c0 = 0; c0 < ncalls; c0 += DENS_THREADS) {
-    const int c = c0 + tid;
+  for (int q0 = 0; q0 < npairs; q0 += DENS_THREADS) {
+    const int q = q0 + tid;
     bool hit = false;
-    CallFO cf;
-    if (c < ncalls) {
-      cf = cfo[(size_t)c * cfo_ld + k];
-      hit = cf.npot == 1 || tile_class(lo, hi, cf.cg[0], cf.cg[1], cf.cg[2], cf.rcut2) != 1;
+    int c = 0;
+    if (q < npairs) {
+      c = pairs[q].call;
+      const CallFO& f = cfo[(size_t)c * cfo_ld + k];
+      hit = f.npot == 1 || tile_class(lo, hi, f.cg[0], f.cg[1], f.cg[2], f.rcut2) != 1;
     }
     const unsigned b = __ballot_sync(0xffffffffu, hit);
     if (lane == 0) s_cnt[warp] = __popc(b);
-    __syncthreads();
-    int before = 0, total = 0;
+    __syncthreads();  // and every thread is done with the previous window
+    int before = 0, qn = 0;
 #pragma unroll
     for (int w = 0; w < DENS_THREADS / 32; ++w) {
       before += (w < warp) ? s_cnt[w] : 0;
-      total += s_cnt[w];
+      qn += s_cnt[w];
     }
     if (hit) {
       const int i = before + __popc(b & ((1u << lane) - 1u));
-      const CallInfo ci = calls[c];
-      s_cg[i][0] = cf.cg[0];
-      s_cg[i][1] = cf.cg[1];
-      s_cg[i][2] = cf.cg[2];
-      s_cg[i][3] = cf.rcut2;
-      s_p0[i] = ci.p0;
-      s_np[i] = ci.np;
+      const CallFO& f = cfo[(size_t)c * cfo_ld + k];
+      const PairGeo& g = pairs[q];
+      s_pair[i] = q;
+      for (int d = 0; d < 3; ++d) {
+        s_cg[i][d] = f.cg[d];
+        s_geo[i][d] = g.C[d];
+      }
+      s_cg[i][3] = f.rcut2;
+      s_geo[i][3] = g.delta;
     }
     __syncthreads();
-    // the copy side walks (call, pair) DENS_NBUF-1 stages ahead of the compute side
-    int fi = 0, fq = 0;
-    while (fi < total && s_np[fi] == 0) ++fi;
-    auto issue = [&](int buf) {
-      if (fi < total) {
-        const int q = s_p0[fi] + fq;
-        const double* src = dc + ((size_t)q * nfo + k) * LDC;
-        if (tid < LDC / 2) cp_async16(&s_row[buf][2 * tid], src + 2 * tid);
-        if (tid >= DENS_THREADS - 2) {
-          const int h = tid - (DENS_THREADS - 2);
-          cp_async16(&s_geo[buf][2 * h], reinterpret_cast<const char*>(pairs + q) + 64 + 16 * h);
-        }
-        if (++fq == s_np[fi]) {
-          fq = 0;
-          ++fi;
-          while (fi < total && s_np[fi] == 0) ++fi;
-        }
+    auto copy = [&](int e0, int buf) {
+      const int ne = min(DENS_CHUNK, qn - e0);
+      for (int i = tid; i < ne * (DENS_LD / 2); i += DENS_THREADS) {
+        const int e = i / (DENS_LD / 2), o = i - e * (DENS_LD / 2);
+        cp_async16(&s_row[buf][e][2 * o], dc + ((size_t)s_pair[e0 + e] * nfo + k) * DENS_LD + 2 * o);
       }
       cp_async_commit();
     };
-#pragma unroll
-    for (int j = 0; j < DENS_NBUF - 1; ++j) issue(j);
-    int ci = 0, cq = 0;
-    while (ci < total && s_np[ci] == 0) ++ci;
-    bool near = false;
-    for (int st = 0; ci < total; ++st) {
-      asm volatile("cp.async.wait_group %0;\n" ::"n"(DENS_NBUF - 2) : "memory");
-      __syncthreads();  // stage st has landed for every thread; stage st-1's buffer is free
-      issue((st + DENS_NBUF - 1) % DENS_NBUF);
-      if (cq == 0)
-        near = valid && !(sqdist_rn2(x, y, z, s_cg[ci][0], s_cg[ci][1], s_cg[ci][2]) > s_cg[ci][3]);
-      if (near) {
-        const int buf = st % DENS_NBUF;
-        PairGeo g;
-        g.C[0] = s_geo[buf][0];
-        g.C[1] = s_geo[buf][1];
-        g.C[2] = s_geo[buf][2];
-        g.delta = s_geo[buf][3];
-        double p[35];
-        const double chgd = pair_poly(x, y, z, g, p);
+    if (qn > 0) copy(0, 0);
+    for (int e0 = 0, buf = 0; e0 < qn; e0 += DENS_CHUNK, buf ^= 1) {
+      cp_async_wait_all();
+      __syncthreads();  // this chunk has arrived and the other buffer is free
+      if (e0 + DENS_CHUNK < qn) copy(e0 + DENS_CHUNK, buf ^ 1);
+      const int ne = min(DENS_CHUNK, qn - e0);
+      for (int i = 0; i < ne; ++i) {
+        const double* cg = s_cg[e0 + i];
+        const bool near = valid && !(sqdist_rn2(x, y, z, cg[0], cg[1], cg[2]) > cg[3]);
+        if (!near) continue;
+        const double* g = s_geo[e0 + i];
+        const double rx = x - g[0], ry = y - g[1], rz = z - g[2], delta = g[3];
+        const double chgd = exp(-(delta * (rz * rz + ry * ry + rx * rx)));
         double a[NCH];
-        pair_channels<NCH>(p, g.delta, s_row[buf], a);
+        pair_channels<NCH>(rx, ry, rz, delta, s_row[buf][i], a);
 #pragma unroll
         for (int ch = 0; ch < NCH; ++ch) acc[ch] += chgd * a[ch];
       }
-      if (++cq == s_np[ci]) {
-        cq = 0;
-        ++ci;
-        while (ci < total && s_np[ci] == 0) ++ci;
-      }
     }
-    cp_async_wait_all();
-    __syncthreads();  // the lists and stage buffers are rewritten by the next batch of calls
   }
   if (valid) {
 #pragma unroll
@@ -346,21 +295,17 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int nc
 
 }  // namespace
 
-int pair_density_ld(int nch) { return nch == 1 ? 36 : (nch == 4 ? 96 : 156); }
+int pair_density_ld() { return DENS_LD; }
 
-void launch_pair_density(int npairs, const PairGeo* pairs, int ncalls, const CallInfo* calls, const CallFO* cfo,
-                         int cfo_ld, int nfo, int nprim, const double* u, int nch, const MeshDev& M, double* dc, double* rhog,
-                         size_t ldr, cudaStream_t st) {
+void launch_pair_density(int npairs, const PairGeo* pairs, const CallFO* cfo, int cfo_ld, int nfo, int nprim,
+                         const double* u, int nch, const MeshDev& M, double* dc, double* rhog, size_t ldr,
+                         cudaStream_t st) {
   if (nfo <= 0 || M.ntiles <= 0) return;
-  const int ldc = pair_density_ld(nch);
-  if (npairs > 0) k_pair_dens_coef<<<npairs, 128, 0, st>>>(pairs, nfo, nprim, u, nch, dc, ldc);
-  dim3 grid(M.ntiles, nfo);
-  if (nch == 1)
-    k_pair_density<1, 36><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
-  else if (nch == 4)
-    k_pair_density<4, 96><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
-  else
-    k_pair_density<10, 156><<<grid, DENS_THREADS, 0, st>>>(M, ncalls, calls, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
+  if (npairs > 0) k_pair_dens_coef<<<npairs, 128, 0, st>>>(pairs, nfo, nprim, u, dc);
+  const dim3 grid(M.ntiles, nfo);
+  if (nch == 1) k_pair_density<1><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
+  else if (nch == 4) k_pair_density<4><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
+  else k_pair_density<10><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
 }
 
 }  // namespace flosic
