@@ -44,24 +44,29 @@ __device__ __forceinline__ void cp_wait() {
 // ---------------------------------------------------------------------------
 // General product
 // ---------------------------------------------------------------------------
-constexpr int GM = 64, GN = 64, GK = 16;     // CTA tile
-constexpr int GLD_M = GM + 4, GLD_N = GN + 4;  // shared pitches (4 mod 16 doubles)
-constexpr int G_THREADS = 256;                // 8 warps: 2 along M (32 rows) x 4 along N (16 columns)
+constexpr int GM = 64, GK = 16;               // CTA tile GM x GN x GK
+constexpr int GLD_M = GM + 4;                 // shared pitches (4 mod 16 doubles)
+constexpr int G_THREADS = 256;                // 8 warps
+// Tile width by the columns: up to 32 (the FOs of a small molecule) half of a
+// 64-wide tile would be padding (324 x 21 x 37,843: 108 -> 66 us).  64: warps 2 along
+// M (32 rows) x 4 along N; 32: 4 along M (16 rows) x 2 along N; 16 columns a warp.
+inline int dgemm_gn(int N) { return N <= 32 ? 32 : 64; }
 
-template <bool TA, bool TB>
+template <bool TA, bool TB, int GN>
 __global__ void __launch_bounds__(G_THREADS) k_dgemm(int M, int N, int K, int kchunk, const double* __restrict__ A,
                                                      int lda, const double* __restrict__ B, int ldb,
                                                      double* __restrict__ out, int ldo, size_t split_stride,
                                                      double alpha, double beta, int direct) {
+  constexpr int GLD_N = GN + 4, WARPS_N = GN / 16, WARPS_M = 8 / WARPS_N, WMT = GM / WARPS_M / 8;
   __shared__ __align__(16) double As[2][GK][GLD_M];
   __shared__ __align__(16) double Bs[2][GK][GLD_N];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp & 1, wn = warp >> 1;
+  const int wm = warp % WARPS_M, wn = warp / WARPS_M;
   const int m0 = blockIdx.x * GM, n0 = blockIdx.y * GN;
   const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-  double acc[4][2][2];
+  double acc[WMT][2][2];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < WMT; ++a)
 #pragma unroll
     for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 
@@ -114,13 +119,13 @@ __global__ void __launch_bounds__(G_THREADS) k_dgemm(int M, int N, int K, int kc
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < GK; kk += 4) {
-      double af[4], bf[2];
+      double af[WMT], bf[2];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) af[mt] = As[buf][kk + (lane & 3)][wm * 32 + mt * 8 + (lane >> 2)];
+      for (int mt = 0; mt < WMT; ++mt) af[mt] = As[buf][kk + (lane & 3)][(wm * WMT + mt) * 8 + (lane >> 2)];
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) bf[nt] = Bs[buf][kk + (lane & 3)][wn * 16 + nt * 8 + (lane >> 2)];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < WMT; ++mt)
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) dmma(acc[mt][nt][0], acc[mt][nt][1], af[mt], bf[nt]);
     }
@@ -128,12 +133,12 @@ __global__ void __launch_bounds__(G_THREADS) k_dgemm(int M, int N, int K, int kc
   }
   double* o = direct ? out : out + blockIdx.z * split_stride;
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < WMT; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int m = m0 + wm * 32 + mt * 8 + (lane >> 2);
+        const int m = m0 + (wm * WMT + mt) * 8 + (lane >> 2);
         const int n = n0 + wn * 16 + nt * 8 + 2 * (lane & 3) + i;
         if (m >= M || n >= N) continue;
         double* c = o + (size_t)n * ldo + m;
@@ -142,21 +147,39 @@ __global__ void __launch_bounds__(G_THREADS) k_dgemm(int M, int N, int K, int kc
       }
 }
 
-// C = alpha sum_z W_z + beta C, the partial products summed in split order.
-__global__ void k_dgemm_reduce(int M, int N, int nsplit, const double* __restrict__ ws, double alpha, double beta,
-                               double* __restrict__ C, int ldc) {
+// C = alpha sum_z W_z + beta C.  Each of eight lanes of threads adds every eighth
+// partial product in order, the eight sums are added in order (one thread per
+// element and up to 300 dependent loads took 131 us for a 21 x 21 SIC matrix, this
+// 12 us).
+constexpr int RED_E = 32, RED_Z = 8;
+__global__ void __launch_bounds__(RED_E * RED_Z) k_dgemm_reduce(int M, int N, int nsplit,
+                                                                const double* __restrict__ ws, double alpha,
+                                                                double beta, double* __restrict__ C, int ldc) {
+  __shared__ double part[RED_Z][RED_E];
   const size_t MN = (size_t)M * N;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < MN; e += (size_t)gridDim.x * blockDim.x) {
+  const int j = threadIdx.x % RED_E, z0 = threadIdx.x / RED_E;
+  for (size_t e0 = blockIdx.x * (size_t)RED_E; e0 < MN; e0 += (size_t)gridDim.x * RED_E) {
+    const size_t e = e0 + j;
     double s = 0.0;
-    for (int z = 0; z < nsplit; ++z) s += ws[(size_t)z * MN + e];
-    const int n = (int)(e / M), m = (int)(e - (size_t)n * M);
-    double* c = C + (size_t)n * ldc + m;
-    *c = (beta == 0.0) ? alpha * s : alpha * s + beta * *c;
+    if (e < MN) {
+#pragma unroll 4
+      for (int z = z0; z < nsplit; z += RED_Z) s += ws[(size_t)z * MN + e];
+    }
+    part[z0][j] = s;
+    __syncthreads();
+    if (z0 == 0 && e < MN) {
+#pragma unroll
+      for (int z = 1; z < RED_Z; ++z) s += part[z][j];
+      const int n = (int)(e / M), m = (int)(e - (size_t)n * M);
+      double* c = C + (size_t)n * ldc + m;
+      *c = (beta == 0.0) ? alpha * s : alpha * s + beta * *c;
+    }
+    __syncthreads();
   }
 }
 
 int dgemm_splits(int M, int N, int K) {
-  const int tiles = ((M + GM - 1) / GM) * ((N + GN - 1) / GN);
+  const int gn = dgemm_gn(N), tiles = ((M + GM - 1) / GM) * ((N + gn - 1) / gn);
   const int want = (2 * 148 + tiles - 1) / tiles;  // about two CTAs per SM
   const int maxs = (K + 4 * GK - 1) / (4 * GK);    // at least four k-steps per split
   return std::max(1, std::min(want, maxs));
@@ -174,19 +197,24 @@ void dgemm(bool ta, bool tb, int M, int N, int K, double alpha, const double* A,
   const int kchunk = (s > 1) ? ((K + s - 1) / s + GK - 1) / GK * GK : std::max(K, 1);
   const int ns = (s > 1) ? (K + kchunk - 1) / kchunk : 1;
   const bool direct = ns == 1;
-  dim3 grid((M + GM - 1) / GM, (N + GN - 1) / GN, ns);
+  const int gn = dgemm_gn(N);
+  dim3 grid((M + GM - 1) / GM, (N + gn - 1) / gn, ns);
   double* out = direct ? C : work;
   const int ldo = direct ? ldc : M;
   const size_t ss = (size_t)M * N;
-#define DG(a, b) k_dgemm<a, b><<<grid, G_THREADS, 0, st>>>(M, N, K, kchunk, A, lda, B, ldb, out, ldo, ss, alpha, beta, direct)
+#define DG(a, b)                                                                                              \
+  (gn == 32 ? k_dgemm<a, b, 32><<<grid, G_THREADS, 0, st>>>(M, N, K, kchunk, A, lda, B, ldb, out, ldo, ss, alpha, \
+                                                            beta, direct)                                     \
+            : k_dgemm<a, b, 64><<<grid, G_THREADS, 0, st>>>(M, N, K, kchunk, A, lda, B, ldb, out, ldo, ss, alpha, \
+                                                            beta, direct))
   if (!ta && !tb) DG(false, false);
   else if (ta && !tb) DG(true, false);
   else if (!ta && tb) DG(false, true);
   else DG(true, true);
 #undef DG
   if (!direct) {
-    const int nblk = (int)std::min<size_t>(1024, (ss + 255) / 256);
-    k_dgemm_reduce<<<nblk, 256, 0, st>>>(M, N, ns, work, alpha, beta, C, ldc);
+    const int nblk = (int)std::min<size_t>(4096, (ss + RED_E - 1) / RED_E);
+    k_dgemm_reduce<<<nblk, RED_E * RED_Z, 0, st>>>(M, N, ns, work, alpha, beta, C, ldc);
   }
 }
 

@@ -466,7 +466,8 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
             }
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
-              const int s = max(min(mt * 8 + n, na - 1), 0);
+              if (mt * 8 >= na) break;
+              const int s = min(mt * 8 + n, na - 1);
               const int r = isfull ? s : (int)(S.slot[warp][s] & 127);
               row[mt] = r * 16 + 2 * (q ^ ((r & 1) << 2));
             }

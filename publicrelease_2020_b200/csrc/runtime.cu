@@ -316,6 +316,7 @@ struct flosic_ctx {
   int device = 0;
   cudaStream_t st = nullptr;
   DevBuf<double> d_gemm_ws;  // split-K partial products of dgemm
+  DevBuf<double> d_wk[3];    // results of the basis-space sums and the DFT side, kept between calls
   DevBuf<CoulombJob> d_jobs;  // batched Coulomb launch led by this context
   DevBuf<int4> d_items;
   DevBuf<int> d_batch_counters;
@@ -1173,7 +1174,7 @@ void adjoint_device(flosic_ctx* c, int s, DevBuf<double>& dg) {
   const int nderv = c->mgga ? 1 : 0;
   const size_t budget = (size_t)3 << 30;
   int chunk = (int)std::min<size_t>(P, std::max<size_t>(TILE, budget / (sizeof(double) * nyc * nb)));
-  chunk = std::max(TILE, chunk / TILE * TILE);
+  if (chunk < P) chunk = std::max(TILE, chunk / TILE * TILE);
   c->d_basis.ensure((size_t)nyc * nb * chunk);
   dg.ensure((size_t)nb * nf);
   const double alpha = -4.0 / c->nspn;
@@ -1268,7 +1269,7 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
 }
 
 void fod_gradient(flosic_ctx* c, int s, double* grad) {
-  DevBuf<double> dg, dm;
+  DevBuf<double>&dg = c->d_wk[0], &dm = c->d_wk[1];
   adjoint_device(c, s, dg);
   SpinCache& S = c->spin[s];
   const int n = S.nf, nw = S.nw, nb = c->nbasis;
@@ -1377,6 +1378,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_eig_a.release(); c->d_eig_w.release(); c->d_eig_v.release(); c->d_eig_work.release(); c->d_eig_info.release();
   c->d_coef_hl.release(); c->d_momv_hl.release(); c->d_tc_err.release(); c->d_dens_coef.release();
   c->d_gemm_ws.release();
+  for (auto& w : c->d_wk) w.release();
   c->d_jobs.release();
   c->d_items.release();
   c->d_batch_counters.release();
@@ -2170,13 +2172,12 @@ int flosic_sic_adjoint(flosic_ctx* c, int lspn, double* g, int ldg) {
     if (!g) fail(FLOSIC_ERR_ARG, "null array argument");
     if (ldg < c->nbasis) fail(FLOSIC_ERR_ARG, "ldg smaller than the number of basis functions");
     const int s = lspn - 1;
-    DevBuf<double> dg;
+    DevBuf<double>& dg = c->d_wk[0];
     adjoint_device(c, s, dg);
     const int nf = c->spin[s].nf, nb = c->nbasis;
     std::vector<double> h((size_t)nb * nf);
     CUDA_CHECK(cudaMemcpyAsync(h.data(), dg.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->st));
     CUDA_CHECK(cudaStreamSynchronize(c->st));
-    dg.release();
     for (int k = 0; k < nf; ++k)
       for (int mu = 0; mu < nb; ++mu) g[(size_t)k * ldg + mu] = h[(size_t)k * nb + mu];
   });
@@ -2209,7 +2210,7 @@ int flosic_sic_siclag_der(flosic_ctx* c, double* dersic, int ldo) {
     const int nderv = c->mgga ? 2 : 1, nbch = c->mgga ? 10 : 4;
     const size_t budget = (size_t)3 << 30;
     int chunk = (int)std::min<size_t>(P, std::max<size_t>(TILE, budget / (sizeof(double) * nbch * nb)));
-    chunk = std::max(TILE, chunk / TILE * TILE);
+    if (chunk < P) chunk = std::max(TILE, chunk / TILE * TILE);
     for (int s = 0; s < c->nspn; ++s) {
       const int nf = c->nfrm[s];
       if (nf == 0) continue;
@@ -2217,7 +2218,7 @@ int flosic_sic_siclag_der(flosic_ctx* c, double* dersic, int ldo) {
       SpinCache& S = c->spin[s];
       c->d_basis.ensure((size_t)nbch * nb * chunk);
       // H_ix = B_{1+ix}^T Y_0 (+ sum_c B_{h(ix,c)}^T Y_{1+c}), nb x nf each
-      DevBuf<double> dh;
+      DevBuf<double>& dh = c->d_wk[0];
       dh.ensure((size_t)3 * nb * nf);
       bool first = true;
       for (int p0 = 0; p0 < P; p0 += chunk) {
@@ -2240,7 +2241,6 @@ int flosic_sic_siclag_der(flosic_ctx* c, double* dersic, int ldo) {
       CUDA_CHECK(cudaMemcpyAsync(h.data(), dh.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->st));
       CUDA_CHECK(cudaMemcpyAsync(cf.data(), S.cfo.p, sizeof(double) * cf.size(), cudaMemcpyDeviceToHost, c->st));
       CUDA_CHECK(cudaStreamSynchronize(c->st));
-      dh.release();
       // DERSIC(ix, lfn, A) = sum_{mu on A} C_mu,k H_ix[mu, k]
       const double fac = c->nspn == 1 ? 2.0 : 1.0;
       for (int a = 0; a < c->natoms; ++a) {
@@ -2278,12 +2278,12 @@ int flosic_sic_sicham(flosic_ctx* c, int lspn, double* ham, int ldh, int packed)
     const int nderv = c->mgga ? 1 : 0;
     const size_t budget = (size_t)3 << 30;
     int chunk = (int)std::min<size_t>(P, std::max<size_t>(TILE, budget / (sizeof(double) * nyc * nb)));
-    chunk = std::max(TILE, chunk / TILE * TILE);
+    if (chunk < P) chunk = std::max(TILE, chunk / TILE * TILE);
     c->d_basis.ensure((size_t)nyc * nb * chunk);
     c->d_tmp.ensure((size_t)nf * P);
     launch_scale_rows(P, nf, S.phi.p, P, c->d_w.p + c->eval_p0, c->d_tmp.p, P, c->st);
     c->launches++;
-    DevBuf<double> dab, dh;
+    DevBuf<double>&dab = c->d_wk[0], &dh = c->d_wk[1];
     dab.ensure((size_t)2 * nb * nf);
     dh.ensure((size_t)nb * nb);
     double* da = dab.p;
@@ -2307,8 +2307,6 @@ int flosic_sic_sicham(flosic_ctx* c, int lspn, double* ham, int ldh, int packed)
     std::vector<double> h((size_t)nb * nb);
     CUDA_CHECK(cudaMemcpyAsync(h.data(), dh.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->st));
     CUDA_CHECK(cudaStreamSynchronize(c->st));
-    dab.release();
-    dh.release();
     if (packed) {
       // HSTOR order of a C1 calculation: IBAS = 1..N outer, JBAS = IBAS..N inner
       size_t indx = 0;
@@ -2332,8 +2330,8 @@ int flosic_sic_densold(flosic_ctx* c, int ngrad, double* rhog, double* phig) {
     const int nderv = ngrad == 10 ? 2 : 0;
     const size_t budget = (size_t)3 << 30;
     int chunk = (int)std::min<size_t>(P, std::max<size_t>(TILE, budget / (sizeof(double) * ngrad * (nb + nwf))));
-    chunk = std::max(TILE, chunk / TILE * TILE);
-    DevBuf<double> dv, dr, dph;
+    if (chunk < P) chunk = std::max(TILE, chunk / TILE * TILE);
+    DevBuf<double>&dv = c->d_wk[0], &dr = c->d_wk[1], &dph = c->d_wk[2];
     dv.ensure((size_t)ngrad * std::max(nwf, 1) * chunk);
     dr.ensure((size_t)ns * ngrad * P);
     if (phig) dph.ensure((size_t)ns * P);
@@ -2370,7 +2368,7 @@ int flosic_sic_coupot1(flosic_ctx* c, double* coulomb) {
     const int npairs = (int)c->pairs.size();
     c->d_u.ensure((size_t)std::max(nwf, 1) * c->nprim * 10);
     if (nwf > 0) launch_prim_u(c->basis_dev(), nwf, c->d_psi.p, c->nbasis, c->d_u.p, c->st);
-    DevBuf<double> ddm, dvh;
+    DevBuf<double>&ddm = c->d_wk[0], &dvh = c->d_wk[1];
     ddm.ensure((size_t)std::max(npairs, 1) * 100);
     dvh.ensure((size_t)P);
     launch_pair_dm(npairs, c->d_pairs.p, nwf, c->nprim, c->d_u.p, ddm.p, c->st);
