@@ -11,8 +11,8 @@
 //                 fragments of mma.sync m8n8k4 .f64 (lane 4 n + q holds row q of
 //                 each k-step at point n; one column per (pair, point), the Boys
 //                 values of four pairs at once over the four lanes of a point),
-//                 and multiplies the coefficient rows of its own near FOs into
-//                 FP64 accumulators, added call by call, masked point by
+//                 and multiplies the listed FOs' coefficient rows into FP64
+//                 accumulators, added call by call, masked point by
 //                 point where a sphere cuts the warp's box.
 //   k_perfo_far   One warp owns 64 points (two per lane) and one FO and adds
 //                 the L <= 6 multipole expansions of the far calls as Clenshaw
@@ -144,18 +144,21 @@ constexpr int NEAR_THREADS = 32 * NEAR_WARPS;
 constexpr int NEAR_CTA_PTS = NEAR_WARPS * NEAR_PTS;
 constexpr int NEAR_PER_TILE = TILE / NEAR_CTA_PTS;
 constexpr int NEAR_WIN = 128;                  // pairs classified at once
-constexpr int near_rows_cap(int mt) { return mt <= 4 ? 192 : (mt <= 8 ? 224 : 384); }
+constexpr int near_rows_cap(int mt) { return mt <= 4 ? 192 : (mt <= 8 ? 224 : 448); }
 
 struct __align__(16) NearEntry {
   int pre;                                     // coefficient rows of the entries before it
   int call, pair;
-  uint8_t lead, nl, fmt, flags;                // index into lead, listed FOs, Boys variant, 1 first + 2 last of its call
+  uint8_t lead, nl, fmt, flags;                // index into lead, listed FOs, Boys variant, NEAR_FIRST ...
 };
+constexpr int NEAR_FIRST = 1, NEAR_LAST = 2;   // of its call
+constexpr int NEAR_CUT = 4;                    // last of a call some sphere of which cuts the CTA's box: after its
+                                               // coefficient rows come the listed FOs' CallFO records, two per row
 
 template <int MT>
 struct NearSmem {
   static constexpr int ROWS = near_rows_cap(MT);  // coefficient rows (16 doubles) per buffer
-  static_assert(ROWS >= 3 * 8 * MT, "a pair's rows of all FOs fit");
+  static_assert(ROWS >= 3 * 8 * MT + 4 * MT, "a pair's rows of all FOs and their spheres fit");
   double A[2][ROWS * 16];
   double V[NEAR_WARPS][8 * MT * NEAR_PTS];     // the warps' potentials, [FO][point]
   double p[NEAR_CTA_PTS][3];
@@ -166,7 +169,6 @@ struct NearSmem {
   int cnt[NEAR_WIN];                           // FOs of the block with near points in the CTA's box
   int wcount[NEAR_WIN / 32][2];
   uint8_t list[NEAR_WIN][8 * MT];              // those FOs, ascending
-  uint8_t slot[NEAR_WARPS][8 * MT];            // a warp's slots: position in list, + 128 when all points are near
 };
 
 // The column values of one (pair, point) for lane residue q: four k-steps of
@@ -228,18 +230,18 @@ __device__ __forceinline__ void near_boys(const double* __restrict__ tab, T x, T
 }
 
 // Four k-steps of one group: two 16-byte fragment loads and four MMAs per eight
-// FO slots.  row[mt]: double offset of the
-// slot's coefficient row, with the lane's piece.
+// listed FOs.  A0, A1: the lane's two pieces of the first rows.
 template <int MT, typename T, int g>
-__device__ __forceinline__ void near_mma(double (&acc)[MT][2], const double* __restrict__ A, const int (&row)[MT],
-                                         int nmt, const NearLane<T>& L, const T (&F)[5], bool q0) {
+__device__ __forceinline__ void near_mma(double (&acc)[MT][2], const double* __restrict__ A0,
+                                         const double* __restrict__ A1, int nmt, const NearLane<T>& L,
+                                         const T (&F)[5], bool q0) {
   double b[4];
   near_group<T, g>(L, F, q0, b);
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) {
     if (mt >= nmt) break;
-    const double2 a0 = *reinterpret_cast<const double2*>(A + row[mt]);
-    const double2 a1 = *reinterpret_cast<const double2*>(A + (row[mt] ^ 8));
+    const double2 a0 = *reinterpret_cast<const double2*>(A0 + mt * 128);
+    const double2 a1 = *reinterpret_cast<const double2*>(A1 + mt * 128);
     dmma(acc[mt], a0.x, b[0]);
     dmma(acc[mt], a0.y, b[1]);
     dmma(acc[mt], a1.x, b[2]);
@@ -300,10 +302,10 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
   const double(*pts)[3] = &S.p[warp * NEAR_PTS];
   const double* box = S.box[warp];
   double T[MT][2];
-  int row[MT];
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) T[mt][0] = T[mt][1] = 0.0, row[mt] = 0;
-  int na = 0, np = 0;  // of the open call: FO slots, pairs
+  for (int mt = 0; mt < MT; ++mt) T[mt][0] = T[mt][1] = 0.0;
+  int np = 0;  // pairs of the open call
+  const int piece = n * 16 + 2 * (q ^ ((n & 1) << 2));  // of the lane's coefficient rows
   PT Fq[5] = {};  // Boys values of one pair of the current four
   const int cyc = max(q - 1, 0);  // the lane's coordinates: (x,y,z), (x,y,z), (y,z,x), (z,x,y)
   const double pa = pts[n][cyc], pb_ = pts[n][cyc == 2 ? 0 : cyc + 1], pc = pts[n][cyc == 0 ? 2 : cyc - 1];
@@ -323,6 +325,11 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
           const int r = i >> 3, pc = i & 7;
           cp_async16(dst + r * 16 + 2 * (pc ^ ((r & 1) << 2)), src + (int)list[r] * 16 + 2 * pc);
         }
+      }
+      if (w.flags & NEAR_CUT) {
+        const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
+        for (int i = lane; i < nl * 4; i += 32)
+          cp_async16(dst + 2 * i, reinterpret_cast<const double*>(cf + list[i >> 2]) + 2 * (i & 3));
       }
     }
     cp_async_commit();
@@ -380,7 +387,8 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
     // 3. the queue: the pairs of the calls that keep an FO
     act = act && S.cnt[mycall] > 0;
     bal = __ballot_sync(0xffffffffu, act);
-    int rows = act ? S.cnt[mycall] * (my.fmt - 2) : 0;
+    const bool cut = act && my.last && !(S.lead[mycall] >> 30);
+    int rows = act ? S.cnt[mycall] * (my.fmt - 2) + (cut ? (S.cnt[mycall] + 1) / 2 : 0) : 0;
     const int mine = rows;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -405,7 +413,8 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
     if (act) {
       const int e = before + __popc(bal & ((1u << lane) - 1u));
       S.queue[e] = NearEntry{rbefore + rows - mine, my.call, my.pair, (uint8_t)mycall, (uint8_t)S.cnt[mycall],
-                             (uint8_t)my.fmt, (uint8_t)(my.first + 2 * my.last)};
+                             (uint8_t)my.fmt,
+                             (uint8_t)(my.first * NEAR_FIRST + my.last * NEAR_LAST + (cut ? NEAR_CUT : 0))};
       const PairGeo& g = J.pairs[my.pair];
       S.geo[e][0] = S.geo[e][3] = g.C[0];
       S.geo[e][1] = S.geo[e][4] = g.C[1];
@@ -440,41 +449,10 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
           const int i = __ffs(todo) - 1, e = e0 + i;
           todo &= todo - 1;
           const NearEntry w = S.queue[e];
-          const int nl = w.nl;
-          const uint8_t* list = S.list[w.lead];
+          const int nl = w.nl, nmt = (nl + 7) >> 3;
           const double* Ae = A + w.pre * 16;
-          const bool isfull = (full >> i) & 1u;
-          if (w.flags & 1) {
-            np = 0;
-            na = nk;  // a call that is near for every FO lists them all
-            if (!isfull) {  // the FOs with near points of this warp, compacted into slots
-              const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
-              const double lo[3] = {box[0], box[1], box[2]}, hi[3] = {box[3], box[4], box[5]};
-              na = 0;
-              for (int sb = 0; sb < nl; sb += 32) {
-                const int s = sb + lane;
-                int st = 1;
-                if (s < nl) {
-                  const CallFO& f = cf[list[s]];
-                  st = (f.npot == 1) ? 0 : tile_class(lo, hi, f.cg[0], f.cg[1], f.cg[2], f.rcut2);
-                }
-                const unsigned on = __ballot_sync(0xffffffffu, st != 1);
-                if (st != 1) S.slot[warp][na + __popc(on & ((1u << lane) - 1u))] = (uint8_t)(s | (st == 0 ? 128 : 0));
-                na += __popc(on);
-              }
-              __syncwarp();
-            }
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-              if (mt * 8 >= na) break;
-              const int s = min(mt * 8 + n, na - 1);
-              const int r = isfull ? s : (int)(S.slot[warp][s] & 127);
-              row[mt] = r * 16 + 2 * (q ^ ((r & 1) << 2));
-            }
-          }
+          if (w.flags & NEAR_FIRST) np = 0;
           ++np;
-          if (na == 0) continue;
-          const int nmt = (na + 7) >> 3;
           if ((e >> 2) != fquad) {
             // Boys values of four pairs at once: lane residue q takes pair 4 fquad + q
             fquad = e >> 2;
@@ -493,42 +471,38 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
           PT F[5];
 #pragma unroll
           for (int j = 0; j < 3; ++j) F[j] = __shfl_sync(0xffffffffu, Fq[j], src);
-          near_mma<MT, PT, 0>(T, Ae, row, nmt, L, F, q == 0);
+          const double *A0 = Ae + piece, *A1 = Ae + (piece ^ 8);
+          near_mma<MT, PT, 0>(T, A0, A1, nmt, L, F, q == 0);
           if (w.fmt >= 4) {
             F[3] = __shfl_sync(0xffffffffu, Fq[3], src);
-            near_mma<MT, PT, 1>(T, Ae + nl * 16, row, nmt, L, F, q == 0);
+            near_mma<MT, PT, 1>(T, A0 + nl * 16, A1 + nl * 16, nmt, L, F, q == 0);
           }
           if (w.fmt >= 5) {
             F[4] = __shfl_sync(0xffffffffu, Fq[4], src);
-            near_mma<MT, PT, 2>(T, Ae + 2 * nl * 16, row, nmt, L, F, q == 0);
+            near_mma<MT, PT, 2>(T, A0 + 2 * nl * 16, A1 + 2 * nl * 16, nmt, L, F, q == 0);
           }
-          if (!(w.flags & 2)) continue;
+          if (!(w.flags & NEAR_LAST)) continue;
           // the call's sum goes to V (call by call, so that no sum depends on how
           // FOs are blocked); a point counts for an FO when it is inside the FO's sphere
-          const CallFO* cf = J.cfo + (size_t)w.call * J.nfo + k0;
+          const uint8_t* list = S.list[w.lead];
+          const CallFO* sph = reinterpret_cast<const CallFO*>(Ae + (w.fmt - 2) * nl * 16);
+          const bool isfull = (full >> i) & 1u;  // then every FO is listed
+          const double *p0 = pts[2 * q], *p1 = pts[2 * q + 1];
           if (isfull && lane == 0) near += (unsigned long long)(nk * npt) * np;
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
             if (mt >= nmt) break;
             const int s = mt * 8 + n;
-            if (s < na) {
-              int k = s;
+            if (s < nl) {
               bool n0 = true, n1 = true;  // points past the end: never stored
               if (!isfull) {
-                const int sl = S.slot[warp][s];
-                k = list[sl & 127];
-                n0 = 2 * q < npt;
-                n1 = 2 * q + 1 < npt;
-                if (sl < 128) {
-                  const CallFO& f = cf[k];
-                  const double cx = f.cg[0], cy = f.cg[1], cz = f.cg[2], rc2 = f.rcut2;
-                  const double *p0 = pts[2 * q], *p1 = pts[2 * q + 1];
-                  n0 = n0 && !(sqdist_rn2(p0[0], p0[1], p0[2], cx, cy, cz) > rc2);
-                  n1 = n1 && !(sqdist_rn2(p1[0], p1[1], p1[2], cx, cy, cz) > rc2);
-                }
+                const CallFO& f = sph[s];
+                const double cx = f.cg[0], cy = f.cg[1], cz = f.cg[2], rc2 = f.rcut2;
+                n0 = 2 * q < npt && !(sqdist_rn2(p0[0], p0[1], p0[2], cx, cy, cz) > rc2);
+                n1 = 2 * q + 1 < npt && !(sqdist_rn2(p1[0], p1[1], p1[2], cx, cy, cz) > rc2);
                 near += (unsigned)(((int)n0 + (int)n1) * np);
               }
-              double2* ch = reinterpret_cast<double2*>(V + k * NEAR_PTS + 2 * q);
+              double2* ch = reinterpret_cast<double2*>(V + (int)list[s] * NEAR_PTS + 2 * q);
               double2 v = *ch;
               if (n0) v.x += T[mt][0];
               if (n1) v.y += T[mt][1];
@@ -536,7 +510,6 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
             }
             T[mt][0] = T[mt][1] = 0.0;
           }
-          if (!isfull) __syncwarp();
         }
       }
       e0 = e1;
