@@ -609,7 +609,8 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                                const double* coef, const int8_t* maxfmt, const CallFO* cfo, const double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
-                               unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st, bool one_density) {
+                               unsigned long long* cnt, cudaEvent_t mid, const SideStream& side, cudaStream_t st,
+                               bool one_density) {
   // one density in FP64: every call by k_one_near and k_perfo_far
   const bool per_fo_only = cfg.per_fo_only || one_density;
   launch_coulomb_classify(ncalls, calls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
@@ -662,7 +663,7 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
     return cudaGetLastError();
   }
   J.nseg = perfo_parts(M.ntiles);
-  launch_perfo(J, cfg.perfo_wm > 0 ? cfg.perfo_wm : perfo_default_wm(nfo), mixed, boys_tab, st);
+  launch_perfo(J, cfg.perfo_wm > 0 ? cfg.perfo_wm : perfo_default_wm(nfo), mixed, boys_tab, side, st);
   return cudaGetLastError();
 }
 

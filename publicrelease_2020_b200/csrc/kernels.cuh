@@ -121,7 +121,7 @@ struct CoulombJob {
   MeshDev M;
   double* vh;
   int nseg, spare;                // the per-FO calls in nseg parts, each a CTA of its own
-  double* seg;                    // nseg > 1: [part][FO][ldv], near parts then far parts
+  double* seg;                    // [part][FO][ldv]: near parts (none if nseg = 1), then far parts
   unsigned long long* cnt;        // work counts of the shared-geometry calls
   unsigned long long* cnt_perfo;  // and of the per-FO calls
 };
@@ -148,11 +148,19 @@ inline int perfo_default_wm(int nfo) { return nfo > 32 ? 2 : 1; }
 // order (from the mesh alone, so that every launch form makes the same sums).
 // Measured: water (31 tiles) near 0.34 -> 0.14 ms in 4 parts, far 0.10 -> 0.05.
 inline int perfo_parts(int ntiles) { return ntiles <= 0 ? 1 : std::max(1, std::min(8, 148 / ntiles)); }
+// One near part adds to vh itself; several, and the far parts, go to seg.
+__host__ __device__ inline int perfo_near_parts(int nseg) { return nseg > 1 ? nseg : 0; }
 inline size_t perfo_seg_size(int ntiles, int nfo, int ldv) {
   const int n = perfo_parts(ntiles);
-  return n > 1 ? (size_t)2 * n * nfo * ldv : 1;
+  return (size_t)(perfo_near_parts(n) + n) * nfo * ldv;
 }
-void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* boys_tab, cudaStream_t st);
+// A context's second stream and the events that fork it from and join it to the first.
+struct SideStream {
+  cudaStream_t st = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* boys_tab, const SideStream& side,
+                  cudaStream_t st);
 // The potential of one density (nfo = 1, FP64) added to vh: near field by one
 // point per thread, far field as above; seg holds one_density_parts * 2 * ldv doubles.
 int one_density_parts(int ntiles);
@@ -177,7 +185,8 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                                const double* coef, const int8_t* maxfmt, const CallFO* cfo, const double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
-                               unsigned long long* cnt, cudaEvent_t mid, cudaStream_t st, bool one_density = false);
+                               unsigned long long* cnt, cudaEvent_t mid, const SideStream& side, cudaStream_t st,
+                               bool one_density = false);
 
 // Exchange-correlation of the FO densities (fully polarised, NSPN forced to 2 as
 // in apotnl_sic.F:419) from the FO values/derivatives phi[(ch*nfo+k)*ldp+p];

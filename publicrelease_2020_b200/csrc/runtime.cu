@@ -315,6 +315,7 @@ struct SpinCache {
 struct flosic_ctx {
   int device = 0;
   cudaStream_t st = nullptr;
+  SideStream side;           // far field of the per-FO calls
   DevBuf<double> d_gemm_ws;  // split-K partial products of dgemm
   DevBuf<double> d_wk[3];    // results of the basis-space sums and the DFT side, kept between calls
   DevBuf<CoulombJob> d_jobs;  // batched Coulomb launch led by this context
@@ -812,9 +813,9 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
                      c->d_bound.p,   c->d_seg.p};
   CUDA_CHECK(launch_coulomb_mma(ncalls, c->d_calls.p, c->d_pairs.p, npairs, nf, c->d_coef.p, c->d_maxfmt.p,
                                 c->d_callfo.p, c->d_mom.p, c->eval_mesh(), c->d_boys.p, vh, P, c->coulomb_cfg, mixed,
-                                scr, c->d_cnt.p, c->ev[8], st, one));
+                                scr, c->d_cnt.p, c->ev[8], c->side, st, one));
   CUDA_CHECK(cudaEventRecord(c->ev[9], st));
-  c->launches += c->coulomb_cfg.per_fo_only ? 8 : 9;
+  c->launches += c->coulomb_cfg.per_fo_only ? 9 : 10;
   unsigned long long cnt[6];
   int tc_err = 0;
   CUDA_CHECK(cudaMemcpyAsync(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost, st));
@@ -1340,6 +1341,9 @@ int flosic_sic_create(int device, flosic_ctx** out) {
     }
     CUDA_CHECK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
     for (auto& e : c->ev) CUDA_CHECK(cudaEventCreate(&e));
+    CUDA_CHECK(cudaStreamCreateWithFlags(&c->side.st, cudaStreamNonBlocking));
+    CUDA_CHECK(cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming));
+    CUDA_CHECK(cudaEventCreateWithFlags(&c->side.join, cudaEventDisableTiming));
     std::vector<double> ang, w;
     lebedev19(ang, w);
     upload_constants(ang.data(), w.data());
@@ -1382,6 +1386,9 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_jobs.release();
   c->d_items.release();
   c->d_batch_counters.release();
+  if (c->side.fork) cudaEventDestroy(c->side.fork);
+  if (c->side.join) cudaEventDestroy(c->side.join);
+  if (c->side.st) cudaStreamDestroy(c->side.st);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
   return FLOSIC_OK;
@@ -2078,7 +2085,7 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       launch_perfo_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), parts, wm,
                          c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, c0->st);
       CUDA_CHECK(cudaGetLastError());
-      c0->launches += 3;
+      c0->launches += 4;
     }
     CUDA_CHECK(cudaEventRecord(c0->ev[4], c0->st));
     for (int m = 1; m < n; ++m) CUDA_CHECK(cudaStreamWaitEvent(ctxs[m]->st, c0->ev[4], 0));
