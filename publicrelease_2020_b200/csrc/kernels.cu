@@ -647,7 +647,8 @@ __global__ void __launch_bounds__(THREADS) k_call_moments(const int* __restrict_
                                                               const double* __restrict__ coef,
                                                               const int8_t* __restrict__ maxfmt,
                                                               const double* __restrict__ boys_tab,
-                                                              CallFO* __restrict__ out, double* __restrict__ momv) {
+                                                              CallFO* __restrict__ out, double* __restrict__ momv,
+                                                          int* __restrict__ again) {
   __shared__ double v[8 * MOM_VLD];
   __shared__ double mom[8][WY_N];
   __shared__ double s_cg[FOS][3], s_rcut[FOS];
@@ -707,28 +708,39 @@ __global__ void __launch_bounds__(THREADS) k_call_moments(const int* __restrict_
   const int f = warp;
   if (f >= nk || !s_on[f]) return;
   const double rcut = s_rcut[f], h = sqrt(rcut * rcut), ri1 = 1.0 / rcut;
+  const double* vf = v + f * MOM_VLD;
+  double vmax = 0.0;
+  for (int i = lane; i < NANG; i += 32) vmax = fmax(vmax, fabs(vf[i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
   double val[2];
   unsigned long long keep = 0ull;
+  bool unsure = false;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int m = lane + 32 * j;
-    bool kept = false;
-    val[j] = 0.0;
-    if (m < NMOM) {
-      int l = 0;
-      while ((l + 1) * (l + 1) <= m) ++l;
-      double rl = h, rt = ri1;
-      for (int i = 1; i <= l; ++i) {
-        rl = h * rl;
-        rt *= ri1;
-      }
-      const double x = mom[f][m] * rl;
-      kept = !(fabs((2 * l + 1) * x * rt) < 1.0e-12);
-      val[j] = kept ? x * c_mom_vf[m] : 0.0;
+    int l = 0;
+    while ((l + 1) * (l + 1) <= m) ++l;
+    double rl = h, rt = ri1;
+    for (int i = 1; i <= l; ++i) {
+      rl = h * rl;
+      rt *= ri1;
     }
+    const double x = m < NMOM ? mom[f][m] * rl : 0.0;
+    // A moment that vanishes by symmetry is rounding of the sum, and where the
+    // potential is large that rounding is near the skip rule's 1e-12: the FO is
+    // left to k_call_moments_again.
+    const double eps = (2 * l + 1) * 7.0e-15 * vmax * fmax(1.0, 0.125 * ci.np);
+    unsure = unsure || (m < NMOM && fabs(fabs((2 * l + 1) * x * rt) - 1.0e-12) < eps);
+    const bool kept = m < NMOM && !(fabs((2 * l + 1) * x * rt) < 1.0e-12);
+    val[j] = kept ? x * c_mom_vf[m] : 0.0;
     keep |= (unsigned long long)__ballot_sync(0xffffffffu, kept) << (32 * j);
   }
   const size_t ck = (size_t)c * nfo + k0 + f;
+  if (__any_sync(0xffffffffu, unsure)) {
+    if (lane == 0) again[1 + atomicAdd(again, 1)] = (int)ck;
+    return;
+  }
   double* mv = momv + ck * MOM_LD;
   mv[lane] = val[0];
   if (lane + 32 < MOM_LD) mv[lane + 32] = val[1];
@@ -740,6 +752,81 @@ __global__ void __launch_bounds__(THREADS) k_call_moments(const int* __restrict_
     }
     out[ck].keep = keep;
     out[ck].lmax = lmx;
+  }
+}
+
+// The moments of the listed (call, FO)s with the skip rule near its threshold,
+// each term and sum formed point by point: harmonics at the FO's own sphere
+// points, 146 terms added in order.  A block per entry.
+constexpr int AGAIN_THREADS = 160;
+__global__ void __launch_bounds__(AGAIN_THREADS) k_call_moments_again(const int* __restrict__ again, int nfo,
+                                                                      const CallInfo* __restrict__ calls,
+                                                                      const PairGeo* __restrict__ pairs,
+                                                                      const double* __restrict__ coef,
+                                                                      const int8_t* __restrict__ maxfmt,
+                                                                      const double* __restrict__ boys_tab,
+                                                                      CallFO* __restrict__ out,
+                                                                      double* __restrict__ momv) {
+  extern __shared__ double prod[];  // [NANG][NMOM]
+  __shared__ unsigned ballot[2];
+  const int tid = threadIdx.x, n = again[0];
+  for (int e = blockIdx.x; e < n; e += gridDim.x) {
+    const int ck = again[1 + e], c = ck / nfo, k = ck - c * nfo;
+    const CallInfo ci = calls[c];
+    const double cg[3] = {out[ck].cg[0], out[ck].cg[1], out[ck].cg[2]}, rcut = out[ck].rcut;
+    if (tid < NANG) {
+      const double q[3] = {cg[0] + c_leb_ang[3 * tid] * rcut, cg[1] + c_leb_ang[3 * tid + 1] * rcut,
+                           cg[2] + c_leb_ang[3 * tid + 2] * rcut};
+      double v = 0.0;
+      for (int qq = 0; qq < ci.np; ++qq) {
+        const PairGeo& g = pairs[ci.p0 + qq];
+        const double rx = q[0] - g.C[0], ry = q[1] - g.C[1], rz = q[2] - g.C[2];
+        const double xx = g.delta * (rz * rz + ry * ry + rx * rx);
+        const double chgd = exp(-xx);
+        double s3[3], s4[4], s5[5], mono[35];
+        boys_all(boys_tab, xx, chgd, s3, s4, s5);
+        monomials(rx, ry, rz, mono);
+        const size_t pk = (size_t)(ci.p0 + qq) * nfo + k;
+        v += pair_potential(coef + pk * COEF_LD, mono, maxfmt[pk], s3, s4, s5);
+      }
+      const double hn = 1.0 / sqrt(rcut * rcut);
+      double Y[NMOM];
+      harmonics6(LM, hn * (c_leb_ang[3 * tid] * rcut), hn * (c_leb_ang[3 * tid + 1] * rcut),
+                 hn * (c_leb_ang[3 * tid + 2] * rcut), Y);
+      for (int m = 0; m < NMOM; ++m) prod[tid * NMOM + m] = c_leb_w[tid] * Y[m] * v;
+    }
+    __syncthreads();
+    bool kept = false;
+    double x = 0.0;
+    int l = 0;
+    if (tid < NMOM) {
+      double s = 0.0;
+      for (int i = 0; i < NANG; ++i) s += prod[i * NMOM + tid];
+      while ((l + 1) * (l + 1) <= tid) ++l;
+      const double h = sqrt(rcut * rcut), ri1 = 1.0 / rcut;
+      double rl = h, rt = ri1;
+      for (int j = 1; j <= l; ++j) {
+        rl = h * rl;
+        rt *= ri1;
+      }
+      x = s * rl;
+      kept = !(fabs((2 * l + 1) * x * rt) < 1.0e-12);
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, kept);
+    if (tid == 0 || tid == 32) ballot[tid >> 5] = b;
+    if (tid < MOM_LD) momv[(size_t)ck * MOM_LD + tid] = kept ? x * c_mom_vf[tid] : 0.0;
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned long long keep = ballot[0] | ((unsigned long long)ballot[1] << 32);
+      int lmx = 0;
+      if (keep) {
+        const int top = 63 - __clzll((long long)keep);
+        while ((lmx + 1) * (lmx + 1) <= top) ++lmx;
+      }
+      out[ck].keep = keep;
+      out[ck].lmax = lmx;
+    }
+    __syncthreads();
   }
 }
 
@@ -876,13 +963,16 @@ __global__ void __launch_bounds__(SETUP1_THREADS) k_call_setup_single(
 }
 
 void init_call_setup() {
+  cudaFuncSetAttribute(k_call_moments_again, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(sizeof(double) * NANG * NMOM));
   cudaFuncSetAttribute(k_call_setup_single, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)(sizeof(double) * NANG * (GEO_LD + NMOM)));
 }
 
 void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo* calls, const PairGeo* pairs,
                        int nfo, int nspn, const double* coef, const int8_t* maxfmt, const double* cgp,
-                       const MeshDev& M, const double* boys_tab, CallFO* cfo, double* momv, cudaStream_t st) {
+                       const MeshDev& M, const double* boys_tab, CallFO* cfo, double* momv, int* again,
+                       cudaStream_t st) {
   if (ncalls <= 0) return;
   if (nsingle > 0)
     k_call_setup_single<<<nsingle, SETUP1_THREADS, sizeof(double) * NANG * (GEO_LD + NMOM), st>>>(
@@ -890,14 +980,17 @@ void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo*
   const int nmulti = ncalls - nsingle;
   if (nmulti > 0) {
     const size_t warps = (size_t)nmulti * nfo;
+    cudaMemsetAsync(again, 0, sizeof(int), st);
     k_call_geom<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(nmulti, list + nsingle, calls, pairs, nfo, nspn, cgp, M,
                                                               cfo, momv);
     if ((size_t)nmulti * ((nfo + 7) / 8) < 4 * 148)  // less than two waves of the eight-FO blocks
       k_call_moments<2, 320><<<dim3(nmulti, (nfo + 1) / 2), 320, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
-                                                                          maxfmt, boys_tab, cfo, momv);
+                                                                          maxfmt, boys_tab, cfo, momv, again);
     else
       k_call_moments<8, 256><<<dim3(nmulti, (nfo + 7) / 8), 256, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
-                                                                          maxfmt, boys_tab, cfo, momv);
+                                                                          maxfmt, boys_tab, cfo, momv, again);
+    k_call_moments_again<<<(int)std::min<size_t>(3 * 148, warps), AGAIN_THREADS, sizeof(double) * NANG * NMOM, st>>>(
+        again, nfo, calls, pairs, coef, maxfmt, boys_tab, cfo, momv);
   }
 }
 

@@ -252,6 +252,7 @@ struct CoulBufs {
   DevBuf<double> coef, cgp, mom, coefp, momp, seg;
   DevBuf<CallBound> bound;
   DevBuf<PerfoPair> plist;
+  DevBuf<int> again;
   DevBuf<int8_t> maxfmt, pairfmt;
   DevBuf<CallFO> callfo;
   DevBuf<CallShare> share;
@@ -266,6 +267,7 @@ struct CoulBufs {
     seg.release();
     bound.release();
     plist.release();
+    again.release();
     maxfmt.release();
     pairfmt.release();
     callfo.release();
@@ -366,6 +368,7 @@ struct flosic_ctx {
   DevBuf<double> d_coefp, d_momp, d_seg;
   DevBuf<CallBound> d_bound;
   DevBuf<PerfoPair> d_plist;
+  DevBuf<int> d_again;
   DevBuf<int> d_lists, d_tc_err;
   DevBuf<int> d_setup_list;  // one-slot calls first (nsingle), then the others
   int nsingle = 0;
@@ -781,12 +784,14 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
   c->d_cgp.ensure((size_t)std::max(npairs, 1) * nf * 4);
   c->d_callfo.ensure((size_t)std::max(ncalls, 1) * nf);
   c->d_mom.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
+  c->d_again.ensure((size_t)1 + (size_t)(ncalls - c->nsingle) * nf);
   CUDA_CHECK(cudaEventRecord(c->ev[2], st));
   launch_pair_coef(npairs, c->d_pairs.p, c->d_calls.p, nf, c->nprim, c->d_u.p, dm, c->nspn, c->d_coef.p,
                    c->d_maxfmt.p, c->d_cgp.p, st);
   c->launches++;
   launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn, c->d_coef.p,
-                    c->d_maxfmt.p, c->d_cgp.p, c->mesh_dev(), c->d_boys.p, c->d_callfo.p, c->d_mom.p, st);
+                    c->d_maxfmt.p, c->d_cgp.p, c->mesh_dev(), c->d_boys.p, c->d_callfo.p, c->d_mom.p,
+                    c->d_again.p, st);
   c->launches++;
   CUDA_CHECK(cudaEventRecord(c->ev[3], st));
   c->d_pairfmt.ensure((size_t)std::max(npairs, 1));
@@ -1223,6 +1228,7 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   B.cgp.ensure((size_t)std::max(npairs, 1) * nf * 4);
   B.callfo.ensure((size_t)std::max(ncalls, 1) * nf);
   B.mom.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
+  B.again.ensure((size_t)1 + (size_t)(ncalls - c->nsingle) * nf);
   B.pairfmt.ensure((size_t)std::max(npairs, 1));
   B.share.ensure((size_t)std::max(ncalls, 1));
   B.lists.ensure((size_t)2 * ncalls + 3);
@@ -1231,7 +1237,7 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   launch_pair_coef(npairs, c->d_pairs.p, c->d_calls.p, nf, c->nprim, c->d_u.p, nullptr, c->nspn, B.coef.p,
                    B.maxfmt.p, B.cgp.p, st);
   launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn, B.coef.p,
-                    B.maxfmt.p, B.cgp.p, c->mesh_dev(), c->d_boys.p, B.callfo.p, B.mom.p, st);
+                    B.maxfmt.p, B.cgp.p, c->mesh_dev(), c->d_boys.p, B.callfo.p, B.mom.p, B.again.p, st);
   CUDA_CHECK(cudaMemsetAsync(B.cnt.p, 0, 3 * sizeof(unsigned long long), st));
   B.coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
   B.momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
@@ -1377,7 +1383,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_basis.release(); c->d_fodpts.release(); c->d_psig.release(); c->d_tmat.release(); c->d_u.release();
   c->d_coef.release(); c->d_cgp.release(); c->d_mom.release(); c->d_part.release(); c->d_sums.release();
   c->d_sic.release(); c->d_tmp.release(); c->d_maxfmt.release(); c->d_callfo.release(); c->d_cnt.release(); c->d_pairfmt.release();
-  c->d_coefp.release(); c->d_momp.release(); c->d_seg.release(); c->d_bound.release(); c->d_plist.release();
+  c->d_coefp.release(); c->d_momp.release(); c->d_seg.release(); c->d_bound.release(); c->d_plist.release(); c->d_again.release();
   c->d_share.release(); c->d_lists.release(); c->d_setup_list.release();
   c->d_eig_a.release(); c->d_eig_w.release(); c->d_eig_v.release(); c->d_eig_work.release(); c->d_eig_info.release();
   c->d_coef_hl.release(); c->d_momv_hl.release(); c->d_tc_err.release(); c->d_dens_coef.release();
