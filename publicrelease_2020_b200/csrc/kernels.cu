@@ -1134,22 +1134,32 @@ void launch_xc(const MeshDev& M, int nfo, int gga, int mgga, int nspn, const int
 }
 
 // Compensated (Neumaier) sums of the block partials, in block order.
-__global__ void k_reduce_parts(int nfo, int nblk, const double* __restrict__ part, double* __restrict__ sums) {
-  const int k = blockIdx.x, j = threadIdx.x;
-  if (j >= NPART) return;
+// Block partial sums added up, compensated: a warp per (FO, quantity), each lane
+// the blocks of its residue in order, then the lanes' sums in a fixed tree (one
+// thread and a dependent chain over all blocks took 10-50 us).
+__global__ void __launch_bounds__(32 * NPART) k_reduce_parts(int nblk, const double* __restrict__ part,
+                                                             double* __restrict__ sums) {
+  const int k = blockIdx.x, j = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double s = 0.0, cmp = 0.0;
-  for (int b = 0; b < nblk; ++b) {
-    const double x = part[((size_t)k * nblk + b) * NPART + j];
+  auto add = [&](double x) {
     const double t = s + x;
     if (fabs(s) >= fabs(x)) cmp += (s - t) + x;
     else cmp += (x - t) + s;
     s = t;
+  };
+#pragma unroll 4
+  for (int b = lane; b < nblk; b += 32) add(part[((size_t)k * nblk + b) * NPART + j]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double x = __shfl_down_sync(0xffffffffu, s, o), c = __shfl_down_sync(0xffffffffu, cmp, o);
+    add(x);
+    cmp += c;
   }
-  sums[(size_t)k * NPART + j] = s + cmp;
+  if (lane == 0) sums[(size_t)k * NPART + j] = s + cmp;
 }
 
 void launch_reduce_parts(int nfo, int nblk, const double* part, double* sums, cudaStream_t st) {
-  k_reduce_parts<<<nfo, 32, 0, st>>>(nfo, nblk, part, sums);
+  k_reduce_parts<<<nfo, 32 * NPART, 0, st>>>(nblk, part, sums);
 }
 
 // FO density channels RHOG(ldr, nch) from the phi channels: nch = 1 (LDA),
@@ -1270,23 +1280,48 @@ void launch_xc_mgga_rhog(const MeshDev& M, const double* rhog, int ldr, const do
   k_xc_mgga_rhog<<<nblk, XC_THREADS, 0, st>>>(M, rhog, ldr, tau, vxc, mixin, part, nblk);
 }
 
-__global__ void __launch_bounds__(XC_THREADS) k_xc_rhog(MeshDev M, int gga, XCParams xp,
-                                                        const double* __restrict__ rhog, int ldr,
-                                                        double* __restrict__ vxc, double* __restrict__ part,
-                                                        int nblk) {
-  double pv[NPART];
-#pragma unroll
-  for (int j = 0; j < NPART; ++j) pv[j] = 0.0;
-  for (int p = blockIdx.x * XC_THREADS + threadIdx.x; p < M.n; p += nblk * XC_THREADS) {
-    double r[10];
-    for (int d = 0; d < 10; ++d) r[d] = (d == 0 || gga) ? rhog[(size_t)d * ldr + p] : 0.0;
-    double vup, vdn, e4[4] = {0, 0, 0, 0};
-    xc_point_sic(xp, r, M.w[p], vup, vdn, e4);
-    vxc[p] = vup;
-    vxc[M.n + p] = vdn;
-    for (int j = 0; j < 4; ++j) pv[4 + j] += e4[j];
+// GETVLXC of given density channels.  One point is a chain of some 15 pow, exp,
+// log and sqrt calls, and a call on a few 10,000 points has about one warp per
+// scheduler: half of a block's warps take the exchange and half the correlation
+// of the same 64 points (20,011 points, PBE: whole call 51 -> 36 us, with the sums below).
+constexpr int RHOG_PTS = 64;
+int xc_rhog_blocks(int npts) { return std::min(1024, (npts + RHOG_PTS - 1) / RHOG_PTS); }
+
+__global__ void __launch_bounds__(2 * RHOG_PTS) k_xc_rhog(MeshDev M, int gga, XCParams xp,
+                                                          const double* __restrict__ rhog, int ldr,
+                                                          double* __restrict__ vxc, double* __restrict__ part,
+                                                          int nblk) {
+  __shared__ double vx[RHOG_PTS], red[2 * RHOG_PTS / 32][2];
+  const int tid = threadIdx.x, i = tid % RHOG_PTS;
+  const bool corr = tid >= RHOG_PTS;
+  double e[2] = {0.0, 0.0};
+  for (int p0 = blockIdx.x * RHOG_PTS; p0 < M.n; p0 += nblk * RHOG_PTS) {
+    const int p = p0 + i;
+    double vup = 0.0, vdn = 0.0;
+    if (p < M.n) {
+      double r[10];
+      for (int d = 0; d < 10; ++d) r[d] = (d == 0 || gga) ? rhog[(size_t)d * ldr + p] : 0.0;
+      if (corr) xc_point_correlation(xp, r, M.w[p], vup, vdn, e[0], e[1]);
+      else vx[i] = xc_point_exchange(xp, r, M.w[p], e[0], e[1]);
+    }
+    __syncthreads();
+    if (corr && p < M.n) {
+      vxc[p] = vx[i] + vup;
+      vxc[M.n + p] = vdn;
+    }
+    __syncthreads();
   }
-  block_reduce_parts(pv, part + (size_t)blockIdx.x * NPART);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    for (int o = 16; o > 0; o >>= 1) e[j] += __shfl_down_sync(0xffffffffu, e[j], o);
+    if ((tid & 31) == 0) red[tid >> 5][j] = e[j];
+  }
+  __syncthreads();
+  if (tid < NPART) {
+    const int j = tid - 4;  // 4..7: ERGXL, ERGXN, ERGCL, ERGCN
+    part[(size_t)blockIdx.x * NPART + tid] =
+        j >= 0 && j < 4 ? red[2 * (j >> 1)][j & 1] + red[2 * (j >> 1) + 1][j & 1] : 0.0;
+  }
 }
 
 // Loads the two kernels of the GETVLXC-on-device-buffers path on the current
@@ -1306,7 +1341,7 @@ void launch_xc_rhog(const MeshDev& M, int gga, const int* xc, const double* rhog
   xp.idftyp[0] = xc[1];
   xp.igga[1] = xc[2];
   xp.idftyp[1] = xc[3];
-  k_xc_rhog<<<nblk, XC_THREADS, 0, st>>>(M, gga, xp, rhog, ldr, vxc, part, nblk);
+  k_xc_rhog<<<nblk, 2 * RHOG_PTS, 0, st>>>(M, gga, xp, rhog, ldr, vxc, part, nblk);
 }
 
 }  // namespace flosic

@@ -229,8 +229,10 @@ void launch_scale_rows(int P, int N, const double* a, int lda, const double* w, 
 // v[k*n + m] = component k of eigenvector m; info 0, or 1 without convergence.
 cudaError_t init_sym_eigen();
 size_t sym_eigen_work(int n);
+size_t sym_eigen_info(int n);  // ints of info; info[0] is the status
 bool launch_sym_eigen(int n, const double* a, double* work, double* w, double* v, int* info, cudaStream_t st);
 cudaError_t preload_xc_rhog();
+int xc_rhog_blocks(int npts);
 void launch_xc_rhog(const MeshDev& M, int gga, const int* xc, const double* rhog, int ldr, double* vxc,
                     double* part, int nblk, cudaStream_t st);
 

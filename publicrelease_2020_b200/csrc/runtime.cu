@@ -318,6 +318,7 @@ struct flosic_ctx {
   int device = 0;
   cudaStream_t st = nullptr;
   SideStream side;           // far field of the per-FO calls
+  double* h_sums = nullptr;  // NPART doubles of mapped host memory (flosic_sic_getvlxc_device)
   DevBuf<double> d_gemm_ws;  // split-K partial products of dgemm
   DevBuf<double> d_wk[3];    // results of the basis-space sums and the DFT side, kept between calls
   DevBuf<CoulombJob> d_jobs;  // batched Coulomb launch led by this context
@@ -670,10 +671,10 @@ auto device_eigen(flosic_ctx* c) {
     c->d_eig_w.ensure(n);
     c->d_eig_v.ensure((size_t)n * n);
     c->d_eig_work.ensure(sym_eigen_work(n));
-    c->d_eig_info.ensure(1);
+    c->d_eig_info.ensure(sym_eigen_info(n));
     if (!launch_sym_eigen(n, c->d_eig_a.p, c->d_eig_work.p, c->d_eig_w.p, c->d_eig_v.p, c->d_eig_info.p, st))
       fail(FLOSIC_ERR_CAPACITY, "LOWSIC: more FOs per spin than the eigen-solver holds");
-    c->launches++;
+    c->launches += 2;
     CUDA_CHECK(cudaGetLastError());
     v.resize((size_t)n * n);
     w.resize(n);
@@ -1139,14 +1140,15 @@ void require_whole_mesh(flosic_ctx* c) {
 // ---------------------------------------------------------------------------
 // flosic_sic_getvlxc_device keeps its per-block energy partial sums in this
 // file-scope device array instead of allocating: XC_SCRATCH_BLOCKS blocks of
-// 256 points (4,194,304 points at most) times NPART partials, then the NPART
-// final sums.  Every call overwrites the partials of its nblk blocks and the
-// sums before reading them, so no part of the array has to start at zero.  All
+// 256 points (4,194,304 points at most) times NPART partials.  Every call
+// overwrites the partials of its nblk blocks before reading them, so no part of
+// the array has to start at zero; the final sums go to the context's own mapped
+// host memory.  All
 // calls on one device share it: calls that overlap in time (other host threads,
 // other contexts or streams on the same device) race on it.
 constexpr int XC_SCRATCH_BLOCKS = 16384;
 constexpr int XC_SCRATCH_POINTS = XC_SCRATCH_BLOCKS * 256;
-static __device__ __align__(256) double g_xc_scratch[(XC_SCRATCH_BLOCKS + 1) * NPART];
+static __device__ __align__(256) double g_xc_scratch[XC_SCRATCH_BLOCKS * NPART];
 
 // Device address of g_xc_scratch for the current device, looked up once per
 // device with that device current.  flosic_sic_create calls it, so the module
@@ -1350,6 +1352,7 @@ int flosic_sic_create(int device, flosic_ctx** out) {
     CUDA_CHECK(cudaStreamCreateWithFlags(&c->side.st, cudaStreamNonBlocking));
     CUDA_CHECK(cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming));
     CUDA_CHECK(cudaEventCreateWithFlags(&c->side.join, cudaEventDisableTiming));
+    CUDA_CHECK(cudaHostAlloc(&c->h_sums, sizeof(double) * NPART, cudaHostAllocMapped));
     std::vector<double> ang, w;
     lebedev19(ang, w);
     upload_constants(ang.data(), w.data());
@@ -1392,6 +1395,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_jobs.release();
   c->d_items.release();
   c->d_batch_counters.release();
+  if (c->h_sums) cudaFreeHost(c->h_sums);
   if (c->side.fork) cudaEventDestroy(c->side.fork);
   if (c->side.join) cudaEventDestroy(c->side.join);
   if (c->side.st) cudaStreamDestroy(c->side.st);
@@ -1722,7 +1726,7 @@ int flosic_sic_getvlxc(flosic_ctx* c, int ndim, const double* rhog, double* vxc,
     DevBuf<double> dr, dv;
     dr.upload(r.data(), r.size(), c->st);
     dv.ensure(2 * (size_t)P);
-    const int nblk = std::min(1024, (P + 255) / 256);
+    const int nblk = xc_rhog_blocks(P);
     c->d_part.ensure((size_t)nblk * NPART);
     c->d_sums.ensure(NPART);
     launch_xc_rhog(c->mesh_dev(), c->gga, c->xc, dr.p, P, dv.p, c->d_part.p, nblk, c->st);
@@ -1904,18 +1908,15 @@ int flosic_sic_getvlxc_device(flosic_ctx* c, int npts, const double* d_rhog, int
                                     std::to_string(XC_SCRATCH_POINTS) +
                                     "-point capacity of the allocation-free GETVLXC scratch");
     double* part = xc_scratch_address(c->device);
-    double* sums = part + (size_t)XC_SCRATCH_BLOCKS * NPART;
-    const int nblk = std::min(1024, (npts + 255) / 256);  // k_xc_rhog strides over the rest
+    const int nblk = xc_rhog_blocks(npts);  // k_xc_rhog strides over the rest
     MeshDev M{};
     M.n = npts;
     M.w = d_wmsh;
     launch_xc_rhog(M, c->gga, c->xc, d_rhog, ldr, d_vxc, part, nblk, c->st);
-    launch_reduce_parts(1, nblk, part, sums, c->st);
+    launch_reduce_parts(1, nblk, part, c->h_sums, c->st);  // straight into the context's mapped host memory
     CUDA_CHECK(cudaGetLastError());
-    double s[NPART];
-    CUDA_CHECK(cudaMemcpyAsync(s, sums, sizeof(s), cudaMemcpyDeviceToHost, c->st));
     CUDA_CHECK(cudaStreamSynchronize(c->st));
-    for (int j = 0; j < 4; ++j) ergs[j] = s[4 + j];
+    for (int j = 0; j < 4; ++j) ergs[j] = c->h_sums[4 + j];
   });
 }
 

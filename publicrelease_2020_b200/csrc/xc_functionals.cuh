@@ -252,62 +252,57 @@ __device__ __forceinline__ void xc_pbecor(double rs, double zet, double t, doubl
 }
 
 // One mesh point of SUBVLXC with NSPN=2: r[0..9] total-density channels, the
-// spin-down density zero (the SIC call of apotnl_sic.F:419-445).  Returns the
-// spin-up/down potentials and adds ERGXL,ERGXN,ERGCL,ERGCN contributions.
-__device__ __forceinline__ void xc_point_sic(const XCParams& P, const double r[10], double wgt, double& vup,
-                                             double& vdn, double e4[4]) {
+// spin-down density zero (the SIC call of apotnl_sic.F:419-445), in two halves.
+// Exchange of the spin-up density (the spin-down density has none): its potential,
+// and the ERGXL, ERGXN contributions.
+__device__ __forceinline__ double xc_point_exchange(const XCParams& P, const double r[10], double wgt, double& ergxl,
+                                                    double& ergxn) {
+  const bool isgga = P.igga[0] >= 1 || P.igga[1] >= 1;
+  const double THIRD = 0.3333333333333333, TRPI2 = 29.6088132032680759, EPS = 1.0e-20;
+  double den0 = r[0];
+  if (den0 < 0.0) den0 = 0.0;
+  if (P.idftyp[0] == 0 || den0 < EPS) return 0.0;
+  const double D = 2.0 * den0;
+  if (!(D > EPS)) return 0.0;
+  double dkf = pow(TRPI2 * D, THIRD);
+  double S = 0, U = 0, V = 0;
+  if (isgga && P.igga[0] != 0) {
+    // spin-up channels = total - 0 (subvlxc_libxc.F90:271-286)
+    const double dg2 = r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+    const double dgg = r[4] * r[1] * r[1] + r[5] * r[2] * r[2] + r[6] * r[3] * r[3] +
+                       2 * (r[7] * r[1] * r[2] + r[8] * r[1] * r[3] + r[9] * r[2] * r[3]);
+    const double dlp = r[4] + r[5] + r[6];
+    double dgrad = 2.0 * sqrt(dg2);
+    double dlap = 2.0 * dlp;
+    double rec2 = 0.5 / (dkf * D);
+    double rec1 = rec2 * D;
+    double rec22 = rec2 * rec2;
+    S = dgrad * rec2;
+    V = dlap * rec1 * rec2;
+    U = (dgrad > EPS) ? 8.0 * dgg * rec1 * rec22 / dgrad : 0.0;
+  }
+  double ex = 0, dex = 0, vx = 0;
+  if (P.idftyp[0] <= 6) xc_pw91ex(dkf, S, U, V, ex, dex, vx);
+  else if (P.idftyp[0] == 7) xc_pbeex(1, D, S, U, V, ex, dex, vx);
+  else if (P.idftyp[0] == 8) xc_pbeex(2, D, S, U, V, ex, dex, vx);
+  else xc_pbeex(3, D, S, U, V, ex, dex, vx);
+  ergxl += 1.0 * 0.5 * ex * D * wgt;
+  ergxn += 1.0 * 0.5 * dex * D * wgt;
+  return vx;
+}
+
+// Correlation: the spin-up and spin-down potentials and the ERGCL, ERGCN contributions.
+__device__ __forceinline__ void xc_point_correlation(const XCParams& P, const double r[10], double wgt, double& vup,
+                                                     double& vdn, double& ergcl, double& ergcn) {
   const bool isgga = P.igga[0] >= 1 || P.igga[1] >= 1;
   const double THIRD = 0.3333333333333333, THIRD2 = 0.6666666666666667;
   const double TRPI2 = 29.6088132032680759, FRDPI = 1.2732395447351627, DKF2RS = 1.9191582926775128;
   const double EPS = 1.0e-20;
-  double rt0 = r[0];
-  if (rt0 < 0.0) rt0 = 0.0;
-  double den0 = rt0, den2 = 0.0;
-  double den1 = den0 - den2;
-  double dg2_0 = 0, dg2_1 = 0, dgg_0 = 0, dgg_1 = 0, dlp_0 = 0, dlp_1 = 0;
-  if (isgga) {
-    dg2_0 = r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
-    dgg_0 = r[4] * r[1] * r[1] + r[5] * r[2] * r[2] + r[6] * r[3] * r[3] +
-            2 * (r[7] * r[1] * r[2] + r[8] * r[1] * r[3] + r[9] * r[2] * r[3]);
-    dlp_0 = r[4] + r[5] + r[6];
-    // spin-up channels = total - 0 (subvlxc_libxc.F90:271-286)
-    double u1 = r[1] - 0.0, u2 = r[2] - 0.0, u3 = r[3] - 0.0;
-    double u4 = r[4] - 0.0, u5 = r[5] - 0.0, u6 = r[6] - 0.0, u7 = r[7] - 0.0, u8 = r[8] - 0.0,
-           u9 = r[9] - 0.0;
-    dg2_1 = u1 * u1 + u2 * u2 + u3 * u3;
-    dgg_1 = u4 * u1 * u1 + u5 * u2 * u2 + u6 * u3 * u3 + 2 * (u7 * u1 * u2 + u8 * u1 * u3 + u9 * u2 * u3);
-    dlp_1 = u4 + u5 + u6;
-  }
+  double D = r[0];
+  if (D < 0.0) D = 0.0;
+  const double den1 = D, den2 = 0.0;
   vup = 0.0;
   vdn = 0.0;
-  // exchange, spin up only (spin-down density is zero)
-  if (!(P.idftyp[0] == 0 || den0 < EPS)) {
-    double D = 2.0 * den1;
-    if (D > EPS) {
-      double dkf = pow(TRPI2 * D, THIRD);
-      double S = 0, U = 0, V = 0;
-      if (P.igga[0] != 0) {
-        double dgrad = 2.0 * sqrt(dg2_1);
-        double dlap = 2.0 * dlp_1;
-        double rec2 = 0.5 / (dkf * D);
-        double rec1 = rec2 * D;
-        double rec22 = rec2 * rec2;
-        S = dgrad * rec2;
-        V = dlap * rec1 * rec2;
-        U = (dgrad > EPS) ? 8.0 * dgg_1 * rec1 * rec22 / dgrad : 0.0;
-      }
-      double ex = 0, dex = 0, vx = 0;
-      if (P.idftyp[0] <= 6) xc_pw91ex(dkf, S, U, V, ex, dex, vx);
-      else if (P.idftyp[0] == 7) xc_pbeex(1, D, S, U, V, ex, dex, vx);
-      else if (P.idftyp[0] == 8) xc_pbeex(2, D, S, U, V, ex, dex, vx);
-      else xc_pbeex(3, D, S, U, V, ex, dex, vx);
-      vup += vx;
-      e4[0] += 1.0 * 0.5 * ex * D * wgt;
-      e4[1] += 1.0 * 0.5 * dex * D * wgt;
-    }
-  }
-  // correlation
-  double D = den0;
   if (P.idftyp[1] == 0 || D < EPS) return;
   double drec = 1.0 / D;
   double zet = (den1 - den2) * drec;
@@ -317,9 +312,12 @@ __device__ __forceinline__ void xc_point_sic(const XCParams& P, const double r[1
   double g = 0.5 * (pow(1.0 + zet, THIRD2) + pow(1.0 - zet, THIRD2));
   if (zet == -1.0 || zet == 1.0) g = 0.5 * pow(2.0, THIRD2);
   double T = 0, UU = 0, VV = 0, WW = 0;
-  if (P.igga[1] != 0) {
-    double dgrad = sqrt(dg2_0);
-    double dlap = dlp_0;
+  if (isgga && P.igga[1] != 0) {
+    const double dg2 = r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+    const double dgg = r[4] * r[1] * r[1] + r[5] * r[2] * r[2] + r[6] * r[3] * r[3] +
+                       2 * (r[7] * r[1] * r[2] + r[8] * r[1] * r[3] + r[9] * r[2] * r[3]);
+    double dgrad = sqrt(dg2);
+    double dlap = r[4] + r[5] + r[6];
     double rec3 = drec;
     double rec1 = 0.5 / (dks * g);
     double rec2 = rec1 * rec3;
@@ -327,10 +325,10 @@ __device__ __forceinline__ void xc_point_sic(const XCParams& P, const double r[1
     T = dgrad * rec2;
     VV = dlap * rec1 * rec2;
     // WW = D*(DG2(2)-DG2(3)) - (DUP-DDN)*DG2(1): DG2(2) is the spin-up |grad|^2
-    WW = D * (dg2_1 - 0.0);
-    WW = WW - (den1 - den2) * dg2_0;
+    WW = D * (dg2 - 0.0);
+    WW = WW - (den1 - den2) * dg2;
     WW = WW * rec3 * rec22;
-    UU = (dgrad > EPS) ? dgg_0 * rec1 * rec22 / dgrad : 0.0;
+    UU = (dgrad > EPS) ? dgg * rec1 * rec22 / dgrad : 0.0;
   }
   double ec = 0, vcup = 0, vcdn = 0, dec = 0, dvcup = 0, dvcdn = 0;
   if (P.idftyp[1] == 6) {
@@ -340,10 +338,19 @@ __device__ __forceinline__ void xc_point_sic(const XCParams& P, const double r[1
   } else {
     xc_pbecor(rs, zet, T, UU, VV, WW, ec, vcup, vcdn, dec, dvcup, dvcdn);
   }
-  e4[2] += ec * D * wgt;
-  e4[3] += dec * D * wgt;
+  ergcl += ec * D * wgt;
+  ergcn += dec * D * wgt;
   vup += vcup + dvcup;
   vdn += vcdn + dvcdn;
+}
+
+// Both: the spin-up/down potentials; adds ERGXL, ERGXN, ERGCL, ERGCN contributions.
+__device__ __forceinline__ void xc_point_sic(const XCParams& P, const double r[10], double wgt, double& vup,
+                                             double& vdn, double e4[4]) {
+  double cup;
+  const double vx = xc_point_exchange(P, r, wgt, e4[0], e4[1]);
+  xc_point_correlation(P, r, wgt, cup, vdn, e4[2], e4[3]);
+  vup = vx + cup;
 }
 
 }  // namespace flosic
