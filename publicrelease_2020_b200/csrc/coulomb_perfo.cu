@@ -834,15 +834,17 @@ __device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp
   count_add(J.cnt_perfo, 0, far, terms);
 }
 
+// Three CTAs per SM in FP32 (80 registers; benzene beside the near field 22.9 -> 21.6
+// ms); in FP64 that limit spills and slows both fields (24.8 -> 31.4 ms).
 template <int FOS, bool MIXED>
-__global__ void __launch_bounds__(far_threads(FOS)) k_perfo_far(const __grid_constant__ CoulombJob J) {
+__global__ void __launch_bounds__(far_threads(FOS), MIXED ? 3 : 2) k_perfo_far(const __grid_constant__ CoulombJob J) {
   far_block<FOS, MIXED>(J, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // items[i] = {job, tile, FO block of fob FOs, 0}; blockIdx.y: group of FAR_FOS FOs of the block,
 // blockIdx.z: part.
 template <bool MIXED>
-__global__ void __launch_bounds__(far_threads(FAR_FOS))
+__global__ void __launch_bounds__(far_threads(FAR_FOS), MIXED ? 3 : 2)
 k_perfo_far_batch(const CoulombJob* __restrict__ jobs, const int4* __restrict__ items, int fob) {
   __shared__ CoulombJob J;
   const int4 w = items[blockIdx.x];
