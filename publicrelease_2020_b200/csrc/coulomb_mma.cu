@@ -616,8 +616,8 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
   launch_coulomb_classify(ncalls, calls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
   if (!per_fo_only && mixed && cfg.shared_tc) {
     const size_t nc = (size_t)npairs * nfo * COEF_LD, nm = (size_t)ncalls * nfo * MOM_LD;
-    launch_split_tf32((size_t)npairs, nfo, coef, scr.coef_hl, st);
-    launch_split_tf32((size_t)ncalls, nfo, momv, scr.momv_hl, st);
+    launch_split_tf32((size_t)npairs, nfo, scr.share, pairs, coef, scr.coef_hl, st);
+    launch_split_tf32((size_t)ncalls, nfo, scr.share, nullptr, momv, scr.momv_hl, st);
     const cudaError_t e = launch_coulomb_shared_tc(ncalls, scr.lists, scr.share, calls, nfo, scr.coef_hl, nc,
                                                    scr.pair_fmt, pairs, scr.momv_hl, nm, M, boys_tab, vh, ldv, cnt,
                                                    scr.err, cfg.wait_limit, st);

@@ -309,6 +309,16 @@ k_coulomb_shared_tc(int ncalls, const int* __restrict__ lists, const CallShare* 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int p0 = tile * TILE;
   const int np = min(TILE, M.n - p0);
+  // no shared-geometry call (NSPN=2): the tile is zero and nothing below has
+  // work, so the block writes it and leaves before any barrier or tensor memory.
+  // The idle pipeline took 1.9 of 27.2 ms of a benzene cycle (merged spins) and
+  // 2 of 4.2 ms of water's.
+  if (lists[2 * ncalls] == 0) {
+    const int col = tid & (TILE - 1);
+    if (col < np)
+      for (int k = tid / TILE; k < nk; k += TC_THREADS / TILE) vh[(size_t)(k0 + k) * ldv + p0 + col] = 0.0;
+    return;
+  }
   volatile int* abort = &S.abort;
   for (int i = tid; i < TILE; i += TC_THREADS) {
     const bool a = i < np;
@@ -653,19 +663,23 @@ k_coulomb_shared_tc(int ncalls, const int* __restrict__ lists, const CallShare* 
 // hi/lo TF32 split of rows [nrow][nfo][KSEG] doubles into the chunk-major
 // layout the producers copy from, [nrow][KSEG/4][nfo][4] floats (hi at out,
 // lo at out + part): the 128 FOs' values of one 4-row chunk are contiguous, so
-// a warp's copies of a chunk are coalesced.
-__global__ void k_split_tf32(size_t nrow, int nfo, const double* __restrict__ src, float* __restrict__ out,
-                             size_t part) {
-  const size_t n = nrow * nfo * KSEG;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = i / ((size_t)nfo * KSEG);
-    const int k = (int)((i / KSEG) % nfo), t = (int)(i % KSEG);
-    const double x = src[i];
-    const float hi = tf32_round((float)x);
-    const float lo = tf32_round((float)(x - (double)hi));
-    const size_t o = ((r * (KSEG / 4) + t / 4) * nfo + k) * 4 + (t & 3);
-    out[o] = hi;
-    out[part + o] = lo;
+// a warp's copies of a chunk are coalesced.  Only rows of shared calls are read
+// there: the others are left out (pairs = nullptr: row = call, else row = pair).
+__global__ void k_split_tf32(size_t nrow, int nfo, const CallShare* __restrict__ share,
+                             const PairGeo* __restrict__ pairs, const double* __restrict__ src,
+                             float* __restrict__ out, size_t part) {
+  const int w = nfo * KSEG;
+  for (size_t r = blockIdx.x; r < nrow; r += gridDim.x) {
+    if (!share[pairs ? pairs[r].call : (int)r].shared) continue;
+    for (int i = threadIdx.x; i < w; i += blockDim.x) {
+      const int k = i / KSEG, t = i % KSEG;
+      const double x = src[r * w + i];
+      const float hi = tf32_round((float)x);
+      const float lo = tf32_round((float)(x - (double)hi));
+      const size_t o = ((r * (KSEG / 4) + t / 4) * nfo + k) * 4 + (t & 3);
+      out[o] = hi;
+      out[part + o] = lo;
+    }
   }
 }
 
@@ -673,11 +687,11 @@ void init_coulomb_tc() {
   cudaFuncSetAttribute(k_coulomb_shared_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
 }
 
-void launch_split_tf32(size_t nrow, int nfo, const double* src, float* out, cudaStream_t st) {
-  const size_t n = nrow * nfo * KSEG;
-  if (n == 0) return;
-  const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-  k_split_tf32<<<blocks, 256, 0, st>>>(nrow, nfo, src, out, n);
+void launch_split_tf32(size_t nrow, int nfo, const CallShare* share, const PairGeo* pairs, const double* src,
+                       float* out, cudaStream_t st) {
+  if (nrow == 0 || nfo == 0) return;
+  const int blocks = (int)std::min<size_t>(nrow, 148 * 16);
+  k_split_tf32<<<blocks, 256, 0, st>>>(nrow, nfo, share, pairs, src, out, nrow * nfo * KSEG);
 }
 
 namespace {

@@ -173,7 +173,8 @@ void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, i
 void init_coulomb_tc();
 // TF32 hi/lo split of nrow x nfo rows of KSEG doubles into the chunk-major
 // [nrow][KSEG/4][nfo][4] layout (hi, then lo at + nrow*nfo*KSEG floats).
-void launch_split_tf32(size_t nrow, int nfo, const double* src, float* out, cudaStream_t st);
+void launch_split_tf32(size_t nrow, int nfo, const CallShare* share, const PairGeo* pairs, const double* src,
+                       float* out, cudaStream_t st);
 // Mixed-precision shared-geometry Coulomb GEMM on tcgen05 (csrc/coulomb_tc.cu);
 // the A rows reach shared memory by TMA through tensor maps built here.
 cudaError_t launch_coulomb_shared_tc(int ncalls, const int* lists, const CallShare* share, const CallInfo* calls,
