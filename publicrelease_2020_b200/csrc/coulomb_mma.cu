@@ -192,20 +192,37 @@ __device__ __forceinline__ void copy_rows(double* dst, int off, int nrow, int ro
 }
 
 // Consumer MMA over one stage: V[k][p] += A[k][0:rows] B[0:rows][p] for the
-// warp's 32 x WPTS tile; m-tiles with mt_active false are skipped.
-template <int NT>
+// warp's NMT 8-FO tiles wm, wm + WM, ... and its 8-point tiles wn, wn + WN, ...
+// (interleaved, so that the warps share a ragged FO block or a partly dead point
+// tile evenly).  A point tile without a point of the segment's kind is skipped
+// (live: per group of 4 rows, one byte per producer warp, one bit per point
+// tile): on tiles cut by a call's sphere both the near and the far segment run,
+// a quarter of all MMAs for zero columns.  Each point tile has a loop of its own
+// over the rows of equal mask, and NMT is known at compile time, because a
+// skipped MMA that the compiler predicates off still takes its slot of the pipe.
+// 128 FOs, 100,003 points: 83.0 ms without masks, 70.3 with masks inside the
+// k loop, 65.5 this way; 75 FOs, 30,001 points: 23.0, 18.2, 14.3.
+template <int NMT, int NT, int WM, int WN>
 __device__ __forceinline__ void stage_mma(double (&V)[4][NT][2], const double* __restrict__ As,
-                                          const double* __restrict__ Bs, int rows, const bool (&mt_active)[4]) {
-  for (int kk = 0; kk < rows; kk += 4) {
-    double af[4];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt) af[mt] = As[mt * 8 * KSEG + kk];
+                                          const double* __restrict__ Bs, const uint32_t* __restrict__ live, int wn,
+                                          int rows) {
+  for (int k0 = 0, k1; k0 < rows; k0 = k1) {
+    const uint32_t lv = live[k0 >> 2];
+    for (k1 = k0 + 4; k1 < rows && live[k1 >> 2] == lv;) k1 += 4;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      const double bf = Bs[(size_t)kk * G_LD + nt * 8];
+      const int pt = nt * WN + wn;
+      if (!((lv >> (8 * (pt >> 2) + (pt & 3))) & 1u)) continue;
+#pragma unroll 4
+      for (int kk = k0; kk < k1; kk += 4) {
+        const double bf = Bs[(size_t)kk * G_LD + nt * WN * 8];
+        double af[NMT];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-        if (mt_active[mt]) dmma884(V[mt][nt][0], V[mt][nt][1], af[mt], bf);
+        for (int mt = 0; mt < NMT; ++mt) af[mt] = As[mt * WM * 8 * KSEG + kk];
+#pragma unroll
+        for (int mt = 0; mt < NMT; ++mt)
+          dmma884(V[mt][nt][0], V[mt][nt][1], af[mt], bf);
+      }
     }
   }
 }
@@ -247,6 +264,7 @@ struct SharedSmem {
   double A[2][32 * WM * KSEG];  // FO rows of the stage's coefficients / moments
   double B[2][KSEG * G_LD];     // G or H columns
   double px[TILE], py[TILE], pz[TILE];
+  uint32_t live[2][KSEG / 4];   // 8-point tiles with a near / far point, per group of 4 rows
   int rows[2];                  // rows of the stage in each buffer, -1 = end
 };
 
@@ -261,7 +279,7 @@ __device__ __forceinline__ void shared_tile(int tile, int fob, int ncalls, const
                                             const double* __restrict__ momv, const MeshDev& M,
                                             const double* __restrict__ boys_tab, double* __restrict__ vh, int ldv,
                                             unsigned long long* __restrict__ cnt) {
-  constexpr int FOB = 32 * WM, WN = CONS_WARPS / WM, WPTS = TILE / WN, NT = WPTS / 8;
+  constexpr int FOB = 32 * WM, WN = CONS_WARPS / WM, NT = TILE / WN / 8;
   using PT = typename std::conditional<MIXED, float, double>::type;  // producer arithmetic
   extern __shared__ __align__(128) unsigned char smraw[];
   SharedSmem<WM>& S = *reinterpret_cast<SharedSmem<WM>*>(smraw);
@@ -321,23 +339,30 @@ __device__ __forceinline__ void shared_tile(int tile, int fob, int ncalls, const
         const int p = pt + j * NPROD;
         double* g = &S.B[b][(size_t)off * G_LD + p];
         const double x = S.px[p], y = S.py[p], z = S.pz[p];
+        double r2 = 0.0;
+        bool on = p < np;
+        if (on && (s.far || s.cls == 2)) {
+          r2 = sqdist_rn2(x, y, z, s.cx, s.cy, s.cz);
+          if (s.cls == 2) on = (r2 > s.rc2) == (s.far != 0);
+        }
+        // which of the warp's four 8-point tiles have such a point
+        const unsigned any = __ballot_sync(0xffffffffu, on);
+        const int wl = pt & 31;
+        if (4 * wl < s.rows) {
+          const unsigned t4 = ((any & 0xffu) ? 1u : 0u) | ((any & 0xff00u) ? 2u : 0u) |
+                              ((any & 0xff0000u) ? 4u : 0u) | ((any & 0xff000000u) ? 8u : 0u);
+          reinterpret_cast<unsigned char*>(&S.live[b][(off >> 2) + wl])[p >> 5] = (unsigned char)t4;
+        }
+        if (!((any >> (wl & 24)) & 0xffu)) continue;  // a dead tile's columns are not read
         if (!s.far) {
-          bool nr = p < np;
-          if (nr && s.cls == 2) nr = !(sqdist_rn2(x, y, z, s.cx, s.cy, s.cz) > s.rc2);
-          if (nr) {
+          if (on) {
             ++my_near;
             write_g_point<PT>(g, s.rows, pairs[s.idx], x, y, z, boys_tab);
           } else {
             zero_rows(g, s.rows);
           }
         } else {
-          double r2 = 0.0;
-          bool fr = p < np;
-          if (fr) {
-            r2 = sqdist_rn2(x, y, z, s.cx, s.cy, s.cz);
-            if (s.cls == 2) fr = r2 > s.rc2;
-          }
-          if (fr) {
+          if (on) {
             ++my_far;
             if (count_terms) my_terms += (unsigned long long)s.ksum;
             write_h<PT>(g, s.rows, PT(x - s.cx), PT(y - s.cy), PT(z - s.cz), PT(r2));
@@ -356,28 +381,32 @@ __device__ __forceinline__ void shared_tile(int tile, int fob, int ncalls, const
     for (int a = 0; a < 4; ++a)
 #pragma unroll
       for (int b = 0; b < NT; ++b) V[a][b][0] = V[a][b][1] = 0.0;
-    bool mt_active[4];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt) mt_active[mt] = wm * 32 + mt * 8 < nk;
+    const int nmt = min(4, max(0, ((nk + 7) / 8 - wm + WM - 1) / WM));  // m-tiles with an FO
     for (int qi = 0;; ++qi) {
       const int b = qi & 1;
       named_sync(BAR_FULL + b);
       const int r = S.rows[b];
       if (r > 0)
-        stage_mma(V, &S.A[b][(wm * 32 + (lane >> 2)) * KSEG + (lane & 3)],
-                  &S.B[b][(lane & 3) * G_LD + wn * WPTS + (lane >> 2)], r, mt_active);
+      {
+        const double* As = &S.A[b][(wm * 8 + (lane >> 2)) * KSEG + (lane & 3)];
+        const double* Bs = &S.B[b][(lane & 3) * G_LD + wn * 8 + (lane >> 2)];
+        if (nmt == 4) stage_mma<4, NT, WM, WN>(V, As, Bs, S.live[b], wn, r);
+        else if (nmt == 3) stage_mma<3, NT, WM, WN>(V, As, Bs, S.live[b], wn, r);
+        else if (nmt == 2) stage_mma<2, NT, WM, WN>(V, As, Bs, S.live[b], wn, r);
+        else if (nmt == 1) stage_mma<1, NT, WM, WN>(V, As, Bs, S.live[b], wn, r);
+      }
       named_arrive(BAR_EMPTY + b);
       if (r < 0) break;
     }
 #pragma unroll
     for (int mt = 0; mt < 4; ++mt) {
-      const int k = wm * 32 + mt * 8 + (lane >> 2);
+      const int k = (mt * WM + wm) * 8 + (lane >> 2);
       if (k >= nk) continue;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const int p = wn * WPTS + nt * 8 + 2 * (lane & 3) + i;
+          const int p = (nt * WN + wn) * 8 + 2 * (lane & 3) + i;
           if (p < np) vh[(size_t)(k0 + k) * ldv + p0 + p] = V[mt][nt][i];
         }
     }
@@ -391,9 +420,28 @@ k_coulomb_shared(int ncalls, const int* __restrict__ lists, const CallShare* __r
                  const CallInfo* __restrict__ calls, int nfo, const double* __restrict__ coef,
                  const int8_t* __restrict__ pair_fmt, const PairGeo* __restrict__ pairs,
                  const double* __restrict__ momv, MeshDev M, const double* __restrict__ boys_tab,
-                 double* __restrict__ vh, int ldv, unsigned long long* __restrict__ cnt) {
-  shared_tile<WM, MIXED>(blockIdx.x, blockIdx.y, ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M,
-                         boys_tab, vh, ldv, cnt);
+                 double* __restrict__ vh, int ldv, unsigned long long* __restrict__ cnt, int whole, int cut) {
+  // blocks [0, whole): one (tile, FO block); the rest: 1/cut of a tile's FO block
+  const int bid = blockIdx.x, item = bid < whole ? bid : whole + (bid - whole) / cut;
+  const int tile = item % M.ntiles, fob = item / M.ntiles, sub = bid < whole ? 0 : (bid - whole) % cut;
+  if constexpr (WM >= 4) {
+    if (bid >= whole && cut == 4) {
+      if (fob * 4 * 32 + sub * 32 < nfo)
+        shared_tile<WM / 4, MIXED>(tile, 4 * fob + sub, ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv,
+                                   M, boys_tab, vh, ldv, cnt);
+      return;
+    }
+  }
+  if constexpr (WM >= 2) {
+    if (bid >= whole && cut == 2) {
+      if ((fob * 2 + sub) * 16 * WM < nfo)
+        shared_tile<WM / 2, MIXED>(tile, 2 * fob + sub, ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv,
+                                   M, boys_tab, vh, ldv, cnt);
+      return;
+    }
+  }
+  shared_tile<WM, MIXED>(tile, fob, ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh,
+                         ldv, cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -567,13 +615,21 @@ static void launch_shared(int ncalls, const int* lists, const CallShare* share, 
                           const double* coef, const int8_t* pair_fmt, const PairGeo* pairs, const double* momv,
                           const MeshDev& M, const double* boys_tab, double* vh, int ldv, unsigned long long* cnt,
                           bool mixed, cudaStream_t st) {
-  dim3 grid(M.ntiles, (nfo + 32 * WM - 1) / (32 * WM));
+  // The last wave: when it fills at most half (a quarter) of the SMs, its tiles
+  // are given out as halves (quarters) of their FOs, each the same sums.  A half
+  // builds the same columns, so a fuller wave would gain nothing.  128 FOs, 782
+  // tiles (42 in the last wave): 65.5 -> 63.4 ms.
+  const int items = M.ntiles * ((nfo + 32 * WM - 1) / (32 * WM)), tail = items % 148;
+  int cut = 1;
+  if (tail > 0 && WM >= 2 && 2 * tail <= 148) cut = WM >= 4 && 4 * tail <= 148 ? 4 : 2;
+  const int whole = cut > 1 ? items - tail : items;
+  const int grid = whole + cut * (items - whole);
   if (mixed)
     k_coulomb_shared<WM, true><<<grid, WS_THREADS, sizeof(SharedSmem<WM>), st>>>(
-        ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh, ldv, cnt);
+        ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh, ldv, cnt, whole, cut);
   else
     k_coulomb_shared<WM, false><<<grid, WS_THREADS, sizeof(SharedSmem<WM>), st>>>(
-        ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh, ldv, cnt);
+        ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh, ldv, cnt, whole, cut);
 }
 
 void launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
