@@ -242,7 +242,8 @@ constexpr int FV_KC = 32;                // basis functions per stage (one atom,
 constexpr int FV_CONS = 256;             // 8 consumer warps, 32 FO columns each
 constexpr int FV_PROD = 256;             // 8 producer warps
 constexpr int FV_THREADS = FV_CONS + FV_PROD;
-constexpr int FV_BAR_FULL = 1, FV_BAR_EMPTY = 3, FV_BAR_PROD = 5;  // named barriers 1-2, 3-4, 5
+constexpr int FV_BAR_FULL = 1, FV_BAR_EMPTY = 3, FV_BAR_PROD = 5;  // named barriers 1-2, 3-4, 5-6
+constexpr int FV_ATOMS = 1024;           // atoms screened at a time
 
 // A CTA's product: ROWS = NCH x BP rows of (channel, point) by BN FO columns.
 // BN = 64: 4 warp rows x 2 warp columns; BN = 128: half the points, 2 x 4, so
@@ -257,18 +258,26 @@ struct FoValShape {
   static constexpr int MTW = ROWS / 8 / WR;             // m-tiles per consumer warp
   static constexpr int LDR = ROWS + 4;
   static constexpr int GA = BP <= 32 ? 4 : 2;           // atoms per stage at most (their exponentials in smem)
+  // Producer groups: with two, each builds every other stage, so the chain of
+  // dependent phases behind a stage (exponentials, radial sums, Cartesian
+  // factors; a few thousand cycles for 16 points) overlaps the other group's.
+  // Values alone (128 points a stage, less work per point, no room for a second
+  // set of exponentials) keep one.
+  static constexpr int NG = NDERV == 0 ? 1 : 2;
+  static constexpr int GT = FV_PROD / NG;               // threads of a group
+  static constexpr int NB = NG == 1 ? 3 : 4;            // coefficient buffers
 };
 
 template <int NDERV, int BN>
 struct FoValSmem {
   using S = FoValShape<NDERV, BN>;
   double As[2][FV_KC][S::LDR];     // basis values: k = function, row = channel * BP + point
-  double Bs[3][FV_KC][BN + 4];     // coefficients: k = function, column = FO (stage qi in Bs[qi % 3])
-  double g[S::GA][S::BP][MAX_BARE];  // exp(-alpha r^2) of each stage atom's bare primitives
-  double rel[S::GA][S::BP][3];       // point - atom centre
+  double Bs[S::NB][FV_KC][BN + 4];  // coefficients: k = function, column = FO (stage qi in Bs[qi % NB])
+  double g[S::NG][S::GA][S::BP][MAX_BARE];  // exp(-alpha r^2) of each stage atom's bare primitives
+  double rel[S::NG][S::GA][S::BP][3];       // point - atom centre
   double px[S::BP], py[S::BP], pz[S::BP];
   int kpad[2];                     // k rows of the stage in each buffer, -1 = end
-  unsigned near[3];                // per window of atoms (mod 3): bit j set when atom j has a point in range
+  unsigned near[S::NG][FV_ATOMS / 32];  // atoms that some point is in range of
 };
 
 __device__ __forceinline__ void fv_bar_sync(int id, int n) {
@@ -316,18 +325,17 @@ __device__ __forceinline__ void fv_function(int a, int b, int cz, double R0, dou
   }
 }
 
-// The Cartesian components of one contraction of angular momentum L (s; x y z;
-// xx yy zz xy xz yz, the order of gorbdrv.f) whose function index lies in the
-// stage: component mu is function fbase + mu * ncon of the stage.
-template <int NDERV, int L>
+// Cartesian components MU0 .. MU1-1 of one contraction of angular momentum L (s;
+// x y z; xx yy zz xy xz yz, the order of gorbdrv.f) whose function index lies in
+// the stage: component mu is function fbase + mu * ncon of the stage.
+template <int NDERV, int L, int MU0, int MU1>
 __device__ __forceinline__ void fv_contraction(double R0, double R1, double R2, const double* xyz, double* As_b,
                                                int ldr, int bp, int i, int fbase, int ncon, int nfc) {
-  constexpr int NCOMP = L == 0 ? 1 : (L == 1 ? 3 : 6);
   constexpr int SHIFT = L == 0 ? 0 : (L == 1 ? 1 : 4);
   constexpr int PW[10][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0},
                              {0, 2, 0}, {0, 0, 2}, {1, 1, 0}, {1, 0, 1}, {0, 1, 1}};
 #pragma unroll
-  for (int mu = 0; mu < NCOMP; ++mu) {
+  for (int mu = MU0; mu < MU1; ++mu) {
     const int fi = fbase + mu * ncon;
     if (fi < 0 || fi >= nfc) continue;
     fv_function<NDERV>(PW[SHIFT + mu][0], PW[SHIFT + mu][1], PW[SHIFT + mu][2], R0, R1, R2, xyz,
@@ -336,13 +344,20 @@ __device__ __forceinline__ void fv_contraction(double R0, double R1, double R2, 
 }
 
 // out[(ch * ncol + k) * ldo + p] = sum_f B_ch(p, f) coef[k * ldc + f] for the
-// npts points (px, py, pz) and ncol columns of coef.  Warp specialised: four
-// producer warps form the basis values of one atom (or 32 of its functions)
-// and its coefficient rows into one of two stage buffers while eight consumer
-// warps multiply the other on the FP64 tensor cores.  Stage hand-over by named
-// barriers FULL+b (producers arrive, consumers wait) and EMPTY+b (consumers
-// arrive, producers wait before refilling); every stage, including the final
-// end marker, is waited on exactly once on each side.
+// npts points (px, py, pz) and ncol columns of coef.  Warp specialised: eight
+// producer warps in NG groups form the basis values of up to 32 functions and
+// their coefficient rows into one of two stage buffers while eight consumer
+// warps multiply the other on the FP64 tensor cores.  Every group walks all
+// atoms and builds the stages qi with qi % NG equal to its number, so with two
+// groups each owns a buffer.  Stage hand-over by named barriers FULL+b (the
+// group arrives, consumers wait) and EMPTY+b (consumers arrive, the group waits
+// before refilling); every stage, including the final end marker, is waited on
+// exactly once on each side.
+//
+// Bound by the producers' issue: 40 atoms, 512 functions, 128 FOs, 100,003
+// points with second derivatives took 9.47 ms against 4.0 of FP64 MMAs.  Two
+// groups: 7.98; items by kind, longest first, d in halves: 7.74; coefficient
+// rows without a division and a row search per element: 6.96.
 template <int NDERV, int BN>
 __global__ void __launch_bounds__(FV_THREADS, 1)
 k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* __restrict__ py,
@@ -360,27 +375,29 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
     sm.py[i] = v ? py[p0 + i] : 0.0;
     sm.pz[i] = v ? pz[p0 + i] : 0.0;
   }
-  if (tid < 3) sm.near[tid] = 0;
   __syncthreads();
 
+  constexpr int HAND = FV_CONS + S::GT;  // threads of a hand-over
   if (warp >= FV_CONS / 32) {
     // ---------------- producers
-    const int pt = tid - FV_CONS;
-    int qi = 0;  // stages handed over
+    const int grp = (tid - FV_CONS) / S::GT, pt = (tid - FV_CONS) % S::GT;
+    int qi = 0;  // stages before the current one, of every group
+    auto mine = [&]() { return qi % S::NG == grp; };
     auto begin = [&](int b) {
-      if (qi >= 2) fv_bar_sync(FV_BAR_EMPTY + b, FV_THREADS);
+      if (qi >= 2) fv_bar_sync(FV_BAR_EMPTY + b, HAND);
     };
     auto finish = [&](int b, int kp) {
       if (pt == 0) sm.kpad[b] = kp;
-      fv_bar_arrive(FV_BAR_FULL + b, FV_THREADS);
-      ++qi;
+      fv_bar_arrive(FV_BAR_FULL + b, HAND);
     };
+    auto group_sync = [&]() { fv_bar_sync(FV_BAR_PROD + grp, S::GT); };
     // The atoms go to the tensor cores in stages of up to 32 basis functions:
     // consecutive atoms that some point of the block reaches (primitive
     // screen of gorbdrv.f:186-195; the others' values are all zero) are
     // packed into one stage while they fit, at most GA of them; an atom with
     // more than 32 functions takes stages of its own, 32 functions each.
     constexpr int GA = S::GA;
+    constexpr bool HALVES = NDERV == 2;
     struct Member {
       int atom, type, nbare, nc0, nc1, nc2, nfa, boff, off;
       double ax, ay, az, amin;
@@ -404,21 +421,27 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
       return m;
     };
     // coefficient rows of the stage (function fi of the stage is row
-    // row_of(fi) of coef) into Bs[qi % 3] by cp.async (zero outside the
+    // row_of(fi) of coef) into Bs[qi % NB] by cp.async (zero outside the
     // matrix); issued early so their latency overlaps the basis values.
-    // Bs[qi % 3] was last read by stage qi - 3, which the consumers released
-    // before the producers passed begin() of stage qi - 1.
+    // Bs[qi % NB] was last read by stage qi - NB, which the consumers released
+    // before the group passed begin() of its previous stage qi - NG.
+    // A lane takes one function: its row is worked out once for all columns.
     auto fetch_coef = [&](int q, int nfc, int kp, auto row_of) {
-      for (int e = pt; e < kp * BN; e += FV_PROD) {
-        const int n = e / kp, fi = e - n * kp;
-        const bool v = fi < nfc && n0 + n < ncol;
-        cp_async8(&sm.Bs[q % 3][fi][n], v ? coef + (size_t)(n0 + n) * ldc + row_of(fi) : coef, v);
+      const int fi = pt & 31;
+      if (fi < kp) {
+        const bool v = fi < nfc;
+        const double* src = coef + (v ? row_of(fi) : 0);
+        double* dst = &sm.Bs[q % S::NB][fi][0];
+        for (int n = pt >> 5; n < BN; n += S::GT / 32) {
+          const bool w = v && n0 + n < ncol;
+          cp_async8(dst + n, w ? src + (size_t)(n0 + n) * ldc : coef, w);
+        }
       }
       cp_commit();
     };
     // exp(-alpha r^2) of member slot ms at the block's points
     auto exps = [&](int ms, const Member& m) {
-      for (int e = pt; e < S::BP * m.nbare; e += FV_PROD) {
+      for (int e = pt; e < S::BP * m.nbare; e += S::GT) {
         const int i = e / m.nbare, ib = e - i * m.nbare;
         const double x = sm.px[i] - m.ax, y = sm.py[i] - m.ay, z = sm.pz[i] - m.az;
         const double r2 = x * x + y * y + z * z;
@@ -427,24 +450,24 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
           const double rex = B.type_alpha[m.type * MAX_BARE + ib] * r2;
           v = (rex < CUTEXP) ? exp(-rex) : 0.0;
         }
-        sm.g[ms][i][ib] = v;
+        sm.g[grp][ms][i][ib] = v;
         if (ib == 0) {
-          sm.rel[ms][i][0] = x;
-          sm.rel[ms][i][1] = y;
-          sm.rel[ms][i][2] = z;
+          sm.rel[grp][ms][i][0] = x;
+          sm.rel[grp][ms][i][1] = y;
+          sm.rel[grp][ms][i][2] = z;
         }
       }
     };
-    // one item per (point, contraction of member slot ms): its radial sums,
-    // then the components whose stage column fbase + mu * ncon lies in [0, nfc)
-    auto item = [&](int ms, const Member& m, int lc, int i, int f0, double* As_b, int nfc) {
-      const int l = lc < m.nc0 ? 0 : (lc < m.nc0 + m.nc1 ? 1 : 2);
-      const int c = lc - (l == 0 ? 0 : (l == 1 ? m.nc0 : m.nc0 + m.nc1));
+    // one item per (point, contraction of member slot ms; kinds: s, p, d or the
+    // two halves of d): its radial sums, then the components whose stage column
+    // fbase + mu * ncon lies in [0, nfc)
+    auto item = [&](int ms, const Member& m, int kind, int c, int i, int f0, double* As_b, int nfc) {
+      const int l = min(kind, 2);
       const double* con = B.type_bfcon + ((size_t)(m.type * 3 + l) * MAX_CON + c) * MAX_BARE;
       const double* alp = B.type_alpha + m.type * MAX_BARE;
       double R0 = 0.0, R1 = 0.0, R2 = 0.0;
       for (int ib = 0; ib < m.nbare; ++ib) {
-        const double cg = con[ib] * sm.g[ms][i][ib];
+        const double cg = con[ib] * sm.g[grp][ms][i][ib];
         R0 += cg;
         if (NDERV > 0) {
           const double a2 = 2.0 * alp[ib];
@@ -452,48 +475,81 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
           if (NDERV > 1) R2 += cg * a2 * a2;
         }
       }
-      const int base = m.off - f0;
-      if (l == 0) fv_contraction<NDERV, 0>(R0, R1, R2, sm.rel[ms][i], As_b, S::LDR, S::BP, i, base + c, m.nc0, nfc);
-      else if (l == 1)
-        fv_contraction<NDERV, 1>(R0, R1, R2, sm.rel[ms][i], As_b, S::LDR, S::BP, i, base + m.nc0 + c, m.nc1, nfc);
-      else
-        fv_contraction<NDERV, 2>(R0, R1, R2, sm.rel[ms][i], As_b, S::LDR, S::BP, i, base + m.nc0 + 3 * m.nc1 + c,
-                                 m.nc2, nfc);
+      const int base = m.off - f0, bp1 = base + m.nc0 + c, bp2 = base + m.nc0 + 3 * m.nc1 + c;
+      const double* rel = sm.rel[grp][ms][i];
+      if (kind == 0) fv_contraction<NDERV, 0, 0, 1>(R0, R1, R2, rel, As_b, S::LDR, S::BP, i, base + c, m.nc0, nfc);
+      else if (kind == 1) fv_contraction<NDERV, 1, 0, 3>(R0, R1, R2, rel, As_b, S::LDR, S::BP, i, bp1, m.nc1, nfc);
+      else if (kind == 2)
+        fv_contraction<NDERV, 2, 0, HALVES ? 3 : 6>(R0, R1, R2, rel, As_b, S::LDR, S::BP, i, bp2, m.nc2, nfc);
+      else if (HALVES) fv_contraction<NDERV, 2, 3, 6>(R0, R1, R2, rel, As_b, S::LDR, S::BP, i, bp2, m.nc2, nfc);
+    };
+    // the items of members [0, ng) over the group's threads, the longest first:
+    // d (in halves), p, s, so that a warp has one kind and the rounds are even
+    auto items = [&](const Member* mem, int ng, int f0, double* As_b, int nfc) {
+      int n2 = 0, n1 = 0, n0 = 0;
+      for (int k = 0; k < ng; ++k) {
+        n2 += mem[k].nc2;
+        n1 += mem[k].nc1;
+        n0 += mem[k].nc0;
+      }
+      const int nd = HALVES ? 2 * n2 : n2;
+      for (int e = pt; e < S::BP * (nd + n1 + n0); e += S::GT) {
+        const int i = e % S::BP;
+        int c = e / S::BP, kind = 2;
+        if (c >= nd + n1) {
+          c -= nd + n1;
+          kind = 0;
+        } else if (c >= nd) {
+          c -= nd;
+          kind = 1;
+        } else if (c >= n2) {
+          c -= n2;
+          kind = 3;
+        }
+        int k = 0;
+        for (; k + 1 < ng; ++k) {
+          const int nc = kind == 0 ? mem[k].nc0 : (kind == 1 ? mem[k].nc1 : mem[k].nc2);
+          if (c < nc) break;
+          c -= nc;
+        }
+        item(k, mem[k], kind, c, i, f0, As_b, nfc);
+      }
     };
     auto pad_rows = [&](int b, int nfc, int kp) {  // zero rows up to the k-step of 4
-      for (int e = pt; e < S::BP * (kp - nfc); e += FV_PROD) {
+      for (int e = pt; e < S::BP * (kp - nfc); e += S::GT) {
         const int fi = nfc + e / S::BP, i = e % S::BP;
 #pragma unroll
         for (int ch = 0; ch < S::NCH; ++ch) sm.As[b][fi][ch * S::BP + i] = 0.0;
       }
     };
-    int win = 0;
+    int scr0 = 0, scr1 = 0;  // atoms [scr0, scr1) are screened
     for (int a = 0; a < B.natoms;) {
-      // screen the window a .. a + GA - 1; every producer passed the previous
-      // stage's items, so g and rel may be rewritten after this barrier
       const int wn = min(GA, B.natoms - a);
-      unsigned bits = 0;
-      for (int j = 0; j < wn; ++j) {
-        const int at = a + j;
-        const int t = B.atom_type[at];
-        const double ax = B.atom_pos[3 * at], ay = B.atom_pos[3 * at + 1], az = B.atom_pos[3 * at + 2];
-        const double amin = B.type_amin[t];
-        for (int i = pt; i < np; i += FV_PROD) {
-          const double x = sm.px[i] - ax, y = sm.py[i] - ay, z = sm.pz[i] - az;
-          if ((x * x + y * y + z * z) * amin < CUTEXP) bits |= 1u << j;
+      if (a + wn > scr1) {
+        // which of the next atoms have a point in range (each group for itself;
+        // its threads are past the previous screen's flags and, below, past the
+        // previous stage's g and rel)
+        scr0 = a;
+        scr1 = min(B.natoms, a + FV_ATOMS);
+        group_sync();
+        for (int j = pt; j < FV_ATOMS / 32; j += S::GT) sm.near[grp][j] = 0u;
+        group_sync();
+        for (int e = pt; e < (scr1 - scr0) * S::BP; e += S::GT) {
+          const int at = scr0 + e / S::BP, i = e % S::BP;
+          if (i >= np) continue;
+          const double x = sm.px[i] - B.atom_pos[3 * at], y = sm.py[i] - B.atom_pos[3 * at + 1],
+                       z = sm.pz[i] - B.atom_pos[3 * at + 2];
+          if ((x * x + y * y + z * z) * B.type_amin[B.atom_type[at]] < CUTEXP)
+            atomicOr(&sm.near[grp][(at - scr0) >> 5], 1u << ((at - scr0) & 31));
         }
+        group_sync();
       }
-      if (bits) atomicOr(&sm.near[win % 3], bits);
-      if (pt == 0) sm.near[(win + 1) % 3] = 0u;
-      fv_bar_sync(FV_BAR_PROD, FV_PROD);
-      const unsigned mask = sm.near[win % 3];
-      ++win;
       // the stage's atoms (the same on every producer)
       Member mem[GA];
       int ng = 0, tot = 0, next = a + wn;
       bool big = false;
       for (int j = 0; j < wn; ++j) {
-        if (!((mask >> j) & 1u)) continue;
+        if (!((sm.near[grp][(a + j - scr0) >> 5] >> ((a + j - scr0) & 31)) & 1u)) continue;
         Member m = member(a + j);
         if (m.nfa > FV_KC) {
           if (ng == 0) {
@@ -518,21 +574,29 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
       if (ng == 0) continue;
       if (big) {
         const Member& m = mem[0];
-        const int nlc = m.nc0 + m.nc1 + m.nc2;
-        fetch_coef(qi, min(FV_KC, m.nfa), (min(FV_KC, m.nfa) + 3) & ~3, [&](int fi) { return m.boff + fi; });
-        exps(0, m);
-        fv_bar_sync(FV_BAR_PROD, FV_PROD);
-        for (int f0 = 0; f0 < m.nfa; f0 += FV_KC) {
+        bool formed = false;  // the group's exponentials of this atom
+        for (int f0 = 0; f0 < m.nfa; f0 += FV_KC, ++qi) {
+          if (!mine()) continue;
           const int nfc = min(FV_KC, m.nfa - f0), kp = (nfc + 3) & ~3;
           const int b = qi & 1;
-          if (f0 > 0) fetch_coef(qi, nfc, kp, [&](int fi) { return m.boff + f0 + fi; });
+          fetch_coef(qi, nfc, kp, [&](int fi) { return m.boff + f0 + fi; });
+          if (!formed) {
+            group_sync();
+            exps(0, m);
+            group_sync();
+            formed = true;
+          }
           begin(b);
           double* As_b = &sm.As[b][0][0];
-          for (int e = pt; e < S::BP * nlc; e += FV_PROD) item(0, m, e / S::BP, e % S::BP, f0, As_b, nfc);
+          items(mem, 1, f0, As_b, nfc);
           pad_rows(b, nfc, kp);
           cp_wait<0>();  // this thread's coefficient copies have landed
           finish(b, kp);
         }
+        continue;
+      }
+      if (!mine()) {
+        ++qi;
         continue;
       }
       const int kp = (tot + 3) & ~3;
@@ -541,32 +605,25 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
         while (k + 1 < ng && fi >= mem[k + 1].off) ++k;
         return mem[k].boff + fi - mem[k].off;
       });
+      group_sync();
       for (int k = 0; k < ng; ++k) exps(k, mem[k]);
-      fv_bar_sync(FV_BAR_PROD, FV_PROD);
+      group_sync();
       const int b = qi & 1;
       begin(b);
       double* As_b = &sm.As[b][0][0];
-      // all members' items in one range, so that every producer has work
-      int start[GA + 1];
-      start[0] = 0;
-      for (int k = 0; k < ng; ++k) start[k + 1] = start[k] + S::BP * (mem[k].nc0 + mem[k].nc1 + mem[k].nc2);
-      for (int e = pt; e < start[ng]; e += FV_PROD) {
-        int k = 0;
-        while (e >= start[k + 1]) ++k;
-        const int r = e - start[k];
-        item(k, mem[k], r / S::BP, r % S::BP, 0, As_b, tot);
-      }
+      items(mem, ng, 0, As_b, tot);
       pad_rows(b, tot, kp);
       cp_wait<0>();
       finish(b, kp);
+      ++qi;
     }
     // end marker, then release of the last two stages
-    {
-      const int b = qi & 1;
-      begin(b);
-      finish(b, -1);
-      for (int j = max(qi - 2, 0); j < qi; ++j) fv_bar_sync(FV_BAR_EMPTY + (j & 1), FV_THREADS);
+    if (mine()) {
+      begin(qi & 1);
+      finish(qi & 1, -1);
     }
+    for (int j = max(qi - 1, 0); j <= qi; ++j)
+      if (j % S::NG == grp) fv_bar_sync(FV_BAR_EMPTY + (j & 1), HAND);
   } else {
     // ---------------- consumers
     const int wr = warp % S::WR, wc = warp / S::WR;
@@ -577,20 +634,20 @@ k_fo_values(BasisDev B, int npts, const double* __restrict__ px, const double* _
       for (int y = 0; y < 4; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
     for (int qi = 0;; ++qi) {
       const int b = qi & 1;
-      fv_bar_sync(FV_BAR_FULL + b, FV_THREADS);
+      fv_bar_sync(FV_BAR_FULL + b, HAND);
       const int kp = sm.kpad[b];
       for (int kk = 0; kk < kp; kk += 4) {
         double af[S::MTW], bf[4];
 #pragma unroll
         for (int mt = 0; mt < S::MTW; ++mt) af[mt] = sm.As[b][kk + (lane & 3)][(wr * S::MTW + mt) * 8 + (lane >> 2)];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) bf[nt] = sm.Bs[qi % 3][kk + (lane & 3)][wc * 32 + nt * 8 + (lane >> 2)];
+        for (int nt = 0; nt < 4; ++nt) bf[nt] = sm.Bs[qi % S::NB][kk + (lane & 3)][wc * 32 + nt * 8 + (lane >> 2)];
 #pragma unroll
         for (int mt = 0; mt < S::MTW; ++mt)
 #pragma unroll
           for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt][0], acc[mt][nt][1], af[mt], bf[nt]);
       }
-      fv_bar_arrive(FV_BAR_EMPTY + b, FV_THREADS);
+      fv_bar_arrive(FV_BAR_EMPTY + b, HAND);
       if (kp < 0) break;
     }
 #pragma unroll
