@@ -243,7 +243,7 @@ constexpr int FV_CONS = 256;             // 8 consumer warps, 32 FO columns each
 constexpr int FV_PROD = 256;             // 8 producer warps
 constexpr int FV_THREADS = FV_CONS + FV_PROD;
 constexpr int FV_BAR_FULL = 1, FV_BAR_EMPTY = 3, FV_BAR_PROD = 5;  // named barriers 1-2, 3-4, 5-6
-constexpr int FV_ATOMS = 1024;           // atoms screened at a time
+constexpr int FV_ATOMS = 64;             // atoms screened at a time
 
 // A CTA's product: ROWS = NCH x BP rows of (channel, point) by BN FO columns.
 // BN = 64: 4 warp rows x 2 warp columns; BN = 128: half the points, 2 x 4, so

@@ -24,9 +24,9 @@
 // one 384-thread CTA per 128 points with producer and consumer warps, spent 9-14
 // us per (call, tile) in CTA barriers, stage hand-overs and per-call FO status,
 // whatever the call's size; with NSPN=2 most calls are one 16-48-row pair.
-// Measured, FP64, both kernels: benzene (37,843 points, 21 + 21 FOs) 85.9 -> 35.2
-// ms, the 40-atom system (100,003 points, 128 FOs) 108 -> 66 ms (near 46, far
-// 20), water (3,942 points) 2.0 -> 0.8 ms.
+// Measured, FP64, both kernels: benzene (37,843 points, 21 + 21 FOs) 85.9 -> 24.5
+// ms (near 16.9, far 11.5 when alone; far on a side stream), the 40-atom system
+// (100,003 points, 128 FOs) 108 -> 62 ms, water (3,942 points) 2.0 -> 0.13 ms.
 #include <algorithm>
 
 #include "coulomb_common.cuh"
@@ -230,22 +230,28 @@ __device__ __forceinline__ void near_boys(const double* __restrict__ tab, T x, T
 }
 
 // Four k-steps of one group: two 16-byte fragment loads and four MMAs per eight
-// listed FOs.  A0, A1: the lane's two pieces of the first rows.
+// listed FOs.  A0, A1: the lane's two pieces of the first rows.  An entry lists at
+// least one FO, so the first eight need no test (benzene: 24.8 -> 24.5 ms, 128 FOs
+// and 100,003 points: 63.3 -> 62.2).
 template <int MT, typename T, int g>
 __device__ __forceinline__ void near_mma(double (&acc)[MT][2], const double* __restrict__ A0,
                                          const double* __restrict__ A1, int nmt, const NearLane<T>& L,
                                          const T (&F)[5], bool q0) {
   double b[4];
   near_group<T, g>(L, F, q0, b);
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    if (mt >= nmt) break;
+  auto step = [&](int mt) {
     const double2 a0 = *reinterpret_cast<const double2*>(A0 + mt * 128);
     const double2 a1 = *reinterpret_cast<const double2*>(A1 + mt * 128);
     dmma(acc[mt], a0.x, b[0]);
     dmma(acc[mt], a0.y, b[1]);
     dmma(acc[mt], a1.x, b[2]);
     dmma(acc[mt], a1.y, b[3]);
+  };
+  step(0);
+#pragma unroll
+  for (int mt = 1; mt < MT; ++mt) {
+    if (mt >= nmt) break;
+    step(mt);
   }
 }
 
