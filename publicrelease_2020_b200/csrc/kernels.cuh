@@ -209,6 +209,12 @@ void launch_fo_tau(int npts, int nfo, int k, const double* phi, int ldp, double*
 void launch_xc_mgga_rhog(const MeshDev& M, const double* rhog, int ldr, const double* tau, double* vxc,
                          double* mixin, double* part, int nblk, cudaStream_t st);
 
+// Products of the FO construction in the order of the host loops, and the FOD
+// force's matrix in the eigenbasis (contract.cu).
+void launch_ordered_product(int M, int N, int K, const double* A, int ai, int am, const double* B, int bj, int bm,
+                            const double* e, double* out, int ldo, cudaStream_t st);
+void launch_force_ham(int n, const double* G, const double* Q, double* out, cudaStream_t st);
+
 // Vxc of given density channels (GETVLXC entry point): vxc[2*n], parts as above (1 FO).
 // Dense products on the FP64 tensor cores (csrc/contract.cu).
 // dgemm: C = alpha op(A) op(B) + beta C, column-major as BLAS DGEMM; work holds

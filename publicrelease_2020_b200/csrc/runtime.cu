@@ -78,21 +78,22 @@ struct DevBuf {
 
 // ---------------------------------------------------------------------------
 // LOWSIC (lowden_files.f:2-172): S^{-1/2} of the FO overlap from its
-// eigen-decomposition (the role of DIAGGE_FO, diagon_sic.f:45); sym_eigen(n, a,
-// w, v) returns the eigenvalues w and v[k*n + m] = component k of eigenvector m.
+// eigen-decomposition (the role of DIAGGE_FO, diagon_sic.f:45).  From the
+// eigenvalues w: e = 1/sqrt(w) and lam = 1/e^2.
 // ---------------------------------------------------------------------------
-template <class Eig>
-void lowsic(Eig&& sym_eigen, int n, const std::vector<double>& over, std::vector<double>& sm12,
-            std::vector<double>& filo, std::vector<double>& lam) {
-  std::vector<double> w;
-  sym_eigen(n, over, w, filo);
+void lowsic_scale(const std::vector<double>& w, std::vector<double>& e, std::vector<double>& lam) {
+  const int n = (int)w.size();
   for (int i = 0; i < n; ++i)
     if (w[i] < 1.0e-8)
       fail(FLOSIC_ERR_LOWDEN, "LOWSIC: LOWDEN EIGENVALUES TOO SMALL (< 1e-8): BAD POSITIONS IN FRMORB");
-  std::vector<double> e(n);
-  for (int i = 0; i < n; ++i) e[i] = 1.0 / std::sqrt(w[i]);
+  e.resize(n);
   lam.resize(n);
+  for (int i = 0; i < n; ++i) e[i] = 1.0 / std::sqrt(w[i]);
   for (int i = 0; i < n; ++i) lam[i] = 1.0 / (e[i] * e[i]);
+}
+
+// S^{-1/2} on the host from the eigenvectors (filo[k*n + m] = component k of vector m).
+void lowsic_sm12(int n, const std::vector<double>& filo, const std::vector<double>& e, std::vector<double>& sm12) {
   sm12.assign((size_t)n * n, 0.0);
   for (int i = 0; i < n; ++i)
     for (int j = 0; j < n; ++j) {
@@ -101,6 +102,12 @@ void lowsic(Eig&& sym_eigen, int n, const std::vector<double>& over, std::vector
       sm12[(size_t)i * n + j] = s;
     }
 }
+
+// From this many FOs per spin the n^3 products of the FO construction and of the
+// FOD force run on the GPU; below, copies and launches take more than the host
+// loops.  FO construction + force of a cycle, host against GPU: 21 + 21 FOs 0.76
+// and 0.92 ms, 29 + 29 1.18 and 1.25, 75 3.9 and 2.2, 128 9.9 and 5.0.
+constexpr int DEVICE_PRODUCTS_MIN = 32;
 
 // Boys-function table of fffmtc.F:25-97 (series for F_19, downward recursion),
 // columns F2 F3 F4 F5 F4/2 F5/2 F6/2 F5/6 F6/6 F7/6.
@@ -325,6 +332,7 @@ struct flosic_ctx {
   DevBuf<int4> d_items;
   DevBuf<int> d_batch_counters;
   DevBuf<double> d_eig_a, d_eig_w, d_eig_v, d_eig_work;
+  DevBuf<double> d_fot, d_force;  // products of the FO construction and of the FOD force
   DevBuf<int> d_eig_info;
   bool have_geom = false, have_orb = false;
   // geometry
@@ -662,29 +670,27 @@ void gemm(flosic_ctx* c, bool ta, bool tb, int M, int N, int K, double alpha, co
   c->launches += w ? 2 : 1;
 }
 
-// Symmetric eigen-decomposition on the GPU (k_sym_eigen, cyclic Jacobi,
-// FP64, ascending eigenvalues) in the convention lowsic expects.
-auto device_eigen(flosic_ctx* c) {
-  return [c](int n, const std::vector<double>& a, std::vector<double>& w, std::vector<double>& v) {
-    cudaStream_t st = c->st;
-    c->d_eig_a.upload(a.data(), (size_t)n * n, st);
-    c->d_eig_w.ensure(n);
-    c->d_eig_v.ensure((size_t)n * n);
-    c->d_eig_work.ensure(sym_eigen_work(n));
-    c->d_eig_info.ensure(sym_eigen_info(n));
-    if (!launch_sym_eigen(n, c->d_eig_a.p, c->d_eig_work.p, c->d_eig_w.p, c->d_eig_v.p, c->d_eig_info.p, st))
-      fail(FLOSIC_ERR_CAPACITY, "LOWSIC: more FOs per spin than the eigen-solver holds");
-    c->launches += 2;
-    CUDA_CHECK(cudaGetLastError());
-    v.resize((size_t)n * n);
-    w.resize(n);
-    int info = 0;
-    CUDA_CHECK(cudaMemcpyAsync(v.data(), c->d_eig_v.p, sizeof(double) * v.size(), cudaMemcpyDeviceToHost, st));
-    CUDA_CHECK(cudaMemcpyAsync(w.data(), c->d_eig_w.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    CUDA_CHECK(cudaMemcpyAsync(&info, c->d_eig_info.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_CHECK(cudaStreamSynchronize(st));
-    if (info != 0) fail(FLOSIC_ERR_LOWDEN, "LOWSIC: eigen-decomposition of the FO overlap did not converge");
-  };
+// Eigen-decomposition of the symmetric n x n matrix in d_eig_a on the GPU (cyclic
+// Jacobi, FP64, ascending eigenvalues): w, and v[k*n + m] = component k of
+// eigenvector m (left in d_eig_v too).
+void device_eigen(flosic_ctx* c, int n, std::vector<double>& w, std::vector<double>& v) {
+  cudaStream_t st = c->st;
+  c->d_eig_w.ensure(n);
+  c->d_eig_v.ensure((size_t)n * n);
+  c->d_eig_work.ensure(sym_eigen_work(n));
+  c->d_eig_info.ensure(sym_eigen_info(n));
+  if (!launch_sym_eigen(n, c->d_eig_a.p, c->d_eig_work.p, c->d_eig_w.p, c->d_eig_v.p, c->d_eig_info.p, st))
+    fail(FLOSIC_ERR_CAPACITY, "LOWSIC: more FOs per spin than the eigen-solver holds");
+  c->launches += 2;
+  CUDA_CHECK(cudaGetLastError());
+  v.resize((size_t)n * n);
+  w.resize(n);
+  int info = 0;
+  CUDA_CHECK(cudaMemcpyAsync(v.data(), c->d_eig_v.p, sizeof(double) * v.size(), cudaMemcpyDeviceToHost, st));
+  CUDA_CHECK(cudaMemcpyAsync(w.data(), c->d_eig_w.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+  CUDA_CHECK(cudaMemcpyAsync(&info, c->d_eig_info.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_CHECK(cudaStreamSynchronize(st));
+  if (info != 0) fail(FLOSIC_ERR_LOWDEN, "LOWSIC: eigen-decomposition of the FO overlap did not converge");
 }
 
 void fo_setup(flosic_ctx* c, int s) {
@@ -727,29 +733,51 @@ void fo_setup(flosic_ctx* c, int s) {
       }
   }
   // TMAT (frmiorb.f:351-480)
-  std::vector<double> T((size_t)nf * nw), over((size_t)nf * nf);
+  std::vector<double> T((size_t)nf * nw);
   for (int k = 0; k < nf; ++k) {
     double rho = 0.0;
     for (int j = 0; j < nw; ++j) rho = rho + PS(0, k, j) * PS(0, k, j);
     if (!(rho > 0.0)) fail(FLOSIC_ERR_ZERO_DENSITY, "FRMIORB: zero density at an FOD");
     for (int j = 0; j < nw; ++j) T[(size_t)k * nw + j] = PS(0, k, j) / std::sqrt(rho);
   }
-  for (int i = 0; i < nf; ++i)
-    for (int j = 0; j < nf; ++j) {
-      double v = 0.0;
-      for (int w = 0; w < nw; ++w) v = v + T[(size_t)i * nw + w] * T[(size_t)j * nw + w];
-      over[(size_t)i * nf + j] = v;
-    }
-  std::vector<double> sm12;
-  lowsic(device_eigen(c), nf, over, sm12, S.filo, S.lam);
-  S.tmat.assign((size_t)nf * nw, 0.0);
-  for (int i = 0; i < nf; ++i)
-    for (int k = 0; k < nf; ++k) {
-      const double h = sm12[(size_t)k * nf + i];
-      for (int w = 0; w < nw; ++w) S.tmat[(size_t)i * nw + w] += h * T[(size_t)k * nw + w];
-    }
+  // overlap T T^T, its S^-1/2 and TMAT = S^-1/2 T: on the GPU in the order and with
+  // the roundings of the host loops
+  std::vector<double> w, e;
+  if (nf >= DEVICE_PRODUCTS_MIN) {
+    c->d_fot.upload(T.data(), T.size(), st);
+    c->d_eig_a.ensure((size_t)nf * nf);
+    launch_ordered_product(nf, nf, nw, c->d_fot.p, nw, 1, c->d_fot.p, nw, 1, nullptr, c->d_eig_a.p, nf, st);
+    device_eigen(c, nf, w, S.filo);
+    lowsic_scale(w, e, S.lam);
+    c->d_eig_w.upload(e.data(), nf, st);
+    launch_ordered_product(nf, nf, nf, c->d_eig_v.p, nf, 1, c->d_eig_v.p, nf, 1, c->d_eig_w.p, c->d_eig_a.p, nf, st);
+    c->d_tmat.ensure(T.size());
+    launch_ordered_product(nf, nw, nf, c->d_eig_a.p, 1, nf, c->d_fot.p, 1, nw, nullptr, c->d_tmat.p, nw, st);
+    c->launches += 3;
+    S.tmat.resize(T.size());
+    CUDA_CHECK(cudaMemcpyAsync(S.tmat.data(), c->d_tmat.p, sizeof(double) * T.size(), cudaMemcpyDeviceToHost, st));
+    CUDA_CHECK(cudaStreamSynchronize(st));
+  } else {
+    std::vector<double> over((size_t)nf * nf), sm12;
+    for (int i = 0; i < nf; ++i)
+      for (int j = 0; j < nf; ++j) {
+        double v = 0.0;
+        for (int m = 0; m < nw; ++m) v = v + T[(size_t)i * nw + m] * T[(size_t)j * nw + m];
+        over[(size_t)i * nf + j] = v;
+      }
+    c->d_eig_a.upload(over.data(), over.size(), st);
+    device_eigen(c, nf, w, S.filo);
+    lowsic_scale(w, e, S.lam);
+    lowsic_sm12(nf, S.filo, e, sm12);
+    S.tmat.assign((size_t)nf * nw, 0.0);
+    for (int i = 0; i < nf; ++i)
+      for (int k = 0; k < nf; ++k) {
+        const double h = sm12[(size_t)k * nf + i];
+        for (int m = 0; m < nw; ++m) S.tmat[(size_t)i * nw + m] += h * T[(size_t)k * nw + m];
+      }
+    c->d_tmat.upload(S.tmat.data(), S.tmat.size(), st);
+  }
   // FO coefficients C_FO(nb x nf) = C_KS(nb x nw) * TMAT^T (unravel2.f:200-240)
-  c->d_tmat.upload(S.tmat.data(), S.tmat.size(), st);
   S.cfo.ensure((size_t)nb * nf);
   const double* cks = c->d_psi.p + (size_t)s * c->nwfs[0] * nb;
   gemm(c, false, false, nb, nf, nw, 1.0, cks, nb, c->d_tmat.p, nw, 0.0, S.cfo.p, nb);
@@ -1067,15 +1095,8 @@ void spin_force(flosic_ctx* c, int s, const double* sic /* SIC(j,l) at [l*ld + j
   const std::vector<double>& Fm = S.filo;
   const std::vector<double>& Q = S.lam;
   const size_t n2 = (size_t)nf * nf;
-  std::vector<double> FmT(n2), sicm(n2), tmp(n2), G(n2);
-  for (int i = 0; i < nf; ++i)
-    for (int a = 0; a < nf; ++a) {
-      FmT[(size_t)a * nf + i] = Fm[(size_t)i * nf + a];
-      sicm[(size_t)i * nf + a] = sic[(size_t)a * ld + i];  // SIC(i,a)
-    }
+  std::vector<double> M((size_t)nf * nw);
   // G = FILO^T SIC FILO  ->  HAM(b,a) = (G[a][b] - G[b][a]) / sqrt(Qa Qb)
-  mat_mul(FmT.data(), sicm.data(), tmp.data(), nf, nf, nf);
-  mat_mul(tmp.data(), Fm.data(), G.data(), nf, nf, nf);
   // Both terms of frmorb2.F:612-717 in one matrix:
   //   term 1: -sum_a FILO(m,a) (HAM^T FILO^T X_kx)[a][m]           (frmorb2.F:616-667)
   //   term 2: +1/4 sum_ab HAM'(b,a) [FILO(m,a) Y_b(m) + FILO(m,b) Y_a(m)],
@@ -1083,20 +1104,49 @@ void spin_force(flosic_ctx* c, int s, const double* sic /* SIC(j,l) at [l*ld + j
   // with X_kx[n][m] = sum_w F(w,n,1) F(w,m,kx+1), so that
   //   DEBDAX(kx,m) = sum_n L[m][n] X_kx[n][m],  L = FILO (HAM'^T/2 + HAM'/2 - HAM^T) FILO^T
   // (H[a][b] = HAM(b,a)), i.e. sum_w M[m][w] F(w,m,kx+1) with M = L F_0.
-  std::vector<double> A1(n2);
-  for (int a = 0; a < nf; ++a)
-    for (int b = 0; b < nf; ++b) {
-      const double sa = std::sqrt(Q[a]), sb = std::sqrt(Q[b]);
-      const double hab = (G[(size_t)a * nf + b] - G[(size_t)b * nf + a]) / (sb * sa);
-      const double hba = (G[(size_t)b * nf + a] - G[(size_t)a * nf + b]) / (sa * sb);
-      const double hpab = hab * (sb - sa) / (sb + sa);
-      const double hpba = hba * (sa - sb) / (sa + sb);
-      A1[(size_t)a * nf + b] = 0.5 * (hpab + hpba) - hab;
-    }
-  std::vector<double> T(n2), L(n2), M((size_t)nf * nw);
-  mat_mul(Fm.data(), A1.data(), T.data(), nf, nf, nf);
-  mat_mul(T.data(), FmT.data(), L.data(), nf, nf, nf);
-  mat_mul(L.data(), &S.fmat[0], M.data(), nf, nf, nw);  // F_0[n][w] = F(w,n,1)
+  if (nf >= DEVICE_PRODUCTS_MIN) {
+    // row-major matrices as column-major transposes: d0 = FILO^T, d1 = SIC
+    cudaStream_t st = c->st;
+    c->d_force.ensure(4 * n2 + (size_t)nf * nw + nf);
+    double *d0 = c->d_force.p, *d1 = d0 + n2, *d2 = d1 + n2, *dm = d2 + n2, *df = dm + (size_t)nf * nw, *dq = df + n2;
+    CUDA_CHECK(cudaMemcpyAsync(d0, Fm.data(), sizeof(double) * n2, cudaMemcpyHostToDevice, st));
+    CUDA_CHECK(cudaMemcpyAsync(dq, Q.data(), sizeof(double) * nf, cudaMemcpyHostToDevice, st));
+    CUDA_CHECK(cudaMemcpyAsync(df, S.fmat.data(), sizeof(double) * nf * nw, cudaMemcpyHostToDevice, st));
+    CUDA_CHECK(cudaMemcpy2DAsync(d1, sizeof(double) * nf, sic, sizeof(double) * ld, sizeof(double) * nf, nf,
+                                 cudaMemcpyHostToDevice, st));
+    gemm(c, false, true, nf, nf, nf, 1.0, d0, nf, d1, nf, 0.0, d2, nf);   // FILO^T SIC^T
+    gemm(c, false, true, nf, nf, nf, 1.0, d2, nf, d0, nf, 0.0, d1, nf);   // G^T
+    launch_force_ham(nf, d1, dq, d2, st);                                 // A1^T
+    c->launches++;
+    gemm(c, false, false, nf, nf, nf, 1.0, d2, nf, d0, nf, 0.0, d1, nf);  // (FILO A1)^T
+    gemm(c, true, false, nf, nf, nf, 1.0, d0, nf, d1, nf, 0.0, d2, nf);   // L^T
+    gemm(c, false, false, nw, nf, nf, 1.0, df, nw, d2, nf, 0.0, dm, nw);  // (L F_0)^T
+    CUDA_CHECK(cudaMemcpyAsync(M.data(), dm, sizeof(double) * M.size(), cudaMemcpyDeviceToHost, st));
+    CUDA_CHECK(cudaStreamSynchronize(st));
+  } else {
+    std::vector<double> FmT(n2), sicm(n2), tmp(n2), G(n2);
+    for (int i = 0; i < nf; ++i)
+      for (int a = 0; a < nf; ++a) {
+        FmT[(size_t)a * nf + i] = Fm[(size_t)i * nf + a];
+        sicm[(size_t)i * nf + a] = sic[(size_t)a * ld + i];  // SIC(i,a)
+      }
+    mat_mul(FmT.data(), sicm.data(), tmp.data(), nf, nf, nf);
+    mat_mul(tmp.data(), Fm.data(), G.data(), nf, nf, nf);
+    std::vector<double> A1(n2);
+    for (int a = 0; a < nf; ++a)
+      for (int b = 0; b < nf; ++b) {
+        const double sa = std::sqrt(Q[a]), sb = std::sqrt(Q[b]);
+        const double hab = (G[(size_t)a * nf + b] - G[(size_t)b * nf + a]) / (sb * sa);
+        const double hba = (G[(size_t)b * nf + a] - G[(size_t)a * nf + b]) / (sa * sb);
+        const double hpab = hab * (sb - sa) / (sb + sa);
+        const double hpba = hba * (sa - sb) / (sa + sb);
+        A1[(size_t)a * nf + b] = 0.5 * (hpab + hpba) - hab;
+      }
+    std::vector<double> T(n2), L(n2);
+    mat_mul(Fm.data(), A1.data(), T.data(), nf, nf, nf);
+    mat_mul(T.data(), FmT.data(), L.data(), nf, nf, nf);
+    mat_mul(L.data(), &S.fmat[0], M.data(), nf, nf, nw);  // F_0[n][w] = F(w,n,1)
+  }
   for (int m = 0; m < nf; ++m)
     for (int kx = 0; kx < 3; ++kx) {
       const double* fk = &S.fmat[((size_t)(kx + 1) * nf + m) * nw];
@@ -1389,6 +1439,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_coefp.release(); c->d_momp.release(); c->d_seg.release(); c->d_bound.release(); c->d_plist.release(); c->d_again.release();
   c->d_share.release(); c->d_lists.release(); c->d_setup_list.release();
   c->d_eig_a.release(); c->d_eig_w.release(); c->d_eig_v.release(); c->d_eig_work.release(); c->d_eig_info.release();
+  c->d_fot.release(); c->d_force.release();
   c->d_coef_hl.release(); c->d_momv_hl.release(); c->d_tc_err.release(); c->d_dens_coef.release();
   c->d_gemm_ws.release();
   for (auto& w : c->d_wk) w.release();

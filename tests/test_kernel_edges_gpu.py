@@ -74,8 +74,9 @@ def test_fo_values_stages(natoms, nbasis, npts):
         ctx.close()
 
 
-# alkanes have 4 n + 1 FOs per spin: the largest one below the limit of 160, the
-# smallest beyond; small and odd sizes by the first FOs of nonane
+# alkanes have 4 n + 1 FOs per spin: the largest one below the eigen-solver's limit
+# of 160, the smallest beyond; small and odd sizes by the first FOs of nonane, 31 and
+# 32 on both sides of the rule that moves the n^3 products to the GPU
 @pytest.mark.parametrize("ncarbon,nfo", [(9, 1), (9, 2), (9, 31), (9, 32), (39, 157), (40, 161)])
 def test_lowdin_sizes(ncarbon, nfo):
     sysm = W.alkane(ncarbon, seed=3, nrad=1)
@@ -83,13 +84,18 @@ def test_lowdin_sizes(ncarbon, nfo):
     sysm.psi = np.ascontiguousarray(np.concatenate([sysm.psi[:nfo], sysm.psi[n0:n0 + nfo]]))
     sysm.nwfs = (nfo, nfo)
     sysm.fods = [f[:nfo] for f in sysm.fods]
-    to, eo = O.Oracle(sysm).frmiorb()
+    orc = O.Oracle(sysm)
+    to, eo = orc.frmiorb()
+    sic = np.random.default_rng(1).normal(size=(nfo, nfo))
     ctx = S.open_system(sysm)
     try:
         tg, eg = ctx.frmiorb()
+        fg = [ctx.frmorb2_force(s, sic) for s in (1, 2)]
     finally:
         ctx.close()
     for s in range(2):
+        fo = orc.frmorb2_force(s + 1, sic)
+        assert np.max(np.abs(fg[s][:nfo] - fo[:nfo])) < 1e-9 * max(1.0, np.abs(fo[:nfo]).max())
         assert np.allclose(tg[s, :nfo, :nfo], to[s, :nfo, :nfo], rtol=1e-10, atol=1e-10)
         assert np.allclose(np.sort(eg[s, :nfo]), np.sort(eo[s, :nfo]), rtol=1e-11)
 
