@@ -34,11 +34,12 @@ sys.path.insert(0, ROOT)
 METRIC = "s per FLO-SIC SCF cycle (all FOs + FOD forces), mixed vs FP64, |ΔE_SIC|≤10µHa"
 COULOMB_FLOPS_NEAR = 92.0    # per near (pair, point, FO): 46 polynomial coefficients x Boys-monomial terms
 COULOMB_FLOPS_TERM = 2.0     # per multipole term kept by the skip rule in a far (call, point, FO) evaluation
-# DRAM bytes of the two Coulomb kernels per tile of 128 points on the C2 shape:
+# DRAM bytes of the Coulomb kernels per tile of 128 points on the C2 shape:
 # ncu dram__bytes_read.sum + dram__bytes_write.sum on 296 tiles (k_coulomb_shared
-# 7.951 GB + 0.041 GB, k_coulomb_perfo 1.828 GB + 0.179 GB); the traffic is
-# re-reads of the per-call A operands, proportional to the tile count.
-COULOMB_DRAM_BYTES_PER_TILE = (7.951e9 + 0.041e9 + 1.828e9 + 0.179e9) / 296
+# 5.311 GB + 0.033 GB, k_perfo_near 0.506 GB + 0.032 GB, k_perfo_far 0.012 GB); the
+# traffic is re-reads of the per-call A operands, proportional to the tile count.
+# k_coulomb_perfo in the line below is the two per-FO kernels together.
+COULOMB_DRAM_BYTES_PER_TILE = (5.311e9 + 0.033e9 + 0.506e9 + 0.032e9 + 0.012e9) / 296
 # (the Boys values, monomials and harmonics depend on geometry only and are
 # formed once per (pair or call, point); the per-FO work is the contraction)
 
@@ -417,7 +418,7 @@ def run_ours(args, rank, world, local_rank):
         "gpu_launches": int(st_acc["launches"]),
         "roofline": {"bound": "tensor", "kernel": "k_coulomb_shared + k_coulomb_perfo", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
-                     "traffic": traffic, "traffic_note": "ncu DRAM bytes of both kernels on the 296-tile C2 "
+                     "traffic": traffic, "traffic_note": "ncu DRAM bytes of the kernels on the 296-tile C2 "
                                                          "shape, scaled by tile count",
                      "peak_kind": "FP64 cuBLAS DGEMM measured in this run (MEASURED_PEAKS.json has no FP64 figure)",
                      "work": f"{st_acc['near'] / args.steps:.4g} near (pair,point,FO) x {COULOMB_FLOPS_NEAR:.0f} + "
@@ -450,7 +451,7 @@ def run_ours(args, rank, world, local_rank):
 def run_batch(args, rank, world, local_rank):
     """C4: 64 alkane-like chains and rings of uneven size in one batch on one
     GPU (batch.Batch): the Coulomb potentials of all FOs of all molecules in
-    two persistent launches (flosic_sic_batch_cycle), FO block width chosen by
+    one set of launches (flosic_sic_batch_cycle), FO block width chosen by
     the batch autotuner.  A step is one SIC cycle of every molecule; with N
     GPUs the molecules are dealt round-robin to the ranks (independent objects,
     no collective) and the step time is the maximum over ranks.  The earlier
@@ -562,7 +563,7 @@ def run_batch(args, rank, world, local_rank):
     nfo = [max(m.nfrm) for m in systems]
     cfg = {"workload": f"C4 batch: 64 alkane-like chains and rings (seeds 100-163, 2-29 atoms), {min(nb)}-{max(nb)} "
                        f"functions, {min(npt)}-{max(npt)} mesh points ({sum(npt)} in all), {min(nfo)}-{max(nfo)} FOs "
-                       "per spin, LDA-PW91, NSPN=2; the Coulomb potentials of all molecules in two persistent "
+                       "per spin, LDA-PW91, NSPN=2; the Coulomb potentials of all molecules in one set of "
                        "launches",
            "molecules": len(systems), "parallelism": (f"molecules dealt to {world} GPUs" if world > 1 else "single GPU"),
            "l2": "working set >> L2 (126 MB)", "precision": headline, "autotune": tuned or "off",

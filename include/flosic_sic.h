@@ -209,9 +209,9 @@ int flosic_sic_cycle(flosic_ctx* ctx, int ld, double* results, double* sic, doub
    in one precision, each with its own geometry, orbitals and FODs.  Every
    molecule's FO construction, FO values, pair coefficients and call set-up run
    on its own stream; then the Coulomb potentials of all FOs of all molecules
-   and both spins are evaluated by two persistent launches over one list of
+   and both spins are evaluated by one set of launches over one list of
    (molecule-spin, 128-point tile, block of 32*wm FOs) items (shared-geometry
-   calls, then per-FO calls added); then each molecule's XC, energies, SIC
+   calls, then the per-FO calls' near and far field added); then each molecule's XC, energies, SIC
    matrix and forces.  wm = 1, 2 or 4 sets the FO block (0: from the largest
    FO count).  Outputs per molecule m at the offsets of flosic_sic_cycle times
    m: RESULTS(13,ld,2), SIC(ld,ld,2), DEBDAX(3,ld,2), CFRM(3,ld,2) and
@@ -322,9 +322,9 @@ int flosic_sic_stats(flosic_ctx* ctx, int64_t* launches, double* stage_ms, int64
 /* The Coulomb evaluation of the last cycle split by kernel (no counterpart in
    the reference): ms[0] = the shared-geometry calls (call classification,
    operand splits and the shared-geometry kernel: k_coulomb_shared_tc or
-   k_coulomb_shared), ms[1] = the per-FO kernel (k_coulomb_perfo), device
-   milliseconds summed over the spins; work[0..2] = near / far / kept-term
-   counts of the shared-geometry kernel, work[3..5] of the per-FO kernel. */
+   k_coulomb_shared), ms[1] = the per-FO kernels (k_perfo_near and
+   k_perfo_far, which overlap), device milliseconds summed over the spins; work[0..2] = near / far / kept-term
+   counts of the shared-geometry kernel, work[3..5] of the per-FO kernels. */
 int flosic_sic_kernel_stats(flosic_ctx* ctx, double* ms, int64_t* work);
 
 #ifdef __cplusplus

@@ -4,12 +4,12 @@ Each molecule has its own context (geometry, orbitals, FODs, device buffers,
 CUDA stream).  Batch.cycle runs one SIC cycle of every molecule through
 flosic_sic_batch_cycle: each molecule's FO construction, FO values, pair
 coefficients and POISSON1 call set-up on its own stream, then the Coulomb
-potentials of all FOs of all molecules and both spins in two persistent
+potentials of all FOs of all molecules and both spins in one set of
 launches over one list of (molecule-spin, 128-point tile, FO block) items,
 then each molecule's XC, energies, SIC matrix and forces.  This is the B200
 form of the reference's orbital-parallel GROUP mode (global_call.F90:113-160),
-where MPI groups take the FOs of a molecule; here the persistent CTAs take
-tiles of every molecule.  Batch.autotune times the FO block widths (32, 64 or
+where MPI groups take the FOs of a molecule; here the CTAs of one launch
+take tiles of every molecule.  Batch.autotune times the FO block widths (32, 64 or
 128 FOs per item) on the batch itself and keeps the fastest.
 
 Batch.cycle_streams is the earlier form kept for comparison: every molecule's

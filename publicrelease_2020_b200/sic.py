@@ -363,7 +363,7 @@ class FlosicSIC:
 
 def batch_cycle(ctxs, wm=0):
     """One SIC cycle of every context in ctxs (flosic_sic_batch_cycle: the
-    Coulomb potentials of all molecules in two persistent launches); a list of
+    Coulomb potentials of all molecules in one set of launches); a list of
     outputs shaped as FlosicSIC.cycle's."""
     n = len(ctxs)
     L = load_library()
