@@ -311,8 +311,7 @@ k_coulomb_shared_tc(int ncalls, const int* __restrict__ lists, const CallShare* 
   const int np = min(TILE, M.n - p0);
   // no shared-geometry call (NSPN=2): the tile is zero and nothing below has
   // work, so the block writes it and leaves before any barrier or tensor memory.
-  // The idle pipeline took 1.9 of 27.2 ms of a benzene cycle (merged spins) and
-  // 2 of 4.2 ms of water's.
+  // The idle pipeline took 2.1 of 27.2 ms of a benzene cycle.
   if (lists[2 * ncalls] == 0) {
     const int col = tid & (TILE - 1);
     if (col < np)
