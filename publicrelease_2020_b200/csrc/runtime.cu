@@ -286,7 +286,6 @@ struct CoulBufs {
 
 struct SpinCache {
   bool fo_valid = false;       // FMAT/TMAT/CFO
-  bool vh_valid = false;       // raw Coulomb potentials at vhp
   bool pot_valid = false;      // potentials, RESULTS
   int nf = 0, nw = 0;
   std::vector<double> fmat;    // [(K*nf + jfm)*nw + jwf]
@@ -643,7 +642,7 @@ void sort_mesh(flosic_ctx* c, const double* rmsh, const double* wmsh) {
 
 void invalidate(flosic_ctx* c) {
   for (auto& s : c->spin) {
-    s.fo_valid = s.vh_valid = s.pot_valid = s.sic_valid = false;
+    s.fo_valid = s.pot_valid = s.sic_valid = false;
   }
 }
 
@@ -908,7 +907,6 @@ int coulomb_set(flosic_ctx* c, int s0, int ns) {
 void coulomb(flosic_ctx* c, int s0, int ns = 1) {
   const int nf = coulomb_set(c, s0, ns);
   coulomb_eval(c, nf, nullptr, c->spin[s0].vh.p);
-  for (int s = s0; s < s0 + ns; ++s) c->spin[s].vh_valid = true;
 }
 
 // Whether a cycle evaluates the Coulomb potentials of both spins together: the
@@ -938,7 +936,11 @@ void results_from_parts(const flosic_ctx* c, int nf, const double* parts, const 
 void spin_xc(flosic_ctx* c, int s);
 
 // Everything of APOTNL_SIC for all FOs of spin s (apotnl_sic.F:232-623).
-void spin_potentials(flosic_ctx* c, int s) {
+// evaluated: the last evaluation on this context was cycle_coulomb, in the same
+// call.  The raw Coulomb potentials are not kept across calls on their own: the
+// pair-route density also needs d_u and d_callfo as that evaluation left them,
+// and every other evaluation (of the other spin, COUPOT1, a batch) refills both.
+void spin_potentials(flosic_ctx* c, int s, bool evaluated = false) {
   SpinCache& S = c->spin[s];
   if (S.pot_valid) return;
   cudaStream_t st = c->st;
@@ -947,14 +949,13 @@ void spin_potentials(flosic_ctx* c, int s) {
   CUDA_CHECK(cudaEventRecord(c->ev[1], st));
   fo_values(c, s);
   CUDA_CHECK(cudaEventRecord(c->ev[7], st));
-  const bool eval = !S.vh_valid;
-  if (eval) coulomb(c, s);
+  if (!evaluated) coulomb(c, s);
   CUDA_CHECK(cudaEventRecord(c->ev[4], st));
   pair_density(c, s, c->d_callfo.p);  // FLOSIC_DENSITY_PAIRS only; timed with XC
   spin_xc(c, s);
   c->stage_ms[0] += elapsed(c->ev[0], c->ev[1]);
   c->stage_ms[1] += elapsed(c->ev[1], c->ev[7]);
-  if (eval) {
+  if (!evaluated) {
     c->stage_ms[2] += elapsed(c->ev[7], c->ev[3]);
     c->stage_ms[3] += elapsed(c->ev[3], c->ev[4]);
   }
@@ -1048,10 +1049,10 @@ void results_from_parts(const flosic_ctx* c, int nf, const double* parts, const 
 
 // SICLAGM (frmorb_mpi.F:456-517): SIC(j,l) = -sum_p phi_j w V_l phi_l; for a
 // meta-GGA -sum_c sum_p d_c phi_j Y_c,l over the four channels of Y (k_xc).
-void spin_sic(flosic_ctx* c, int s) {
+void spin_sic(flosic_ctx* c, int s, bool evaluated = false) {
   SpinCache& S = c->spin[s];
   if (S.sic_valid) return;
-  spin_potentials(c, s);
+  spin_potentials(c, s, evaluated);
   const int nf = S.nf, P = c->eval_n;
   cudaStream_t st = c->st;
   CUDA_CHECK(cudaEventRecord(c->ev[0], st));
@@ -1853,7 +1854,7 @@ int flosic_sic_set_density_mode(flosic_ctx* c, int mode) {
     if (mode != c->density) {
       c->density = mode;
       for (auto& s : c->spin) {
-        s.vh_valid = s.pot_valid = false;
+        s.pot_valid = false;
         s.sic_valid = false;
         if (mode == FLOSIC_DENSITY_PHI2) s.rhog.release();
       }
@@ -1869,7 +1870,7 @@ int flosic_sic_set_precision(flosic_ctx* c, int mode) {
     if (mode != c->precision) {
       c->precision = mode;
       for (auto& s : c->spin) {
-        s.vh_valid = s.pot_valid = false;
+        s.pot_valid = false;
         s.sic_valid = false;
       }
     }
@@ -1902,7 +1903,7 @@ int flosic_sic_autotune(flosic_ctx* c, int reps, int* perfo_fos, float* ms) {
     if (c->nfrm[s] < 1) fail(FLOSIC_ERR_STATE, "no FOs to tune on");
     // The timing runs overwrite these potentials: drop the cached ones first,
     // and put the width and counters back on every way out.
-    for (int t = s; t < s + ns; ++t) c->spin[t].vh_valid = c->spin[t].pot_valid = c->spin[t].sic_valid = false;
+    for (int t = s; t < s + ns; ++t) c->spin[t].pot_valid = c->spin[t].sic_valid = false;
     struct Restore {
       flosic_ctx* c;
       int wm;
@@ -2041,12 +2042,13 @@ int flosic_sic_cycle(flosic_ctx* c, int ld, double* results, double* sic, double
     c->kernel_ms[0] = c->kernel_ms[1] = 0.0;
     for (auto& w : c->kernel_work) w = 0;
     invalidate(c);
-    if (spins_together(c)) cycle_coulomb(c);
+    const bool both = spins_together(c);
+    if (both) cycle_coulomb(c);
     double zsic = 0.0;
     for (int s = 0; s < c->nspn; ++s) {
       const int nf = c->nfrm[s];
       if (nf == 0) continue;
-      spin_sic(c, s);
+      spin_sic(c, s, both);
       const SpinCache& S = c->spin[s];
       for (int k = 0; k < nf; ++k) {
         for (int i = 0; i < 13; ++i) results[((size_t)s * ld + k) * 13 + i] = S.results[(size_t)k * 13 + i];
@@ -2158,10 +2160,7 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       c->work_far += cnt[1];
       c->work_terms += cnt[2];
       const int s0 = owner[j].second;
-      for (int s = s0; s < s0 + (spins_together(c) ? 2 : 1); ++s) {
-        c->spin[s].vh_valid = true;
-        spin_xc(c, s);
-      }
+      for (int s = s0; s < s0 + (spins_together(c) ? 2 : 1); ++s) spin_xc(c, s);
     }
     for (int m = 0; m < n; ++m) {
       flosic_ctx* c = ctxs[m];
@@ -2488,13 +2487,14 @@ int flosic_sic_cycle_partial(flosic_ctx* c, double* d_partial) {
     c->kernel_ms[0] = c->kernel_ms[1] = 0.0;
     for (auto& w : c->kernel_work) w = 0;
     invalidate(c);
-    if (spins_together(c)) cycle_coulomb(c);
+    const bool both = spins_together(c);
+    if (both) cycle_coulomb(c);
     std::vector<double> h(partial_doubles(c), 0.0);
     size_t o = 0;
     for (int s = 0; s < c->nspn; ++s) {
       const int nf = c->nfrm[s];
       if (nf == 0) continue;
-      spin_sic(c, s);
+      spin_sic(c, s, both);
       const SpinCache& S = c->spin[s];
       std::copy(S.sic.begin(), S.sic.end(), h.begin() + o);
       o += (size_t)nf * nf;
