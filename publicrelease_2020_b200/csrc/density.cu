@@ -11,11 +11,11 @@
 // density is the reference's truncated one rather than phi^2.
 //
 //   k_pair_dens_coef   RHOC (35) per (pair, FO), thresholded as the reference
-//                      skips its entries.  Every RHOD entry is a power times one
+//                      skips its entries.  Every RHOD entry is a power f times one
 //                      RHOC entry (gtdncf.F), so the derivative channels are the
-//                      derivatives of the one polynomial.  (The reference drops
-//                      an RHOD entry by its own magnitude: it keeps f RHOC with
-//                      f = 2..12 where RHOC is between 1e-14 / f and 1e-14.)
+//                      derivatives of the one polynomial, except where RHOC is
+//                      between 1e-14 / f and 1e-14: the entry is then kept in the
+//                      channels of those f alone, and listed apart.
 //   k_pair_density     all pairs of one FO over one mesh tile: near test per
 //                      point, the polynomial with its derivatives, channel sums
 //                      in call order
@@ -36,7 +36,8 @@ constexpr double DENS_EPS = 1.0e-14;  // poisson1.f:860,870,880
 constexpr int DENS_THREADS = TILE;    // one mesh point per thread
 
 // A coefficient row: 35 entries in the order pair_channels reads them (x power
-// descending, then y, then z), one of padding.
+// descending, then y, then z), then a bit per monomial m that only derivative
+// channels keep.  The values of those are in a second array of rows, at m.
 constexpr int DENS_LD = 36;
 __device__ __forceinline__ int dens_pos(int px, int py, int pz) {
   const int n = 4 - px, u = n - py, s = u - pz;
@@ -61,7 +62,8 @@ __device__ __forceinline__ void mono_powers(int m, int& px, int& py, int& pz) {
 }
 
 __global__ void __launch_bounds__(128) k_pair_dens_coef(const PairGeo* __restrict__ pairs, int nfo, int nprim,
-                                                        const double* __restrict__ u, double* __restrict__ dc) {
+                                                        const double* __restrict__ u, int nch,
+                                                        double* __restrict__ dc, double* __restrict__ dronly) {
   __shared__ double P1[10][10][3][5];
   const int ip = blockIdx.x, tid = threadIdx.x;
   const PairGeo g = pairs[ip];
@@ -90,6 +92,7 @@ __global__ void __launch_bounds__(128) k_pair_dens_coef(const PairGeo* __restric
       for (int y = 0; y <= nb; ++y) e[x + y] += pa[x] * pb[y];
     for (int j = 0; j < 5; ++j) P1[mu][nu][d][j] = e[j];
   }
+  for (int k = tid; k < nfo; k += blockDim.x) dc[((size_t)ip * nfo + k) * DENS_LD + 35] = 0.0;  // no bit set
   __syncthreads();
   const double ex = exp(-arg);
   for (int q = tid; q < nfo * 35; q += blockDim.x) {
@@ -113,9 +116,15 @@ __global__ void __launch_bounds__(128) k_pair_dens_coef(const PairGeo* __restric
       }
     }
     const double rc = s * ex;
-    double* row = dc + ((size_t)ip * nfo + k) * DENS_LD;
-    row[dens_pos(px, py, pz)] = dens_keep(rc);
-    if (m == 0) row[35] = 0.0;
+    const size_t r0 = ((size_t)ip * nfo + k) * DENS_LD;
+    dc[r0 + dens_pos(px, py, pz)] = dens_keep(rc);
+    // the largest factor of the monomial's RHOD entries
+    const int lo = min(px, min(py, pz)), hi = max(px, max(py, pz)), mid = px + py + pz - lo - hi;
+    const int f = nch == 1 ? 0 : (nch == 4 ? hi : max(hi, max(hi * (hi - 1), hi * mid)));
+    if (dens_keep(rc) == 0.0 && dens_keep(f * rc) != 0.0) {
+      dronly[r0 + m] = rc;
+      atomicOr(reinterpret_cast<unsigned long long*>(dc + r0 + 35), 1ull << m);
+    }
   }
 }
 
@@ -132,12 +141,48 @@ struct Horner {
   }
 };
 
+// Channels 1.. of the monomials that only derivative channels keep, before the
+// Gaussian factor: every RHOD entry f c above the threshold, with its product-rule
+// terms.  Out of line, since a row with such an entry is the exception.
+template <int NCH>
+__device__ __noinline__ void derivative_only(unsigned long long bits, const double* __restrict__ c_of, double x,
+                                             double y, double z, double delta, double* a) {
+  const double v[3] = {x, y, z};
+  double g[3] = {0.0, 0.0, 0.0}, h[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (; bits; bits &= bits - 1) {
+    const int m = __ffsll((long long)bits) - 1;
+    const double c = c_of[m];
+    int p[3];
+    mono_powers(m, p[0], p[1], p[2]);
+    auto mono = [&](int i, int j) {  // the monomial without one power of i and of j (j < 0: of i alone)
+      double t = 1.0;
+      for (int d = 0; d < 3; ++d)
+        for (int e = p[d] - (d == i) - (d == j); e > 0; --e) t *= v[d];
+      return t;
+    };
+    for (int d = 0; d < 3; ++d) {
+      const double fc = dens_keep(p[d] * c);
+      if (fc != 0.0) g[d] += fc * mono(d, -1);
+    }
+    for (int q = 0; NCH == 10 && q < 6; ++q) {  // xx yy zz xy xz yz
+      const int i = q < 3 ? q : (q < 5 ? 0 : 1), j = q < 3 ? q : (q == 3 ? 1 : 2);
+      const double fc = dens_keep((i == j ? p[i] * (p[i] - 1) : p[i] * p[j]) * c);
+      if (fc != 0.0) h[q] += fc * mono(i, j);
+    }
+  }
+  for (int d = 0; d < 3; ++d) a[d] = g[d];
+  for (int q = 0; NCH == 10 && q < 6; ++q) {
+    const int i = q < 3 ? q : (q < 5 ? 0 : 1), j = q < 3 ? q : (q == 3 ? 1 : 2);
+    a[3 + q] = h[q] - 2.0 * delta * (v[j] * g[i] + v[i] * g[j]);
+  }
+}
+
 // Channels of one pair and one FO at offset (x, y, z) before the Gaussian
 // factor: the polynomial RHOC and its derivatives by nested Horner schemes (z
 // inside y inside x, 90 multiply-adds for all ten channels against 155 with the
 // monomials and RHOD tables), then the product-rule terms of the Gaussian's
-// derivatives (poisson1.f:849-940).  row: 36 coefficients in shared memory, read
-// in order.
+// derivatives (poisson1.f:849-940).  row: its 35 coefficients in shared memory,
+// read in order.
 template <int NCH>
 __device__ __forceinline__ void pair_channels(double x, double y, double z, double delta,
                                               const double* __restrict__ row, double (&a)[NCH]) {
@@ -209,6 +254,7 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int np
                                                                const PairGeo* __restrict__ pairs,
                                                                const CallFO* __restrict__ cfo, int cfo_ld, int nfo,
                                                                const double* __restrict__ dc,
+                                                               const double* __restrict__ dronly,
                                                                double* __restrict__ rhog, size_t ldr) {
   __shared__ __align__(16) double s_row[2][DENS_CHUNK][DENS_LD];
   __shared__ double s_geo[DENS_THREADS][4];  // queue: C[3], delta
@@ -284,6 +330,15 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int np
         pair_channels<NCH>(rx, ry, rz, delta, s_row[buf][i], a);
 #pragma unroll
         for (int ch = 0; ch < NCH; ++ch) acc[ch] += chgd * a[ch];
+        if constexpr (NCH > 1) {
+          const unsigned long long bits = (unsigned long long)__double_as_longlong(s_row[buf][i][35]);
+          if (bits) {
+            double e[NCH - 1];
+            derivative_only<NCH>(bits, dronly + ((size_t)s_pair[e0 + i] * nfo + k) * DENS_LD, rx, ry, rz, delta, e);
+#pragma unroll
+            for (int ch = 1; ch < NCH; ++ch) acc[ch] += chgd * e[ch - 1];
+          }
+        }
       }
     }
   }
@@ -295,17 +350,21 @@ __global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int np
 
 }  // namespace
 
-int pair_density_ld() { return DENS_LD; }
+// The rows, and with derivative channels as many again for the entries that only those keep.
+int pair_density_ld(int nch) { return nch > 1 ? 2 * DENS_LD : DENS_LD; }
 
 void launch_pair_density(int npairs, const PairGeo* pairs, const CallFO* cfo, int cfo_ld, int nfo, int nprim,
                          const double* u, int nch, const MeshDev& M, double* dc, double* rhog, size_t ldr,
                          cudaStream_t st) {
   if (nfo <= 0 || M.ntiles <= 0) return;
-  if (npairs > 0) k_pair_dens_coef<<<npairs, 128, 0, st>>>(pairs, nfo, nprim, u, dc);
+  double* dronly = dc + (size_t)npairs * nfo * DENS_LD;
+  if (npairs > 0) k_pair_dens_coef<<<npairs, 128, 0, st>>>(pairs, nfo, nprim, u, nch, dc, dronly);
   const dim3 grid(M.ntiles, nfo);
-  if (nch == 1) k_pair_density<1><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
-  else if (nch == 4) k_pair_density<4><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
-  else k_pair_density<10><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, rhog, ldr);
+#define PD(n) k_pair_density<n><<<grid, DENS_THREADS, 0, st>>>(M, npairs, pairs, cfo, cfo_ld, nfo, dc, dronly, rhog, ldr)
+  if (nch == 1) PD(1);
+  else if (nch == 4) PD(4);
+  else PD(10);
+#undef PD
 }
 
 }  // namespace flosic

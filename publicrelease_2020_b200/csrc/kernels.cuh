@@ -247,8 +247,8 @@ void launch_xc_rhog(const MeshDev& M, int gga, const int* xc, const double* rhog
 // 4 or 10) of each of nfo FOs, rhog[(ch*nfo + k)*ldr + p] over the mesh M,
 // from the pairs of every call at the points inside the call's RCUT sphere
 // (poisson1.f:849-948).  u: the FOs' primitive projections; cfo: the calls'
-// per-FO geometry (cfo_ld FOs per call); dc: npairs*nfo*pair_density_ld() doubles of scratch.
-int pair_density_ld();
+// per-FO geometry (cfo_ld FOs per call); dc: npairs*nfo*pair_density_ld(nch) doubles of scratch.
+int pair_density_ld(int nch);
 void launch_pair_density(int npairs, const PairGeo* pairs, const CallFO* cfo, int cfo_ld, int nfo, int nprim,
                          const double* u, int nch, const MeshDev& M, double* dc, double* rhog, size_t ldr,
                          cudaStream_t st);

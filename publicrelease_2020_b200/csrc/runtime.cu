@@ -873,7 +873,7 @@ void pair_density(flosic_ctx* c, int s, const CallFO* cfo) {
   SpinCache& S = c->spin[s];
   const int nf = S.nf, P = c->eval_n, nch = c->nch();
   const int npairs = (int)c->pairs.size();
-  c->d_dens_coef.ensure((size_t)std::max(npairs, 1) * nf * pair_density_ld());
+  c->d_dens_coef.ensure((size_t)std::max(npairs, 1) * nf * pair_density_ld(nch));
   S.rhog.ensure((size_t)nch * nf * P);
   launch_pair_density(npairs, c->d_pairs.p, cfo + S.kofs, S.kld, nf, c->nprim,
                       c->d_u.p + (size_t)S.kofs * c->nprim * 10, nch, c->eval_mesh(), c->d_dens_coef.p, S.rhog.p,
