@@ -662,7 +662,7 @@ void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems,
 }
 
 cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo* pairs, int npairs, int nfo,
-                               const double* coef, const int8_t* maxfmt, const CallFO* cfo, const double* momv,
+                               double* coef, const int8_t* maxfmt, const CallFO* cfo, double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
                                unsigned long long* cnt, cudaEvent_t mid, const SideStream& side, cudaStream_t st,
@@ -691,8 +691,8 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
   }
   if (mid) cudaEventRecord(mid, st);
   if (per_fo_only) cudaMemset2DAsync(vh, sizeof(double) * ldv, 0, sizeof(double) * M.n, nfo, st);
-  launch_perfo_setup(ncalls, npairs, nfo, calls, pairs, cfo, scr.share, per_fo_only, mixed, coef, momv, scr.coefp,
-                     scr.momp, scr.bound, st);
+  launch_perfo_setup(ncalls, npairs, nfo, calls, pairs, cfo, scr.share, per_fo_only, mixed, one_density, coef, momv,
+                     scr.bound, st);
   CoulombJob J{};
   J.ncalls = ncalls;
   J.nfo = nfo;
@@ -704,8 +704,6 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
   J.pair_fmt = scr.pair_fmt;
   J.cfo = cfo;
   J.momv = momv;
-  J.coefp = scr.coefp;
-  J.momp = scr.momp;
   J.bound = scr.bound;
   J.plist = scr.plist;
   J.M = M;

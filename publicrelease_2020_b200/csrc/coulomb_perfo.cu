@@ -45,20 +45,24 @@ __constant__ int8_t c_mma_row[NEAR_K] = {0,  5,  4,  3,  1,  8,  7,  6,  2,  14,
                                          26, 20, 17, 15, 28, 19, 16, 18, 27, 30, 24, 21, 22, 29, 23, 25,
                                          41, 45, 35, 31, 38, 44, 34, 36, 37, 43, 39, 32, -1, 42, 33, 40};
 
-// Coefficient rows of the per-FO calls' pairs in the order the lanes read them:
-// [pair][group g of four k-steps][FO][16].  The 16-byte piece of a row that
-// holds k-steps 4 g + 2 h and 4 g + 2 h + 1 of residue q is number 4 h + q.
+// Brings the coefficient rows of the per-FO calls' pairs into the order the lanes
+// read them, in place: nothing reads the former order after the call set-up, and a
+// second array would be as large as the coefficients.  A row is [group g of four
+// k-steps][16]; the 16-byte piece that holds k-steps 4 g + 2 h and 4 g + 2 h + 1 of
+// residue q is number 4 h + q of its group.  A warp takes a row at a time.
 __global__ void __launch_bounds__(256) k_perfo_pack(int nfo, const PairGeo* __restrict__ pairs,
                                                     const CallShare* __restrict__ share, int per_fo_only,
-                                                    const double* __restrict__ coef, double* __restrict__ out) {
-  const int pr = blockIdx.x;
+                                                    double* __restrict__ coef) {
+  const int pr = blockIdx.x, lane = threadIdx.x & 31;
   if (!per_fo_only && share[pairs[pr].call].shared) return;
-  const double* src = coef + (size_t)pr * nfo * COEF_LD;
-  double* dst = out + (size_t)pr * nfo * NEAR_K;
-  for (int e = threadIdx.x; e < nfo * NEAR_K; e += blockDim.x) {
-    const int g = e / (nfo * 16), f = e - g * nfo * 16, k = f >> 4;
-    const int row = c_mma_row[4 * (4 * g + 2 * ((f >> 3) & 1) + (f & 1)) + ((f >> 1) & 3)];
-    dst[e] = row >= 0 ? src[(size_t)k * COEF_LD + row] : 0.0;
+  auto from = [](int e) { return (int)c_mma_row[4 * (4 * (e >> 4) + 2 * ((e >> 3) & 1) + (e & 1)) + ((e >> 1) & 3)]; };
+  const int r0 = from(lane), r1 = lane < NEAR_K - 32 ? from(lane + 32) : -1;
+  for (int k = threadIdx.x >> 5; k < nfo; k += blockDim.x >> 5) {
+    double* row = coef + ((size_t)pr * nfo + k) * COEF_LD;
+    const double v0 = r0 >= 0 ? row[r0] : 0.0, v1 = r1 >= 0 ? row[r1] : 0.0;
+    __syncwarp();
+    row[lane] = v0;
+    if (lane < NEAR_K - 32) row[lane + 32] = v1;
   }
 }
 
@@ -326,10 +330,10 @@ __device__ __forceinline__ void near_block(const CoulombJob& J, int blk, int fob
       const uint8_t* list = S.list[w.lead];
       double* dst = S.A[b] + (w.pre - S.queue[e0].pre) * 16;
       for (int g = 0; g < w.fmt - 2; ++g, dst += nl * 16) {
-        const double* src = J.coefp + (((size_t)w.pair * 3 + g) * J.nfo + k0) * 16;
+        const double* src = J.coef + ((size_t)w.pair * J.nfo + k0) * COEF_LD + g * 16;
         for (int i = lane; i < nl * 8; i += 32) {
           const int r = i >> 3, pc = i & 7;
-          cp_async16(dst + r * 16 + 2 * (pc ^ ((r & 1) << 2)), src + (int)list[r] * 16 + 2 * pc);
+          cp_async16(dst + r * 16 + 2 * (pc ^ ((r & 1) << 2)), src + (int)list[r] * COEF_LD + 2 * pc);
         }
       }
       if (w.flags & NEAR_CUT) {
@@ -634,15 +638,15 @@ __device__ __forceinline__ float far_sum(const float* __restrict__ mv, float ux,
   return pot;
 }
 
-// Moments of the per-FO calls for k_perfo_far, rows of MOM_LD doubles: in FP64
-// times the leading factors of far_sum's recursion, prod_{i=m+1..l} (2i-1)/(i-m)
-// and prod_{i=2..m} (2i-1), in its order; in the mixed path rounded to FP32 in
-// the order of the moments (MOM_LD floats, then unused space).
+// Brings the moments of the per-FO calls into the form k_perfo_far reads, in place,
+// rows of MOM_LD doubles: in FP64 times the leading factors of far_sum's recursion,
+// prod_{i=m+1..l} (2i-1)/(i-m) and prod_{i=2..m} (2i-1), in its order; in the mixed
+// path rounded to FP32 in the order of the moments (MOM_LD floats, then unused space).
 __global__ void __launch_bounds__(64) k_perfo_pack_mom(int nfo, int mixed, int per_fo_only,
                                                        const CallShare* __restrict__ share,
-                                                       const double* __restrict__ momv, double* __restrict__ out) {
+                                                       double* __restrict__ momv) {
   const int c = blockIdx.x, j = threadIdx.x;
-  if ((!per_fo_only && share[c].shared) || j >= MOM_LD) return;
+  if (!per_fo_only && share[c].shared) return;
   int pos = j;
   double f = j < NMOM ? 1.0 : 0.0;
   if (!mixed && j < NMOM) {
@@ -656,10 +660,12 @@ __global__ void __launch_bounds__(64) k_perfo_pack_mom(int nfo, int mixed, int p
     pos = j == NMOM ? 7 : j;  // the positions far_pos leaves out
   }
   for (int k = blockIdx.y; k < nfo; k += gridDim.y) {
-    const size_t r = ((size_t)c * nfo + k) * MOM_LD;
-    const double v = j < NMOM ? momv[r + j] * f : 0.0;
-    if (mixed) reinterpret_cast<float*>(out + r)[j] = (float)v;
-    else out[r + pos] = v;
+    double* row = momv + ((size_t)c * nfo + k) * MOM_LD;
+    const double v = j < NMOM ? row[j] * f : 0.0;
+    __syncthreads();
+    if (j >= MOM_LD) continue;
+    if (mixed) reinterpret_cast<float*>(row)[j] = (float)v;
+    else row[pos] = v;
   }
 }
 
@@ -728,7 +734,7 @@ __device__ __forceinline__ void far_block(const CoulombJob& J, int tile, int grp
       if (r < nk * MP) {
         const int kk = r / MP, o = r - kk * MP;
         cp_async16(reinterpret_cast<char*>(S.mv[b][i][kk]) + 16 * o,
-                   reinterpret_cast<const char*>(J.momp + (ck + kk) * MOM_LD) + 16 * o);
+                   reinterpret_cast<const char*>(J.momv + (ck + kk) * MOM_LD) + 16 * o);
       } else {
         cp_async16(reinterpret_cast<char*>(S.f[b][i]) + 16 * (r - nk * MP),
                    reinterpret_cast<const char*>(J.cfo + ck) + 16 * (r - nk * MP));
@@ -1025,14 +1031,13 @@ cudaError_t init_coulomb_perfo() {
 }
 
 void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
-                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed,
-                        const double* coef, const double* momv, double* coefp, double* momp, CallBound* bound,
-                        cudaStream_t st) {
+                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed, bool one_density,
+                        double* coef, double* momv, CallBound* bound, cudaStream_t st) {
   if (ncalls <= 0 || npairs <= 0) return;
   k_perfo_bounds<<<(ncalls + 7) / 8, 256, 0, st>>>(ncalls, nfo, calls, pairs, cfo, bound);
-  k_perfo_pack<<<npairs, 256, 0, st>>>(nfo, pairs, share, per_fo_only ? 1 : 0, coef, coefp);
-  k_perfo_pack_mom<<<dim3(ncalls, std::min(nfo, 32)), 64, 0, st>>>(nfo, mixed ? 1 : 0, per_fo_only ? 1 : 0, share, momv,
-                                                                  momp);
+  if (!one_density)  // k_one_near reads the coefficients in their first order
+    k_perfo_pack<<<npairs, 256, 0, st>>>(nfo, pairs, share, per_fo_only ? 1 : 0, coef);
+  k_perfo_pack_mom<<<dim3(ncalls, std::min(nfo, 32)), 64, 0, st>>>(nfo, mixed ? 1 : 0, per_fo_only ? 1 : 0, share, momv);
 }
 
 template <int MT>

@@ -86,10 +86,8 @@ struct CoulombScratch {
   float* coef_hl;      // mixed path: TF32 hi/lo split of the coefficients (2 x npairs*nfo*COEF_LD)
   float* momv_hl;      // mixed path: TF32 hi/lo split of the moments (2 x ncalls*nfo*MOM_LD)
   int* err;            // mixed path: set when a tensor-core pipeline wait reached its limit
-  double* coefp;       // npairs*nfo*NEAR_K: the per-FO calls' coefficients in MMA order
-  double* momp;        // ncalls*nfo*MOM_LD: their moments as the far kernel reads them
   CallBound* bound;    // ncalls
-  double* seg;         // perfo_seg_size doubles
+  double* seg;         // perfo_seg_size doubles (one density: 2 * one_density_parts * ldv)
 };
 // Kernel choices (all evaluate the same sums; the results differ only by the
 // rounding of the chosen arithmetic).  per_fo_only: every call through the
@@ -112,12 +110,10 @@ struct CoulombJob {
   const CallShare* share;
   const CallInfo* calls;
   const PairGeo* pairs;
-  const double* coef;
+  const double* coef;             // of the per-FO calls' pairs in MMA order
   const int8_t* pair_fmt;
   const CallFO* cfo;
-  const double* momv;
-  const double* coefp;
-  const double* momp;
+  const double* momv;             // of the per-FO calls as the far kernel reads them
   const CallBound* bound;
   const PerfoPair* plist;
   MeshDev M;
@@ -137,13 +133,13 @@ void launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int 
 // in list order from a device counter (zeroed here) by nctas CTAs.
 void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
                           const double* boys_tab, int nctas, cudaStream_t st);
-// Per-FO calls (csrc/coulomb_perfo.cu): spheres of the calls and coefficients
-// in MMA order, then the far and the near field added to vh.
+// Per-FO calls (csrc/coulomb_perfo.cu): spheres of the calls, and their
+// coefficients and moments brought into the kernels' order in place (the
+// coefficients not for one density), then the far and the near field added to vh.
 cudaError_t init_coulomb_perfo();
 void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
-                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed,
-                        const double* coef, const double* momv, double* coefp, double* momp, CallBound* bound,
-                        cudaStream_t st);
+                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed, bool one_density,
+                        double* coef, double* momv, CallBound* bound, cudaStream_t st);
 inline int perfo_default_wm(int nfo) { return nfo > 32 ? 2 : 1; }
 // Parts of the call list: a small mesh does not fill the chip with one CTA per
 // 64 points, so its calls are walked in up to 8 parts whose sums are added in
@@ -183,9 +179,10 @@ cudaError_t launch_coulomb_shared_tc(int ncalls, const int* lists, const CallSha
                                      const double* boys_tab, double* vh, int ldv, unsigned long long* cnt, int* err,
                                      long long wait_limit, cudaStream_t st);
 // cnt[0..2]: near/far/terms of the shared-geometry kernel, cnt[3..5]: of the per-FO kernel;
-// mid (may be null) is recorded between the two kernels.
+// mid (may be null) is recorded between the two kernels.  coef and momv of the
+// per-FO calls are left in the order of their kernels.
 cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo* pairs, int npairs, int nfo,
-                               const double* coef, const int8_t* maxfmt, const CallFO* cfo, const double* momv,
+                               double* coef, const int8_t* maxfmt, const CallFO* cfo, double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
                                unsigned long long* cnt, cudaEvent_t mid, const SideStream& side, cudaStream_t st,

@@ -256,7 +256,7 @@ struct TypeInfo {
 // Coulomb inputs of one spin for a batched launch over many molecules (the
 // per-molecule path keeps them in the context and reuses them per spin).
 struct CoulBufs {
-  DevBuf<double> coef, cgp, mom, coefp, momp, seg;
+  DevBuf<double> coef, cgp, mom;
   DevBuf<CallBound> bound;
   DevBuf<PerfoPair> plist;
   DevBuf<int> again;
@@ -269,9 +269,6 @@ struct CoulBufs {
     coef.release();
     cgp.release();
     mom.release();
-    coefp.release();
-    momp.release();
-    seg.release();
     bound.release();
     plist.release();
     again.release();
@@ -373,7 +370,6 @@ struct flosic_ctx {
   DevBuf<double> d_basis, d_fodpts, d_psig, d_tmat, d_u, d_coef, d_cgp, d_mom, d_part, d_sums, d_sic, d_tmp;
   DevBuf<int8_t> d_maxfmt, d_pairfmt;
   DevBuf<CallShare> d_share;
-  DevBuf<double> d_coefp, d_momp, d_seg;
   DevBuf<CallBound> d_bound;
   DevBuf<PerfoPair> d_plist;
   DevBuf<int> d_again;
@@ -835,15 +831,13 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
     c->d_tc_err.ensure(1);
     CUDA_CHECK(cudaMemsetAsync(c->d_tc_err.p, 0, sizeof(int), st));
   }
-  c->d_coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
-  c->d_momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
   c->d_bound.ensure((size_t)std::max(ncalls, 1));
   // one density (COUPOT1) in FP64 has kernels of its own
   const bool one = dm != nullptr && !mixed && !c->coulomb_cfg.per_fo_only;
-  c->d_seg.ensure(one ? (size_t)2 * one_density_parts(c->eval_nt) * P : perfo_seg_size(c->eval_nt, nf, P));
+  // the parts' sums in the buffer that XC fills with the scaled potentials afterwards
+  c->d_tmp.ensure(one ? (size_t)2 * one_density_parts(c->eval_nt) * P : perfo_seg_size(c->eval_nt, nf, P));
   CoulombScratch scr{c->d_pairfmt.p, c->d_share.p,  c->d_lists.p, c->d_plist.p, c->d_coef_hl.p,
-                     c->d_momv_hl.p, c->d_tc_err.p, c->d_coefp.p, c->d_momp.p,
-                     c->d_bound.p,   c->d_seg.p};
+                     c->d_momv_hl.p, c->d_tc_err.p, c->d_bound.p, c->d_tmp.p};
   CUDA_CHECK(launch_coulomb_mma(ncalls, c->d_calls.p, c->d_pairs.p, npairs, nf, c->d_coef.p, c->d_maxfmt.p,
                                 c->d_callfo.p, c->d_mom.p, c->eval_mesh(), c->d_boys.p, vh, P, c->coulomb_cfg, mixed,
                                 scr, c->d_cnt.p, c->ev[8], c->side, st, one));
@@ -1292,15 +1286,14 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn, B.coef.p,
                     B.maxfmt.p, B.cgp.p, c->mesh_dev(), c->d_boys.p, B.callfo.p, B.mom.p, B.again.p, st);
   CUDA_CHECK(cudaMemsetAsync(B.cnt.p, 0, 3 * sizeof(unsigned long long), st));
-  B.coefp.ensure((size_t)std::max(npairs, 1) * nf * NEAR_K);
-  B.momp.ensure((size_t)std::max(ncalls, 1) * nf * MOM_LD);
   B.bound.ensure((size_t)std::max(ncalls, 1));
-  B.seg.ensure(perfo_seg_size(c->eval_nt, nf, P));
-  CoulombScratch scr{B.pairfmt.p, B.share.p, B.lists.p, B.plist.p, nullptr, nullptr, nullptr, B.coefp.p, B.momp.p,
-                     B.bound.p, B.seg.p};
+  // the parts' sums in the buffer that XC fills with the SIC potentials afterwards
+  DevBuf<double>& seg = c->spin[s0].vpot;
+  seg.ensure(perfo_seg_size(c->eval_nt, nf, P));
+  CoulombScratch scr{B.pairfmt.p, B.share.p, B.lists.p, B.plist.p, nullptr, nullptr, nullptr, B.bound.p, seg.p};
   launch_coulomb_classify(ncalls, c->d_calls.p, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
   launch_perfo_setup(ncalls, npairs, nf, c->d_calls.p, c->d_pairs.p, B.callfo.p, B.share.p, false,
-                     c->precision == FLOSIC_PRECISION_MIXED, B.coef.p, B.mom.p, B.coefp.p, B.momp.p, B.bound.p, st);
+                     c->precision == FLOSIC_PRECISION_MIXED, false, B.coef.p, B.mom.p, B.bound.p, st);
   c->launches += 8;
   for (int s = s0; s < s0 + ns; ++s) pair_density(c, s, B.callfo.p);
   CoulombJob J{};
@@ -1315,13 +1308,11 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   J.pair_fmt = B.pairfmt.p;
   J.cfo = B.callfo.p;
   J.momv = B.mom.p;
-  J.coefp = B.coefp.p;
-  J.momp = B.momp.p;
   J.bound = B.bound.p;
   J.plist = B.plist.p;
   J.M = c->eval_mesh();
   J.nseg = perfo_parts(c->eval_nt);
-  J.seg = B.seg.p;
+  J.seg = seg.p;
   J.vh = c->spin[s0].vh.p;
   J.cnt = B.cnt.p;
   J.cnt_perfo = B.cnt.p;
@@ -1437,7 +1428,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_basis.release(); c->d_fodpts.release(); c->d_psig.release(); c->d_tmat.release(); c->d_u.release();
   c->d_coef.release(); c->d_cgp.release(); c->d_mom.release(); c->d_part.release(); c->d_sums.release();
   c->d_sic.release(); c->d_tmp.release(); c->d_maxfmt.release(); c->d_callfo.release(); c->d_cnt.release(); c->d_pairfmt.release();
-  c->d_coefp.release(); c->d_momp.release(); c->d_seg.release(); c->d_bound.release(); c->d_plist.release(); c->d_again.release();
+  c->d_bound.release(); c->d_plist.release(); c->d_again.release();
   c->d_share.release(); c->d_lists.release(); c->d_setup_list.release();
   c->d_eig_a.release(); c->d_eig_w.release(); c->d_eig_v.release(); c->d_eig_work.release(); c->d_eig_info.release();
   c->d_fot.release(); c->d_force.release();
