@@ -632,12 +632,13 @@ static void launch_shared(int ncalls, const int* lists, const CallShare* share, 
         ncalls, lists, share, calls, nfo, coef, pair_fmt, pairs, momv, M, boys_tab, vh, ldv, cnt, whole, cut);
 }
 
-void launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
-                             const CallFO* cfo, const CoulombScratch& scr, bool per_fo_only, cudaStream_t st) {
+int launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
+                            const CallFO* cfo, const CoulombScratch& scr, bool per_fo_only, cudaStream_t st) {
   if (npairs > 0) k_pair_fmt<<<(npairs + 127) / 128, 128, 0, st>>>(npairs, nfo, maxfmt, scr.pair_fmt);
   if (ncalls > 0) k_call_share<<<(ncalls + 7) / 8, 256, 0, st>>>(ncalls, nfo, cfo, scr.share);
   k_call_lists<<<1, LIST_THREADS, 0, st>>>(ncalls, per_fo_only ? 1 : 0, scr.share, calls, scr.pair_fmt, scr.lists,
                                            scr.plist);
+  return 1 + (npairs > 0 ? 1 : 0) + (ncalls > 0 ? 1 : 0);
 }
 
 template <int WM>
@@ -651,14 +652,15 @@ static void launch_batch_wm(const CoulombJob* jobs, const int4* items, int nitem
                                                                                            boys_tab);
 }
 
-void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
-                          const double* boys_tab, int nctas, cudaStream_t st) {
-  if (nitems <= 0) return;
+int launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
+                         const double* boys_tab, int nctas, cudaStream_t st) {
+  if (nitems <= 0) return 0;
   nctas = std::max(1, std::min(nctas, nitems));
   cudaMemsetAsync(counter, 0, sizeof(int), st);
   if (wm == 4) launch_batch_wm<4>(jobs, items, nitems, counter, mixed, boys_tab, nctas, st);
   else if (wm == 2) launch_batch_wm<2>(jobs, items, nitems, counter, mixed, boys_tab, nctas, st);
   else launch_batch_wm<1>(jobs, items, nitems, counter, mixed, boys_tab, nctas, st);
+  return 1;
 }
 
 cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo* pairs, int npairs, int nfo,
@@ -666,14 +668,15 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
                                unsigned long long* cnt, cudaEvent_t mid, const SideStream& side, cudaStream_t st,
-                               bool one_density) {
+                               bool one_density, long long* launched) {
   // one density in FP64: every call by k_one_near and k_perfo_far
   const bool per_fo_only = cfg.per_fo_only || one_density;
-  launch_coulomb_classify(ncalls, calls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
+  *launched += launch_coulomb_classify(ncalls, calls, npairs, nfo, maxfmt, cfo, scr, per_fo_only, st);
+  if (!per_fo_only) ++*launched;  // the shared-geometry kernel
   if (!per_fo_only && mixed && cfg.shared_tc) {
     const size_t nc = (size_t)npairs * nfo * COEF_LD, nm = (size_t)ncalls * nfo * MOM_LD;
-    launch_split_tf32((size_t)npairs, nfo, scr.share, pairs, coef, scr.coef_hl, st);
-    launch_split_tf32((size_t)ncalls, nfo, scr.share, nullptr, momv, scr.momv_hl, st);
+    *launched += launch_split_tf32((size_t)npairs, nfo, scr.share, pairs, coef, scr.coef_hl, st);
+    *launched += launch_split_tf32((size_t)ncalls, nfo, scr.share, nullptr, momv, scr.momv_hl, st);
     const cudaError_t e = launch_coulomb_shared_tc(ncalls, scr.lists, scr.share, calls, nfo, scr.coef_hl, nc,
                                                    scr.pair_fmt, pairs, scr.momv_hl, nm, M, boys_tab, vh, ldv, cnt,
                                                    scr.err, cfg.wait_limit, st);
@@ -691,8 +694,8 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
   }
   if (mid) cudaEventRecord(mid, st);
   if (per_fo_only) cudaMemset2DAsync(vh, sizeof(double) * ldv, 0, sizeof(double) * M.n, nfo, st);
-  launch_perfo_setup(ncalls, npairs, nfo, calls, pairs, cfo, scr.share, per_fo_only, mixed, one_density, coef, momv,
-                     scr.bound, st);
+  *launched += launch_perfo_setup(ncalls, npairs, nfo, calls, pairs, cfo, scr.share, per_fo_only, mixed, one_density,
+                                  coef, momv, scr.bound, st);
   CoulombJob J{};
   J.ncalls = ncalls;
   J.nfo = nfo;
@@ -713,11 +716,11 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
   J.coef = coef;
   if (one_density) {
     J.nseg = one_density_parts(M.ntiles);
-    launch_one_density(J, boys_tab, st);
+    *launched += launch_one_density(J, boys_tab, st);
     return cudaGetLastError();
   }
   J.nseg = perfo_parts(M.ntiles);
-  launch_perfo(J, cfg.perfo_wm > 0 ? cfg.perfo_wm : perfo_default_wm(nfo), mixed, boys_tab, side, st);
+  *launched += launch_perfo(J, cfg.perfo_wm > 0 ? cfg.perfo_wm : perfo_default_wm(nfo), mixed, boys_tab, side, st);
   return cudaGetLastError();
 }
 

@@ -1030,14 +1030,15 @@ cudaError_t init_coulomb_perfo() {
   return e;
 }
 
-void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
-                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed, bool one_density,
-                        double* coef, double* momv, CallBound* bound, cudaStream_t st) {
-  if (ncalls <= 0 || npairs <= 0) return;
+int launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
+                       const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed, bool one_density,
+                       double* coef, double* momv, CallBound* bound, cudaStream_t st) {
+  if (ncalls <= 0 || npairs <= 0) return 0;
   k_perfo_bounds<<<(ncalls + 7) / 8, 256, 0, st>>>(ncalls, nfo, calls, pairs, cfo, bound);
   if (!one_density)  // k_one_near reads the coefficients in their first order
     k_perfo_pack<<<npairs, 256, 0, st>>>(nfo, pairs, share, per_fo_only ? 1 : 0, coef);
   k_perfo_pack_mom<<<dim3(ncalls, std::min(nfo, 32)), 64, 0, st>>>(nfo, mixed ? 1 : 0, per_fo_only ? 1 : 0, share, momv);
+  return one_density ? 2 : 3;
 }
 
 template <int MT>
@@ -1050,9 +1051,9 @@ static void launch_near(const CoulombJob& J, bool mixed, const double* tab, cuda
 // The near field starts on st, the far field on the side stream: its small CTAs
 // fill the SMs as the near field's uneven ones end (benzene, 296 tiles: 28.6 ->
 // 24.7 ms both).
-void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* tab, const SideStream& side,
-                  cudaStream_t st) {
-  if (J.M.ntiles <= 0 || J.nfo <= 0) return;
+int launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* tab, const SideStream& side,
+                 cudaStream_t st) {
+  if (J.M.ntiles <= 0 || J.nfo <= 0) return 0;
   cudaEventRecord(side.fork, st);
   cudaStreamWaitEvent(side.st, side.fork, 0);
   if (wm == 4) launch_near<16>(J, mixed, tab, st);
@@ -1064,16 +1065,18 @@ void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* tab, co
   cudaEventRecord(side.join, side.st);
   cudaStreamWaitEvent(st, side.join, 0);
   k_perfo_add<<<dim3(J.M.ntiles, J.nfo), TILE, 0, st>>>(J);
+  return 3;
 }
 
 // Enough CTAs for eight per SM, at least a window of pairs each.
 int one_density_parts(int ntiles) { return std::max(2, std::min(32, 8 * 148 / std::max(ntiles, 1))); }
 
-void launch_one_density(const CoulombJob& J, const double* tab, cudaStream_t st) {
-  if (J.M.ntiles <= 0) return;
+int launch_one_density(const CoulombJob& J, const double* tab, cudaStream_t st) {
+  if (J.M.ntiles <= 0) return 0;
   k_perfo_far<1, false><<<dim3(J.M.ntiles, 1, J.nseg), far_threads(1), 0, st>>>(J);
   k_one_near<<<dim3(J.M.ntiles, J.nseg), TILE, 0, st>>>(J, tab);
   k_perfo_add<<<dim3(J.M.ntiles, 1), TILE, 0, st>>>(J);
+  return 3;
 }
 
 template <int MT>
@@ -1084,9 +1087,9 @@ static void launch_near_batch(const CoulombJob* jobs, const int4* items, int nit
   else k_perfo_near_batch<MT, false><<<grid, NEAR_THREADS, sizeof(NearSmem<MT>), st>>>(jobs, items, tab);
 }
 
-void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, int wm, bool mixed,
-                        const double* tab, cudaStream_t st) {
-  if (nitems <= 0) return;
+int launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, int wm, bool mixed,
+                       const double* tab, cudaStream_t st) {
+  if (nitems <= 0) return 0;
   const dim3 grid(nitems, 32 * wm / FAR_FOS, parts);
   if (mixed) k_perfo_far_batch<true><<<grid, far_threads(FAR_FOS), 0, st>>>(jobs, items, 32 * wm);
   else k_perfo_far_batch<false><<<grid, far_threads(FAR_FOS), 0, st>>>(jobs, items, 32 * wm);
@@ -1094,6 +1097,7 @@ void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, i
   else if (wm == 2) launch_near_batch<8>(jobs, items, nitems, parts, mixed, tab, st);
   else launch_near_batch<4>(jobs, items, nitems, parts, mixed, tab, st);
   k_perfo_add_batch<<<nitems, TILE, 0, st>>>(jobs, items, 32 * wm);
+  return 3;
 }
 
 }  // namespace flosic

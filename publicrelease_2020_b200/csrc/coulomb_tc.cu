@@ -686,11 +686,12 @@ void init_coulomb_tc() {
   cudaFuncSetAttribute(k_coulomb_shared_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
 }
 
-void launch_split_tf32(size_t nrow, int nfo, const CallShare* share, const PairGeo* pairs, const double* src,
-                       float* out, cudaStream_t st) {
-  if (nrow == 0 || nfo == 0) return;
+int launch_split_tf32(size_t nrow, int nfo, const CallShare* share, const PairGeo* pairs, const double* src,
+                      float* out, cudaStream_t st) {
+  if (nrow == 0 || nfo == 0) return 0;
   const int blocks = (int)std::min<size_t>(nrow, 148 * 16);
   k_split_tf32<<<blocks, 256, 0, st>>>(nrow, nfo, share, pairs, src, out, nrow * nfo * KSEG);
+  return 1;
 }
 
 namespace {

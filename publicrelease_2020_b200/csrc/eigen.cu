@@ -288,16 +288,16 @@ size_t sym_eigen_work(int n) {
 }
 size_t sym_eigen_info(int n) { return (size_t)n + 2; }
 
-bool launch_sym_eigen(int n, const double* a, double* work, double* w, double* v, int* info, cudaStream_t st) {
-  if (n < 1 || n > EIG_MAX_N) return false;
+int launch_sym_eigen(int n, const double* a, double* work, double* w, double* v, int* info, cudaStream_t st) {
+  if (n < 1 || n > EIG_MAX_N) return 0;
   if (n <= EIG_SMEM_MAX_N) {
     double2* rot = reinterpret_cast<double2*>(work);
     k_sym_eigen_rot<<<1, EIG_THREADS, sizeof(double) * n * (n + 1), st>>>(n, a, rot, w, info);
     k_sym_eigen_vec<<<n, 32, 0, st>>>(n, rot, info, v);
-  } else {
-    k_sym_eigen<<<1, EIG_THREADS, 0, st>>>(n, a, work, work + (size_t)n * (n + 1), w, v, info);
+    return 2;
   }
-  return true;
+  k_sym_eigen<<<1, EIG_THREADS, 0, st>>>(n, a, work, work + (size_t)n * (n + 1), w, v, info);
+  return 1;
 }
 
 }  // namespace flosic

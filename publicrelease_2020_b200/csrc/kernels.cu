@@ -969,11 +969,11 @@ void init_call_setup() {
                        (int)(sizeof(double) * NANG * (GEO_LD + NMOM)));
 }
 
-void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo* calls, const PairGeo* pairs,
-                       int nfo, int nspn, const double* coef, const int8_t* maxfmt, const double* cgp,
-                       const MeshDev& M, const double* boys_tab, CallFO* cfo, double* momv, int* again,
-                       cudaStream_t st) {
-  if (ncalls <= 0) return;
+int launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo* calls, const PairGeo* pairs,
+                      int nfo, int nspn, const double* coef, const int8_t* maxfmt, const double* cgp,
+                      const MeshDev& M, const double* boys_tab, CallFO* cfo, double* momv, int* again,
+                      cudaStream_t st) {
+  if (ncalls <= 0) return 0;
   if (nsingle > 0)
     k_call_setup_single<<<nsingle, SETUP1_THREADS, sizeof(double) * NANG * (GEO_LD + NMOM), st>>>(
         list, calls, pairs, nfo, nspn, coef, maxfmt, M, boys_tab, cfo, momv);
@@ -992,6 +992,7 @@ void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo*
     k_call_moments_again<<<(int)std::min<size_t>(3 * 148, warps), AGAIN_THREADS, sizeof(double) * NANG * NMOM, st>>>(
         again, nfo, calls, pairs, coef, maxfmt, boys_tab, cfo, momv);
   }
+  return (nsingle > 0 ? 1 : 0) + (nmulti > 0 ? 3 : 0);
 }
 
 // ---------------------------------------------------------------------------

@@ -7,6 +7,8 @@
 
 namespace flosic {
 
+// The launch_* functions that return int return how many kernels they launched.
+
 // Basis tables in device memory (general-contraction NRLMOL layout).
 struct BasisDev {
   int natoms, ntypes, nbasis, nprim;
@@ -64,10 +66,10 @@ void init_call_setup();
 // list: the nsingle calls of one slot (one pair, NSPN=1; CG/RCUT/NPOT shared
 // by all FOs, set up once per call), then the other calls (once per FO).
 // again: scratch of 1 + (ncalls - nsingle)*nfo ints.
-void launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo* calls, const PairGeo* pairs,
-                       int nfo, int nspn, const double* coef, const int8_t* maxfmt, const double* cgp,
-                       const MeshDev& M, const double* boys_tab, CallFO* cfo, double* momv, int* again,
-                       cudaStream_t st);
+int launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo* calls, const PairGeo* pairs,
+                      int nfo, int nspn, const double* coef, const int8_t* maxfmt, const double* cgp,
+                      const MeshDev& M, const double* boys_tab, CallFO* cfo, double* momv, int* again,
+                      cudaStream_t st);
 
 // Coulomb potential of every FO at every mesh point, vh[k*ldv + p], on the
 // FP64 tensor cores (csrc/coulomb_mma.cu).  Calls whose near/far geometry is
@@ -126,20 +128,20 @@ struct CoulombJob {
 void init_coulomb_mma();
 // Pair Boys variants, shared-geometry flags and the two call lists (the set-up
 // of launch_coulomb_mma before its kernels).
-void launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
-                             const CallFO* cfo, const CoulombScratch& scr, bool per_fo_only, cudaStream_t st);
+int launch_coulomb_classify(int ncalls, const CallInfo* calls, int npairs, int nfo, const int8_t* maxfmt,
+                            const CallFO* cfo, const CoulombScratch& scr, bool per_fo_only, cudaStream_t st);
 // The shared-geometry calls of every (job, tile, FO block) item of a batch in
 // one persistent launch: items[i] = {job, tile, FO block of 32*wm FOs, 0}, taken
 // in list order from a device counter (zeroed here) by nctas CTAs.
-void launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
-                          const double* boys_tab, int nctas, cudaStream_t st);
+int launch_coulomb_batch(const CoulombJob* jobs, const int4* items, int nitems, int* counter, int wm, bool mixed,
+                         const double* boys_tab, int nctas, cudaStream_t st);
 // Per-FO calls (csrc/coulomb_perfo.cu): spheres of the calls, and their
 // coefficients and moments brought into the kernels' order in place (the
 // coefficients not for one density), then the far and the near field added to vh.
 cudaError_t init_coulomb_perfo();
-void launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
-                        const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed, bool one_density,
-                        double* coef, double* momv, CallBound* bound, cudaStream_t st);
+int launch_perfo_setup(int ncalls, int npairs, int nfo, const CallInfo* calls, const PairGeo* pairs,
+                       const CallFO* cfo, const CallShare* share, bool per_fo_only, bool mixed, bool one_density,
+                       double* coef, double* momv, CallBound* bound, cudaStream_t st);
 inline int perfo_default_wm(int nfo) { return nfo > 32 ? 2 : 1; }
 // Parts of the call list: a small mesh does not fill the chip with one CTA per
 // 64 points, so its calls are walked in up to 8 parts whose sums are added in
@@ -157,20 +159,20 @@ struct SideStream {
   cudaStream_t st = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
-void launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* boys_tab, const SideStream& side,
-                  cudaStream_t st);
+int launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* boys_tab, const SideStream& side,
+                 cudaStream_t st);
 // The potential of one density (nfo = 1, FP64) added to vh: near field by one
 // point per thread, far field as above; seg holds one_density_parts * 2 * ldv doubles.
 int one_density_parts(int ntiles);
-void launch_one_density(const CoulombJob& J, const double* boys_tab, cudaStream_t st);
+int launch_one_density(const CoulombJob& J, const double* boys_tab, cudaStream_t st);
 // parts: the largest nseg of the jobs
-void launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, int wm, bool mixed,
-                        const double* boys_tab, cudaStream_t st);
+int launch_perfo_batch(const CoulombJob* jobs, const int4* items, int nitems, int parts, int wm, bool mixed,
+                       const double* boys_tab, cudaStream_t st);
 void init_coulomb_tc();
 // TF32 hi/lo split of nrow x nfo rows of KSEG doubles into the chunk-major
 // [nrow][KSEG/4][nfo][4] layout (hi, then lo at + nrow*nfo*KSEG floats).
-void launch_split_tf32(size_t nrow, int nfo, const CallShare* share, const PairGeo* pairs, const double* src,
-                       float* out, cudaStream_t st);
+int launch_split_tf32(size_t nrow, int nfo, const CallShare* share, const PairGeo* pairs, const double* src,
+                      float* out, cudaStream_t st);
 // Mixed-precision shared-geometry Coulomb GEMM on tcgen05 (csrc/coulomb_tc.cu);
 // the A rows reach shared memory by TMA through tensor maps built here.
 cudaError_t launch_coulomb_shared_tc(int ncalls, const int* lists, const CallShare* share, const CallInfo* calls,
@@ -180,13 +182,13 @@ cudaError_t launch_coulomb_shared_tc(int ncalls, const int* lists, const CallSha
                                      long long wait_limit, cudaStream_t st);
 // cnt[0..2]: near/far/terms of the shared-geometry kernel, cnt[3..5]: of the per-FO kernel;
 // mid (may be null) is recorded between the two kernels.  coef and momv of the
-// per-FO calls are left in the order of their kernels.
+// per-FO calls are left in the order of their kernels; *launched += the kernels launched.
 cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo* pairs, int npairs, int nfo,
                                double* coef, const int8_t* maxfmt, const CallFO* cfo, double* momv,
                                const MeshDev& M, const double* boys_tab, double* vh, int ldv,
                                const CoulombConfig& cfg, bool mixed, const CoulombScratch& scr,
                                unsigned long long* cnt, cudaEvent_t mid, const SideStream& side, cudaStream_t st,
-                               bool one_density = false);
+                               bool one_density, long long* launched);
 
 // Exchange-correlation of the FO densities (fully polarised, NSPN forced to 2 as
 // in apotnl_sic.F:419) from the FO values/derivatives phi[(ch*nfo+k)*ldp+p];
@@ -231,10 +233,11 @@ void launch_scale_rows(int P, int N, const double* a, int lda, const double* w, 
 // Symmetric eigen-decomposition (one CTA, cyclic Jacobi; csrc/eigen.cu): a is
 // n x n row-major, work holds sym_eigen_work(n) doubles; w ascending,
 // v[k*n + m] = component k of eigenvector m; info 0, or 1 without convergence.
+// Returns the kernels launched, 0 for an n the solver does not hold.
 cudaError_t init_sym_eigen();
 size_t sym_eigen_work(int n);
 size_t sym_eigen_info(int n);  // ints of info; info[0] is the status
-bool launch_sym_eigen(int n, const double* a, double* work, double* w, double* v, int* info, cudaStream_t st);
+int launch_sym_eigen(int n, const double* a, double* work, double* w, double* v, int* info, cudaStream_t st);
 cudaError_t preload_xc_rhog();
 int xc_rhog_blocks(int npts);
 void launch_xc_rhog(const MeshDev& M, int gga, const int* xc, const double* rhog, int ldr, double* vxc,

@@ -674,9 +674,9 @@ void device_eigen(flosic_ctx* c, int n, std::vector<double>& w, std::vector<doub
   c->d_eig_v.ensure((size_t)n * n);
   c->d_eig_work.ensure(sym_eigen_work(n));
   c->d_eig_info.ensure(sym_eigen_info(n));
-  if (!launch_sym_eigen(n, c->d_eig_a.p, c->d_eig_work.p, c->d_eig_w.p, c->d_eig_v.p, c->d_eig_info.p, st))
-    fail(FLOSIC_ERR_CAPACITY, "LOWSIC: more FOs per spin than the eigen-solver holds");
-  c->launches += 2;
+  const int ran = launch_sym_eigen(n, c->d_eig_a.p, c->d_eig_work.p, c->d_eig_w.p, c->d_eig_v.p, c->d_eig_info.p, st);
+  if (ran == 0) fail(FLOSIC_ERR_CAPACITY, "LOWSIC: more FOs per spin than the eigen-solver holds");
+  c->launches += ran;
   CUDA_CHECK(cudaGetLastError());
   v.resize((size_t)n * n);
   w.resize(n);
@@ -812,11 +812,10 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
   CUDA_CHECK(cudaEventRecord(c->ev[2], st));
   launch_pair_coef(npairs, c->d_pairs.p, c->d_calls.p, nf, c->nprim, c->d_u.p, dm, c->nspn, c->d_coef.p,
                    c->d_maxfmt.p, c->d_cgp.p, st);
-  c->launches++;
-  launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn, c->d_coef.p,
-                    c->d_maxfmt.p, c->d_cgp.p, c->mesh_dev(), c->d_boys.p, c->d_callfo.p, c->d_mom.p,
-                    c->d_again.p, st);
-  c->launches++;
+  c->launches += npairs > 0 ? 1 : 0;
+  c->launches += launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn,
+                                   c->d_coef.p, c->d_maxfmt.p, c->d_cgp.p, c->mesh_dev(), c->d_boys.p, c->d_callfo.p,
+                                   c->d_mom.p, c->d_again.p, st);
   CUDA_CHECK(cudaEventRecord(c->ev[3], st));
   c->d_pairfmt.ensure((size_t)std::max(npairs, 1));
   c->d_share.ensure((size_t)std::max(ncalls, 1));
@@ -840,9 +839,8 @@ void coulomb_eval(flosic_ctx* c, int nf, const double* dm, double* vh) {
                      c->d_momv_hl.p, c->d_tc_err.p, c->d_bound.p, c->d_tmp.p};
   CUDA_CHECK(launch_coulomb_mma(ncalls, c->d_calls.p, c->d_pairs.p, npairs, nf, c->d_coef.p, c->d_maxfmt.p,
                                 c->d_callfo.p, c->d_mom.p, c->eval_mesh(), c->d_boys.p, vh, P, c->coulomb_cfg, mixed,
-                                scr, c->d_cnt.p, c->ev[8], c->side, st, one));
+                                scr, c->d_cnt.p, c->ev[8], c->side, st, one, &c->launches));
   CUDA_CHECK(cudaEventRecord(c->ev[9], st));
-  c->launches += c->coulomb_cfg.per_fo_only ? 9 : 10;
   unsigned long long cnt[6];
   int tc_err = 0;
   CUDA_CHECK(cudaMemcpyAsync(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost, st));
@@ -1283,18 +1281,19 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   B.cnt.ensure(3);
   launch_pair_coef(npairs, c->d_pairs.p, c->d_calls.p, nf, c->nprim, c->d_u.p, nullptr, c->nspn, B.coef.p,
                    B.maxfmt.p, B.cgp.p, st);
-  launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn, B.coef.p,
-                    B.maxfmt.p, B.cgp.p, c->mesh_dev(), c->d_boys.p, B.callfo.p, B.mom.p, B.again.p, st);
+  c->launches += npairs > 0 ? 1 : 0;
+  c->launches += launch_call_setup(ncalls, c->d_setup_list.p, c->nsingle, c->d_calls.p, c->d_pairs.p, nf, c->nspn,
+                                   B.coef.p, B.maxfmt.p, B.cgp.p, c->mesh_dev(), c->d_boys.p, B.callfo.p, B.mom.p,
+                                   B.again.p, st);
   CUDA_CHECK(cudaMemsetAsync(B.cnt.p, 0, 3 * sizeof(unsigned long long), st));
   B.bound.ensure((size_t)std::max(ncalls, 1));
   // the parts' sums in the buffer that XC fills with the SIC potentials afterwards
   DevBuf<double>& seg = c->spin[s0].vpot;
   seg.ensure(perfo_seg_size(c->eval_nt, nf, P));
   CoulombScratch scr{B.pairfmt.p, B.share.p, B.lists.p, B.plist.p, nullptr, nullptr, nullptr, B.bound.p, seg.p};
-  launch_coulomb_classify(ncalls, c->d_calls.p, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
-  launch_perfo_setup(ncalls, npairs, nf, c->d_calls.p, c->d_pairs.p, B.callfo.p, B.share.p, false,
-                     c->precision == FLOSIC_PRECISION_MIXED, false, B.coef.p, B.mom.p, B.bound.p, st);
-  c->launches += 8;
+  c->launches += launch_coulomb_classify(ncalls, c->d_calls.p, npairs, nf, B.maxfmt.p, B.callfo.p, scr, false, st);
+  c->launches += launch_perfo_setup(ncalls, npairs, nf, c->d_calls.p, c->d_pairs.p, B.callfo.p, B.share.p, false,
+                                    c->precision == FLOSIC_PRECISION_MIXED, false, B.coef.p, B.mom.p, B.bound.p, st);
   for (int s = s0; s < s0 + ns; ++s) pair_density(c, s, B.callfo.p);
   CoulombJob J{};
   J.ncalls = ncalls;
@@ -2129,14 +2128,13 @@ int flosic_sic_batch_cycle(flosic_ctx** ctxs, int n, int wm, int ld, double* res
       CUDA_CHECK(cudaMemcpyAsync(c0->d_items.p, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice,
                                  c0->st));
       c0->d_batch_counters.ensure(1);
-      launch_coulomb_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), c0->d_batch_counters.p, wm,
-                           c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, nsm, c0->st);
+      c0->launches += launch_coulomb_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), c0->d_batch_counters.p, wm,
+                                           c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, nsm, c0->st);
       int parts = 1;
       for (const CoulombJob& J : jobs) parts = std::max(parts, J.nseg);
-      launch_perfo_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), parts, wm,
-                         c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, c0->st);
+      c0->launches += launch_perfo_batch(c0->d_jobs.p, c0->d_items.p, (int)items.size(), parts, wm,
+                                         c0->precision == FLOSIC_PRECISION_MIXED, c0->d_boys.p, c0->st);
       CUDA_CHECK(cudaGetLastError());
-      c0->launches += 4;
     }
     CUDA_CHECK(cudaEventRecord(c0->ev[4], c0->st));
     for (int m = 1; m < n; ++m) CUDA_CHECK(cudaStreamWaitEvent(ctxs[m]->st, c0->ev[4], 0));
@@ -2423,11 +2421,11 @@ int flosic_sic_coupot1(flosic_ctx* c, double* coulomb) {
     const int npairs = (int)c->pairs.size();
     c->d_u.ensure((size_t)std::max(nwf, 1) * c->nprim * 10);
     if (nwf > 0) launch_prim_u(c->basis_dev(), nwf, c->d_psi.p, c->nbasis, c->d_u.p, c->st);
+    c->launches += (nwf > 0 ? 1 : 0) + (npairs > 0 ? 1 : 0);
     DevBuf<double>&ddm = c->d_wk[0], &dvh = c->d_wk[1];
     ddm.ensure((size_t)std::max(npairs, 1) * 100);
     dvh.ensure((size_t)P);
     launch_pair_dm(npairs, c->d_pairs.p, nwf, c->nprim, c->d_u.p, ddm.p, c->st);
-    c->launches += 2;
     coulomb_eval(c, 1, ddm.p, dvh.p);
     std::vector<double> v(P);
     CUDA_CHECK(cudaMemcpyAsync(v.data(), dvh.p, sizeof(double) * P, cudaMemcpyDeviceToHost, c->st));
