@@ -492,12 +492,12 @@ __global__ void k_call_share(int ncalls, int nfo, const CallFO* __restrict__ cfo
   const int lane = threadIdx.x & 31;
   if (c >= ncalls) return;
   const CallFO f0 = cfo[(size_t)c * nfo];
-  bool same = true;
+  bool same = true;  // of one FO, whatever its CG: launch_coulomb_mma then has no per-FO call
   int lmx = -1, ksum = 0;
   for (int k = lane; k < nfo; k += 32) {
     const CallFO f = cfo[(size_t)c * nfo + k];
-    same = same && f.cg[0] == f0.cg[0] && f.cg[1] == f0.cg[1] && f.cg[2] == f0.cg[2] && f.rcut2 == f0.rcut2 &&
-           f.npot == f0.npot;
+    same = same && (nfo == 1 || (f.cg[0] == f0.cg[0] && f.cg[1] == f0.cg[1] && f.cg[2] == f0.cg[2] &&
+                                 f.rcut2 == f0.rcut2 && f.npot == f0.npot));
     if (f.npot == 2 && f.keep != 0ull) {
       lmx = max(lmx, f.lmax);
       ksum += __popcll(f.keep);
@@ -693,6 +693,9 @@ cudaError_t launch_coulomb_mma(int ncalls, const CallInfo* calls, const PairGeo*
                        ldv, cnt, mixed, st);
   }
   if (mid) cudaEventRecord(mid, st);
+  // One FO or density: every call has its geometry, and what follows would be six
+  // launches without work.
+  if (nfo == 1 && !per_fo_only) return cudaGetLastError();
   if (per_fo_only) cudaMemset2DAsync(vh, sizeof(double) * ldv, 0, sizeof(double) * M.n, nfo, st);
   *launched += launch_perfo_setup(ncalls, npairs, nfo, calls, pairs, cfo, scr.share, per_fo_only, mixed, one_density,
                                   coef, momv, scr.bound, st);

@@ -539,12 +539,14 @@ __device__ int call_far_count(const CallInfo& ci, const MeshDev& M, const double
 // CG, RCUT and NPOT of every call of more than one slot and FO (poisson1.f:503-583),
 // one warp each.  The far count first adds the tiles that lie wholly outside the
 // sphere and stops once NPOT=2 is certain; only a call with few of them looks at
-// the points of the tiles its sphere cuts.
+// the points of the tiles its sphere cuts.  again (may be null): the (call, FO)s
+// with far points are listed there for k_call_moments_again.
 __global__ void __launch_bounds__(256) k_call_geom(int nmulti, const int* __restrict__ list,
                                                    const CallInfo* __restrict__ calls,
                                                    const PairGeo* __restrict__ pairs, int nfo, int nspn,
                                                    const double* __restrict__ cgp, MeshDev M,
-                                                   CallFO* __restrict__ out, double* __restrict__ momv) {
+                                                   CallFO* __restrict__ out, double* __restrict__ momv,
+                                                   int* __restrict__ again) {
   const size_t wi = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wi >= (size_t)nmulti * nfo) return;
@@ -622,6 +624,7 @@ __global__ void __launch_bounds__(256) k_call_geom(int nmulti, const int* __rest
     f.lmax = 0;
     f.pad = 0;
     out[ck] = f;
+    if (again && npot == 2 && nfar > 0) again[1 + atomicAdd(again, 1)] = (int)ck;
   }
   if (npot == 1 || nfar == 0)
     for (int m = lane; m < MOM_LD; m += 32) momv[ck * MOM_LD + m] = 0.0;
@@ -755,10 +758,10 @@ __global__ void __launch_bounds__(THREADS) k_call_moments(const int* __restrict_
   }
 }
 
-// The moments of the listed (call, FO)s with the skip rule near its threshold,
-// each term and sum formed point by point: harmonics at the FO's own sphere
-// points, 146 terms added in order.  A block per entry.
-constexpr int AGAIN_THREADS = 160;
+// The moments of the listed (call, FO)s (those with the skip rule near its
+// threshold, or all of a few), each term and sum formed point by point: harmonics
+// at the FO's own sphere points, 146 terms added in order.  A block per entry.
+constexpr int AGAIN_THREADS = 160, AGAIN_WAVE = 3 * 148;  // three blocks per SM
 __global__ void __launch_bounds__(AGAIN_THREADS) k_call_moments_again(const int* __restrict__ again, int nfo,
                                                                       const CallInfo* __restrict__ calls,
                                                                       const PairGeo* __restrict__ pairs,
@@ -978,21 +981,29 @@ int launch_call_setup(int ncalls, const int* list, int nsingle, const CallInfo* 
     k_call_setup_single<<<nsingle, SETUP1_THREADS, sizeof(double) * NANG * (GEO_LD + NMOM), st>>>(
         list, calls, pairs, nfo, nspn, coef, maxfmt, M, boys_tab, cfo, momv);
   const int nmulti = ncalls - nsingle;
+  int launched = nsingle > 0 ? 1 : 0;
   if (nmulti > 0) {
     const size_t warps = (size_t)nmulti * nfo;
+    // So few (call, FO)s that one wave of k_call_moments_again takes them all: the
+    // product form would only come before it, each a chain of ~100 us (water's one
+    // density, 85 calls: 230 us in three kernels, 140 in two).
+    const bool few = warps <= (size_t)AGAIN_WAVE;
     cudaMemsetAsync(again, 0, sizeof(int), st);
     k_call_geom<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(nmulti, list + nsingle, calls, pairs, nfo, nspn, cgp, M,
-                                                              cfo, momv);
-    if ((size_t)nmulti * ((nfo + 7) / 8) < 4 * 148)  // less than two waves of the eight-FO blocks
-      k_call_moments<2, 320><<<dim3(nmulti, (nfo + 1) / 2), 320, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
-                                                                          maxfmt, boys_tab, cfo, momv, again);
-    else
-      k_call_moments<8, 256><<<dim3(nmulti, (nfo + 7) / 8), 256, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
-                                                                          maxfmt, boys_tab, cfo, momv, again);
-    k_call_moments_again<<<(int)std::min<size_t>(3 * 148, warps), AGAIN_THREADS, sizeof(double) * NANG * NMOM, st>>>(
+                                                              cfo, momv, few ? again : nullptr);
+    if (!few) {
+      if ((size_t)nmulti * ((nfo + 7) / 8) < 4 * 148)  // less than two waves of the eight-FO blocks
+        k_call_moments<2, 320><<<dim3(nmulti, (nfo + 1) / 2), 320, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
+                                                                            maxfmt, boys_tab, cfo, momv, again);
+      else
+        k_call_moments<8, 256><<<dim3(nmulti, (nfo + 7) / 8), 256, 0, st>>>(list + nsingle, calls, pairs, nfo, coef,
+                                                                            maxfmt, boys_tab, cfo, momv, again);
+    }
+    k_call_moments_again<<<(int)std::min<size_t>(AGAIN_WAVE, warps), AGAIN_THREADS, sizeof(double) * NANG * NMOM, st>>>(
         again, nfo, calls, pairs, coef, maxfmt, boys_tab, cfo, momv);
+    launched += few ? 2 : 3;
   }
-  return (nsingle > 0 ? 1 : 0) + (nmulti > 0 ? 3 : 0);
+  return launched;
 }
 
 // ---------------------------------------------------------------------------
