@@ -154,12 +154,13 @@ int flosic_sic_set_wait_limit(flosic_ctx* ctx, int64_t polls);
 
 /* Tile-shape autotuner (no counterpart in the reference, whose POISSON1 batch
    shapes are compile-time constants: MXPR pairs per call, coupot_sic.F:46, and
-   MPX points per block, poisson1.f:62).  Times the per-FO Coulomb kernel with
-   tiles of 128 mesh points by 32, 64 and 128 FO slots on this context's own
-   COUPOT_SIC evaluation (as a cycle makes it: both spins together when their FOs
-   fit one block, else the spin with the most FOs; the current precision mode and
+   MPX points per block, poisson1.f:62).  Times the near-field kernel of the
+   per-FO calls with blocks of 64 mesh points by 32, 64 and 128 FOs on this
+   context's own COUPOT_SIC evaluation (as a cycle makes it: both spins together
+   when their FOs fit one block of 64, else the spin with the most FOs; also the
+   latter when one spin's FODs cannot be used; the current precision mode and
    mesh shard; best of reps >= 1 runs after one untimed run) and keeps the
-   fastest for the following calls.  Widths that would leave half a tile or more
+   fastest for the following calls.  Widths that would leave half a block or more
    empty are skipped.  All widths give the same potentials bit for bit.
    perfo_fos: the chosen width; ms[3] (may be NULL): the times of widths
    32, 64, 128 in milliseconds, -1 for a skipped width.  Needs

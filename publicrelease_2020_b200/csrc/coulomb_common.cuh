@@ -174,7 +174,6 @@ __device__ __forceinline__ int far_degree(int kf) {
   return kf <= 4 ? 1 : (kf <= 12 ? 2 : (kf <= 16 ? 3 : (kf <= 28 ? 4 : (kf <= 36 ? 5 : 6))));
 }
 
-// H column (rows [0, kf)) of one far point: harmonics times 1/r^(l+1), zero padded.
 // One segment of the shared GEMM: the near part of one pair or the far part of
 // one call, restricted to this tile.
 struct Segment {

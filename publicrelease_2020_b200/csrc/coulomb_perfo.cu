@@ -1068,7 +1068,8 @@ int launch_perfo(const CoulombJob& J, int wm, bool mixed, const double* tab, con
   return 3;
 }
 
-// Enough CTAs for eight per SM, at least a window of pairs each.
+// Enough CTAs for eight per SM, from the mesh alone (a short pair list leaves some of
+// the parts without a pair).
 int one_density_parts(int ntiles) { return std::max(2, std::min(32, 8 * 148 / std::max(ntiles, 1))); }
 
 int launch_one_density(const CoulombJob& J, const double* tab, cudaStream_t st) {

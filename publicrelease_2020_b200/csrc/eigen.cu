@@ -25,9 +25,9 @@ constexpr int EIG_MAX_N = 1024;          // pairs held in shared memory: EIG_MAX
 constexpr int EIG_SMEM_MAX_N = 160;      // matrix in shared memory up to 160 x 161 doubles (206 KB)
 constexpr int EIG_MAX_SWEEPS = 60;
 
-// More than EIG_SMEM_MAX_N FOs.  A(i, j) at A[i * (n + 1) + j].  The rotations are accumulated transposed, Vt(m, k) =
-// component k of vector m, so that a column update of V is a row update of Vt
-// (contiguous in memory).
+// More than EIG_SMEM_MAX_N FOs.  A(i, j) at A[i * (n + 1) + j].  The rotations are
+// accumulated transposed, Vt(m, k) = component k of vector m, so that a column
+// update of V is a row update of Vt (contiguous in memory).
 __global__ void __launch_bounds__(EIG_THREADS, 1)
 k_sym_eigen(int n, const double* __restrict__ ain, double* __restrict__ aglob, double* __restrict__ vt,
             double* __restrict__ wout, double* __restrict__ vout, int* __restrict__ info) {

@@ -732,7 +732,9 @@ __global__ void __launch_bounds__(THREADS) k_call_moments(const int* __restrict_
     const double x = m < NMOM ? mom[f][m] * rl : 0.0;
     // A moment that vanishes by symmetry is rounding of the sum, and where the
     // potential is large that rounding is near the skip rule's 1e-12: the FO is
-    // left to k_call_moments_again.
+    // left to k_call_moments_again.  (The bound leaves out that the harmonics of
+    // large m reach 1e4: of those a few in a million cross 1e-12 by rounding alone,
+    // one way or the other, and the count of kept terms with them.)
     const double eps = (2 * l + 1) * 7.0e-15 * vmax * fmax(1.0, 0.125 * ci.np);
     unsure = unsure || (m < NMOM && fabs(fabs((2 * l + 1) * x * rt) - 1.0e-12) < eps);
     const bool kept = m < NMOM && !(fabs((2 * l + 1) * x * rt) < 1.0e-12);
@@ -1145,8 +1147,7 @@ void launch_xc(const MeshDev& M, int nfo, int gga, int mgga, int nspn, const int
   else k_xc<false><<<grid, XC_THREADS, 0, st>>>(M, nfo, gga, nspn, xp, phi, ldp, rhog, vh, vpot, y, part, nblk);
 }
 
-// Compensated (Neumaier) sums of the block partials, in block order.
-// Block partial sums added up, compensated: a warp per (FO, quantity), each lane
+// Block partial sums added up, compensated (Neumaier): a warp per (FO, quantity), each lane
 // the blocks of its residue in order, then the lanes' sums in a fixed tree (one
 // thread and a dependent chain over all blocks took 10-50 us).
 __global__ void __launch_bounds__(32 * NPART) k_reduce_parts(int nblk, const double* __restrict__ part,

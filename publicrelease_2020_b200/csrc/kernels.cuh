@@ -214,7 +214,6 @@ void launch_ordered_product(int M, int N, int K, const double* A, int ai, int am
                             const double* e, double* out, int ldo, cudaStream_t st);
 void launch_force_ham(int n, const double* G, const double* Q, double* out, cudaStream_t st);
 
-// Vxc of given density channels (GETVLXC entry point): vxc[2*n], parts as above (1 FO).
 // Dense products on the FP64 tensor cores (csrc/contract.cu).
 // dgemm: C = alpha op(A) op(B) + beta C, column-major as BLAS DGEMM; work holds
 // dgemm_work(M, N, K) doubles (split-K partial products; 0: none needed).
@@ -238,6 +237,8 @@ cudaError_t init_sym_eigen();
 size_t sym_eigen_work(int n);
 size_t sym_eigen_info(int n);  // ints of info; info[0] is the status
 int launch_sym_eigen(int n, const double* a, double* work, double* w, double* v, int* info, cudaStream_t st);
+// Vxc of given density channels (GETVLXC entry point): vxc[2*n], parts as above (1
+// FO), in xc_rhog_blocks(npts) blocks.
 cudaError_t preload_xc_rhog();
 int xc_rhog_blocks(int npts);
 void launch_xc_rhog(const MeshDev& M, int gga, const int* xc, const double* rhog, int ldr, double* vxc,

@@ -1185,13 +1185,13 @@ void require_whole_mesh(flosic_ctx* c) {
 // Allocation-free GETVLXC scratch
 // ---------------------------------------------------------------------------
 // flosic_sic_getvlxc_device keeps its per-block energy partial sums in this
-// file-scope device array instead of allocating: XC_SCRATCH_BLOCKS blocks of
-// 256 points (4,194,304 points at most) times NPART partials.  Every call
+// file-scope device array instead of allocating: NPART partials of each block
+// (today at most 1024 blocks, which stride over the points; the array and the
+// limit of 4,194,304 points are those of one block per 256 points).  Every call
 // overwrites the partials of its nblk blocks before reading them, so no part of
 // the array has to start at zero; the final sums go to the context's own mapped
-// host memory.  All
-// calls on one device share it: calls that overlap in time (other host threads,
-// other contexts or streams on the same device) race on it.
+// host memory.  All calls on one device share it: calls that overlap in time
+// (other host threads, other contexts or streams on the same device) race on it.
 constexpr int XC_SCRATCH_BLOCKS = 16384;
 constexpr int XC_SCRATCH_POINTS = XC_SCRATCH_BLOCKS * 256;
 static __device__ __align__(256) double g_xc_scratch[XC_SCRATCH_BLOCKS * NPART];
@@ -1247,16 +1247,6 @@ void adjoint_device(flosic_ctx* c, int s, DevBuf<double>& dg) {
   }
 }
 
-// dE_SIC/dFOD of spin s, grad[k*3 + d], from the adjoint G by the chain rule
-// through the FO construction.  C_FO = U C_KS with U = S^-1/2 T the
-// Lowdin-orthonormalised Fermi transformation (frmiorb.f:351-480), T_kj =
-// psi_j(a_k)/sqrt(rho(a_k)) = FMAT(j,k,1), S = T T^T = V diag(q) V^T (the
-// eigenpairs LOWSIC kept); row k of T depends on FOD a_k only, with
-// derivatives FMAT(.,k,2:4) (frmorb2.F:296-346).  With M = C_KS G and A = T M:
-//   W = V ((V^T A V) o F) V^T,  F_ab = -1 / (sqrt q_a sqrt q_b (sqrt q_a + sqrt q_b)),
-//   dE/dT = (W + W^T) T + (M S^-1/2)^T,  dE/da_m = sum_j (dE/dT)_mj dT_mj/da_m.
-// This is the reference's FOD force (frmorb2.F:586-717, times 2/NSPN) reached
-// through the basis-space adjoint instead of the SIC matrix.
 // Batch of molecules: everything of spins [s0, s0 + ns) before their Coulomb
 // evaluation -- FO construction, FO values, pair coefficients, POISSON1 call
 // set-up and call classification -- into the first spin's own buffers, on the
@@ -1321,6 +1311,16 @@ CoulombJob batch_prepare(flosic_ctx* c, int s0, int ns) {
   return J;
 }
 
+// dE_SIC/dFOD of spin s, grad[k*3 + d], from the adjoint G by the chain rule
+// through the FO construction.  C_FO = U C_KS with U = S^-1/2 T the
+// Lowdin-orthonormalised Fermi transformation (frmiorb.f:351-480), T_kj =
+// psi_j(a_k)/sqrt(rho(a_k)) = FMAT(j,k,1), S = T T^T = V diag(q) V^T (the
+// eigenpairs LOWSIC kept); row k of T depends on FOD a_k only, with
+// derivatives FMAT(.,k,2:4) (frmorb2.F:296-346).  With M = C_KS G and A = T M:
+//   W = V ((V^T A V) o F) V^T,  F_ab = -1 / (sqrt q_a sqrt q_b (sqrt q_a + sqrt q_b)),
+//   dE/dT = (W + W^T) T + (M S^-1/2)^T,  dE/da_m = sum_j (dE/dT)_mj dT_mj/da_m.
+// This is the reference's FOD force (frmorb2.F:586-717, times 2/NSPN) reached
+// through the basis-space adjoint instead of the SIC matrix.
 void fod_gradient(flosic_ctx* c, int s, double* grad) {
   DevBuf<double>&dg = c->d_wk[0], &dm = c->d_wk[1];
   adjoint_device(c, s, dg);
@@ -1878,14 +1878,15 @@ int flosic_sic_set_precision(flosic_ctx* c, int mode) {
   });
 }
 
-// Tile-shape autotuner of the per-FO Coulomb kernel: its tiles are 128 mesh
-// points by 32, 64 or 128 compacted FO slots.  Each width is timed (CUDA
-// events on the context's stream, best of reps after one untimed run) on the
-// full COUPOT_SIC Coulomb evaluation of the spin with the most FOs, under the
-// context's precision mode and mesh shard, and the fastest is kept.  The
-// widths only regroup FOs into CTAs; every potential is formed by the same
-// operations in the same order, so the choice changes time, not results.
-// Work counters and launch counts are left as they were.
+// Tile-shape autotuner of the near-field kernel of the per-FO calls: its blocks
+// are 64 mesh points by 32, 64 or 128 FOs.  Each width is timed (CUDA events on
+// the context's stream, best of reps after one untimed run) on the full
+// COUPOT_SIC Coulomb evaluation that a cycle makes -- of both spins together, or
+// of the spin with the most FOs -- under the context's precision mode and mesh
+// shard, and the fastest is kept.  The widths only regroup FOs into CTAs; every
+// potential is formed by the same operations in the same order, so the choice
+// changes time, not results.  Work counters and launch counts are left as they
+// were, and no potentials of the timed runs are kept.
 int flosic_sic_autotune(flosic_ctx* c, int reps, int* perfo_fos, float* ms) {
   return guarded([&] {
     require(c, true);
@@ -1897,7 +1898,7 @@ int flosic_sic_autotune(flosic_ctx* c, int reps, int* perfo_fos, float* ms) {
       try {
         for (int t = 0; t < 2; ++t) fo_setup(c, t);
       } catch (const Fail&) {
-        both = false;  // one spin's FODs cannot be used: tune on the other
+        both = false;  // one spin's FODs cannot be used: tune on the larger spin alone, if it is not that one
       }
     }
     const int s = !both && c->nspn == 2 && c->nfrm[1] > c->nfrm[0] ? 1 : 0, ns = both ? 2 : 1;
