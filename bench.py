@@ -36,10 +36,10 @@ COULOMB_FLOPS_NEAR = 92.0    # per near (pair, point, FO): 46 polynomial coeffic
 COULOMB_FLOPS_TERM = 2.0     # per multipole term kept by the skip rule in a far (call, point, FO) evaluation
 # DRAM bytes of the Coulomb kernels per tile of 128 points on the C2 shape:
 # ncu dram__bytes_read.sum + dram__bytes_write.sum on 296 tiles (k_coulomb_shared
-# 5.311 GB + 0.033 GB, k_perfo_near 0.506 GB + 0.032 GB, k_perfo_far 0.012 GB); the
+# 5.463 GB + 0.032 GB, k_perfo_near 1.173 GB + 0.035 GB, k_perfo_far 0.012 GB); the
 # traffic is re-reads of the per-call A operands, proportional to the tile count.
 # k_coulomb_perfo in the line below is the two per-FO kernels together.
-COULOMB_DRAM_BYTES_PER_TILE = (5.311e9 + 0.033e9 + 0.506e9 + 0.032e9 + 0.012e9) / 296
+COULOMB_DRAM_BYTES_PER_TILE = (5.463e9 + 0.032e9 + 1.173e9 + 0.035e9 + 0.012e9) / 296
 # (the Boys values, monomials and harmonics depend on geometry only and are
 # formed once per (pair or call, point); the per-FO work is the contraction)
 
