@@ -141,40 +141,52 @@ struct Horner {
   }
 };
 
+// x^e for e <= 3 (1 for e < 0, where the factor is zero).
+__device__ __forceinline__ double power3(double x, int e) {
+  const double x2 = x * x;
+  return e <= 0 ? 1.0 : (e == 1 ? x : (e == 2 ? x2 : x2 * x));
+}
+
 // Channels 1.. of the monomials that only derivative channels keep, before the
 // Gaussian factor: every RHOD entry f c above the threshold, with its product-rule
-// terms.  Out of line, since a row with such an entry is the exception (a cycle of 20
-// atoms, 64 FOs, 50,021 points, PBE: 45.5 ms without these entries, 46.4 with them).
+// terms.  of: their values.  Out of line, since a row with such an entry is the
+// exception (20 atoms, 64 FOs, 50,021 points, PBE: k_pair_density 26.6 ms without
+// these entries, 27.5 with them; 28.3 with the first value loaded ahead).
 template <int NCH>
-__device__ __noinline__ void derivative_only(unsigned long long bits, const double* __restrict__ c_of, double x,
+__device__ __noinline__ void derivative_only(unsigned long long bits, const double* __restrict__ of, double x,
                                              double y, double z, double delta, double* a) {
-  const double v[3] = {x, y, z};
   double g[3] = {0.0, 0.0, 0.0}, h[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (; bits; bits &= bits - 1) {
     const int m = __ffsll((long long)bits) - 1;
-    const double c = c_of[m];
-    int p[3];
-    mono_powers(m, p[0], p[1], p[2]);
-    auto mono = [&](int i, int j) {  // the monomial without one power of i and of j (j < 0: of i alone)
-      double t = 1.0;
-      for (int d = 0; d < 3; ++d)
-        for (int e = p[d] - (d == i) - (d == j); e > 0; --e) t *= v[d];
-      return t;
-    };
-    for (int d = 0; d < 3; ++d) {
-      const double fc = dens_keep(p[d] * c);
-      if (fc != 0.0) g[d] += fc * mono(d, -1);
-    }
-    for (int q = 0; NCH == 10 && q < 6; ++q) {  // xx yy zz xy xz yz
-      const int i = q < 3 ? q : (q < 5 ? 0 : 1), j = q < 3 ? q : (q == 3 ? 1 : 2);
-      const double fc = dens_keep((i == j ? p[i] * (p[i] - 1) : p[i] * p[j]) * c);
-      if (fc != 0.0) h[q] += fc * mono(i, j);
+    const double c = of[m];
+    int px, py, pz;
+    mono_powers(m, px, py, pz);
+    const double X = px == 4 ? x * power3(x, 3) : power3(x, px), Y = py == 4 ? y * power3(y, 3) : power3(y, py),
+                 Z = pz == 4 ? z * power3(z, 3) : power3(z, pz);
+    const double X1 = power3(x, px - 1), Y1 = power3(y, py - 1), Z1 = power3(z, pz - 1);
+    g[0] += dens_keep(px * c) * (X1 * Y * Z);
+    g[1] += dens_keep(py * c) * (X * Y1 * Z);
+    g[2] += dens_keep(pz * c) * (X * Y * Z1);
+    if constexpr (NCH == 10) {
+      h[0] += dens_keep(px * (px - 1) * c) * (power3(x, px - 2) * Y * Z);
+      h[1] += dens_keep(py * (py - 1) * c) * (X * power3(y, py - 2) * Z);
+      h[2] += dens_keep(pz * (pz - 1) * c) * (X * Y * power3(z, pz - 2));
+      h[3] += dens_keep(px * py * c) * (X1 * Y1 * Z);
+      h[4] += dens_keep(px * pz * c) * (X1 * Y * Z1);
+      h[5] += dens_keep(py * pz * c) * (X * Y1 * Z1);
     }
   }
-  for (int d = 0; d < 3; ++d) a[d] = g[d];
-  for (int q = 0; NCH == 10 && q < 6; ++q) {
-    const int i = q < 3 ? q : (q < 5 ? 0 : 1), j = q < 3 ? q : (q == 3 ? 1 : 2);
-    a[3 + q] = h[q] - 2.0 * delta * (v[j] * g[i] + v[i] * g[j]);
+  const double d2 = 2.0 * delta;
+  a[0] = g[0];
+  a[1] = g[1];
+  a[2] = g[2];
+  if constexpr (NCH == 10) {
+    a[3] = h[0] - 2.0 * d2 * x * g[0];
+    a[4] = h[1] - 2.0 * d2 * y * g[1];
+    a[5] = h[2] - 2.0 * d2 * z * g[2];
+    a[6] = h[3] - d2 * (y * g[0] + x * g[1]);
+    a[7] = h[4] - d2 * (z * g[0] + x * g[2]);
+    a[8] = h[5] - d2 * (z * g[1] + y * g[2]);
   }
 }
 
@@ -250,8 +262,11 @@ __device__ __forceinline__ void pair_channels(double x, double y, double z, doub
 // Measured, 40 atoms, 128 FOs, 37,888 points, PBE: 288 -> 164 ms (before: one barrier
 // per pair and rows of 156 entries, 78 16-byte shared-memory loads each).
 constexpr int DENS_CHUNK = 16;
+// resident blocks per SM that the registers of the sums allow (the function called
+// out of line would take more: 152, 30.3 ms)
+constexpr int dens_blocks(int nch) { return nch == 10 ? 4 : (nch == 4 ? 7 : 8); }
 template <int NCH>
-__global__ void __launch_bounds__(DENS_THREADS) k_pair_density(MeshDev M, int npairs,
+__global__ void __launch_bounds__(DENS_THREADS, dens_blocks(NCH)) k_pair_density(MeshDev M, int npairs,
                                                                const PairGeo* __restrict__ pairs,
                                                                const CallFO* __restrict__ cfo, int cfo_ld, int nfo,
                                                                const double* __restrict__ dc,
