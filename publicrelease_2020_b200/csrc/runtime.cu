@@ -14,6 +14,8 @@
 #include <cfloat>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -75,6 +77,61 @@ struct DevBuf {
     n = 0;
   }
 };
+
+// Mapped host memory for the contexts' results (flosic_sic_getvlxc_device), a slot
+// each.  Registering a page takes 0.3 ms (cudaHostAlloc 1.1-3.5 when no other pinned
+// block is alive), so the contexts alive, of any thread and device, share pages of 32
+// slots; a page without a context is given back.
+class MappedSlots {
+ public:
+  double* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    for (Page& g : pages_)
+      if (g.used != ~0u) return slot(g);
+    void* p = std::aligned_alloc(32 * SLOT, 32 * SLOT);
+    if (!p) throw std::bad_alloc();
+    const cudaError_t e = cudaHostRegister(p, 32 * SLOT, cudaHostRegisterMapped | cudaHostRegisterPortable);
+    if (e != cudaSuccess) std::free(p);
+    CUDA_CHECK(e);
+    pages_.push_back({static_cast<char*>(p), 0u});
+    return slot(pages_.back());
+  }
+  void give(double* s) {
+    std::lock_guard<std::mutex> lock(mu_);
+    for (size_t i = 0; i < pages_.size(); ++i) {
+      Page& g = pages_[i];
+      const std::uintptr_t o = reinterpret_cast<std::uintptr_t>(s) - reinterpret_cast<std::uintptr_t>(g.p);
+      if (o >= 32 * SLOT) continue;
+      g.used &= ~(1u << (o / SLOT));
+      if (g.used == 0u) {
+        cudaHostUnregister(g.p);
+        std::free(g.p);
+        pages_.erase(pages_.begin() + i);
+      }
+      return;
+    }
+  }
+
+ private:
+  static constexpr std::size_t SLOT = 128;
+  static_assert(sizeof(double) * NPART <= SLOT, "a context's results fit its slot");
+  struct Page {
+    char* p;
+    unsigned used;  // a bit per slot
+  };
+  static double* slot(Page& g) {
+    int b = 0;
+    while ((g.used >> b) & 1u) ++b;
+    g.used |= 1u << b;
+    return reinterpret_cast<double*>(g.p + b * SLOT);
+  }
+  std::mutex mu_;
+  std::vector<Page> pages_;
+};
+MappedSlots& mapped_slots() {
+  static MappedSlots* m = new MappedSlots;  // contexts may be closed while the process ends
+  return *m;
+}
 
 // ---------------------------------------------------------------------------
 // LOWSIC (lowden_files.f:2-172): S^{-1/2} of the FO overlap from its
@@ -321,10 +378,7 @@ struct flosic_ctx {
   int device = 0;
   cudaStream_t st = nullptr;
   SideStream side;           // far field of the per-FO calls
-  // NPART doubles of mapped host memory (flosic_sic_getvlxc_device) and their device
-  // address.  A registered page takes 0.3 ms of flosic_sic_create where cudaHostAlloc
-  // took 1.1-3.5.
-  double *h_sums = nullptr, *d_hsums = nullptr;
+  double *h_sums = nullptr, *d_hsums = nullptr;  // a slot of MappedSlots and its device address
   DevBuf<double> d_gemm_ws;  // split-K partial products of dgemm
   DevBuf<double> d_wk[3];    // results of the basis-space sums and the DFT side, kept between calls
   DevBuf<CoulombJob> d_jobs;  // batched Coulomb launch led by this context
@@ -1396,14 +1450,8 @@ int flosic_sic_create(int device, flosic_ctx** out) {
     CUDA_CHECK(cudaStreamCreateWithFlags(&c->side.st, cudaStreamNonBlocking));
     CUDA_CHECK(cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming));
     CUDA_CHECK(cudaEventCreateWithFlags(&c->side.join, cudaEventDisableTiming));
-    constexpr size_t PAGE = 4096;
-    void* page = std::aligned_alloc(PAGE, PAGE);
-    if (!page) throw std::bad_alloc();
-    const cudaError_t reg = cudaHostRegister(page, PAGE, cudaHostRegisterMapped);
-    if (reg != cudaSuccess) std::free(page);
-    CUDA_CHECK(reg);
-    c->h_sums = static_cast<double*>(page);
-    CUDA_CHECK(cudaHostGetDevicePointer(&c->d_hsums, page, 0));
+    c->h_sums = mapped_slots().take();
+    CUDA_CHECK(cudaHostGetDevicePointer(&c->d_hsums, c->h_sums, 0));
     std::vector<double> ang, w;
     lebedev19(ang, w);
     upload_constants(ang.data(), w.data());
@@ -1447,8 +1495,7 @@ int flosic_sic_destroy(flosic_ctx* c) {
   c->d_jobs.release();
   c->d_items.release();
   c->d_batch_counters.release();
-  if (c->h_sums) cudaHostUnregister(c->h_sums);
-  std::free(c->h_sums);
+  if (c->h_sums) mapped_slots().give(c->h_sums);
   if (c->side.fork) cudaEventDestroy(c->side.fork);
   if (c->side.join) cudaEventDestroy(c->side.join);
   if (c->side.st) cudaStreamDestroy(c->side.st);
